@@ -11,6 +11,7 @@
 // the last CTA to finish (deterministic).  PDL: the weight ring is filled before griddepcontrol.wait.
 // Warp roles: 0 = TMA producer, 1 = MMA issuer (one elected thread), 2..5 = epilogue (TMEM -> registers -> HBM).
 #include "common.cuh"
+#include "gemm_pair.cuh"
 #include "tmap.cuh"
 #include "../../include/b200_tgis.h"
 
@@ -38,6 +39,9 @@ __device__ __forceinline__ void gemm_store(void* y, size_t i, float v) {
 constexpr int kGemmThreads = 192;
 constexpr int kTileM = 128;  // features per tile
 constexpr int kTileK = 64;   // fp16 elements per k-block = one 128-byte swizzle row
+// Calls of more tokens go to the SM pairs (gemm_pair.cuh).  Measured on B200 (us, this kernel / pairs) at 64 tokens: 4096 x 4096 14.8 / 12.9,
+// 4096 -> 22016 37.1 / 40.0, 11008 -> 4096 23.6 / 28.8; at 96: 18.2 / 13.1, 42.9 / 41.3; at 128: 20.5 / 13.4, 45.8 / 42.3, 30.0 / 29.9.
+constexpr int kF16DecodeT = 64;
 constexpr int64_t kCounterBytes = 64 * 1024;
 
 template <int TN>
@@ -52,14 +56,13 @@ struct GemmF16Cfg {
 
 struct F16Params {
   void* y;
-  float* partial;  // [token tile][feature tile][contributor][TN][128] fp32
-  int* counters;   // [token tile][feature tile]
+  float* partial;  // [feature tile][contributor][TN][128] fp32
+  int* counters;   // [feature tile]
   const void* bias;
   int T, N;
   int nkb;            // 64-wide k-blocks per tile
-  int n_tiles_n;      // feature tiles
   int units_per_cta;  // contiguous (tile, k-block) units per CTA
-  int total_units;    // per token tile
+  int total_units;
   int max_contrib;    // partial slots per tile
   int defer;          // 1: leave every tile segment as an fp32 partial for the consumer kernel (B200SplitK), no fix-up
 };
@@ -79,7 +82,6 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
 
   pdl_launch_dependents();
   const int warp = warp_id(), lane = lane_id();
-  const int t0 = blockIdx.y * TN;
   const int u0 = blockIdx.x * p.units_per_cta;
   const int u1 = min(p.total_units, u0 + p.units_per_cta);
   const int n_units = u1 - u0;
@@ -118,7 +120,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       pdl_wait();
       int kbx = kb0;
       for (int i = 0; i < npre; ++i) {
-        tma_load_2d_hint(smem + i * C::kStageBytes + C::kABytes, &tmap_x, kbx * kTileK, t0, &full_bar[i], pol_x);
+        tma_load_2d_hint(smem + i * C::kStageBytes + C::kABytes, &tmap_x, kbx * kTileK, 0, &full_bar[i], pol_x);
         if (++kbx == p.nkb) kbx = 0;
       }
       for (int i = npre; i < n_units; ++i) {
@@ -127,7 +129,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
         mbar_arrive_expect_tx(&full_bar[s], C::kStageBytes);
         unsigned char* a = smem + s * C::kStageBytes;
         tma_load_2d_hint(a, &tmap_w, kb * kTileK, tile * kTileM, &full_bar[s], pol_w);
-        tma_load_2d_hint(a + C::kABytes, &tmap_x, kb * kTileK, t0, &full_bar[s], pol_x);
+        tma_load_2d_hint(a + C::kABytes, &tmap_x, kb * kTileK, 0, &full_bar[s], pol_x);
         if (++kb == p.nkb) { kb = 0; ++tile; }
       }
     }
@@ -172,11 +174,10 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       const int c_last = ((tile + 1) * p.nkb - 1) / p.units_per_cta;
       const int n_contrib = c_last - c_first + 1;
       const int my_contrib = (int)blockIdx.x - c_first;
-      const int tix = blockIdx.y * p.n_tiles_n + tile;
       mbar_wait(tmem_full, seg & 1);
       tcgen05_fence_after();
       const float bv = (p.bias && n_ok) ? gemm_load_bias<FMT>(p.bias, n) : 0.f;
-      float* part = p.partial + ((size_t)tix * p.max_contrib + my_contrib) * (TN * kTileM);
+      float* part = p.partial + ((size_t)tile * p.max_contrib + my_contrib) * (TN * kTileM);
 #pragma unroll 1
       for (int c = 0; c < TN; c += 16) {
         uint32_t d[16];
@@ -186,7 +187,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
           if (n_ok) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-              const int t = t0 + c + j;
+              const int t = c + j;
               if (t < p.T) gemm_store<FMT>(p.y, (size_t)t * p.N + n, __uint_as_float(d[j]) + bv);
             }
           }
@@ -204,17 +205,17 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (etid == 0) {
           __threadfence();
-          const int prev = atomicAdd(&p.counters[tix], 1);
+          const int prev = atomicAdd(&p.counters[tile], 1);
           s_is_last = prev == n_contrib - 1;
           if (s_is_last) {
-            p.counters[tix] = 0;  // re-armed for the next launch (graph replay safe)
+            p.counters[tile] = 0;  // re-armed for the next launch (graph replay safe)
             __threadfence();
           }
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");
         if (s_is_last) {
-          const float* base = p.partial + (size_t)tix * p.max_contrib * (TN * kTileM);
-          const int n_vec = min(p.T - t0, TN) * (kTileM / 4);
+          const float* base = p.partial + (size_t)tile * p.max_contrib * (TN * kTileM);
+          const int n_vec = min(p.T, TN) * (kTileM / 4);
           const bool vec_ok = (p.N & 3) == 0;
           for (int idx0 = etid; idx0 < n_vec; idx0 += 256) {
             float4 acc[2];
@@ -256,12 +257,12 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
                   uint2 o;
                   o.x = pack_half2(a4[0] + b4[0], a4[1] + b4[1]);
                   o.y = pack_half2(a4[2] + b4[2], a4[3] + b4[3]);
-                  *reinterpret_cast<uint2*>(&reinterpret_cast<__half*>(p.y)[(size_t)(t0 + tt) * p.N + nn]) = o;
+                  *reinterpret_cast<uint2*>(&reinterpret_cast<__half*>(p.y)[(size_t)tt * p.N + nn]) = o;
                 } else {
 #pragma unroll
                   for (int q = 0; q < 4; ++q)
                     if (nn + q < p.N)
-                      gemm_store<FMT>(p.y, (size_t)(t0 + tt) * p.N + nn + q, a4[q] + (p.bias ? gemm_load_bias<FMT>(p.bias, nn + q) : 0.f));
+                      gemm_store<FMT>(p.y, (size_t)tt * p.N + nn + q, a4[q] + (p.bias ? gemm_load_bias<FMT>(p.bias, nn + q) : 0.f));
                 }
               }
             }
@@ -389,12 +390,11 @@ static int launch_gemm_f16(const CUtensorMap* mw, const CUtensorMap* mx, void* y
   p.T = T;
   p.N = N;
   p.nkb = pl.nkb;
-  p.n_tiles_n = pl.n_tiles_n;
   p.units_per_cta = pl.units_per_cta;
   p.total_units = pl.n_tiles_n * pl.nkb;
   p.max_contrib = pl.max_contrib;
   p.defer = defer;
-  dim3 grid(pl.n_ctas, pl.n_tiles_t, 1);
+  const dim3 grid(pl.n_ctas);
   b200_timing_mark(B200_TIME_GEMM_F16, 0, st);
   B200_LAUNCH((gemm_f16_kernel<TN, FMT>), grid, dim3(kGemmThreads), (size_t)C::kSmemBytes, st, *mw, *mx, p);
   b200_timing_mark(B200_TIME_GEMM_F16, 1, st);
@@ -414,6 +414,15 @@ static int gemm_f16_impl(const void* x, const void* w, const void* bias, void* y
   if (defer && (!workspace || T > 256 || N % 8 != 0)) {
     b200_set_last_error("gemm_f16_deferred: needs a workspace, T <= 256 (one token tile) and N % 8 == 0");
     return B200_ERR_UNSUPPORTED;
+  }
+  if (!defer && T > kF16DecodeT) {
+    PairParams pp = {};
+    pp.y = y;
+    pp.bias = bias;
+    pp.T = (int)T;
+    pp.N = pp.ldy = (int)N;
+    pp.n_kb = (int)((K + kPairK - 1) / kPairK);
+    return launch_gemm_pair<FMT>(x, w, K, pp, pair_plan(T, N, pp.n_kb, false, f16_num_sms()), B200_TIME_GEMM_F16, (cudaStream_t)stream);
   }
   F16Plan pl = plan_f16(T, N, K, f16_num_sms(), defer);
   if (!defer && pl.max_contrib > 1 && (!workspace || (int64_t)pl.n_tiles_n * pl.n_tiles_t * 4 > kCounterBytes)) {

@@ -1,5 +1,5 @@
 // GPTQ int4 linear  Y[T,N] = X[T,K] . dequant(Wq)[K,N]  on tcgen05 tensor cores, weights de-quantised in-kernel
-// straight into TMEM (no fp16 scratch matrix, for any T).
+// straight into TMEM (no fp16 scratch matrix, for any T).  This kernel takes calls of up to 128 tokens (kW4DecodeT), gemm_pair.cuh larger ones.
 //
 // Replaces `exllamav2_kernels.make_q_matrix` / `gemm_half_q_half`
 // (/root/reference/server/text_generation_server/utils/gptq/exllamav2.py:14-62,139-144), including its M > 50
@@ -42,7 +42,9 @@
 // observation implies the skipped phase completed (see the ring-depth static_asserts).  Polls whose result is wanted
 // later use test_wait: try_wait may suspend the thread until a time-out while the phase is pending.
 #include "common.cuh"
+#include "gemm_pair.cuh"
 #include "tmap.cuh"
+#include "w4_format.cuh"
 #include "../../include/b200_tgis.h"
 
 #include <cstdlib>
@@ -50,12 +52,6 @@
 
 namespace b200 {
 
-constexpr int kW4TileM = 128;
-constexpr int kW4BlockK = 128;
-constexpr int kW4WordBytes = (kW4BlockK / 8) * kW4TileM * 4;  // 8192
-constexpr int kW4MetaRowBytes = kW4TileM * 4;                 // 512
-constexpr int kW4MaxGroupRows = 4;                            // groupsize >= 32
-constexpr int kW4RecMaxBytes = kW4WordBytes + kW4MaxGroupRows * kW4MetaRowBytes;  // 10240 = shared-memory stage stride
 // Warp roles.  The SM sub-partition arbiter favours the higher warp id, so the three single-thread roles that pace the
 // pipeline (MMA issue, the two TMA producers) get the highest ids, the 16 issue-bound dequant warps sit in the middle and
 // the mostly-waiting epilogue warps get the lowest (and sleep while they wait).
@@ -69,6 +65,10 @@ constexpr int kW4Threads = (kW4XProdWarp + 1) * 32;             // 768
 constexpr int kW4AColsPerStage = 64;  // 128 fp16 per row = 64 x 32-bit columns
 constexpr int64_t kW4CounterBytes = 64 * 1024;
 
+// Most tokens of one token tile; more go to the SM pairs (gemm_pair.cuh).  At 128 tokens the pairs would win on wide outputs and short k only
+// (us, this kernel / pairs: 2048 -> 2560 13.1 / 10.9, 4096 -> 28672 45.2 / 46.3, 4096 -> 4096 15.3 / 19.2, 14336 -> 4096 23.9 / 53.8); at 129 this
+// kernel would need two token tiles (4096 -> 4096 40.1 / 19.6, 14336 -> 4096 107 / 58).
+constexpr int kW4DecodeT = 128;
 constexpr int kW4R = 2;  // feature tiles per super-tile: consecutive units (super-tile, k-block, r = 0..1) share one activation tile
 
 template <int TN>
@@ -93,34 +93,6 @@ struct GemmW4Cfg {
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
 };
 
-__device__ __forceinline__ uint32_t lop3_and_or(uint32_t a, uint32_t b, uint32_t c) {
-  uint32_t r;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(b), "r"(c));  // (a & b) | c
-  return r;
-}
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-  uint32_t r;
-  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-  return r;
-}
-__device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-  return v;
-}
-__device__ __forceinline__ void lds_v4(uint32_t addr, uint32_t* v) {
-  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(addr));
-}
-__device__ __forceinline__ uint32_t hadd2_u(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
-__device__ __forceinline__ uint32_t hmul2_u(uint32_t a, uint32_t b) {
-  uint32_t r;
-  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-  return r;
-}
 __device__ __forceinline__ uint32_t lds_acquire_cta(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
@@ -135,18 +107,6 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
   return v;
 }
 
-// non-blocking poll (mbarrier.try_wait may suspend the thread until a time-out when the phase is still pending)
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred P;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, P;\n\t}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
 // wait of a warp that has nothing else to do for a long time: sleep between polls so it does not take issue slots
 __device__ __forceinline__ void mbar_wait_relaxed(uint64_t* bar, uint32_t parity) {
   uint32_t spins = 0;
@@ -156,55 +116,22 @@ __device__ __forceinline__ void mbar_wait_relaxed(uint64_t* bar, uint32_t parity
   }
 }
 
-// one packed word (8 weights along k) -> 4 half2 (k, k+1) pairs, each fp16(scale * (q - zero)):
-//   low nibbles:  0x6400 | q      = 1024 + q   (ulp 1);     + (-(1024 + zero)) is exact
-//   high nibbles: 0x5400 | q << 4 = 64 + q     (ulp 1/16);  + (-(64 + zero))   is exact
-// then one rounding in the multiplication by the scale, as in fp16(scale * (q - zero)).
-__device__ __forceinline__ void dequant_word(uint32_t w, uint32_t nz1024, uint32_t nz64, uint32_t scale2, uint32_t* out) {
-  const uint32_t w8 = w >> 8;
-  const uint32_t q0 = lop3_and_or(w, 0x000f000fu, 0x64006400u);   // (k0, k1)
-  const uint32_t q1 = lop3_and_or(w, 0x00f000f0u, 0x54005400u);   // (k2, k3)
-  const uint32_t q2 = lop3_and_or(w8, 0x000f000fu, 0x64006400u);  // (k4, k5)
-  const uint32_t q3 = lop3_and_or(w8, 0x00f000f0u, 0x54005400u);  // (k6, k7)
-  out[0] = hmul2_u(hadd2_u(q0, nz1024), scale2);
-  out[1] = hmul2_u(hadd2_u(q1, nz64), scale2);
-  out[2] = hmul2_u(hadd2_u(q2, nz1024), scale2);
-  out[3] = hmul2_u(hadd2_u(q3, nz64), scale2);
-}
-// meta word (fp16 scale | (zero + 1) << 16) -> the three half2 constants of dequant_word
-__device__ __forceinline__ void dequant_consts(uint32_t rec, uint32_t& scale2, uint32_t& nz1024, uint32_t& nz64) {
-  scale2 = prmt(rec, rec, 0x1010);             // fp16 scale in both halves
-  const uint32_t z2 = prmt(rec, rec, 0x3232);  // zero + 1 (1..16) in both halves
-  nz1024 = 0xE400E400u + z2;                   // -(1024 + zero), exact
-  nz64 = 0xD400D400u + (z2 << 4);              // -(64 + zero), exact
-}
-
-// fp16(fp16(silu(fp16 g)) * fp16 u) from the two fp32 accumulators: exactly what the separate linear (fp16 output) followed
-// by silu_mul_kernel (elementwise.cu; torch fp16 SiLU = fp32 x / (1 + exp(-x)), one rounding, then an fp16 multiply) gives
-__device__ __forceinline__ __half silu_mul_f16(float gate_acc, float up_acc) {
-  const float g = __half2float(__float2half_rn(gate_acc));
-  const __half a = __float2half_rn(g / (1.f + expf(-g)));
-  return __hmul(a, __float2half_rn(up_acc));
-}
-
 struct W4Params {
   __half* y;
-  float* partial;   // [token tile][super-tile][contributor][kW4R][TN][128] fp32
-  int* counters;    // [token tile][super-tile][2]: partials written / slices reduced
+  float* partial;   // [super-tile][contributor][kW4R][TN][128] fp32
+  int* counters;    // [super-tile][2]: partials written / slices reduced
   const __half* bias;
   const unsigned char* packed;  // unit records, (super-tile, k-block, r) order
   int T, N;
   int nkb;          // 128-wide k-blocks per tile
   int n_super;      // super-tiles (pairs of 128-feature tiles)
   int su_per_cta;   // contiguous (super-tile, k-block) super-units per CTA
-  int total_su;     // per token tile
+  int total_su;
   int max_contrib;  // partial slots per super-tile
   int rec_bytes;    // 8192 + group_rows * 512
   int half_tiles;   // 0: super-tile s = feature tiles (2s, 2s+1); > 0 ("gate|up" layout): tiles (s, s + half_tiles)
   int act;          // 1: y[t, 128 s + m] = fp16(silu(fp16 gate)) * fp16 up  (needs the gate|up layout), row stride ldy
   int ldy;          // output row stride in halves
-  int persist;      // 1 (several token tiles, prefill): grid.x persistent CTAs take whole (token tile, super-tile) items c, c + grid, ...
-  int n_items;      //    n_token_tiles * n_super items, token tile major (concurrent CTAs share an activation tile in L2)
   int defer;        // 1: every super-tile segment is left as an fp32 partial in the workspace and the NEXT kernel of the stream sums
                     //    them (B200SplitK consumers: rmsnorm / rope / SiLU*up / all-reduce); no counters, no waiting on peer CTAs
   unsigned long long* trace;  // debug: per-CTA phase timestamps (globaltimer ns), NULL in production
@@ -232,30 +159,18 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
   // exactly one per 16 MMAs.)  Monotonic: super-unit j is ready at 9 * (j / 8 + 1).
   __shared__ uint32_t s_ready[8];
   __shared__ uint32_t s_issued;  // super-units whose MMAs have been issued (hand-over between the two MMA warps)
-  __shared__ int s_fix[2][4];  // super-tiles this CTA shares with others: {counter index, super-tile, contributors, my index}
+  __shared__ int s_fix[2][3];  // super-tiles this CTA shares with others: {super-tile, contributors, my index}
   __shared__ int s_nfix;
 
   pdl_launch_dependents();
   const int warp = warp_id(), lane = lane_id();
-  // Two ways to cut the work.  Decode (one token tile): a contiguous range of super-units of the (super-tile, k-block) space.
-  // Prefill (persist): whole items = all k-blocks of one super-tile for one token tile; CTA c takes items c, c + grid, ... so that
-  // launch, set-up and pipeline ramp are paid once per SM instead of once per item (they cost as much as ~30 k-blocks of main loop:
-  // the gate_up projection ran at 43 % of the tensor peak against 67 % for the 3.5 x deeper down projection, ncu r2).
-  const bool persist = p.persist != 0;
-  const int n_items_cta = persist ? (p.n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-  const int t0 = persist ? 0 : blockIdx.y * TN;
-  const int su0 = persist ? 0 : blockIdx.x * p.su_per_cta;
-  const int su1 = persist ? n_items_cta * p.nkb : min(p.total_su, su0 + p.su_per_cta);
+  const int su0 = blockIdx.x * p.su_per_cta;  // a contiguous range of super-units of the (super-tile, k-block) space
+  const int su1 = min(p.total_su, su0 + p.su_per_cta);
   const int n_su = su1 - su0;
   const int n_units = n_su * kW4R;
-  const int kb0 = persist ? 0 : su0 % p.nkb;
-  auto item_of_seg = [&](int seg) { return (int)blockIdx.x + seg * (int)gridDim.x; };
-  auto t0_of_seg = [&](int seg) { return persist ? (item_of_seg(seg) / p.n_super) * TN : t0; };
+  const int kb0 = su0 % p.nkb;
   auto unit_src = [&](int i) -> const unsigned char* {  // HBM address of this CTA's i-th unit record
-    if (!persist) return p.packed + ((size_t)su0 * kW4R + i) * p.rec_bytes;
-    const int per_item = p.nkb * kW4R;
-    const int seg = i / per_item;
-    return p.packed + ((size_t)(item_of_seg(seg) % p.n_super) * per_item + (i - seg * per_item)) * p.rec_bytes;
+    return p.packed + ((size_t)su0 * kW4R + i) * p.rec_bytes;
   };
 #define W4_TRACE(id, who)                                                                              \
   do {                                                                                                 \
@@ -277,7 +192,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
         mbar_init(&empty_w[s], 4);  // the 4 warps of the team that owns the stage
       }
       mbar_fence_init();
-      const uint64_t pol_w = persist ? policy_evict_last() : policy_evict_first();  // prefill re-reads the weights once per token tile
+      const uint64_t pol_w = policy_evict_first();
       const int n0 = min(n_units, C::kWStages);
       for (int i = 0; i < n0; ++i) {
         mbar_arrive_expect_tx(&full_w[i], p.rec_bytes);
@@ -312,7 +227,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
     // ------------------------------------------------------------------ TMA producer: unit records (HBM stream); the first
     // ring was issued above
     if (elect_one()) {
-      const uint64_t pol_w = persist ? policy_evict_last() : policy_evict_first();
+      const uint64_t pol_w = policy_evict_first();
       int s = 0, ph = 0;  // stage 0 again: wait for its first release
       for (int i = w_issued; i < n_units; ++i) {
         mbar_wait(&empty_w[s], ph);
@@ -326,16 +241,13 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
     // one [TN x 128] tile per super-unit; the same thread watches the tiles land and counts them into s_ready
     if (elect_one()) {
       const uint64_t pol_x = policy_evict_last();
-      int kb = kb0, seg_x = 0, t0x = t0_of_seg(0);
+      int kb = kb0;
       auto load_x = [&](int s) {
         mbar_arrive_expect_tx(&full_x[s], C::kXStageBytes);
         unsigned char* st = x_ring + s * C::kXStageBytes;
-        tma_load_2d_hint(st, &tmap_x, kb * kW4BlockK, t0x, &full_x[s], pol_x);
-        tma_load_2d_hint(st + C::kXSubBytes, &tmap_x, kb * kW4BlockK + 64, t0x, &full_x[s], pol_x);
-        if (++kb == p.nkb) {
-          kb = 0;
-          t0x = t0_of_seg(++seg_x);  // persist: the next item may belong to another token tile
-        }
+        tma_load_2d_hint(st, &tmap_x, kb * kW4BlockK, 0, &full_x[s], pol_x);
+        tma_load_2d_hint(st + C::kXSubBytes, &tmap_x, kb * kW4BlockK + 64, 0, &full_x[s], pol_x);
+        if (++kb == p.nkb) kb = 0;
       };
       pdl_wait();  // x is the previous kernel's output; the weight ring is already streaming
       for (int j = 0; j < C::kXStages && j < n_su; ++j) load_x(j);
@@ -482,17 +394,15 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
     int seg = 0, nfix = 0;
     pdl_wait();  // outputs / bias / stream-K workspace belong to the stream order
     for (int u = su0; u < su1; ++seg) {
-      const int sup = persist ? item_of_seg(seg) % p.n_super : u / p.nkb;
-      const int seg_end = persist ? u + p.nkb : min(su1, (sup + 1) * p.nkb);
-      const int t0 = t0_of_seg(seg);  // shadows the CTA-wide value: persistent CTAs change token tile between items
+      const int sup = u / p.nkb;
+      const int seg_end = min(su1, (sup + 1) * p.nkb);
       const int buf = C::kDBufs == 2 ? (seg & 1) : 0;
-      // contributors of this super-tile: CTAs whose range intersects [sup*nkb, (sup+1)*nkb); a persistent CTA owns whole items
-      const int c_first = persist ? (int)blockIdx.x : (sup * p.nkb) / p.su_per_cta;
-      const int c_last = persist ? (int)blockIdx.x : ((sup + 1) * p.nkb - 1) / p.su_per_cta;
+      // contributors of this super-tile: CTAs whose range intersects [sup*nkb, (sup+1)*nkb)
+      const int c_first = (sup * p.nkb) / p.su_per_cta;
+      const int c_last = ((sup + 1) * p.nkb - 1) / p.su_per_cta;
       const int n_contrib = c_last - c_first + 1;
       const int my_contrib = (int)blockIdx.x - c_first;
-      const int tix = blockIdx.y * p.n_super + sup;
-      float* part = p.partial + ((size_t)tix * p.max_contrib + my_contrib) * (kW4R * TN * kW4TileM);
+      float* part = p.partial + ((size_t)sup * p.max_contrib + my_contrib) * (kW4R * TN * kW4TileM);
       mbar_wait_relaxed(&tmem_full[buf], C::kDBufs == 2 ? ((seg >> 1) & 1) : (seg & 1));
       tcgen05_fence_after();
       W4_TRACE(8 + (seg & 3) * 2, 0);
@@ -517,7 +427,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
           if (!direct) {
 #pragma unroll
             for (int j = 0; j < kCh; ++j) {
-              if (t0 + c + j < p.T) {
+              if (c + j < p.T) {
                 part[(c + j) * kW4TileM + m] = __uint_as_float(d0[j]);
                 part[(TN + c + j) * kW4TileM + m] = __uint_as_float(d1[j]);
               }
@@ -526,14 +436,14 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
             if (ok0) {
 #pragma unroll
               for (int j = 0; j < kCh; ++j) {
-                const int t = t0 + c + j;
+                const int t = c + j;
                 if (t < p.T) p.y[(size_t)t * p.ldy + n0] = silu_mul_f16(__uint_as_float(d0[j]) + bv0, __uint_as_float(d1[j]) + bv1);
               }
             }
           } else {
 #pragma unroll
             for (int j = 0; j < kCh; ++j) {
-              const int t = t0 + c + j;
+              const int t = c + j;
               if (t < p.T) {
                 if (ok0) p.y[(size_t)t * p.ldy + n0] = __float2half_rn(__uint_as_float(d0[j]) + bv0);
                 if (ok1) p.y[(size_t)t * p.ldy + n1] = __float2half_rn(__uint_as_float(d1[j]) + bv1);
@@ -551,11 +461,10 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
         asm volatile("bar.sync 1, %0;" ::"n"(kW4EpWarps * 32) : "memory");
         if (threadIdx.x == 0) {
           __threadfence();
-          atomicAdd(&p.counters[2 * tix], 1);
-          s_fix[nfix][0] = tix;
-          s_fix[nfix][1] = sup;
-          s_fix[nfix][2] = n_contrib;
-          s_fix[nfix][3] = my_contrib;
+          atomicAdd(&p.counters[2 * sup], 1);
+          s_fix[nfix][0] = sup;
+          s_fix[nfix][1] = n_contrib;
+          s_fix[nfix][2] = my_contrib;
         }
         ++nfix;
       }
@@ -573,18 +482,18 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
   if (nfix > 0) pdl_wait();
   W4_TRACE(40, 0);
   for (int f = 0; f < nfix; ++f) {
-    const int tix = s_fix[f][0], sup = s_fix[f][1], n_contrib = s_fix[f][2], my_contrib = s_fix[f][3];
+    const int sup = s_fix[f][0], n_contrib = s_fix[f][1], my_contrib = s_fix[f][2];
     if (threadIdx.x == 0) {
       uint32_t spins = 0;
-      while (ld_acquire_gpu(&p.counters[2 * tix]) < n_contrib) {  // all contributors are co-resident (grid <= #SMs, 1 CTA/SM)
+      while (ld_acquire_gpu(&p.counters[2 * sup]) < n_contrib) {  // all contributors are co-resident (grid <= #SMs, 1 CTA/SM)
         __nanosleep(64);
         if (++spins > (1u << 24)) __trap();
       }
     }
     __syncthreads();
     W4_TRACE(41 + f * 3, 0);
-    const float* base = p.partial + (size_t)tix * p.max_contrib * (kW4R * TN * kW4TileM);
-    const int rows = min(p.T - t0, TN);
+    const float* base = p.partial + (size_t)sup * p.max_contrib * (kW4R * TN * kW4TileM);
+    const int rows = min(p.T, TN);
     const int n_vec = kW4R * rows * (kW4TileM / 4);  // float4 elements: [r][row][32]
     const int per = (n_vec + n_contrib - 1) / n_contrib;
     const int hi = min(n_vec, (my_contrib + 1) * per);
@@ -614,7 +523,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
           uint2 o;
           o.x = pack_half2(acc.x, acc.y);
           o.y = pack_half2(acc.z, acc.w);
-          *reinterpret_cast<uint2*>(&p.y[(size_t)(t0 + tt) * p.ldy + nn]) = o;
+          *reinterpret_cast<uint2*>(&p.y[(size_t)tt * p.ldy + nn]) = o;
         }
       }
     } else {
@@ -648,7 +557,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
           u.x += __half2float(p.bias[nu]); u.y += __half2float(p.bias[nu + 1]); u.z += __half2float(p.bias[nu + 2]); u.w += __half2float(p.bias[nu + 3]);
         }
         __half o[4] = {silu_mul_f16(g.x, u.x), silu_mul_f16(g.y, u.y), silu_mul_f16(g.z, u.z), silu_mul_f16(g.w, u.w)};
-        *reinterpret_cast<uint2*>(&p.y[(size_t)(t0 + tt) * p.ldy + nn]) = *reinterpret_cast<uint2*>(o);
+        *reinterpret_cast<uint2*>(&p.y[(size_t)tt * p.ldy + nn]) = *reinterpret_cast<uint2*>(o);
       }
     }
     W4_TRACE(42 + f * 3, 0);
@@ -656,10 +565,10 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
     W4_TRACE(43 + f * 3, 0);
     if (threadIdx.x == 0) {
       // the last contributor to finish its slice re-arms both counters for the next launch (graph replay safe)
-      const int prev = atomicAdd(&p.counters[2 * tix + 1], 1);
+      const int prev = atomicAdd(&p.counters[2 * sup + 1], 1);
       if (prev == n_contrib - 1) {
-        p.counters[2 * tix] = 0;
-        p.counters[2 * tix + 1] = 0;
+        p.counters[2 * sup] = 0;
+        p.counters[2 * sup + 1] = 0;
         __threadfence();
       }
     }
@@ -920,15 +829,7 @@ static int launch_gemm_w4(const CUtensorMap* mx, const void* packed, void* y, vo
   p.ldy = act ? N / 2 : N;
   p.defer = defer;
   p.trace = g_w4_trace;
-  dim3 grid(pl.n_ctas, pl.n_tiles_t, 1);
-  p.persist = 0;
-  p.n_items = 0;
-  if (pl.n_tiles_t > 1) {  // prefill: persistent CTAs over (token tile, super-tile) items
-    p.persist = 1;
-    p.n_items = pl.n_super * pl.n_tiles_t;
-    const int sms = num_sms();
-    grid = dim3(p.n_items < sms ? p.n_items : sms, 1, 1);
-  }
+  const dim3 grid(pl.n_ctas);
   b200_timing_mark(B200_TIME_GEMM_W4A16, 0, st);
   constexpr auto kernel = gemm_w4a16_kernel<TN, kGR>;
   B200_LAUNCH_AS("gemm_w4a16_kernel", kernel, grid, dim3(kW4Threads), (size_t)C::kSmemBytes, st, *mx, p);
@@ -955,6 +856,23 @@ static int gemm_w4a16_impl(const void* x, const void* packed, const void* bias, 
     return B200_ERR_UNSUPPORTED;
   }
   const int gr = w4_group_rows(K, &groupsize);
+  if (!defer && T > kW4DecodeT) {
+    PairParams pp = {};
+    pp.y = y;
+    pp.bias = bias;
+    pp.packed = (const unsigned char*)packed;
+    pp.T = (int)T;
+    pp.N = (int)N;
+    pp.ldy = (int)(act ? N / 2 : N);
+    pp.n_kb = 2 * (int)((K + kW4BlockK - 1) / kW4BlockK);
+    pp.rec_per_tile = w4_nkb(K);
+    pp.rec_bytes = kW4WordBytes + gr * kW4MetaRowBytes;
+    pp.group_rows = gr;
+    pp.half_tiles = half_tiles;
+    const PairPlan pl = pair_plan(T, N, pp.n_kb, true, num_sms());
+    return act ? launch_gemm_pair<kPairW4Silu>(x, nullptr, K, pp, pl, B200_TIME_GEMM_W4A16, (cudaStream_t)stream)
+               : launch_gemm_pair<kPairW4>(x, nullptr, K, pp, pl, B200_TIME_GEMM_W4A16, (cudaStream_t)stream);
+  }
   const W4Plan pl = launch_plan_w4(T, N, K, num_sms(), workspace != nullptr, defer);
   const CUtensorMap* mx = get_tmap_2d(x, T, K, K, pl.TN, 64, TmapDtype::kF16, TmapSwizzle::k128B);
   if (!mx) return B200_ERR_CUDA;
