@@ -1,0 +1,76 @@
+"""Prompt attention over the paged pool (csrc/attn_prefill_paged.cu) where its schedule could go wrong: more items than SMs, head groups that
+pair heads and that pair query tiles (with and without a second tile), maxima that grow slowly, by leaps and late, scores of any sign of the
+scale, and rows whose weights are all alike.  Reference: float64.
+
+Tolerance: a weight is rounded to fp16 once (2^-11 of it), the sum normalises the rounded weights, so an output is off by at most 2 * 2^-11 of the
+weighted mean of |v|, plus its own rounding; scores are fp32 sums of d products (d 2^-24 of the largest, times the weight's slope 1)."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _run(lens, past, H, G, d, scale, shape_keys=None, seed=0):
+    import tgis_b200  # noqa: F401
+    from tgis_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    L = [n + past for n in lens]
+    pages = [(n + 15) // 16 for n in L]
+    perm = torch.randperm(sum(pages) + 3, generator=g, device=DEV).int()
+    table = torch.zeros(len(lens), max(pages), dtype=torch.int32, device=DEV)
+    shape = (sum(pages) + 3, G, 16, d)
+    kp, vp = torch.randn(shape, generator=g, device=DEV).half(), torch.randn(shape, generator=g, device=DEV).half()
+    T = sum(lens)
+    q = torch.randn(T, (H + 2 * G) * d, generator=g, device=DEV).half()[:, :H * d].unflatten(1, (H, d))
+    t, c = torch.arange(16, device=DEV)[:, None], torch.arange(d // 8, device=DEV)[None, :]
+    at = 0
+    for b, n in enumerate(pages):
+        table[b, :n] = perm[at:at + n]
+        at += n
+        if shape_keys is not None:   # a factor per key position
+            f = shape_keys(torch.arange(n * 16, device=DEV)).view(n, 1, 16, 1)
+            idx = table[b, :n].long()
+            kp[idx] = (kp[idx].float() * f).half()
+    out = torch.full((T, H, d), float("nan"), dtype=torch.float16, device=DEV)
+    cu = torch.tensor([0] + lens, device=DEV).cumsum(0).int()
+    ops.attn_prefill_paged(q, kp, vp, table, torch.tensor(L, dtype=torch.int32, device=DEV), cu, max(lens), scale, out=out)
+    plain = [p.unflatten(-1, (-1, 8))[..., t, c ^ (t & 7), :].flatten(-2) for p in (kp, vp)]
+    row = 0
+    for b, (n, Lb) in enumerate(zip(lens, L)):
+        K, V = (p[table[b, :pages[b]].long()].transpose(1, 2).flatten(0, 1)[:Lb].double() for p in plain)
+        ok = torch.arange(Lb, device=DEV)[None] <= past + torch.arange(n, device=DEV)[:, None]
+        for h in range(H):
+            s = q[row:row + n, h].double() @ K[:, h * G // H].T
+            top = (s * scale).masked_fill(~ok, 0).abs().amax(1, keepdim=True)
+            w = torch.softmax((s * scale).masked_fill(~ok, -math.inf), 1)
+            ref, spread = w @ V[:, h * G // H], w @ V[:, h * G // H].abs()
+            tol = 2.0 ** -11 * ref.abs() + (2 * 2.0 ** -11 + 2 * d * 2.0 ** -24 * (1 + top)) * spread + 1e-6
+            err = (out[row:row + n, h].double() - ref).abs()
+            assert bool((err <= tol).all()), (b, h, float((err / tol).max()), int((err > tol).sum()))
+        row += n
+
+
+@pytest.mark.parametrize("H,G,d", [(8, 2, 128), (6, 2, 128), (3, 3, 64), (7, 1, 64), (12, 2, 64)])
+def test_head_and_tile_pairs(H, G, d):
+    _run([1, 128, 129, 255, 256, 257, 385, 40], 0, H, G, d, d ** -0.5)
+    _run([130, 3, 300], 77, H, G, d, d ** -0.5, seed=1)
+
+
+def test_more_items_than_sms():
+    _run([33 + 17 * (i % 9) for i in range(40)], 0, 16, 4, 64, 0.125, seed=2)
+
+
+@pytest.mark.parametrize("grow", ["slow", "leaps", "late", "falling", "flat"])
+def test_maxima_that_move(grow):
+    f = {"slow": lambda p: 0.2 + p / 300.0, "leaps": lambda p: 4.0 ** (p // 300).clamp(max=3), "late": lambda p: torch.where(p > 1300, 12.0, 0.05),
+         "falling": lambda p: 6.0 / (1 + p / 100.0), "flat": lambda p: 0.0 * p}[grow]
+    _run([1500, 700], 0, 4, 2, 128, 128 ** -0.5, shape_keys=f, seed=3)
+    _run([40], 1490, 4, 4, 64, 0.125, shape_keys=f, seed=4)
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.1])
+def test_scales_that_are_not_positive(scale):
+    _run([300, 20], 50, 4, 2, 64, scale, seed=5)

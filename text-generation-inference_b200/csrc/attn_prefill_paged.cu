@@ -7,41 +7,114 @@
 // CACHED context: query i of sequence b sits at absolute position context_lens[b] - n_q(b) + i and attends keys 0 .. that position.
 // That is what an add-on prefill over a prompt prefix, a chunked prefill and a mixed prefill + decode step need.
 //
-// Design (one CTA = 128 queries of one sequence x one query head; 6 warps):
-//   warp 0      TMA producer.  Q tile [128 x d] through a 128B-swizzled tensor map; per 128-key tile 8 KV pages x (K, V) x d/64
+// Design (12 warps, one persistent CTA per SM).  An item is TWO query tiles of 128 rows that meet the same keys, so that the tensor cores work for
+// one while the other is in its soft-max: two query heads of a key / value head when their number is even, else two neighbouring query tiles
+// of a head.  Items are taken longest first.
+//   warp 0      TMA producer.  Q tiles [128 x d] through a 128B-swizzled tensor map; per 128-key tile 8 KV pages x (K, V) x d/64
 //               slabs, each one cp.async.bulk.tensor box [16 tokens x 64 halves] of the pool: the pool stores every token row
 //               with its 16-byte chunks XOR-swizzled by (token & 7), which IS the tcgen05 SWIZZLE_128B image, so
-//               pages land in shared memory ready for the tensor core without any software swizzle.  2-stage ring.
-//   warp 1      MMA issuer (one elected thread).  S = Q K^T: tcgen05.mma kind::f16, both operands K-major from shared memory,
-//               fp32 accumulator in TMEM (two S buffers: QK^T of tile j+1 overlaps the softmax of tile j).
-//               O += P V: A = P from TMEM (fp16, written by the softmax warps over the S buffer), B = V as an MN-major
+//               pages land in shared memory ready for the tensor core without any software swizzle.  2-stage rings of K and V.
+//   warp 1      MMA issuer (one elected thread): P0 V, Q0 K of the next key tile, P1 V, Q1 K of the next key tile, and so on.
+//               S = Q K^T: tcgen05.mma kind::f16, both operands K-major from shared memory, fp32 accumulator in TMEM.
+//               O += P V: A = P from TMEM (fp16, written by the softmax warps over their S), B = V as an MN-major
 //               shared-memory operand (keys are the MMA K dimension, d contiguous), accumulator O in TMEM.
-//   warps 2..5  softmax: thread = one query row = one TMEM lane (no shuffles).  tcgen05.ld S, causal mask, fp32 online softmax
-//               in the log2 domain, P rounded to fp16 (flash-attn semantics) and stored back to TMEM; when the running maximum
-//               moved, O is rescaled in TMEM (tcgen05.ld / st) before the next P V accumulates into it.
-// Causality prunes whole key tiles (a query tile only visits tiles up to its last row's position).
+//   warps 4..7, 8..11   softmax of the first and the second tile: thread = one query row = one TMEM lane (no shuffles).  tcgen05.ld S, causal
+//               mask, fp32 online softmax in the log2 domain, P rounded to fp16 (flash-attn semantics) and stored back to TMEM, O
+//               rescaled in TMEM when a row's reference maximum moves (kPfExactTiles, kPfRescale).  The row's sum adds the rounded P, what the
+//               products weigh.  S of tile j is complete only after P V of tile j - 1 (issue order), so O is quiescent whenever a
+//               softmax warp runs.
+// Causality over absolute positions prunes whole key tiles.  Bound: soft-max exponentials (MUFU, 16 a cycle and SM: 1024 cycles per 128 x 128 tile,
+// as long as its products at d = 128, twice as long at d = 64), and between items the pipeline's drain.  Measured on B200 (us, before: one query
+// tile of one head per CTA): 13 prompts of 300 to 2048 tokens, 32 / 8 heads, d = 128 571 -> 306; 16 x 1024 428 -> 199; 8192 1196 -> 500 (1.10
+// PFLOP/s); d = 64, 32 / 4 heads 440 -> 251; 300 tokens after 1500 cached ones x 4 110 -> 72.  Tried: four more warps for the output (305 instead of
+// 287: the softmax warps are then compiled for 128 registers).
 #include "common.cuh"
 #include "tmap.cuh"
 #include "../../include/b200_tgis.h"
 
 namespace b200 {
 
-constexpr int kPfM = 128;        // queries per CTA
+constexpr int kPfM = 128;        // queries per tile, two tiles per item
 constexpr int kPfN = 128;        // keys per tile = 8 pages
-constexpr int kPfThreads = 192;  // warp 0 TMA, warp 1 MMA, warps 2..5 softmax
+constexpr int kPfThreads = 384;  // warp 0 TMA, warp 1 MMA, warps 4..11 softmax
 constexpr int kPfSlabBytes = 128 * 128;  // 128 rows x 64 halves
 constexpr int kPfPageSlabBytes = kPageTokens * 128;
-constexpr float kPfNegBig = -1.0e30f;
+constexpr int kPfStages = 2;
+// The reference maximum of a row follows the true one through the first key tiles after the first; later it moves only when the maximum has grown
+// past it by more than 2^8.  A largest weight of exactly 1 is worth some precision (against float64, over prompts of 64 to 2500 keys: 0.993 of
+// the error of following it always with unrounded sums, 1.006 with no exact tiles), following it always costs 323 us where this takes 306.
+constexpr int kPfExactTiles = 4;
+constexpr float kPfRescale = 8.f;  // log2
+// registers per thread: the launch has 384 x 168; the two softmax warpgroups take 216 each, the other one keeps 72
+constexpr int kPfSoftmaxRegs = 216, kPfServeRegs = 72;
+
+__device__ int attn_prefill_gave_up;
 
 template <int D>
 struct PfCfg {
   static constexpr int kSlabs = D / 64;
   static constexpr int kTileBytes = kSlabs * kPfSlabBytes;  // a Q, K or V tile
-  static constexpr int kStages = 2;
-  static constexpr int kNumBars = 1 + 3 * kStages + 2 + 2 + 1;  // q_full | k_full, v_full, kv_empty | s_full[2] | p_ready[2] | o_done
-  static constexpr int kSmemBytes = (1 + 2 * kStages) * kTileBytes + kNumBars * 8 + 16 + 1024;
-  static constexpr int kTmemCols = 512;  // S0 [0,128) | S1 [128,256) | O [256, 256 + D)
+  static constexpr int kNumBars = 2 + 4 * kPfStages + 6;    // q_full, q_empty | k_full, k_empty, v_full, v_empty | s_full[2], p_ready[2], o_full[2]
+  static constexpr int kSmemBytes = (2 + 2 * kPfStages) * kTileBytes + kNumBars * 8 + 16 + 1024;
+  static constexpr int kTmemCols = 512;  // S0 [0,128) | S1 [128,256) | O0 [256, 256 + D) | O1 behind it
 };
+
+struct PfParams {
+  const int32_t* block_table;
+  int64_t bt_stride;
+  const int32_t* context_lens;
+  const int32_t* cu_q;
+  __half* out;
+  int64_t out_stride;
+  int n_heads, n_kv, B;
+  int pair_heads;        // 1: an item is two heads, 0: two query tiles
+  int n_units, n_groups; // head (pair)s, query tile (pair)s of the longest sequence
+  float scale_log2;
+};
+
+// one item: the rows and key tiles of its two query tiles
+struct PfItem {
+  int b, q_begin, past, last_page, kv_head;
+  int q0[2], rows[2], head[2], n_kt[2], n;
+};
+
+// item i, longest query tiles first; n = 0: the sequence has no such tile
+__device__ __forceinline__ PfItem pf_item(const PfParams& p, int i) {
+  PfItem it;
+  const int per = p.B * p.n_units, group = p.n_groups - 1 - i / per, r = i % per, unit = r % p.n_units;
+  it.b = r / p.n_units;
+  it.q_begin = p.cu_q[it.b];
+  const int n_q = p.cu_q[it.b + 1] - it.q_begin, L = p.context_lens[it.b];
+  it.past = max(L - n_q, 0);  // cached tokens in front of this step's first query
+  it.last_page = (L - 1) / kPageTokens;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    it.head[u] = p.pair_heads ? 2 * unit + u : unit;
+    it.q0[u] = (p.pair_heads ? group : 2 * group + u) * kPfM;
+    it.rows[u] = min(kPfM, n_q - it.q0[u]);
+    it.n_kt[u] = it.rows[u] > 0 ? (it.past + it.q0[u] + it.rows[u] - 1) / kPfN + 1 : 0;  // key tiles the last row reaches
+  }
+  it.kv_head = it.head[0] / (p.n_heads / p.n_kv);
+  it.n = max(it.n_kt[0], it.n_kt[1]);
+  return it;
+}
+
+__device__ __forceinline__ uint64_t f32x2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f32x2_split(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ float add_f32_f16(float a, uint16_t h) {
+  float r;
+  asm("add.rn.f32.f16 %0, %1, %2;" : "=f"(r) : "h"(h), "f"(a));
+  return r;
+}
 
 // MN-major shared-memory operand, 128-byte swizzle: rows along K (here: keys) of 128 bytes = 64 MN elements, 8-row swizzle atoms
 // `sbo` bytes apart, blocks of 64 MN elements `lbo` bytes apart.  Bit layout as umma_desc_kmajor_sw128 (common.cuh).
@@ -58,234 +131,278 @@ __device__ __forceinline__ uint64_t umma_desc_mnmajor_sw128(uint32_t smem_addr, 
 template <int D>
 __global__ void __launch_bounds__(kPfThreads, 1)
 attn_prefill_paged_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                          const __grid_constant__ CUtensorMap tmap_v, const int32_t* __restrict__ block_table, int64_t bt_stride,
-                          const int32_t* __restrict__ context_lens, const int32_t* __restrict__ cu_q, __half* __restrict__ out,
-                          int64_t out_stride, int n_heads, int n_kv, int tiles_per_seq, float scale_log2) {
+                          const __grid_constant__ CUtensorMap tmap_v, const PfParams p) {
   using C = PfCfg<D>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   unsigned char* sQ = smem;
-  unsigned char* sKV = smem + C::kTileBytes;  // stage s: K at sKV + s * 2 * kTileBytes, V right behind it
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sKV + C::kStages * 2 * C::kTileBytes);
-  uint64_t* q_full = bars;
-  uint64_t* k_full = bars + 1;
-  uint64_t* v_full = k_full + C::kStages;
-  uint64_t* kv_empty = v_full + C::kStages;
-  uint64_t* s_full = kv_empty + C::kStages;
+  unsigned char* sK = sQ + 2 * C::kTileBytes;
+  unsigned char* sV = sK + kPfStages * C::kTileBytes;
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(sV + kPfStages * C::kTileBytes);
+  uint64_t* q_empty = q_full + 1;
+  uint64_t* k_full = q_empty + 1;
+  uint64_t* k_empty = k_full + kPfStages;
+  uint64_t* v_full = k_empty + kPfStages;
+  uint64_t* v_empty = v_full + kPfStages;
+  uint64_t* s_full = v_empty + kPfStages;
   uint64_t* p_ready = s_full + 2;
-  uint64_t* o_done = p_ready + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
+  uint64_t* o_full = p_ready + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
 
   pdl_launch_dependents();
-  pdl_wait();  // q and the pool's newest tokens are the previous kernels' output
   const int warp = warp_id(), lane = lane_id();
-  const int b = blockIdx.x / tiles_per_seq, tile = blockIdx.x % tiles_per_seq;
-  const int head = blockIdx.y;
-  const int hk = head / (n_heads / n_kv);
-  const int q_begin = cu_q[b];
-  const int n_q = cu_q[b + 1] - q_begin;
-  const int q0 = tile * kPfM;
-  if (q0 >= n_q) return;  // the whole CTA: this sequence has fewer query tiles
-  const int L = context_lens[b];
-  const int past = max(L - n_q, 0);  // cached tokens in front of this step's first query
-  const int rows = min(kPfM, n_q - q0);
-  const int n_kt = (past + q0 + rows - 1) / kPfN + 1;  // key tiles the last query row reaches
-  const int last_page = (L - 1) / kPageTokens;
-
+  const int n_items = p.B * p.n_units * p.n_groups;
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_q);
     tma_prefetch_desc(&tmap_k);
     tma_prefetch_desc(&tmap_v);
     mbar_init(q_full, 1);
-    for (int s = 0; s < C::kStages; ++s) {
+    mbar_init(q_empty, 1);
+    for (int s = 0; s < kPfStages; ++s) {
       mbar_init(&k_full[s], 1);
+      mbar_init(&k_empty[s], 1);
       mbar_init(&v_full[s], 1);
-      mbar_init(&kv_empty[s], 1);
+      mbar_init(&v_empty[s], 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&s_full[i], 1);
-      mbar_init(&p_ready[i], 4);
+    for (int u = 0; u < 2; ++u) {
+      mbar_init(&s_full[u], 1);
+      mbar_init(&p_ready[u], 4);
+      mbar_init(&o_full[u], 1);
     }
-    mbar_init(o_done, 1);
     mbar_fence_init();
   }
-  if (warp == 0) tmem_alloc<C::kTmemCols>(tmem_slot);
+  if (warp == 2) tmem_alloc<C::kTmemCols>(tmem_slot);
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_o = tmem_base + 256;
+  bool ok = true;
+  pdl_wait();  // q, the index tensors and the pool's newest tokens are the previous kernels' output
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      mbar_arrive_expect_tx(q_full, C::kTileBytes);
-      for (int s = 0; s < C::kSlabs; ++s) tma_load_2d(sQ + s * kPfSlabBytes, &tmap_q, head * D + s * 64, q_begin + q0, q_full);
-    }
-    const int32_t* bt = block_table + (int64_t)b * bt_stride;
-    for (int j = 0; j < n_kt; ++j) {
-      const int st = j % C::kStages;
-      // 8 pages of this key tile; pages past the sequence's last one repeat it (finite data, masked by the softmax warps)
-      const int page = min(j * (kPfN / kPageTokens) + (lane & 7), last_page);
-      const int blk = bt[page];
-      if (lane == 0) mbar_wait(&kv_empty[st], ((j / C::kStages) & 1) ^ 1);
-      __syncwarp();
-      unsigned char* sK = sKV + st * 2 * C::kTileBytes;
-      unsigned char* sV = sK + C::kTileBytes;
-      if (lane == 0) {
-        mbar_arrive_expect_tx(&k_full[st], C::kTileBytes);
-        mbar_arrive_expect_tx(&v_full[st], C::kTileBytes);
-      }
-      for (int p = 0; p < kPfN / kPageTokens; ++p) {
-        const int bp = __shfl_sync(0xffffffffu, blk, p);
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPfServeRegs));
+    if (warp == 0) {
+      // ------------------------------------------------------------------ TMA producer
+      int st = 0, ph = 1, qph = 1;
+      for (int i = blockIdx.x; i < n_items; i += gridDim.x) {
+        const PfItem it = pf_item(p, i);
+        if (it.n == 0) continue;
+        mbar_wait_soft(q_empty, qph, ok);  // the previous item's last Q K^T
+        qph ^= 1;
         if (lane == 0) {
-          const int row = (bp * n_kv + hk) * kPageTokens;  // row of the pool viewed as [blocks * n_kv * 16, d]
-          for (int s = 0; s < C::kSlabs; ++s)
-            tma_load_2d(sK + s * kPfSlabBytes + p * kPfPageSlabBytes, &tmap_k, s * 64, row, &k_full[st]);
+          mbar_arrive_expect_tx(q_full, ((it.n_kt[0] > 0) + (it.n_kt[1] > 0)) * C::kTileBytes);
+          for (int u = 0; u < 2; ++u)
+            if (it.n_kt[u] > 0)
+              for (int s = 0; s < C::kSlabs; ++s)
+                tma_load_2d(sQ + u * C::kTileBytes + s * kPfSlabBytes, &tmap_q, it.head[u] * D + s * 64, it.q_begin + it.q0[u], q_full);
+        }
+        const int32_t* bt = p.block_table + (int64_t)it.b * p.bt_stride;
+        for (int j = 0; j < it.n; ++j) {
+          // 8 pages of this key tile, a lane each; pages past the sequence's last one repeat it (finite data, masked by the softmax warps)
+          const int page = min(j * (kPfN / kPageTokens) + (lane & 7), it.last_page);
+          const int row = (bt[page] * p.n_kv + it.kv_head) * kPageTokens;  // row of the pool viewed as [blocks * n_kv * 16, d]
+          mbar_wait_soft(&k_empty[st], ph, ok);
+          if (lane == 0) mbar_arrive_expect_tx(&k_full[st], C::kTileBytes);
+          __syncwarp();
+          if (lane < 8)
+            for (int s = 0; s < C::kSlabs; ++s)
+              tma_load_2d(sK + st * C::kTileBytes + s * kPfSlabBytes + lane * kPfPageSlabBytes, &tmap_k, s * 64, row, &k_full[st]);
+          __syncwarp();
+          mbar_wait_soft(&v_empty[st], ph, ok);
+          if (lane == 0) mbar_arrive_expect_tx(&v_full[st], C::kTileBytes);
+          __syncwarp();
+          if (lane < 8)
+            for (int s = 0; s < C::kSlabs; ++s)
+              tma_load_2d(sV + st * C::kTileBytes + s * kPfSlabBytes + lane * kPfPageSlabBytes, &tmap_v, s * 64, row, &v_full[st]);
+          __syncwarp();
+          if (++st == kPfStages) { st = 0; ph ^= 1; }
         }
       }
-      for (int p = 0; p < kPfN / kPageTokens; ++p) {
-        const int bp = __shfl_sync(0xffffffffu, blk, p);
-        if (lane == 0) {
-          const int row = (bp * n_kv + hk) * kPageTokens;
-          for (int s = 0; s < C::kSlabs; ++s)
-            tma_load_2d(sV + s * kPfSlabBytes + p * kPfPageSlabBytes, &tmap_v, s * 64, row, &v_full[st]);
+    } else if (warp == 1) {
+      // ------------------------------------------------------------------ MMA issuer
+      constexpr uint32_t idesc_qk = umma_idesc_f16_f32acc(kPfM, kPfN);
+      constexpr uint32_t idesc_pv = umma_idesc_f16_f32acc(kPfM, D) | (1u << 16);  // B (= V) is MN-major
+      const uint64_t qdesc = umma_desc_kmajor_sw128(smem_u32(sQ)), kdesc = umma_desc_kmajor_sw128(smem_u32(sK));
+      const uint64_t vdesc = umma_desc_mnmajor_sw128(smem_u32(sV), kPfSlabBytes, 1024);
+      int kst = 0, kph = 0, vst = 0, vph = 0, qph = 0, pph[2] = {0, 0};
+      auto issue_qk = [&](int u) {
+        if (elect_one()) {
+          const uint64_t a = qdesc + (uint64_t)((u * C::kTileBytes) >> 4), b = kdesc + (uint64_t)((kst * C::kTileBytes) >> 4);
+#pragma unroll
+          for (int k = 0; k < D / 16; ++k) {
+            const uint64_t off = (uint64_t)((k >> 2) * (kPfSlabBytes >> 4) + (k & 3) * 2);
+            umma_f16_ss(tmem_base + u * kPfN, a + off, b + off, idesc_qk, k > 0 ? 1u : 0u);
+          }
+          umma_commit(&s_full[u]);
         }
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    constexpr uint32_t idesc_qk = umma_idesc_f16_f32acc(kPfM, kPfN);
-    constexpr uint32_t idesc_pv = umma_idesc_f16_f32acc(kPfM, D) | (1u << 16);  // B (= V) is MN-major
-    const uint64_t qdesc = umma_desc_kmajor_sw128(smem_u32(sQ));
-    auto issue_qk = [&](int j) {
-      const int st = j % C::kStages, buf = j & 1;
-      mbar_wait(&k_full[st], (j / C::kStages) & 1);
-      tcgen05_fence_after();
-      if (elect_one()) {
-        const uint64_t kdesc = umma_desc_kmajor_sw128(smem_u32(sKV + st * 2 * C::kTileBytes));
+        __syncwarp();
+      };
+      auto release = [&](uint64_t* bar) {
+        if (elect_one()) umma_commit(bar);
+        __syncwarp();
+      };
+      for (int i = blockIdx.x; i < n_items; i += gridDim.x) {
+        const PfItem it = pf_item(p, i);
+        if (it.n == 0) continue;
+        mbar_wait_soft(q_full, qph, ok);
+        qph ^= 1;
+        for (int j = -1; j < it.n; ++j) {  // P V of key tile j, Q K^T of key tile j + 1
+          const bool more = j + 1 < it.n;
+          if (more) mbar_wait_soft(&k_full[kst], kph, ok);
+          if (j >= 0) mbar_wait_soft(&v_full[vst], vph, ok);
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint64_t off = (uint64_t)((k >> 2) * (kPfSlabBytes >> 4) + (k & 3) * 2);
-          umma_f16_ss(tmem_base + buf * kPfN, qdesc + off, kdesc + off, idesc_qk, k > 0 ? 1u : 0u);
-        }
-        umma_commit(&s_full[buf]);
-      }
-      __syncwarp();
-    };
-    mbar_wait(q_full, 0);
-    issue_qk(0);
-    for (int j = 0; j < n_kt; ++j) {
-      const int st = j % C::kStages, buf = j & 1;
-      if (j + 1 < n_kt) issue_qk(j + 1);  // overlaps the softmax of tile j (the other S buffer)
-      mbar_wait(&p_ready[buf], (j >> 1) & 1);
-      mbar_wait(&v_full[st], (j / C::kStages) & 1);
-      tcgen05_fence_after();
-      if (elect_one()) {
-        const uint32_t v_addr = smem_u32(sKV + st * 2 * C::kTileBytes + C::kTileBytes);
-        const uint64_t vdesc = umma_desc_mnmajor_sw128(v_addr, kPfSlabBytes, 1024);
-        const uint32_t tmem_p = tmem_base + buf * kPfN;  // fp16 P over the first 64 columns of the S buffer
+          for (int u = 0; u < 2; ++u) {
+            if (j >= 0 && j < it.n_kt[u]) {
+              mbar_wait_soft(&p_ready[u], pph[u], ok);
+              pph[u] ^= 1;
+              tcgen05_fence_after();
+              if (elect_one()) {
+                const uint64_t b = vdesc + (uint64_t)((vst * C::kTileBytes) >> 4);
 #pragma unroll
-        for (int kk = 0; kk < kPfN / 16; ++kk)  // 16 keys = 2 swizzle atoms of 8 key rows = 2048 bytes per step
-          umma_f16_ts(tmem_o, tmem_p + kk * 8, vdesc + (uint64_t)((kk * 2048) >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
-        umma_commit(&kv_empty[st]);
-        umma_commit(o_done);
-      }
-      __syncwarp();
-    }
-  } else {
-    // ------------------------------------------------------------------ softmax warps: thread = query row = TMEM lane
-    const int quarter = warp & 3;
-    const int row = quarter * 32 + lane;
-    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
-    const int qpos = past + q0 + row;  // absolute position of this row's query (rows >= `rows` are padding: computed, not stored)
-    float m = kPfNegBig, l = 0.f;
-    for (int j = 0; j < n_kt; ++j) {
-      const int buf = j & 1;
-      const uint32_t tmem_s = tmem_base + lane_base + buf * kPfN;
-      mbar_wait(&s_full[buf], (j >> 1) & 1);
-      tcgen05_fence_after();
-      float s[kPfN];
-#pragma unroll
-      for (int c = 0; c < kPfN / 16; ++c) tmem_ld_32x32b_x16(tmem_s + c * 16, reinterpret_cast<uint32_t(&)[16]>(s[c * 16]));
-      tmem_ld_wait();
-      const int key0 = j * kPfN;
-      float mx = kPfNegBig;
-      if (key0 + kPfN - 1 > past + q0 + quarter * 32) {  // warp-uniform: some row of this warp has keys to mask in this tile
-#pragma unroll
-        for (int c = 0; c < kPfN; ++c) {
-          s[c] = (key0 + c <= qpos) ? s[c] * scale_log2 : -INFINITY;
-          mx = fmaxf(mx, s[c]);
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < kPfN; ++c) {
-          s[c] *= scale_log2;
-          mx = fmaxf(mx, s[c]);
-        }
-      }
-      const float m_new = fmaxf(m, mx);
-      const float alpha = fast_exp2(m - m_new);
-      m = m_new;
-      float sum = 0.f;
-      uint32_t p[kPfN / 2];
-#pragma unroll
-      for (int c = 0; c < kPfN; c += 2) {
-        const float p0 = fast_exp2(s[c] - m_new), p1 = fast_exp2(s[c + 1] - m_new);
-        sum += p0 + p1;
-        p[c / 2] = pack_half2(p0, p1);
-      }
-      l = l * alpha + sum;
-      if (j > 0) {
-        mbar_wait(o_done, (j - 1) & 1);  // P V of tile j-1 has completed: O is quiescent and the P buffer is free
-        tcgen05_fence_after();
-        if (__any_sync(0xffffffffu, alpha != 1.f)) {
-#pragma unroll
-          for (int c = 0; c < D / 16; ++c) {
-            uint32_t o[16];
-            tmem_ld_32x32b_x16(tmem_o + lane_base + c * 16, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_32x32b_x16(tmem_o + lane_base + c * 16, o);
+                for (int kk = 0; kk < kPfN / 16; ++kk)  // 16 keys = 2 swizzle atoms of 8 key rows = 2048 bytes per step
+                  umma_f16_ts(tmem_base + 256 + u * D, tmem_base + u * kPfN + kk * 8, b + (uint64_t)((kk * 2048) >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+                if (j == it.n_kt[u] - 1) umma_commit(&o_full[u]);
+              }
+              __syncwarp();
+            } else {
+              tcgen05_fence_after();
+            }
+            if (j + 1 < it.n_kt[u]) issue_qk(u);
+          }
+          if (j >= 0) {
+            release(&v_empty[vst]);
+            if (++vst == kPfStages) { vst = 0; vph ^= 1; }
+          }
+          if (more) {
+            release(&k_empty[kst]);
+            if (++kst == kPfStages) { kst = 0; kph ^= 1; }
+            if (j + 2 == it.n) release(q_empty);
           }
         }
       }
-#pragma unroll
-      for (int c = 0; c < kPfN / 32; ++c) tmem_st_32x32b_x16(tmem_s + c * 16, reinterpret_cast<const uint32_t(&)[16]>(p[c * 16]));
-      tmem_st_wait();
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&p_ready[buf]);
     }
-    mbar_wait(o_done, (n_kt - 1) & 1);
-    tcgen05_fence_after();
-    const float inv = l > 0.f ? 1.f / l : 0.f;
-    __half* op = out + (int64_t)(q_begin + q0 + row) * out_stride + head * D;
+  } else {
+    // ------------------------------------------------------------------ softmax warps: thread = query row = TMEM lane
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPfSoftmaxRegs));
+    const int u = (warp - 4) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
+    const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+    const uint32_t tmem_s = tmem_base + lane_base + u * kPfN, tmem_o = tmem_base + lane_base + 256 + u * D;
+    int sph = 0, oph = 0;
+    for (int i = blockIdx.x; i < n_items; i += gridDim.x) {
+      const PfItem it = pf_item(p, i);
+      const int n_kt = u ? it.n_kt[1] : it.n_kt[0], q0 = u ? it.q0[1] : it.q0[0];
+      if (n_kt == 0) continue;
+      const int first = it.past + q0 + quarter * 32;  // absolute position of the warp's first query
+      const int qpos = first + lane;                  // rows past the tile's last one are padding: computed, not stored
+      float m = 0.f;
+      float sum[2] = {0.f, 0.f};  // two partial sums of the row
+      for (int j = 0; j < n_kt; ++j) {
+        mbar_wait_soft(&s_full[u], sph, ok);
+        sph ^= 1;
+        tcgen05_fence_after();
+        float s[kPfN];
 #pragma unroll
-    for (int c = 0; c < D / 16; ++c) {
-      uint32_t o[16];
-      tmem_ld_32x32b_x16(tmem_o + lane_base + c * 16, o);
-      tmem_ld_wait();
-      if (row < rows) {
-        uint4 lo, hi;
-        lo.x = pack_half2(__uint_as_float(o[0]) * inv, __uint_as_float(o[1]) * inv);
-        lo.y = pack_half2(__uint_as_float(o[2]) * inv, __uint_as_float(o[3]) * inv);
-        lo.z = pack_half2(__uint_as_float(o[4]) * inv, __uint_as_float(o[5]) * inv);
-        lo.w = pack_half2(__uint_as_float(o[6]) * inv, __uint_as_float(o[7]) * inv);
-        hi.x = pack_half2(__uint_as_float(o[8]) * inv, __uint_as_float(o[9]) * inv);
-        hi.y = pack_half2(__uint_as_float(o[10]) * inv, __uint_as_float(o[11]) * inv);
-        hi.z = pack_half2(__uint_as_float(o[12]) * inv, __uint_as_float(o[13]) * inv);
-        hi.w = pack_half2(__uint_as_float(o[14]) * inv, __uint_as_float(o[15]) * inv);
-        *reinterpret_cast<uint4*>(op + c * 16) = lo;
-        *reinterpret_cast<uint4*>(op + c * 16 + 8) = hi;
+        for (int c = 0; c < kPfN / 32; ++c) tmem_ld_32x32b_x32(tmem_s + c * 32, reinterpret_cast<uint32_t(&)[32]>(s[c * 32]));
+        tmem_ld_wait();
+        const int key0 = j * kPfN;
+        float scale = p.scale_log2;
+        if (key0 + kPfN - 1 > first || scale <= 0.f) {  // warp-uniform: some row of this warp has keys to mask in this tile
+#pragma unroll
+          for (int c = 0; c < kPfN; ++c) s[c] = (key0 + c <= qpos) ? s[c] * scale : -INFINITY;
+          scale = 1.f;
+        }
+        float mx4[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+        for (int c = 4; c < kPfN; c += 4) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) mx4[k] = fmaxf(mx4[k], s[c + k]);
+        }
+        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale;
+        if (j == 0) {
+          m = mx;
+        } else {
+          const bool grew = mx > m + (j <= kPfExactTiles ? 0.f : kPfRescale);
+          if (__any_sync(0xffffffffu, grew)) {
+            const float alpha = grew ? fast_exp2(m - mx) : 1.f;
+            if (grew) m = mx;
+            sum[0] *= alpha;
+            sum[1] *= alpha;
+#pragma unroll
+            for (int c = 0; c < D / 64; ++c) {
+              uint32_t o[64];
+              tmem_ld_32x32b_x32(tmem_o + c * 64, reinterpret_cast<uint32_t(&)[32]>(o[0]));
+              tmem_ld_32x32b_x32(tmem_o + c * 64 + 32, reinterpret_cast<uint32_t(&)[32]>(o[32]));
+              tmem_ld_wait();
+#pragma unroll
+              for (int k = 0; k < 64; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * alpha);
+#pragma unroll
+              for (int k = 0; k < 4; ++k) tmem_st_32x32b_x16(tmem_o + c * 64 + k * 16, reinterpret_cast<const uint32_t(&)[16]>(o[k * 16]));
+            }
+          }
+        }
+        const uint64_t scale2 = f32x2(scale, scale), neg_m = f32x2(-m, -m);
+#pragma unroll
+        for (int h = 0; h < kPfN / 32; ++h) {
+          uint32_t pk[16];
+#pragma unroll
+          for (int c = 0; c < 32; c += 2) {
+            float a, b;
+            f32x2_split(fma_f32x2(f32x2(s[h * 32 + c], s[h * 32 + c + 1]), scale2, neg_m), a, b);
+            pk[c / 2] = pack_half2(fast_exp2(a), fast_exp2(b));
+            sum[0] = add_f32_f16(sum[0], (uint16_t)pk[c / 2]);
+            sum[1] = add_f32_f16(sum[1], (uint16_t)(pk[c / 2] >> 16));
+          }
+          tmem_st_32x32b_x16(tmem_s + h * 16, pk);
+        }
+        tmem_st_wait();
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_ready[u]);
       }
+      mbar_wait_soft(&o_full[u], oph, ok);
+      oph ^= 1;
+      tcgen05_fence_after();
+      const float l = sum[0] + sum[1], inv = l > 0.f ? 1.f / l : 0.f;
+      const int rows = u ? it.rows[1] : it.rows[0], head = u ? it.head[1] : it.head[0];
+      __half* op = p.out + (int64_t)(it.q_begin + q0 + row) * p.out_stride + head * D;
+#pragma unroll
+      for (int c = 0; c < D / 32; ++c) {
+        uint32_t o[32];
+        tmem_ld_32x32b_x32(tmem_o + c * 32, o);
+        tmem_ld_wait();
+        if (row < rows) {
+#pragma unroll
+          for (int k = 0; k < 32; k += 8) {
+            uint4 w;
+            w.x = pack_half2(__uint_as_float(o[k]) * inv, __uint_as_float(o[k + 1]) * inv);
+            w.y = pack_half2(__uint_as_float(o[k + 2]) * inv, __uint_as_float(o[k + 3]) * inv);
+            w.z = pack_half2(__uint_as_float(o[k + 4]) * inv, __uint_as_float(o[k + 5]) * inv);
+            w.w = pack_half2(__uint_as_float(o[k + 6]) * inv, __uint_as_float(o[k + 7]) * inv);
+            *reinterpret_cast<uint4*>(op + c * 32 + k) = w;
+          }
+        }
+      }
+      tcgen05_fence_before();  // the next item's first P V overwrites O: it is issued after this warp's next arrival at p_ready
     }
   }
 
+  if (!ok) {  // gave up: let copies and products in flight end before the block's memory goes
+    atomicAdd(&attn_prefill_gave_up, 1);
+    for (int i = 0; i < 64; ++i) __nanosleep(1000000);
+  }
   tcgen05_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc<C::kTmemCols>(tmem_base);
+  if (warp == 2) tmem_dealloc<C::kTmemCols>(tmem_base);
+}
+
+static int pf_num_sms() {
+  static int n = 0;
+  if (n == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+  }
+  return n;
 }
 
 }  // namespace b200
@@ -308,10 +425,26 @@ static int launch_prefill_paged(const void* q, int64_t q_stride, int64_t T_q, co
   const CUtensorMap* mk = get_tmap_2d(k_pool, pool_rows, D, D, kPageTokens, 64, TmapDtype::kF16, TmapSwizzle::kNone);
   const CUtensorMap* mv = get_tmap_2d(v_pool, pool_rows, D, D, kPageTokens, 64, TmapDtype::kF16, TmapSwizzle::kNone);
   if (!mq || !mk || !mv) return B200_ERR_CUDA;
+  PfParams p;
+  p.block_table = block_table;
+  p.bt_stride = bt_stride;
+  p.context_lens = context_lens;
+  p.cu_q = cu_q;
+  p.out = (__half*)out;
+  p.out_stride = out_stride;
+  p.n_heads = n_heads;
+  p.n_kv = n_kv;
+  p.B = B;
+  // two heads of a key / value head are equally long and share their keys; neighbouring query tiles are not, and a short prompt has no second one
+  p.pair_heads = (n_heads / n_kv) % 2 == 0;
+  p.n_units = p.pair_heads ? n_heads / 2 : n_heads;
   const int tiles = (max_q + kPfM - 1) / kPfM;
-  dim3 grid((unsigned)(B * tiles), (unsigned)n_heads);
-  B200_LAUNCH(attn_prefill_paged_kernel<D>, grid, dim3(kPfThreads), (size_t)C::kSmemBytes, st, *mq, *mk, *mv, block_table, bt_stride,
-              context_lens, cu_q, (__half*)out, out_stride, n_heads, n_kv, tiles, scale * 1.4426950408889634f);
+  p.n_groups = p.pair_heads ? tiles : (tiles + 1) / 2;
+  p.scale_log2 = scale * 1.4426950408889634f;
+  const int64_t items = (int64_t)p.n_units * p.n_groups * B;
+  if (items > (1 << 30)) { b200_set_last_error("attn_prefill_paged: too many query tiles"); return B200_ERR_ARG; }
+  const int grid = (int)(items < pf_num_sms() ? items : pf_num_sms());
+  B200_LAUNCH(attn_prefill_paged_kernel<D>, dim3(grid), dim3(kPfThreads), (size_t)C::kSmemBytes, st, *mq, *mk, *mv, p);
   b200_count_launches(1);
   return B200_OK;
 }

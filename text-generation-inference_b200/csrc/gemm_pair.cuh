@@ -96,17 +96,6 @@ __device__ __forceinline__ void cluster_sync() {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// Bounded: at the limit (a protocol fault, not a slow neighbour: seconds) `ok` falls, and this and every later wait of the thread returns at
-// once.  No loop ends early for it: the counters of the product loop stay warp-uniform, and with them the operands of tcgen05.mma in uniform
-// registers.
-__device__ __forceinline__ void mbar_wait_pair(uint64_t* bar, uint32_t parity, bool& ok) {
-  uint32_t spins = 0;
-  while (ok && !mbar_try_wait(bar, parity))
-    if (++spins > (1u << 24)) {
-      ok = false;
-      atomicAdd(&gemm_pair_gave_up, 1);
-    }
-}
 // tensor copy into this CTA's shared memory whose bytes count in a barrier of either CTA of the pair
 __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* m, int c0, int c1, uint32_t cluster_bar, uint64_t policy) {
   asm volatile(
@@ -128,17 +117,6 @@ __device__ __forceinline__ void umma_pair_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
                "h"((uint16_t)3)
                : "memory");
-}
-__device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,"
-      "%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
-        "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
-        "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]),
-        "=r"(v[31])
-      : "r"(taddr)
-      : "memory");
 }
 __device__ __forceinline__ void sts_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
@@ -235,7 +213,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         const int t0 = tt * p.tn, nn = min(p.tn, (p.T - t0 + 31) & ~31);
         const int row_x = t0 + (int)rank * (nn >> 1), row_w = m * kPairM + (int)rank * 128;
         for (int kb = 0; kb < p.n_stages; ++kb) {
-          mbar_wait_pair(&empty[s], ph, ok);
+          mbar_wait_soft(&empty[s], ph, ok);
           unsigned char* st = smem + s * p.stage_bytes;
           const uint32_t bar = cluster_map(smem_u32(&full[s]), 0);
           if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * p.per_stage * ((C::kInt4 ? 0 : kPairABytes) + p.tn * kPairK));
@@ -259,9 +237,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         pair_tile(p, i, m, tt);
         const int nn = min(p.tn, (p.T - tt * p.tn + 31) & ~31);
         const uint32_t idesc = umma_idesc_f16_f32acc(kPairM, nn) | fmt, d = tmem_d + (it & 1) * kPairMaxN;
-        mbar_wait_pair(&tmem_empty[it & 1], ((it >> 1) & 1) ^ 1, ok);
+        mbar_wait_soft(&tmem_empty[it & 1], ((it >> 1) & 1) ^ 1, ok);
         for (int kb = 0; kb < p.n_stages; ++kb) {
-          mbar_wait_pair(&full[s], ph, ok);
+          mbar_wait_soft(&full[s], ph, ok);
           tcgen05_fence_after();
           const uint64_t da = desc0 + (uint64_t)((s * p.stage_bytes) >> 4), db = da + (uint64_t)((p.per_stage * kPairABytes) >> 4);
           if (elect_one()) {
@@ -288,7 +266,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         int m, tt;
         pair_tile(p, i, m, tt);
         for (int kb = 0; kb < p.n_kb / 2; ++kb) {
-          mbar_wait_pair(&rec_empty[r], ph, ok);
+          mbar_wait_soft(&rec_empty[r], ph, ok);
           mbar_arrive_expect_tx(&rec_full[r], p.rec_bytes);
           unsigned char* dst = recs + r * kW4RecMaxBytes;
           const unsigned char* two = p.packed + ((size_t)m * p.rec_per_tile + kb) * 2 * p.rec_bytes;
@@ -320,7 +298,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     int r = team >> 1, rph = 0, s = team / p.per_stage, ph = 1;
     uint32_t wq[8], mrec[2];
     auto fetch = [&]() {
-      mbar_wait_pair(&rec_full[r], rph, ok);
+      mbar_wait_soft(&rec_full[r], rph, ok);
       lds_v4(words + r * kW4RecMaxBytes, &wq[0]);
       lds_v4(words + r * kW4RecMaxBytes + 2048, &wq[4]);
       // the 64 k of a half lie in one group row, or in two when a group is 32 wide
@@ -340,7 +318,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         dequant_consts(mrec[c >> 2], scale2, nz1024, nz64);
         dequant_word(wq[c], nz1024, nz64, scale2, &v[c * 4]);
       }
-      mbar_wait_pair(&empty[s], ph, ok);
+      mbar_wait_soft(&empty[s], ph, ok);
       const uint32_t dst = dst_row + s * p.stage_bytes;
 #pragma unroll
       for (int c = 0; c < 8; ++c) sts_v4(dst + ((uint32_t)(c << 4) ^ swz), v[c * 4], v[c * 4 + 1], v[c * 4 + 2], v[c * 4 + 3]);
@@ -370,7 +348,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       const int n_w = C::kAct ? n + (lane >> 4) * p.half_tiles * 128 : n;  // the weight row behind this lane
       const bool n_ok = C::kAct || n < p.N;
       const float bv = p.bias && n_ok ? pair_bias<KIND>(p.bias, n_w) : 0.f;
-      mbar_wait_pair(&tmem_full[it & 1], (it >> 1) & 1, ok);
+      mbar_wait_soft(&tmem_full[it & 1], (it >> 1) & 1, ok);
       tcgen05_fence_after();
       for (int c = 0; c < nn; c += 32) {
         uint32_t v[32];
@@ -419,8 +397,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
   }
 
-  if (!ok)
-    for (int i = 0; i < 64; ++i) __nanosleep(1000000);  // gave up: let copies and products in flight end before the pair's memory goes
+  if (!ok) {  // gave up: let copies and products in flight end before the pair's memory goes
+    atomicAdd(&gemm_pair_gave_up, 1);
+    for (int i = 0; i < 64; ++i) __nanosleep(1000000);
+  }
   tcgen05_fence_before();
   __syncthreads();
   cluster_sync();  // the leader's products read the other CTA's shared memory and write its TMEM until the epilogues are done
