@@ -7,9 +7,10 @@
 // CACHED context: query i of sequence b sits at absolute position context_lens[b] - n_q(b) + i and attends keys 0 .. that position.
 // That is what an add-on prefill over a prompt prefix, a chunked prefill and a mixed prefill + decode step need.
 //
-// Design (12 warps, one persistent CTA per SM).  An item is TWO query tiles of 128 rows that meet the same keys, so that the tensor cores work for
+// Design (12 warps, one CTA per SM).  A block takes its own item and then those of blocks that have not started (cluster launch control), longest
+// first: with items dealt out in turn the SMs were busy for 75 % of the time on ragged prompts.  An item is TWO query tiles of 128 rows that meet the same keys, so that the tensor cores work for
 // one while the other is in its soft-max: two query heads of a key / value head when their number is even, else two neighbouring query tiles
-// of a head.  Items are taken longest first.
+// of a head.
 //   warp 0      TMA producer.  Q tiles [128 x d] through a 128B-swizzled tensor map; per 128-key tile 8 KV pages x (K, V) x d/64
 //               slabs, each one cp.async.bulk.tensor box [16 tokens x 64 halves] of the pool: the pool stores every token row
 //               with its 16-byte chunks XOR-swizzled by (token & 7), which IS the tcgen05 SWIZZLE_128B image, so
@@ -25,8 +26,9 @@
 //               softmax warp runs.
 // Causality over absolute positions prunes whole key tiles.  Bound: soft-max exponentials (MUFU, 16 a cycle and SM: 1024 cycles per 128 x 128 tile,
 // as long as its products at d = 128, twice as long at d = 64), and between items the pipeline's drain.  Measured on B200 (us, before: one query
-// tile of one head per CTA): 13 prompts of 300 to 2048 tokens, 32 / 8 heads, d = 128 571 -> 306; 16 x 1024 428 -> 199; 8192 1196 -> 500 (1.10
-// PFLOP/s); d = 64, 32 / 4 heads 440 -> 251; 300 tokens after 1500 cached ones x 4 110 -> 72.  Tried: four more warps for the output (305 instead of
+// tile of one head per CTA): 13 prompts of 300 to 2048 tokens, 32 / 8 heads, d = 128 571 -> 234; 16 x 1024 428 -> 187; 8192 1196 -> 465 (1.18
+// PFLOP/s); d = 64, 32 / 4 heads 440 -> 186; 300 tokens after 1500 cached ones x 4 110 -> 67; 64 tokens x 10 18.1 -> 15.6.  Items dealt out in turn:
+// 294 at the first of these.  Tried: four more warps for the output (305 instead of
 // 287: the softmax warps are then compiled for 128 registers).
 #include "common.cuh"
 #include "tmap.cuh"
@@ -39,7 +41,9 @@ constexpr int kPfN = 128;        // keys per tile = 8 pages
 constexpr int kPfThreads = 384;  // warp 0 TMA, warp 1 MMA, warps 4..11 softmax
 constexpr int kPfSlabBytes = 128 * 128;  // 128 rows x 64 halves
 constexpr int kPfPageSlabBytes = kPageTokens * 128;
+constexpr int kPfCornerBytes = 32 * 128;  // a softmax warp's rows on their way out
 constexpr int kPfStages = 2;
+constexpr int kPfAhead = 2;      // items that are known ahead
 // The reference maximum of a row follows the true one through the first key tiles after the first; later it moves only when the maximum has grown
 // past it by more than 2^8.  A largest weight of exactly 1 is worth some precision (against float64, over prompts of 64 to 2500 keys: 0.993 of
 // the error of following it always with unrounded sums, 1.006 with no exact tiles), following it always costs 323 us where this takes 306.
@@ -54,8 +58,9 @@ template <int D>
 struct PfCfg {
   static constexpr int kSlabs = D / 64;
   static constexpr int kTileBytes = kSlabs * kPfSlabBytes;  // a Q, K or V tile
-  static constexpr int kNumBars = 2 + 4 * kPfStages + 6;    // q_full, q_empty | k_full, k_empty, v_full, v_empty | s_full[2], p_ready[2], o_full[2]
-  static constexpr int kSmemBytes = (2 + 2 * kPfStages) * kTileBytes + kNumBars * 8 + 16 + 1024;
+  static constexpr int kNumBars = 2 + 4 * kPfStages + 8 + 2 * kPfAhead + 1;    // q_full, q_empty | k_full, k_empty, v_full, v_empty | s_full[2], p_ready[2][2 halves], o_full[2]
+  static constexpr int kSmemBytes = (2 + 2 * kPfStages) * kTileBytes + 8 * kPfCornerBytes + kNumBars * 8 + 16 + 1024;
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
   static constexpr int kTmemCols = 512;  // S0 [0,128) | S1 [128,256) | O0 [256, 256 + D) | O1 behind it
 };
 
@@ -69,6 +74,7 @@ struct PfParams {
   int n_heads, n_kv, B;
   int pair_heads;        // 1: an item is two heads, 0: two query tiles
   int n_units, n_groups; // head (pair)s, query tile (pair)s of the longest sequence
+  int more_blocks;       // the grid is larger than the GPU: blocks take more items
   float scale_log2;
 };
 
@@ -99,6 +105,32 @@ __device__ __forceinline__ PfItem pf_item(const PfParams& p, int i) {
   return it;
 }
 
+// Asks for a block of the grid that has not started: its index in x, or -1 when there is none left (no further request may follow then).
+// One thread; `resp` 16 bytes of shared memory, `bar` an mbarrier of one arrival.
+__device__ __forceinline__ int take_block(uint32_t* resp, uint64_t* bar, uint32_t parity, bool& ok) {
+  mbar_arrive_expect_tx(bar, 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(resp)), "r"(smem_u32(bar)) : "memory");
+  mbar_wait_soft(bar, parity, ok);
+  if (!ok) return -1;
+  uint32_t taken, x;
+  asm volatile(
+      "{\n\t.reg .b128 h;\n\t.reg .pred p;\n\t"
+      "ld.shared.b128 h, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
+      : "=r"(taken), "=r"(x)
+      : "r"(smem_u32(resp))
+      : "memory");
+  fence_proxy_async_smem();  // the next request writes the answer's place through the async proxy
+  return taken ? (int)x : -1;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 __device__ __forceinline__ uint64_t f32x2(float a, float b) {
   uint64_t r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
@@ -138,7 +170,8 @@ attn_prefill_paged_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   unsigned char* sQ = smem;
   unsigned char* sK = sQ + 2 * C::kTileBytes;
   unsigned char* sV = sK + kPfStages * C::kTileBytes;
-  uint64_t* q_full = reinterpret_cast<uint64_t*>(sV + kPfStages * C::kTileBytes);
+  unsigned char* sOut = sV + kPfStages * C::kTileBytes;
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(sOut + 8 * kPfCornerBytes);
   uint64_t* q_empty = q_full + 1;
   uint64_t* k_full = q_empty + 1;
   uint64_t* k_empty = k_full + kPfStages;
@@ -146,12 +179,16 @@ attn_prefill_paged_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   uint64_t* v_empty = v_full + kPfStages;
   uint64_t* s_full = v_empty + kPfStages;
   uint64_t* p_ready = s_full + 2;
-  uint64_t* o_full = p_ready + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
+  uint64_t* o_full = p_ready + 4;
+  uint64_t* next_full = o_full + 2;
+  uint64_t* next_empty = next_full + kPfAhead;
+  uint64_t* taken = next_empty + kPfAhead;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(taken + 1);
+  __shared__ __align__(16) uint32_t s_resp[4];
+  __shared__ int s_next[kPfAhead];
 
   pdl_launch_dependents();
   const int warp = warp_id(), lane = lane_id();
-  const int n_items = p.B * p.n_units * p.n_groups;
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_q);
     tma_prefetch_desc(&tmap_k);
@@ -166,9 +203,15 @@ attn_prefill_paged_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
     }
     for (int u = 0; u < 2; ++u) {
       mbar_init(&s_full[u], 1);
-      mbar_init(&p_ready[u], 4);
+      mbar_init(&p_ready[2 * u], 4);
+      mbar_init(&p_ready[2 * u + 1], 4);
       mbar_init(&o_full[u], 1);
     }
+    for (int s = 0; s < kPfAhead; ++s) {
+      mbar_init(&next_full[s], 1);
+      mbar_init(&next_empty[s], 10);  // producer, issuer, eight softmax warps
+    }
+    mbar_init(taken, 1);
     mbar_fence_init();
   }
   if (warp == 2) tmem_alloc<C::kTmemCols>(tmem_slot);
@@ -177,6 +220,16 @@ attn_prefill_paged_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   bool ok = true;
+  // the next item of this CTA, or -1
+  int at = 0, at_ph = 0;
+  auto next_item = [&]() {
+    mbar_wait_soft(&next_full[at], at_ph, ok);
+    const int i = ok ? s_next[at] : -1;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&next_empty[at]);
+    if (++at == kPfAhead) { at = 0; at_ph ^= 1; }
+    return __reduce_max_sync(0xffffffffu, i);  // a warp reduction: the compiler knows its result, and the loops' control, to be uniform
+  };
   pdl_wait();  // q, the index tensors and the pool's newest tokens are the previous kernels' output
 
   if (warp < 4) {
@@ -184,9 +237,9 @@ attn_prefill_paged_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
     if (warp == 0) {
       // ------------------------------------------------------------------ TMA producer
       int st = 0, ph = 1, qph = 1;
-      for (int i = blockIdx.x; i < n_items; i += gridDim.x) {
+      for (int i = blockIdx.x; i >= 0; i = next_item()) {
         const PfItem it = pf_item(p, i);
-        if (it.n == 0) continue;
+        if (it.n == 0) continue;  // only the block's own item can be empty
         mbar_wait_soft(q_empty, qph, ok);  // the previous item's last Q K^T
         qph ^= 1;
         if (lane == 0) {
@@ -241,8 +294,11 @@ attn_prefill_paged_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
         if (elect_one()) umma_commit(bar);
         __syncwarp();
       };
-      for (int i = blockIdx.x; i < n_items; i += gridDim.x) {
-        const PfItem it = pf_item(p, i);
+      for (int i = blockIdx.x; i >= 0; i = next_item()) {
+        PfItem it = pf_item(p, i);
+        it.n_kt[0] = __reduce_max_sync(0xffffffffu, it.n_kt[0]);
+        it.n_kt[1] = __reduce_max_sync(0xffffffffu, it.n_kt[1]);
+        it.n = max(it.n_kt[0], it.n_kt[1]);
         if (it.n == 0) continue;
         mbar_wait_soft(q_full, qph, ok);
         qph ^= 1;
@@ -253,17 +309,20 @@ attn_prefill_paged_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
             if (j >= 0 && j < it.n_kt[u]) {
-              mbar_wait_soft(&p_ready[u], pph[u], ok);
-              pph[u] ^= 1;
-              tcgen05_fence_after();
-              if (elect_one()) {
-                const uint64_t b = vdesc + (uint64_t)((vst * C::kTileBytes) >> 4);
+              const uint64_t b = vdesc + (uint64_t)((vst * C::kTileBytes) >> 4);
 #pragma unroll
-                for (int kk = 0; kk < kPfN / 16; ++kk)  // 16 keys = 2 swizzle atoms of 8 key rows = 2048 bytes per step
-                  umma_f16_ts(tmem_base + 256 + u * D, tmem_base + u * kPfN + kk * 8, b + (uint64_t)((kk * 2048) >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
-                if (j == it.n_kt[u] - 1) umma_commit(&o_full[u]);
+              for (int h = 0; h < 2; ++h) {
+                mbar_wait_soft(&p_ready[2 * u + h], pph[u], ok);
+                tcgen05_fence_after();
+                if (elect_one()) {
+#pragma unroll
+                  for (int kk = h * 4; kk < h * 4 + 4; ++kk)  // 16 keys = 2 swizzle atoms of 8 key rows = 2048 bytes per step
+                    umma_f16_ts(tmem_base + 256 + u * D, tmem_base + u * kPfN + kk * 8, b + (uint64_t)((kk * 2048) >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u);
+                  if (h == 1 && j == it.n_kt[u] - 1) umma_commit(&o_full[u]);
+                }
+                __syncwarp();
               }
-              __syncwarp();
+              pph[u] ^= 1;
             } else {
               tcgen05_fence_after();
             }
@@ -280,6 +339,24 @@ attn_prefill_paged_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
           }
         }
       }
+    } else if (warp == 3) {
+      // ------------------------------------------------------------------ scheduler: after the block's own item those of blocks that have not
+      // started, as long as there are any; items without a tile are passed over here
+      if (lane == 0) {
+        int slot = 0, ph = 1, tph = 0;
+        for (int i; p.more_blocks && (i = take_block(s_resp, taken, tph, ok)) >= 0;) {
+          tph ^= 1;
+          if (pf_item(p, i).n == 0) continue;
+          mbar_wait_soft(&next_empty[slot], ph, ok);
+          s_next[slot] = i;
+          mbar_arrive(&next_full[slot]);
+          if (++slot == kPfAhead) { slot = 0; ph ^= 1; }
+        }
+        mbar_wait_soft(&next_empty[slot], ph, ok);
+        s_next[slot] = -1;
+        mbar_arrive(&next_full[slot]);
+      }
+      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------------ softmax warps: thread = query row = TMEM lane
@@ -288,7 +365,7 @@ attn_prefill_paged_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const uint32_t tmem_s = tmem_base + lane_base + u * kPfN, tmem_o = tmem_base + lane_base + 256 + u * D;
     int sph = 0, oph = 0;
-    for (int i = blockIdx.x; i < n_items; i += gridDim.x) {
+    for (int i = blockIdx.x; i >= 0; i = next_item()) {
       const PfItem it = pf_item(p, i);
       const int n_kt = u ? it.n_kt[1] : it.n_kt[0], q0 = u ? it.q0[1] : it.q0[0];
       if (n_kt == 0) continue;
@@ -313,11 +390,13 @@ attn_prefill_paged_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
         }
         float mx4[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll
-        for (int c = 4; c < kPfN; c += 4) {
+        for (int c = 4; c + 8 <= kPfN; c += 8) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) mx4[k] = fmaxf(mx4[k], s[c + k]);
+          for (int k = 0; k < 4; ++k) mx4[k] = max3(mx4[k], s[c + k], s[c + 4 + k]);
         }
-        const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) mx4[k] = fmaxf(mx4[k], s[kPfN - 4 + k]);
+        const float mx = fmaxf(max3(mx4[0], mx4[1], mx4[2]), mx4[3]) * scale;
         if (j == 0) {
           m = mx;
         } else {
@@ -353,34 +432,46 @@ attn_prefill_paged_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
             sum[1] = add_f32_f16(sum[1], (uint16_t)(pk[c / 2] >> 16));
           }
           tmem_st_32x32b_x16(tmem_s + h * 16, pk);
+          if (h & 1) {  // half of P: its products run under the exponentials of the other half
+            tmem_st_wait();
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&p_ready[2 * u + (h >> 1)]);
+          }
         }
-        tmem_st_wait();
-        tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&p_ready[u]);
       }
       mbar_wait_soft(&o_full[u], oph, ok);
       oph ^= 1;
       tcgen05_fence_after();
       const float l = sum[0] + sum[1], inv = l > 0.f ? 1.f / l : 0.f;
       const int rows = u ? it.rows[1] : it.rows[0], head = u ? it.head[1] : it.head[0];
-      __half* op = p.out + (int64_t)(it.q_begin + q0 + row) * p.out_stride + head * D;
+      // 64 columns at a time through the warp's corner of shared memory, so that a store covers whole lines (16-byte pieces of 32 rows at once cost
+      // thirty-two passes of the store unit)
+      unsigned char* corner = sOut + (warp - 4) * kPfCornerBytes;
+      __half* op = p.out + (int64_t)(it.q_begin + q0 + quarter * 32) * p.out_stride + head * D;
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t o[32];
-        tmem_ld_32x32b_x32(tmem_o + c * 32, o);
+      for (int c = 0; c < D; c += 64) {
+        uint32_t o[64];
+        tmem_ld_32x32b_x32(tmem_o + c, reinterpret_cast<uint32_t(&)[32]>(o[0]));
+        tmem_ld_32x32b_x32(tmem_o + c + 32, reinterpret_cast<uint32_t(&)[32]>(o[32]));
         tmem_ld_wait();
-        if (row < rows) {
 #pragma unroll
-          for (int k = 0; k < 32; k += 8) {
-            uint4 w;
-            w.x = pack_half2(__uint_as_float(o[k]) * inv, __uint_as_float(o[k + 1]) * inv);
-            w.y = pack_half2(__uint_as_float(o[k + 2]) * inv, __uint_as_float(o[k + 3]) * inv);
-            w.z = pack_half2(__uint_as_float(o[k + 4]) * inv, __uint_as_float(o[k + 5]) * inv);
-            w.w = pack_half2(__uint_as_float(o[k + 6]) * inv, __uint_as_float(o[k + 7]) * inv);
-            *reinterpret_cast<uint4*>(op + c * 32 + k) = w;
-          }
+        for (int k = 0; k < 8; ++k) {
+          uint4 w;
+          w.x = pack_half2(__uint_as_float(o[8 * k]) * inv, __uint_as_float(o[8 * k + 1]) * inv);
+          w.y = pack_half2(__uint_as_float(o[8 * k + 2]) * inv, __uint_as_float(o[8 * k + 3]) * inv);
+          w.z = pack_half2(__uint_as_float(o[8 * k + 4]) * inv, __uint_as_float(o[8 * k + 5]) * inv);
+          w.w = pack_half2(__uint_as_float(o[8 * k + 6]) * inv, __uint_as_float(o[8 * k + 7]) * inv);
+          *reinterpret_cast<uint4*>(corner + lane * 128 + ((k ^ (lane & 7)) << 4)) = w;
         }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int r = k * 4 + (lane >> 3), ch = lane & 7;
+          if (quarter * 32 + r < rows)
+            *reinterpret_cast<uint4*>(op + (int64_t)r * p.out_stride + c + ch * 8) = *reinterpret_cast<const uint4*>(corner + r * 128 + ((ch ^ (r & 7)) << 4));
+        }
+        __syncwarp();
       }
       tcgen05_fence_before();  // the next item's first P V overwrites O: it is issued after this warp's next arrival at p_ready
     }
@@ -443,8 +534,8 @@ static int launch_prefill_paged(const void* q, int64_t q_stride, int64_t T_q, co
   p.scale_log2 = scale * 1.4426950408889634f;
   const int64_t items = (int64_t)p.n_units * p.n_groups * B;
   if (items > (1 << 30)) { b200_set_last_error("attn_prefill_paged: too many query tiles"); return B200_ERR_ARG; }
-  const int grid = (int)(items < pf_num_sms() ? items : pf_num_sms());
-  B200_LAUNCH(attn_prefill_paged_kernel<D>, dim3(grid), dim3(kPfThreads), (size_t)C::kSmemBytes, st, *mq, *mk, *mv, p);
+  p.more_blocks = items > pf_num_sms();
+  B200_LAUNCH(attn_prefill_paged_kernel<D>, dim3((unsigned)items), dim3(kPfThreads), (size_t)C::kSmemBytes, st, *mq, *mk, *mv, p);
   b200_count_launches(1);
   return B200_OK;
 }
