@@ -1,0 +1,92 @@
+"""Prompts over token-major bfloat16 pages (csrc/attn_prompt.cuh behind ops_seq.talk_attn): tiles of 128 (token, head) rows for every head ratio, chunk
+borders inside a tile, windows whose first key tile some rows do not see, sinks, portions behind cached tokens, single tokens among prompts, more
+items than SMs, and the forms beside it that stay with the general kernels.  Reference: float64.
+
+Tolerance: queries are given as bfloat16 values, so products are exact; a weight is rounded to bfloat16 once (2^-9 of it) and the sum adds the
+rounded weights: 2 * 2^-9 of the weighted mean of |v|, and d 2^-24 of the largest score times the weight's slope for the fp32 sums."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _run(new, past, H, G, d, chunk=0, window=0, sink=None, page=16, dv=None, pad=0, seed=0, key_scale=1.0):
+    import tgis_b200  # noqa: F401
+    from tgis_b200 import ops_seq
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    dv = dv or d
+    starts = past if isinstance(past, list) else [past] * len(new)
+    L = [s + n for s, n in zip(starts, new)]
+    pages = [(n + page - 1) // page for n in L]
+    perm = torch.randperm(sum(pages) + 2, generator=g, device=DEV).int()
+    table, at = torch.zeros(len(new), max(pages), dtype=torch.int32, device=DEV), 0
+    for b, n in enumerate(pages):
+        table[b, :n] = perm[at:at + n]
+        at += n
+    k_off, v_off = pad, pad + G * d + pad
+    width = v_off + G * dv + pad
+    cache = (torch.randn(sum(pages) + 2, page, width, generator=g, device=DEV) * key_scale).bfloat16()
+    T = sum(new)
+    q = torch.randn(T, H, d, generator=g, device=DEV).bfloat16().float()
+    pos = torch.cat([torch.arange(s, s + n, device=DEV) for s, n in zip(starts, new)])
+    cu = torch.tensor([0] + new, device=DEV).cumsum(0).int()
+    seq = torch.repeat_interleave(torch.arange(len(new), device=DEV, dtype=torch.int32), torch.tensor(new, device=DEV))
+    step = ops_seq.RaggedStep(T=T, B=len(new), position_ids=pos, cu_q=cu, seq_of_token=seq, slot_mapping=pos, block_table=table, state_slots=None)
+    out = ops_seq.talk_attn(q, cache, step, kv_heads=G, vdim=dv, k_off=k_off, v_off=v_off, scale=d ** -0.5, chunk=chunk, window=window, sink=sink)
+    row = 0
+    for b, (n, s0, Lb) in enumerate(zip(new, starts, L)):
+        rows = cache[table[b, :pages[b]].long()].flatten(0, 1)[:Lb].double()
+        K, V = rows[:, k_off:k_off + G * d].unflatten(1, (G, d)), rows[:, v_off:v_off + G * dv].unflatten(1, (G, dv))
+        p, j = s0 + torch.arange(n, device=DEV)[:, None], torch.arange(Lb, device=DEV)[None]
+        ok = j <= p
+        if chunk:
+            ok = ok & (j // chunk == p // chunk)
+        if window:
+            ok = ok & (j > p - window)
+        for h in range(H):
+            s = (q[row:row + n, h].double() @ K[:, h * G // H].T * d ** -0.5).masked_fill(~ok, -math.inf)
+            top = s.masked_fill(~ok, 0).abs().amax(1, keepdim=True)
+            if sink is not None:
+                s = torch.cat([s, sink[h].double().expand(n, 1)], 1)
+            w = torch.softmax(s, 1)[:, :Lb]
+            ref, spread = w @ V[:, h * G // H], w @ V[:, h * G // H].abs()
+            tol = (2 * 2.0 ** -9 + 2 * d * 2.0 ** -24 * (1 + top)) * spread + 1e-6
+            err = (out[row:row + n, h].double() - ref).abs()
+            assert bool((err <= tol).all()), (b, h, float((err / tol).max()), int((err > tol).sum()))
+        row += n
+
+
+@pytest.mark.parametrize("H,G,d", [(4, 4, 64), (4, 2, 128), (16, 4, 128), (8, 1, 64), (16, 1, 128), (6, 2, 64)])   # (6, 2): three heads a key head, the general kernel
+def test_head_ratios(H, G, d):
+    _run([1, 31, 32, 33, 64, 65, 129, 200], 0, H, G, d)
+    _run([100, 3, 77], [5, 400, 128], H, G, d, seed=1)
+
+
+@pytest.mark.parametrize("chunk,window", [(64, 0), (100, 0), (0, 1), (0, 40), (0, 130), (200, 50), (2048, 0)])
+def test_masks(chunk, window):
+    _run([300, 90], [0, 170], 8, 2, 64, chunk=chunk, window=window, seed=2)
+    _run([150], 2000, 4, 1, 128, chunk=chunk, window=window, seed=3)
+
+
+def test_sinks():
+    g = torch.Generator(device=DEV).manual_seed(4)
+    sink = torch.randn(8, generator=g, device=DEV) * 3
+    sink[0], sink[1], sink[2] = 40.0, -40.0, -math.inf
+    _run([70, 200], [0, 300], 8, 2, 128, sink=sink, seed=5)
+    _run([140], 0, 8, 2, 64, window=30, sink=sink, seed=6)
+
+
+def test_more_items_than_sms():
+    _run([25 + 13 * (i % 7) for i in range(60)], [17 * (i % 5) for i in range(60)], 16, 8, 64, chunk=128, seed=7)
+
+
+def test_maxima_that_leap():
+    _run([700], 0, 4, 2, 128, key_scale=6.0, seed=8)
+
+
+@pytest.mark.parametrize("kw", [dict(page=32), dict(dv=128), dict(pad=4), dict(pad=8)])   # other pages, value sizes, offsets (the last one stays with the tcgen05 kernel)
+def test_forms_beside_it(kw):
+    _run([60, 130], [0, 20], 4, 2, 64, seed=9, **kw)

@@ -18,7 +18,10 @@
 //                           warp each).  Prompts, portions and decoded tokens are one case: keys come back from the cache.
 //   group_attn_kernel     : plain form without a mix: one block per (query token, key / value head group, 8 heads of the group).
 //   talk_attn_mma_kernel  : bfloat16 caches, m16n8k16 tensor-core products; see the note above the kernel.
+//   attn_prompt_kernel    : prompts over bfloat16 caches without a mix, tcgen05 products (attn_prompt.cuh).
+#include "attn_prompt.cuh"
 #include "seq_common.cuh"
+#include "tmap.cuh"
 
 #include <cstdlib>
 
@@ -718,6 +721,61 @@ extern "C" int b200_seq_talk_attn_splits(int dt, int64_t T, int B, int H, int G,
   return (int)n;
 }
 
+// Prompts without a mix take the tcgen05 kernel: tiles of 128 (token, head) rows, so it wants steps of enough tokens per sequence to fill them.
+// Measured on B200 (us, the m16n8k16 kernel / this one; 16 / 4 heads, d = 128): 2118 + 1882 tokens in chunks of 2048 387 / 86, 4 x 512 84 / 26, 300 after
+// 800 cached 51 / 34, 4 x 40 after 500 38 / 27, 4 x 24 after 1900 56 / 41, 24 after 20 24.5 / 14.3; 4 x 16 after 1900 55 / 51, 4 x 8 48.5 / 50.
+// What it needs beside that: heads of 64 or 128 columns, whole 128-row tiles (128 % (heads / kv_heads) == 0), pages of 16 tokens, and 16-byte pieces.
+constexpr int kTalkPromptTokens = 24;  // average tokens per sequence from which on
+
+static bool talk_prompt_route(const void* q, const void* cache, int dt, int64_t RW, int k_off, int v_off, const int32_t* cu_q, const float* talk,
+                              const void* out, int64_t T, int B, int H, int G, int d, int dv, int page) {
+  const int rep = H / G;
+  return dt == B200_DT_BF16 && talk == nullptr && cu_q != nullptr && B > 0 && T >= (int64_t)kTalkPromptTokens * B && (d == 64 || d == 128) && dv == d &&
+         page == b200::kPageTokens && rep <= 128 && 128 % rep == 0 && RW % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0 && T <= (1 << 24) &&
+         ((reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+}
+
+template <int D>
+static int launch_talk_prompt(const float* q, const void* cache, int64_t RW, int k_off, int v_off, const int32_t* block_table, int64_t bt_stride,
+                              const int32_t* cu_q, int B, const int64_t* position_ids, float* out, int64_t T, int H, int G, int chunk, int window,
+                              float scale, const float* sink, cudaStream_t st) {
+  using C = b200::PfCfg<D>;
+  static bool cfg = false;
+  if (!cfg) {
+    cudaError_t e = cudaFuncSetAttribute(b200::attn_prompt_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    if (e != cudaSuccess) { b200_set_last_error(cudaGetErrorString(e)); return B200_ERR_CUDA; }
+    cfg = true;
+  }
+  // rows of the cache viewed as [blocks * 16, row width]: the block table is trusted, as everywhere, so the map has no bound of its own
+  const CUtensorMap* m = b200::get_tmap_2d(cache, (uint64_t)1 << 30, (uint64_t)RW, (uint64_t)RW, b200::kPageTokens, 64, b200::TmapDtype::kF16, b200::TmapSwizzle::k128B);
+  if (!m) return B200_ERR_CUDA;
+  b200::PfParams p = {};
+  p.block_table = block_table;
+  p.bt_stride = bt_stride;
+  p.cu_q = cu_q;
+  p.out = out;
+  p.n_heads = H;
+  p.n_kv = G;
+  p.B = B;
+  p.q = q;
+  p.position_ids = position_ids;
+  p.sink = sink;
+  p.k_off = k_off;
+  p.v_off = v_off;
+  p.chunk = chunk;
+  p.window = window;
+  p.rep = H / G;
+  p.tokens = 128 / p.rep;
+  p.n_units = G;
+  p.n_groups = (int)(T / (2 * p.tokens)) + B;  // upper bound of sum_b ceil(n_b / (2 tokens)); surplus items are passed over
+  p.scale_log2 = scale * 1.4426950408889634f;
+  const int64_t items = (int64_t)p.n_units * p.n_groups;
+  p.more_blocks = items > b200::pf_num_sms();
+  B200_LAUNCH((b200::attn_prompt_kernel<D, true>), dim3((unsigned)items), dim3(b200::kPfThreads), (size_t)C::kSmemBytes, st, *m, *m, *m, p);
+  b200_count_launches(1);
+  return B200_OK;
+}
+
 // q fp32 [T, H, d]; cache rows as above; talk fp32 [H, H] or NULL (no mix); chunk / window <= 0: none -> out fp32 [T, H, dv].
 // sink fp32 [H] or NULL: a logit per head that joins the soft-max denominator (after the mix, unscaled) and carries no value.
 // `partial` / nsplit: from b200_seq_talk_attn_splits (NULL / <= 1: no split).
@@ -731,6 +789,11 @@ extern "C" int b200_seq_talk_attn(const float* q, const void* cache, int dt, int
     return B200_ERR_ARG;
   }
   cudaStream_t st = (cudaStream_t)stream;
+  if (talk_prompt_route(q, cache, dt, row_width, k_off, v_off, cu_q, talk, out, T, B, H, G, d, dv, page)) {
+    if (d == 128)
+      return launch_talk_prompt<128>(q, cache, row_width, k_off, v_off, block_table, bt_stride, cu_q, B, position_ids, out, T, H, G, chunk, window, scale, sink, st);
+    return launch_talk_prompt<64>(q, cache, row_width, k_off, v_off, block_table, bt_stride, cu_q, B, position_ids, out, T, H, G, chunk, window, scale, sink, st);
+  }
   const TalkPlan plan = talk_mma_plan(dt, T, B, H, G, d, dv, talk != nullptr);
   if (plan.QT > 0 && cu_q != nullptr && row_width % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0 && (reinterpret_cast<uintptr_t>(cache) & 15) == 0) {
     const int64_t tiles = (T + plan.QT - 1) / plan.QT + B;  // upper bound of sum_b ceil(n_b / QT); surplus blocks return at once
