@@ -4,6 +4,7 @@ Every function requires CUDA tensors and raises if the library is missing — no
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional, Tuple
 
 import torch
@@ -18,7 +19,8 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """the current stream of the current device, without a Stream object around it"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _req(t: torch.Tensor, dtype, name: str):
@@ -199,9 +201,14 @@ def attn_prefill_paged(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tens
 _gemm_ws = {}
 
 
+@functools.lru_cache(maxsize=1024)
+def _gemm_workspace_bytes(N: int, K: int) -> int:
+    return _lib.load().b200_gemm_workspace_bytes_max(N, K)
+
+
 def gemm_workspace(device, T: int, N: int, K: int) -> torch.Tensor:
     """Per-device split-K workspace (counters zeroed once; the kernels re-arm them)."""
-    need = _lib.load().b200_gemm_workspace_bytes_max(N, K)
+    need = _gemm_workspace_bytes(N, K)
     ws = _gemm_ws.get(device)
     if ws is None or ws.numel() < need:
         ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=device)

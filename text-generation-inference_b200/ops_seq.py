@@ -9,6 +9,7 @@ soft-max, recurrences, states and the residual stream are fp32 in both.  CUDA te
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from dataclasses import dataclass
 from typing import Optional
@@ -32,7 +33,8 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """the current stream of the current device, without a Stream object around it"""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _cuda(*ts):
@@ -63,10 +65,15 @@ _on_side = False
 SIDE_STREAM = os.getenv("B200_SEQ_SIDE_STREAM", "1") != "0"
 
 
+@functools.lru_cache(maxsize=1024)
+def _gemm_workspace_bytes(N: int, K: int) -> int:
+    return _lib.load_seq().b200_gemm_workspace_bytes_max(N, K)
+
+
 def _gemm_workspace(device, N: int, K: int, side: Optional[bool] = None) -> torch.Tensor:
     """split-K workspace of the tensor-core product, one per device and stream that products run on side by side (tile counters zeroed
     once; the kernel re-arms them)"""
-    need = _lib.load_seq().b200_gemm_workspace_bytes_max(N, K)
+    need = _gemm_workspace_bytes(N, K)
     key = (device, _on_side if side is None else side)
     ws = _gemm_ws.get(key)
     if ws is None or ws.numel() < need:

@@ -63,12 +63,11 @@ class Ex4bitLinearV2(nn.Module):
     def forward(self, x, force_cuda=False):
         if self.q_handle is None:
             self.post_init()
-        out_shape = x.shape[:-1] + (self.outfeatures,)
-        x2 = x.reshape(-1, x.shape[-1]).contiguous()
+        x2 = x.contiguous() if x.dim() == 2 else x.reshape(-1, x.shape[-1]).contiguous()
         if self.q_perm is not None:
             x2 = _ops().permute_columns(x2, self.q_perm)
         out = _ops().gemm_w4a16(x2, self.q_handle, self.outfeatures, self.group_size, self.bias, layout=self.pack_layout)
-        return out.view(out_shape)
+        return out if x.dim() == 2 else out.view(x.shape[:-1] + (self.outfeatures,))
 
     def temp_dq_size(self):
         return 0
