@@ -42,6 +42,9 @@ constexpr int kTileK = 64;   // fp16 elements per k-block = one 128-byte swizzle
 // Calls of more tokens go to the SM pairs (gemm_pair.cuh).  Measured on B200 (us, this kernel / pairs) at 64 tokens: 4096 x 4096 14.8 / 12.9,
 // 4096 -> 22016 37.1 / 40.0, 11008 -> 4096 23.6 / 28.8; at 96: 18.2 / 13.1, 42.9 / 41.3; at 128: 20.5 / 13.4, 45.8 / 42.3, 30.0 / 29.9.
 constexpr int kF16DecodeT = 64;
+// fp32 results show how long a sum ran in the tensor cores: cut into stream-K pieces that are added in fp32 it is off by 5e-7 (against float64,
+// k = 2048), in one piece by 2e-6.  So they stay here for as long as this kernel cuts them (one token tile).
+constexpr int kF32OutDecodeT = 256;
 constexpr int64_t kCounterBytes = 64 * 1024;
 
 template <int TN>
@@ -415,7 +418,7 @@ static int gemm_f16_impl(const void* x, const void* w, const void* bias, void* y
     b200_set_last_error("gemm_f16_deferred: needs a workspace, T <= 256 (one token tile) and N % 8 == 0");
     return B200_ERR_UNSUPPORTED;
   }
-  if (!defer && T > kF16DecodeT) {
+  if (!defer && T > (FMT == 2 ? kF32OutDecodeT : kF16DecodeT)) {
     PairParams pp = {};
     pp.y = y;
     pp.bias = bias;
