@@ -131,6 +131,108 @@ __global__ void __launch_bounds__(kPrepThreads, TAPS <= 4 ? 4 : 2) delta_prepare
   }
 }
 
+// Prompts and portions, key sizes of 64 or 128, at most four taps, 16-byte rows: a warp has four channels per lane of 128 neighbouring ones and walks
+// kRunTok tokens of a sequence, so that an input is read once instead of once per tap, weights once instead of once per token, and all
+// accesses are 16 bytes wide.  Per channel the arithmetic is that of delta_prepare_kernel, in its order; only the sum of a unit vector's squares is
+// added in another order.  Bound: memory (u, decays in; rows out).
+// Measured on B200 (us, a block per token / runs; 16 heads of 128): 1898 tokens 70 / 33, 690 28 / 18.7, 250 12.9 / 15.9, 21 6.1 / 9.5 (few runs: latency);
+// 32 heads: 3600 tokens 246 / 108, 400 31.4 / 19.9.
+constexpr int kRunTok = 16, kRunMinTokens = 384;
+
+template <typename TP>
+__global__ void __launch_bounds__(256) delta_prepare_run_kernel(
+    const float* __restrict__ u, int64_t ld, int col0, int taps, const TP* __restrict__ w, const float* __restrict__ conv_state,
+    const int32_t* __restrict__ state_slots, const int32_t* __restrict__ cu_q, int B, const int64_t* __restrict__ position_ids,
+    const float* __restrict__ raw, int64_t ldr, int col_b, const float* __restrict__ dec, int64_t ldd, int col_a, int channels,
+    const TP* __restrict__ A_log, const TP* __restrict__ dt_bias, float q_scale, float* __restrict__ out, int H, int G, int dk, int dv) {
+  pdl_launch_dependents();
+  pdl_wait();
+  int b, tile = blockIdx.x;
+  find_ragged_tile(cu_q, B, 1, kRunTok, b, tile);
+  if (b >= B) return;
+  const int lane = lane_id(), row0 = cu_q[b], t0 = row0 + tile * kRunTok, n_tok = min(kRunTok, cu_q[b + 1] - t0);
+  const int64_t s = position_ids[row0], p0 = s + tile * kRunTok;
+  const int C = 2 * G * dk + H * dv;
+  const float* st = conv_state + (int64_t)state_slots[b] * (taps > 1 ? taps - 1 : 1) * C;
+  const DeltaRow lay = delta_row(H, G, dk, dv, channels != 0);
+  const int spans = (C + 127) / 128, n_dec = channels ? H * dk : 0, g_spans = (n_dec + 127) / 128;
+  const int task = blockIdx.y * 8 + warp_id(), c = (task < spans ? task : task - spans) * 128 + lane * 4;
+  float* row = out + (int64_t)t0 * lay.width;
+  if (task < spans) {
+    const bool live = c < C;
+    float wt[4][4], x[4][4];   // weights and the last inputs, tap by tap (taps < 4: the first ones are zero)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int jj = j - (4 - taps);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) wt[j][k] = live && jj >= 0 ? ldf(w + jj * C + c + k) : 0.f;
+      const int64_t pp = p0 - 3 + j;   // inputs ahead of the run's first token
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (j < 3 && live && jj >= 0 && pp >= 0) v = pp >= s ? *reinterpret_cast<const float4*>(u + (row0 + (pp - s)) * ld + col0 + c)
+                                                           : *reinterpret_cast<const float4*>(st + (pp - s + taps - 1) * C + c);
+      x[j][0] = v.x; x[j][1] = v.y; x[j][2] = v.z; x[j][3] = v.w;
+    }
+    const bool unit = c < 2 * G * dk;                        // (a span never holds both kinds: 2 G dk is a multiple of 128 or the spans' lanes differ)
+    const float unit_scale = c < G * dk ? q_scale : 1.f;
+    const float* src = u + (int64_t)t0 * ld + col0 + c;
+    for (int t = 0; t < n_tok; t += 4) {
+      float4 in[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) in[i] = live && t + i < n_tok ? *reinterpret_cast<const float4*>(src + (int64_t)(t + i) * ld) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        x[3][0] = in[i].x; x[3][1] = in[i].y; x[3][2] = in[i].z; x[3][3] = in[i].w;
+        float y[4], sq = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          float acc = 0.f;
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (j >= 4 - taps) acc = fmaf(wt[j][k], x[j][k], acc);
+          y[k] = silu_f(acc);
+          sq = fmaf(y[k], y[k], sq);
+#pragma unroll
+          for (int j = 0; j < 3; ++j) x[j][k] = x[j + 1][k];
+        }
+        if (__any_sync(0xffffffffu, unit)) {   // a head's dk channels are dk / 4 neighbouring lanes
+#pragma unroll
+          for (int o = 1; o < 16; o <<= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+          if (dk == 128) sq += __shfl_xor_sync(0xffffffffu, sq, 16);
+          const float r = unit ? unit_scale / sqrtf(sq + 1e-6f) : 1.f;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) y[k] *= r;
+        }
+        if (live && t + i < n_tok) *reinterpret_cast<float4*>(row + (int64_t)(t + i) * lay.width + c) = make_float4(y[0], y[1], y[2], y[3]);
+      }
+    }
+  } else if (task < spans + g_spans) {
+    if (c >= n_dec) return;
+    float bias[4], a[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      bias[k] = ldf(dt_bias + c + k);
+      a[k] = -expf(ldf(A_log + c / dk));
+    }
+    for (int t = 0; t < n_tok; t += 4) {
+      float4 in[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) in[i] = t + i < n_tok ? *reinterpret_cast<const float4*>(dec + (int64_t)(t0 + t + i) * ldd + col_a + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (t + i < n_tok)
+          *reinterpret_cast<float4*>(row + (int64_t)(t + i) * lay.width + lay.g + c) =
+              make_float4(expf(a[0] * softplus_f(in[i].x + bias[0])), expf(a[1] * softplus_f(in[i].y + bias[1])), expf(a[2] * softplus_f(in[i].z + bias[2])),
+                          expf(a[3] * softplus_f(in[i].w + bias[3])));
+    }
+  } else if (task == spans + g_spans) {   // what there is one of per head
+    for (int i = lane; i < n_tok * H; i += 32) {
+      const int t = i / H, h = i - t * H;
+      row[(int64_t)t * lay.width + lay.b + h] = sigmoid_f(raw[(int64_t)(t0 + t) * ldr + col_b + h]);
+      if (!channels) row[(int64_t)t * lay.width + lay.g + h] = expf(-expf(ldf(A_log + h)) * softplus_f(dec[(int64_t)(t0 + t) * ldd + col_a + h] + ldf(dt_bias + h)));
+    }
+  }
+}
+
 // the state becomes the last taps - 1 inputs of the sequence (older entries shift when the step brought fewer tokens than that)
 __global__ void delta_conv_state_kernel(const float* __restrict__ u, int64_t ld_u, int col0, int C, int taps, float* __restrict__ conv_state,
                                         const int32_t* __restrict__ state_slots, const int32_t* __restrict__ cu_q,
@@ -156,12 +258,12 @@ __device__ __forceinline__ void cp_async_4(void* smem_dst, const void* gmem_src)
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
 }
 
-constexpr int kTileTok = 16, kQuad = 4, kQuads = kTileTok / kQuad, kRowLanes = 16, kColsPerWarp = 8, kABPitch = 24;
+constexpr int kTileTok = 16, kQuad = 4, kQuads = kTileTok / kQuad, kABPitch = 24;
 
 // shared memory of delta_chunk_kernel in floats
 __host__ __device__ inline int delta_raw_row(int dk, int NC, bool channels) { return (channels ? 3 : 2) * ((dk + 3) & ~3) + NC + 8; }
-__host__ __device__ inline int delta_chunk_floats(int NR, int dk, int NC, bool channels) {
-  return kQuads * NR * kRowLanes * 13 + kQuads * 2 * kABPitch + 2 * kTileTok * delta_raw_row(dk, NC, channels);
+__host__ __device__ inline int delta_chunk_floats(int rows, int dk, int NC, bool channels) {  // rows: those that the block's lanes hold
+  return kQuads * rows * 13 + kQuads * 2 * kABPitch + 2 * kTileTok * delta_raw_row(dk, NC, channels);
 }
 
 // values v[0 .. 2^k) summed over the lanes of a group of 2^k' lanes, each lane left with its share: one halving per lane bit
@@ -190,14 +292,27 @@ __device__ __forceinline__ void permute4(float4 f, bool lo, bool hi, float* o) {
   o[3] = hi ? b : d;
 }
 
-template <int NR>  // state rows per lane: dk <= 16 NR
-__global__ void __launch_bounds__(256, NR <= 8 ? 2 : 1) delta_chunk_kernel(
+// a * b + c on two fp32 at once (each rounded as fmaf)
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{ .reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 z, {%6, %7}; fma.rn.f32x2 z, x, y, z; mov.b64 {%0, %1}, z; }"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+
+// The memory's rows lie over kRowLanes lanes, NR each (dk <= kRowLanes NR).  Sixteen lanes and eight columns per warp take fewer instructions; 32 lanes
+// and four columns put twice as many warps on a small grid and shorten the chain from four tokens to the next four, which is what bounds it
+// then.  Measured on B200 (us, 16 / 32 lanes, heads of 128 x 128): 16 heads, 690 tokens 251 / 180, 4 sequences of 256 to 768 281 / 257, 2 of 125 55 / 46;
+// 32 heads, 400 tokens 164 / 134, 8 x 500 557 / 707, 6 of 400 to 800 681 / 775; 16 heads, 16 x 250 305 / 401.
+template <int NR, int kRowLanes>
+__global__ void __launch_bounds__(256, NR * kRowLanes <= 128 ? 2 : 1) delta_chunk_kernel(
     const float* __restrict__ pre, float* __restrict__ S_state, const int32_t* __restrict__ state_slots, const int32_t* __restrict__ cu_q,
     const int64_t* __restrict__ position_ids, float* __restrict__ y, int64_t ld_y, int H, int G, int dk, int dv, int channels, int NC, int vec) {
   pdl_launch_dependents();
   pdl_wait();
   extern __shared__ __align__(16) float sm[];
-  constexpr int dkp = NR * kRowLanes;
+  constexpr int dkp = NR * kRowLanes, kColsPerWarp = kRowLanes == 16 ? 8 : 4;
   float4* KG = reinterpret_cast<float4*>(sm);       // [quad][dkp]: G_j k_j, j = 0 .. 3
   float4* QG = KG + kQuads * dkp;                   // G_j q_j
   float4* KD = QG + kQuads * dkp;                   // D_i k_i
@@ -256,9 +371,9 @@ __global__ void __launch_bounds__(256, NR <= 8 ? 2 : 1) delta_chunk_kernel(
     cp_async_commit();
   };
 
-  // this thread's part of the memory: rows rl + 16 i, columns c0 .. c0 + 3 of the block's.  Entry x of S[i] is column c0 + (x ^ perm): with
+  // this thread's part of the memory: rows rl + kRowLanes i, columns c0 .. c0 + 3 of the block's.  Entry x of S[i] is column c0 + (x ^ perm): with
   // a lane's own column order a reduction over lanes always keeps the lower half of what it has and sends the upper half
-  const int rl = lane & 15, c0 = w * kColsPerWarp + (lane >> 4) * 4;
+  const int rl = lane & (kRowLanes - 1), c0 = w * kColsPerWarp + (kRowLanes == 16 ? (lane >> 4) * 4 : 0);
   const bool b3 = lane & 8, b2 = lane & 4, b1 = lane & 2, b0 = lane & 1;
   const int perm = (lane >> 2) & 3, my_c = c0 + perm;    // my_c: the column whose reductions this lane ends up with
   float* Sp = S_state + ((int64_t)state_slots[b] * H + h) * dk * dv + v0;
@@ -340,22 +455,27 @@ __global__ void __launch_bounds__(256, NR <= 8 ? 2 : 1) delta_chunk_kernel(
     __syncthreads();
     for (int qd = 0; qd < quads; ++qd) {
       float P[16], O[16];   // [column][token]
+      {
+        float2 P2[8], O2[8];  // token pairs: the staged vectors come as such
 #pragma unroll
-      for (int i = 0; i < 16; ++i) P[i] = O[i] = 0.f;
+        for (int i = 0; i < 8; ++i) P2[i] = O2[i] = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int i = 0; i < NR; ++i) {
-        const float4 kg = KG[qd * dkp + rl + kRowLanes * i], qg = QG[qd * dkp + rl + kRowLanes * i];
+        for (int i = 0; i < NR; ++i) {
+          const float4 kg = KG[qd * dkp + rl + kRowLanes * i], qg = QG[qd * dkp + rl + kRowLanes * i];
+          const float2 k01 = make_float2(kg.x, kg.y), k23 = make_float2(kg.z, kg.w), q01 = make_float2(qg.x, qg.y), q23 = make_float2(qg.z, qg.w);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float s = S[i][c];
-          P[c * 4 + 0] = fmaf(kg.x, s, P[c * 4 + 0]);
-          P[c * 4 + 1] = fmaf(kg.y, s, P[c * 4 + 1]);
-          P[c * 4 + 2] = fmaf(kg.z, s, P[c * 4 + 2]);
-          P[c * 4 + 3] = fmaf(kg.w, s, P[c * 4 + 3]);
-          O[c * 4 + 0] = fmaf(qg.x, s, O[c * 4 + 0]);
-          O[c * 4 + 1] = fmaf(qg.y, s, O[c * 4 + 1]);
-          O[c * 4 + 2] = fmaf(qg.z, s, O[c * 4 + 2]);
-          O[c * 4 + 3] = fmaf(qg.w, s, O[c * 4 + 3]);
+          for (int c = 0; c < 4; ++c) {
+            const float2 s2 = make_float2(S[i][c], S[i][c]);
+            P2[c * 2] = fma2(k01, s2, P2[c * 2]);
+            P2[c * 2 + 1] = fma2(k23, s2, P2[c * 2 + 1]);
+            O2[c * 2] = fma2(q01, s2, O2[c * 2]);
+            O2[c * 2 + 1] = fma2(q23, s2, O2[c * 2 + 1]);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          P[2 * i] = P2[i].x; P[2 * i + 1] = P2[i].y;
+          O[2 * i] = O2[i].x; O[2 * i + 1] = O2[i].y;
         }
       }
       // predictions: every group of four lanes ends with the four tokens of one column
@@ -365,6 +485,10 @@ __global__ void __launch_bounds__(256, NR <= 8 ? 2 : 1) delta_chunk_kernel(
       for (int j = 0; j < 4; ++j) P[j] += __shfl_xor_sync(0xffffffffu, P[j], 2);
 #pragma unroll
       for (int j = 0; j < 4; ++j) P[j] += __shfl_xor_sync(0xffffffffu, P[j], 1);
+      if constexpr (kRowLanes == 32) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) P[j] += __shfl_xor_sync(0xffffffffu, P[j], 16);
+      }
       const float* tr = tile + qd * kQuad * rr;
       const float4* ab0 = reinterpret_cast<const float4*>(AB + qd * 2 * kABPitch);
       const float4* ab1 = ab0 + kABPitch / 4;
@@ -392,18 +516,26 @@ __global__ void __launch_bounds__(256, NR <= 8 ? 2 : 1) delta_chunk_kernel(
         const float4 kd = KD[qd * dkp + rl + kRowLanes * i];
         const float ga = GA[qd * dkp + rl + kRowLanes * i];
 #pragma unroll
-        for (int c = 0; c < 4; ++c)
-          S[i][c] = fmaf(kd.w, U[3][c], fmaf(kd.z, U[2][c], fmaf(kd.y, U[1][c], fmaf(kd.x, U[0][c], ga * S[i][c]))));
+        for (int c = 0; c < 4; c += 2) {
+          float2 v = make_float2(ga * S[i][c], ga * S[i][c + 1]);
+          v = fma2(make_float2(kd.x, kd.x), make_float2(U[0][c], U[0][c + 1]), v);
+          v = fma2(make_float2(kd.y, kd.y), make_float2(U[1][c], U[1][c + 1]), v);
+          v = fma2(make_float2(kd.z, kd.z), make_float2(U[2][c], U[2][c + 1]), v);
+          v = fma2(make_float2(kd.w, kd.w), make_float2(U[3][c], U[3][c + 1]), v);
+          S[i][c] = v.x;
+          S[i][c + 1] = v.y;
+        }
       }
       // read-outs: every lane ends with one (token, column)
       fold<16>(O, 8);
       fold<8>(O, 4);
       halve<4>(O, 2, b1);
       halve<2>(O, 1, b0);
+      if constexpr (kRowLanes == 32) O[0] += __shfl_xor_sync(0xffffffffu, O[0], 16);
       const int j = lane & 3, t = t0 + qd * kQuad + j;
       const float4 bj = ab0[2 + j], bx = ab1[2 + j];
       const float o = O[0] + (bj.x + bx.x) * um[0] + (bj.y + bx.y) * um[1] + (bj.z + bx.z) * um[2] + (bj.w + bx.w) * um[3];
-      if (t < t_end && my_c < live_cols) y[(int64_t)t * ld_y + h * dv + v0 + my_c] = o;
+      if ((kRowLanes == 16 || lane < 16) && t < t_end && my_c < live_cols) y[(int64_t)t * ld_y + h * dv + v0 + my_c] = o;
     }
   }
 #pragma unroll
@@ -562,6 +694,19 @@ extern "C" int b200_seq_delta_prepare(const float* u, int64_t ld, int col0, int 
   }
   cudaStream_t st = (cudaStream_t)stream;
   const int shift = (T == B && taps > 1) ? 1 : 0, C = 2 * kv_heads * dk + H * dv;
+  const bool wide = ((reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(conv_state) | reinterpret_cast<uintptr_t>(dec) | reinterpret_cast<uintptr_t>(out)) & 15) == 0 &&
+                    ((ld | col0 | ldd | col_a | (H * dv)) & 3) == 0;
+  if (wide && (dk == 64 || dk == 128) && taps <= 4 && T > 4 * (int64_t)B && T >= kRunMinTokens) {
+    const int run_tasks = (C + 127) / 128 + (channels ? (H * dk + 127) / 128 : 0) + 1;
+    B200_SEQ_DISPATCH(dt, E, B200_LAUNCH((delta_prepare_run_kernel<E>), dim3((unsigned)(T / kRunTok + B), (unsigned)((run_tasks + 7) / 8)), dim3(256), 0, st, u, ld, col0,
+                                         taps, (const E*)w, conv_state, state_slots, cu_q, B, position_ids, raw, ldr, col_b, dec, ldd, col_a, channels,
+                                         (const E*)A_log, (const E*)dt_bias, q_scale, out, H, kv_heads, dk, dv));
+    if (taps > 1)
+      B200_LAUNCH(delta_conv_state_kernel, dim3((unsigned)B, (unsigned)((C + 255) / 256)), dim3(256), 0, st, u, ld, col0, C, taps, conv_state, state_slots, cu_q,
+                  position_ids);
+    b200_count_launches(taps > 1 ? 2 : 1);
+    return B200_OK;
+  }
   const int tasks = 2 * kv_heads + (H * dv + kPrepSpan - 1) / kPrepSpan + ((channels ? H * dk : H) + kPrepSpan - 1) / kPrepSpan +
                     (H + kPrepSpan - 1) / kPrepSpan;
   int parts = (tasks + kPrepThreads / 32 - 1) / (kPrepThreads / 32);   // few rows: a warp per task; many: blocks that loop
@@ -581,14 +726,14 @@ extern "C" int b200_seq_delta_prepare(const float* u, int64_t ld, int col0, int 
   return B200_OK;
 }
 
-template <int NR>
+template <int NR, int LANES>
 static int launch_delta_chunk(const float* pre, float* S_state, const int32_t* state_slots, const int32_t* cu_q, const int64_t* position_ids, float* y,
                               int64_t ld_y, int B, int H, int G, int dk, int dv, int channels, int NC, int vec, cudaStream_t st) {
-  const size_t smem = (size_t)delta_chunk_floats(NR, dk, NC, channels != 0) * 4;
+  const size_t smem = (size_t)delta_chunk_floats(NR * LANES, dk, NC, channels != 0) * 4;
   static bool cfg = false;
-  if (!cfg) { cudaFuncSetAttribute(delta_chunk_kernel<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); cfg = true; }
+  if (!cfg) { cudaFuncSetAttribute(delta_chunk_kernel<NR, LANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); cfg = true; }
   dim3 grid((unsigned)B, (unsigned)H, (unsigned)((dv + NC - 1) / NC));
-  B200_LAUNCH((delta_chunk_kernel<NR>), grid, dim3((unsigned)(NC / kColsPerWarp * 32)), smem, st, pre, S_state, state_slots, cu_q, position_ids, y, ld_y,
+  B200_LAUNCH((delta_chunk_kernel<NR, LANES>), grid, dim3((unsigned)(NC / (LANES == 16 ? 8 : 4) * 32)), smem, st, pre, S_state, state_slots, cu_q, position_ids, y, ld_y,
               H, G, dk, dv, channels, NC, vec);
   b200_count_launches(1);
   return B200_OK;
@@ -636,13 +781,19 @@ extern "C" int b200_seq_delta_rows_scan(const float* pre, int channels, float* S
 #undef DST
   }
   const int vec = (dk % 4 == 0 && dv % 4 == 0 && aligned) ? 1 : 0;
-  // 64 columns per block share each staged vector among more of the memory; 32 spread a small grid over more SMs
-  const int most = (int64_t)B * H * ((dv + 31) / 32) <= 148 ? 32 : 64;
+  // 64 columns per block share each staged vector among more of the memory; a small grid is spread over 32 columns and 32 lanes
+  const bool small = (int64_t)B * H * ((dv + 31) / 32) <= 2 * 148;
+  const int most = small ? 32 : 64;
   const int blocks = (dv + most - 1) / most;
   const int NC = ((dv + blocks - 1) / blocks + 7) / 8 * 8;
-#define DCH(NR) return (launch_delta_chunk<NR>(pre, S_state, state_slots, cu_q, position_ids, y, ld_y, B, H, kv_heads, dk, dv, channels, NC, vec, st))
-  if (dk <= 64) DCH(4);
-  if (dk <= 128) DCH(8);
-  DCH(16);
+#define DCH(NR, LANES) return (launch_delta_chunk<NR, LANES>(pre, S_state, state_slots, cu_q, position_ids, y, ld_y, B, H, kv_heads, dk, dv, channels, NC, vec, st))
+  if (small) {
+    if (dk <= 64) DCH(2, 32);
+    if (dk <= 128) DCH(4, 32);
+    DCH(8, 32);
+  }
+  if (dk <= 64) DCH(4, 16);
+  if (dk <= 128) DCH(8, 16);
+  DCH(16, 16);
 #undef DCH
 }
