@@ -13,8 +13,8 @@
 //   * int4: four teams of four warps turn 64 k of a record each into the SWIZZLE_128B image of an fp16 A tile (thread = feature row, eight
 //     conflict-free 16-byte stores).  One de-quantised tile serves up to 256 tokens, twice as many as the weight-streaming kernel's, and shared
 //     memory as the operand's place leaves TMEM to the accumulators.
-//     Gate|up weights with SiLU(gate) * up: a CTA takes the same 64 features of both tiles of a super-tile, sixteen of each per warp, so
-//     that both factors of an output sit in one warp, sixteen lanes apart.
+//   * Gate|up weights with SiLU(gate) * up: a CTA takes 64 gate features and the 64 up features that belong to them, sixteen of each per epilogue
+//     warp, so that both factors of an output sit in one warp, sixteen lanes apart.
 //   * Lane = feature in the epilogue, transposed through shared memory into 16-byte stores; rows that those do not fit are stored by value.
 //
 // Measured on B200 (us, cold weights; before = one CTA per tile): fp16 4099 x 4096 x 4096 134 -> 98, 300 x 4096 x 4096 31.4 -> 16.2, 3001 x 5120 x
@@ -46,16 +46,20 @@ constexpr int kPairMaxStages = 10;
 __host__ __device__ constexpr int pair_block_bytes(int tn) { return kPairABytes + (tn / 2) * kPairK * 2; }
 
 // what the weights are, and what happens to the result (the first four as FMT of gemm_f16.cu)
-enum PairKind { kPairF16 = 0, kPairBf16 = 1, kPairBf16F32 = 2, kPairBf16Relu2 = 3, kPairW4 = 4, kPairW4Silu = 5 };
+enum PairKind { kPairF16 = 0, kPairBf16 = 1, kPairBf16F32 = 2, kPairBf16Relu2 = 3, kPairW4 = 4, kPairW4Silu = 5,
+  // grouped: rows of X are compact, those of one expert side by side, W is one matrix per expert
+  kPairExpBf16 = 6, kPairExpBf16F32 = 7, kPairExpRelu2 = 8 };
 
 template <int KIND>
 struct PairCfg {
   static constexpr bool kInt4 = KIND == kPairW4 || KIND == kPairW4Silu;
+  static constexpr bool kExperts = KIND >= kPairExpBf16;
+  static constexpr bool kOut32 = KIND == kPairBf16F32 || KIND == kPairExpBf16F32;
   static constexpr bool kAct = KIND == kPairW4Silu;
   static constexpr int kThreads = kInt4 ? 768 : 256;
   static constexpr int kRingBytes = (kInt4 ? 5 : 6) * pair_block_bytes(kPairMaxN);
   static constexpr int kRecs = kInt4 ? 4 : 0;  // ring of int4 records (128 k each)
-  static constexpr int kOutBytes = 4 * 32 * 32 * (KIND == kPairBf16F32 ? 4 : 2);  // 32 tokens of an epilogue warp's features, four warps
+  static constexpr int kOutBytes = 4 * 32 * 32 * (kOut32 ? 4 : 2);  // 32 tokens of an epilogue warp's features, four warps
   static constexpr int kNumBars = 2 * kPairMaxStages + 2 * kRecs + 4;
   static constexpr int kSmemBytes = kRingBytes + kRecs * kW4RecMaxBytes + kOutBytes + kNumBars * 8 + 16 + 1024;
   static constexpr int kDqWarp = 4, kServeWarp = kInt4 ? 20 : 4;
@@ -67,11 +71,14 @@ struct PairParams {
   const void* bias;
   const unsigned char* packed;  // int4 records
   int T, N, ldy;
+  int half;                     // act: weight rows between a gate feature and its up feature; N is the number of outputs then
   int n_kb;                     // 64-wide k-blocks per tile (int4: two per record)
   int rec_per_tile, rec_bytes, group_rows, half_tiles;
   int tn, n_tt, n_m;            // token tile, token tiles, feature tiles
   int per_stage, n_stages;      // k-blocks per stage of the ring, stages per tile
   int stages, stage_bytes;      // depth of the ring
+  const int32_t* offsets;       // experts: first row of each, [E + 1]
+  int E;
   int vec;                      // rows of y can be written in 16-byte pieces
 };
 
@@ -124,9 +131,9 @@ __device__ __forceinline__ void sts_v4(uint32_t addr, uint32_t a, uint32_t b, ui
 
 template <int KIND>
 __device__ __forceinline__ auto pair_value(float v) {
-  if constexpr (KIND == kPairBf16) return __float2bfloat16_rn(v);
-  else if constexpr (KIND == kPairBf16Relu2) return __float2bfloat16_rn(v < 0.f ? 0.f : v * v);
-  else if constexpr (KIND == kPairBf16F32) return v;
+  if constexpr (KIND == kPairBf16 || KIND == kPairExpBf16) return __float2bfloat16_rn(v);
+  else if constexpr (KIND == kPairBf16Relu2 || KIND == kPairExpRelu2) return __float2bfloat16_rn(v < 0.f ? 0.f : v * v);
+  else if constexpr (KIND == kPairBf16F32 || KIND == kPairExpBf16F32) return v;
   else return __float2half_rn(v);
 }
 // SiLU(gate) * up of two tokens' accumulators: lanes 0..15 hold gate features and finish the first token, lanes 16..31 hold the up features
@@ -140,16 +147,49 @@ __device__ __forceinline__ __half act_pair(uint32_t first, uint32_t second, floa
 }
 template <int KIND>
 __device__ __forceinline__ float pair_bias(const void* bias, int n) {
-  if constexpr (KIND == kPairBf16 || KIND == kPairBf16F32 || KIND == kPairBf16Relu2) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(bias)[n]);
+  if constexpr (KIND != kPairF16 && KIND < kPairW4) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(bias)[n]);
   else return __half2float(reinterpret_cast<const __half*>(bias)[n]);
 }
 
-// Tile i of the output in the order in which the pairs take them: sixteen token tiles share a weight tile before the next one, so that the
-// weights come from HBM once per sixteen token tiles and the activations stay in L2.
-__device__ __forceinline__ void pair_tile(const PairParams& p, int i, int& m, int& tt) {
-  const int per = 16 * p.n_m, g = i / per, r = i - g * per, width = min(16, p.n_tt - g * 16);
-  m = r / width;
-  tt = g * 16 + r % width;
+struct PairTile {
+  int m, t0, nn, row_end;  // feature tile; first row, padded rows and end of the rows of its token tile
+  int expert;
+};
+// the tile a role is at, and (experts) where its rows lie: `before` row tiles belong to experts ahead of `e`
+struct PairCursor {
+  int e = 0, before = 0;
+};
+
+// Tile i in the order in which the pairs take them; false: there is none.  Sixteen token tiles share a weight tile before the next one, so that the
+// weights come from HBM once per sixteen token tiles and the activations stay in L2.  Experts: all feature tiles of a row tile side by side; how many
+// row tiles there are is only known here, from the plan's offsets (i ascends, so the cursor only moves on).
+template <int KIND>
+__device__ __forceinline__ bool pair_tile(const PairParams& p, int i, PairCursor& cur, PairTile& t) {
+  if constexpr (PairCfg<KIND>::kExperts) {
+    const int rt = i / p.n_m;
+    t.m = i - rt * p.n_m;
+    for (; cur.e < p.E; ++cur.e) {
+      const int first = p.offsets[cur.e], end = p.offsets[cur.e + 1], n = (end - first + kPairMaxN - 1) / kPairMaxN;
+      if (rt < cur.before + n) {
+        t.expert = cur.e;
+        t.t0 = first + (rt - cur.before) * kPairMaxN;
+        t.nn = min(kPairMaxN, (end - t.t0 + 31) & ~31);
+        t.row_end = end;
+        return true;
+      }
+      cur.before += n;
+    }
+    return false;
+  } else {
+    if (i >= p.n_tt * p.n_m) return false;
+    const int per = 16 * p.n_m, g = i / per, r = i - g * per, width = min(16, p.n_tt - g * 16);
+    t.m = r / width;
+    t.t0 = (g * 16 + r % width) * p.tn;
+    t.nn = min(p.tn, (p.T - t.t0 + 31) & ~31);
+    t.row_end = p.T;
+    t.expert = 0;
+    return true;
+  }
 }
 
 template <int KIND>
@@ -200,6 +240,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   tcgen05_fence_after();
   const uint32_t tmem_d = *tmem_slot;
   bool ok = true;
+  if constexpr (C::kExperts) pdl_wait();  // every role reads the plan's offsets
 
   if (warp == C::kServeWarp + 1) {
     // ------------------------------------------------------------------ TMA: half of the tile's tokens (and fp16 / bf16 features)
@@ -207,11 +248,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       const uint64_t pol = policy_evict_last();
       int s = 0, ph = 1;
       pdl_wait();  // x is the previous kernel's output
-      for (int i = pair; i < n_tiles; i += n_pairs) {
-        int m, tt;
-        pair_tile(p, i, m, tt);
-        const int t0 = tt * p.tn, nn = min(p.tn, (p.T - t0 + 31) & ~31);
-        const int row_x = t0 + (int)rank * (nn >> 1), row_w = m * kPairM + (int)rank * 128;
+      PairCursor cur;
+      PairTile tl;
+      for (int i = pair; pair_tile<KIND>(p, i, cur, tl); i += n_pairs) {
+        const int m = tl.m, row_x = tl.t0 + (int)rank * (tl.nn >> 1), row_w = tl.expert * p.N + m * kPairM + (int)rank * 128;
         for (int kb = 0; kb < p.n_stages; ++kb) {
           mbar_wait_soft(&empty[s], ph, ok);
           unsigned char* st = smem + s * p.stage_bytes;
@@ -232,10 +272,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       constexpr uint32_t fmt = C::kInt4 || KIND == kPairF16 ? 0u : ((1u << 7) | (1u << 10));
       const uint64_t desc0 = umma_desc_kmajor_sw128(smem_u32(smem));
       int s = 0, ph = 0, it = 0;
-      for (int i = pair; i < n_tiles; i += n_pairs, ++it) {
-        int m, tt;
-        pair_tile(p, i, m, tt);
-        const int nn = min(p.tn, (p.T - tt * p.tn + 31) & ~31);
+      PairCursor cur;
+      PairTile tl;
+      for (int i = pair;; i += n_pairs, ++it) {
+        bool more = pair_tile<KIND>(p, i, cur, tl);
+        if constexpr (C::kExperts) {  // values from memory: through a reduction, whose result the compiler knows to be warp-uniform
+          more = __reduce_max_sync(0xffffffffu, (unsigned)more) != 0;
+          tl.nn = __reduce_max_sync(0xffffffffu, tl.nn);
+        }
+        if (!more) break;
+        const int nn = tl.nn;
         const uint32_t idesc = umma_idesc_f16_f32acc(kPairM, nn) | fmt, d = tmem_d + (it & 1) * kPairMaxN;
         mbar_wait_soft(&tmem_empty[it & 1], ((it >> 1) & 1) ^ 1, ok);
         for (int kb = 0; kb < p.n_stages; ++kb) {
@@ -262,9 +308,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     // ------------------------------------------------------------------ TMA: int4 records (immutable: no wait for the previous kernel)
     if (elect_one()) {
       int r = 0, ph = 1;
-      for (int i = pair; i < n_tiles; i += n_pairs) {
-        int m, tt;
-        pair_tile(p, i, m, tt);
+      PairCursor cur;
+      PairTile tl;
+      for (int i = pair; pair_tile<KIND>(p, i, cur, tl); i += n_pairs) {
+        const int m = tl.m;
         for (int kb = 0; kb < p.n_kb / 2; ++kb) {
           mbar_wait_soft(&rec_empty[r], ph, ok);
           mbar_arrive_expect_tx(&rec_full[r], p.rec_bytes);
@@ -337,16 +384,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
     int it = 0;
     pdl_wait();  // y and the bias belong to the stream order
-    for (int i = pair; i < n_tiles; i += n_pairs, ++it) {
-      int m, tt;
-      pair_tile(p, i, m, tt);
-      const int t0 = tt * p.tn, nn = min(p.tn, (p.T - t0 + 31) & ~31);
+    PairCursor cur;
+    PairTile tl;
+    for (int i = pair; pair_tile<KIND>(p, i, cur, tl); i += n_pairs, ++it) {
+      const int m = tl.m, t0 = tl.t0, nn = tl.nn, row_end = tl.row_end;
       // act: lanes 0..15 hold gate features, lanes 16..31 the up features of the same outputs
       const int tile = p.half_tiles ? m + (int)rank * p.half_tiles : 2 * m + (int)rank;  // 128-feature tile of this CTA
       const int n = C::kAct ? m * 128 + (int)rank * 64 + warp * 16 + (lane & 15) : tile * 128 + warp * 32 + lane;
       const int n0 = n - lane % kRow;                                       // the warp's first output feature
-      const int n_w = C::kAct ? n + (lane >> 4) * p.half_tiles * 128 : n;  // the weight row behind this lane
-      const bool n_ok = C::kAct || n < p.N;
+      const int n_w = C::kAct ? n + (lane >> 4) * p.half : n;  // the weight row behind this lane
+      const bool n_ok = n < p.N;
       const float bv = p.bias && n_ok ? pair_bias<KIND>(p.bias, n_w) : 0.f;
       mbar_wait_soft(&tmem_full[it & 1], (it >> 1) & 1, ok);
       tcgen05_fence_after();
@@ -377,7 +424,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 #pragma unroll
             for (int j = 0; j < 32; j += kTokens) {
               const int t = j + lane / kPieces;
-              if (t0 + c + t < p.T)
+              if (t0 + c + t < row_end)
                 *reinterpret_cast<uint4*>(reinterpret_cast<Out*>(p.y) + (size_t)(t0 + c + t) * p.ldy + n0 + f) = *reinterpret_cast<const uint4*>(out + t * kRow + f);
             }
           }
@@ -386,12 +433,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
           for (int j = 0; j < 32; j += 2) {
             const Out o = act_pair(v[j], v[j + 1], bv, lane);
             const int t = t0 + c + j + (lane >> 4);
-            if (t < p.T) reinterpret_cast<Out*>(p.y)[(size_t)t * p.ldy + n] = o;
+            if (t < row_end && n_ok) reinterpret_cast<Out*>(p.y)[(size_t)t * p.ldy + n] = o;
           }
         } else if (n_ok) {
 #pragma unroll
           for (int j = 0; j < 32; ++j)
-            if (t0 + c + j < p.T) reinterpret_cast<Out*>(p.y)[(size_t)(t0 + c + j) * p.ldy + n] = pair_value<KIND>(__uint_as_float(v[j]) + bv);
+            if (t0 + c + j < row_end) reinterpret_cast<Out*>(p.y)[(size_t)(t0 + c + j) * p.ldy + n] = pair_value<KIND>(__uint_as_float(v[j]) + bv);
         }
       }
     }
@@ -441,9 +488,10 @@ static int launch_gemm_pair(const void* x, const void* w, int64_t K, PairParams 
     configured = true;
   }
   const CUtensorMap* mx = get_tmap_2d(x, pp.T, K, K, pl.tn / 2, kPairK, TmapDtype::kF16, TmapSwizzle::k128B);
-  const CUtensorMap* mw = w ? get_tmap_2d(w, pp.N, K, K, 128, kPairK, TmapDtype::kF16, TmapSwizzle::k128B) : mx;
+  const uint64_t rows_w = (uint64_t)pp.N * (C::kExperts ? pp.E : 1);
+  const CUtensorMap* mw = w ? get_tmap_2d(w, rows_w, K, K, 128, kPairK, TmapDtype::kF16, TmapSwizzle::k128B) : mx;
   if (!mx || !mw) return B200_ERR_CUDA;
-  constexpr int kOut = KIND == kPairBf16F32 ? 4 : 2;
+  constexpr int kOut = C::kOut32 ? 4 : 2;
   pp.vec = ((uintptr_t)pp.y & 15) == 0 && (int64_t)pp.ldy * kOut % 16 == 0;
   pp.tn = pl.tn;
   pp.n_tt = pl.n_tt;

@@ -862,8 +862,8 @@ static int gemm_w4a16_impl(const void* x, const void* packed, const void* bias, 
     pp.bias = bias;
     pp.packed = (const unsigned char*)packed;
     pp.T = (int)T;
-    pp.N = (int)N;
-    pp.ldy = (int)(act ? N / 2 : N);
+    pp.N = pp.ldy = (int)(act ? N / 2 : N);
+    pp.half = half_tiles * kW4TileM;
     pp.n_kb = 2 * (int)((K + kW4BlockK - 1) / kW4BlockK);
     pp.rec_per_tile = w4_nkb(K);
     pp.rec_bytes = kW4WordBytes + gr * kW4MetaRowBytes;

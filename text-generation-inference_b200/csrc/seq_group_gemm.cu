@@ -12,6 +12,7 @@
 // Warp roles: 0 = TMA producer, 1 = MMA issuer (one elected thread each), 2..5 = epilogue.
 //
 // Every wait is bounded: a block that gives up counts itself in `group_gemm_gave_up`, waits for its copies in flight, frees its TMEM and ends.
+#include "gemm_pair.cuh"
 #include "seq_common.cuh"
 #include "tmap.cuh"
 
@@ -224,6 +225,11 @@ static int launch_group_gemm(const void* w, int64_t w_rows, int64_t K, const voi
 using namespace b200;
 using namespace b200::seq;
 
+// Average rows per expert from which the pairs take over.  Measured on B200 (us, blocks of this file / pairs; 16 experts, 2048 -> 2112 and back): 82 rows
+// 29.2 + 30.0 / 29.5 + 30.4, 131 rows 31.3 + 31.9 / 31.4 + 32.4, 205 rows 40.6 + 41.3 / 35.7 + 39.0, 819 rows 126 + 126 / 97 + 92; 4096 -> 4224, 205 rows
+// 134 + 136 / 113 + 117.
+constexpr int64_t kPairRowsPerExpert = 160;
+
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // blocks of this process's grouped products that gave up a wait (0 unless something is wrong); -1: the count could not be read
@@ -268,6 +274,24 @@ extern "C" int b200_seq_experts_gemm(const void* x, const void* w, void* y, int 
   if (E < 1 || E > 256 || K <= 0 || K % 8 || !aligned16(x) || !aligned16(w) || (y_dt != B200_DT_BF16 && y_dt != B200_DT_F32)) {
     b200_set_last_error("seq_experts_gemm: need at most 256 experts, K a multiple of 8, 16-byte aligned operands");
     return B200_ERR_ARG;
+  }
+  if (K >= 64 && max_rows / E >= kPairRowsPerExpert && !(act && y_dt == B200_DT_F32)) {
+    // row tiles of up to 256 rows of one expert on pairs of SMs; each is as wide as it has rows
+    PairParams pp = {};
+    pp.y = y;
+    pp.T = (int)max_rows;
+    pp.N = pp.ldy = (int)N;
+    pp.n_kb = (int)((K + kPairK - 1) / kPairK);
+    pp.offsets = offsets;
+    pp.E = E;
+    const int n_m = (int)((N + kPairM - 1) / kPairM), pairs = 148 / 2;
+    const int64_t most = ((max_rows + kPairMaxN - 1) / kPairMaxN + E) * n_m;
+    if (most < (1 << 30)) {
+      const PairPlan pl = {kPairMaxN, 0, n_m, (int)(most < pairs ? most : pairs), 1, 0.f};
+      cudaStream_t ps = (cudaStream_t)stream;
+      return act ? launch_gemm_pair<kPairExpRelu2>(x, w, K, pp, pl, 0, ps)
+                 : y_dt == B200_DT_F32 ? launch_gemm_pair<kPairExpBf16F32>(x, w, K, pp, pl, 0, ps) : launch_gemm_pair<kPairExpBf16>(x, w, K, pp, pl, 0, ps);
+    }
   }
   GgParams p{y, N, 0, 0, offsets, E, (int)max_rows, (int)N, (int)((K + kGgTileK - 1) / kGgTileK), y_dt == B200_DT_F32, act};
   const int TN = max_rows / E >= 160 ? 256 : 128;   // rows per expert, were they dealt out evenly
