@@ -46,7 +46,7 @@ constexpr int kPfAhead = 2;      // items that are known ahead
 // The reference maximum of a row follows the true one through the first key tiles after the first; later it moves only when the maximum has grown
 // past it by more than 2^8.  A largest weight of exactly 1 is worth some precision (against float64, over prompts of 64 to 2500 keys: 0.993 of
 // the error of following it always with unrounded sums, 1.006 with no exact tiles), following it always costs 323 us where this takes 306.
-// (bfloat16 weights, the token-major caches': always followed; lagging by the same rule cost 2 to 5 % of precision.)
+// (bfloat16 weights, the token-major caches': always followed.)
 constexpr int kPfExactTiles = 4;
 constexpr float kPfRescale = 8.f;  // log2
 // registers per thread: the launch has 384 x 168; the two softmax warpgroups take 216 each, the other one keeps 72

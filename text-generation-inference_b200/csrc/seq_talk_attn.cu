@@ -722,8 +722,8 @@ extern "C" int b200_seq_talk_attn_splits(int dt, int64_t T, int B, int H, int G,
 }
 
 // Prompts without a mix take the tcgen05 kernel: tiles of 128 (token, head) rows, so it wants steps of enough tokens per sequence to fill them.
-// Measured on B200 (us, the m16n8k16 kernel / this one; 16 / 4 heads, d = 128): 2118 + 1882 tokens in chunks of 2048 387 / 86, 4 x 512 84 / 26, 300 after
-// 800 cached 51 / 34, 4 x 40 after 500 38 / 27, 4 x 24 after 1900 56 / 41, 24 after 20 24.5 / 14.3; 4 x 16 after 1900 55 / 51, 4 x 8 48.5 / 50.
+// Measured on B200 (us, the m16n8k16 kernel / this one; 16 / 4 heads, d = 128): 2118 + 1882 tokens in chunks of 2048 387 / 94, 4 x 512 84 / 25, 300 after
+// 800 cached 51 / 35, 4 x 40 after 500 38 / 26, 4 x 24 after 1900 56 / 43, 24 after 20 24.5 / 14.3; 4 x 16 after 1900 55 / 53, 4 x 8 48 / 50.
 // What it needs beside that: heads of 64 or 128 columns, whole 128-row tiles (128 % (heads / kv_heads) == 0), pages of 16 tokens, and 16-byte pieces.
 constexpr int kTalkPromptTokens = 24;  // average tokens per sequence from which on
 
