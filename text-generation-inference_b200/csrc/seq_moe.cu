@@ -136,8 +136,8 @@ __device__ __forceinline__ void moe_pick(const float* __restrict__ row, int E, i
 }
 
 // The plan from the experts' counts (a block, counts in shared memory): row offsets and tiles of every expert.  `offs` [E + 1] receives
-// the offsets as well.  The first 32 threads scan 8 experts each.
-__device__ __forceinline__ void moe_offsets(const int* counts, int* offs, int E, const MoePlan& p) {
+// the offsets as well.  The first 32 threads scan 8 experts each.  `write`: this block puts them into the plan.
+__device__ __forceinline__ void moe_offsets(const int* counts, int* offs, int E, const MoePlan& p, bool write) {
   if (threadIdx.x < 32) {
     int c[kMaxExpertsPerLane], rows = 0, tiles = 0;
 #pragma unroll
@@ -155,8 +155,10 @@ __device__ __forceinline__ void moe_offsets(const int* counts, int* offs, int E,
     }
     if (threadIdx.x == 31) {
       offs[E] = r0;
-      p.offsets[E] = r0;
-      *p.n_tiles = t0;
+      if (write) {
+        p.offsets[E] = r0;
+        *p.n_tiles = t0;
+      }
     }
     r0 -= rows;
     t0 -= tiles;
@@ -165,8 +167,8 @@ __device__ __forceinline__ void moe_offsets(const int* counts, int* offs, int E,
       const int e = threadIdx.x * kMaxExpertsPerLane + i;
       if (e >= E) break;
       offs[e] = r0;
-      p.offsets[e] = r0;
-      for (int r = 0; r < c[i]; r += kMoeTile) {
+      if (write) p.offsets[e] = r0;
+      for (int r = 0; write && r < c[i]; r += kMoeTile) {
         p.tile_expert[t0] = e;
         p.tile_row0[t0] = r0 + r;
         ++t0;
@@ -193,19 +195,24 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const float* __restrict_
   });
 }
 
-__global__ void __launch_bounds__(1024) moe_plan_kernel(const int32_t* __restrict__ ids, int64_t R, int top, int E, MoePlan p) {
+// a pick per thread; every block scans the experts' counts itself, the first one writes what belongs to the plan as a whole.  (One block for all
+// picks walked them 1024 at a time, each a chain of three loads: B200, routing and plan of 2048 / 8192 tokens, 16 experts, 14.6 / 31.7 us, now
+// 11.3 / 19.1.)
+constexpr int kPlanThreads = 256;
+
+__global__ void __launch_bounds__(kPlanThreads) moe_plan_kernel(const int32_t* __restrict__ ids, int64_t R, int top, int E, MoePlan p) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ int counts[32 * kMaxExpertsPerLane], offs[32 * kMaxExpertsPerLane + 1];
-  for (int e = threadIdx.x; e < E; e += blockDim.x) counts[e] = p.counts[e];
+  const int64_t i = (int64_t)blockIdx.x * kPlanThreads + threadIdx.x;
+  const int e = i < R ? ids[i] : E, place = e < E ? p.place[i] : 0;
+  for (int k = threadIdx.x; k < E; k += kPlanThreads) counts[k] = p.counts[k];
   __syncthreads();
-  moe_offsets(counts, offs, E, p);
-  for (int64_t i = threadIdx.x; i < R; i += blockDim.x) {
-    const int e = ids[i];
-    const int row = e < E ? offs[e] + p.place[i] : -1;
-    p.row_of[i] = row;
-    if (row >= 0) p.token_of_row[row] = (int32_t)(i / top);
-  }
+  moe_offsets(counts, offs, E, p, blockIdx.x == 0);
+  if (i >= R) return;
+  const int row = e < E ? offs[e] + place : -1;
+  p.row_of[i] = row;
+  if (row >= 0) p.token_of_row[row] = (int32_t)(i / top);
 }
 
 // picks and plan of a step of few tokens (decoding) in one launch: one block, counters in shared memory
@@ -227,7 +234,7 @@ __global__ void __launch_bounds__(1024) moe_route_plan_kernel(const float* __res
       s_place[t * top + k] = e < E ? atomicAdd(counts + e, 1) : -1;
     });
   __syncthreads();
-  moe_offsets(counts, offs, E, p);
+  moe_offsets(counts, offs, E, p, true);
   for (int i = threadIdx.x; i < T * top; i += blockDim.x) {
     const int e = s_id[i], row = e < E ? offs[e] + s_place[i] : -1;
     ids[i] = e;
@@ -457,7 +464,7 @@ extern "C" int b200_seq_moe_route_scored(const float* logits, int64_t ld, int64_
 #undef ROUTE
   b200_count_launches(1);
   if (one_pass) return B200_OK;
-  B200_LAUNCH(moe_plan_kernel, dim3(1), dim3(1024), 0, st, (const int32_t*)ids, T * top, top, E, p);
+  B200_LAUNCH(moe_plan_kernel, dim3((unsigned)((T * top + kPlanThreads - 1) / kPlanThreads)), dim3(kPlanThreads), 0, st, (const int32_t*)ids, T * top, top, E, p);
   b200_count_launches(1);
   return B200_OK;
 }
