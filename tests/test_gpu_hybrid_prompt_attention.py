@@ -90,3 +90,43 @@ def test_maxima_that_leap():
 @pytest.mark.parametrize("kw", [dict(page=32), dict(dv=128), dict(pad=4), dict(pad=8)])   # other pages, value sizes, offsets (the last one stays with the tcgen05 kernel)
 def test_forms_beside_it(kw):
     _run([60, 130], [0, 20], 4, 2, 64, seed=9, **kw)
+
+
+@pytest.mark.parametrize("d,H,G", [(64, 8, 2), (128, 16, 4)])
+@pytest.mark.parametrize("new,past,chunk,window", [([1, 40, 128, 150], [0, 0, 0, 0], 0, 0), ([70, 33, 300], [5, 1003, 130], 0, 0), ([100, 40], [500, 37], 0, 45),
+                                                   ([90, 200], [333, 1000], 128, 0), ([60, 24], [2041, 700], 200, 77)])
+def test_what_no_query_sees_does_not_matter(d, H, G, new, past, chunk, window):
+    """slots that no query of the step sees - behind a sequence's last key, ahead of its first visible one, blocks of no sequence - and table
+    entries of pages without a visible key: NaN and Inf there change no bit of the result"""
+    import tgis_b200  # noqa: F401
+    from tgis_b200 import ops_seq
+    g = torch.Generator(device=DEV).manual_seed(d + sum(new))
+    L = [s + n for s, n in zip(past, new)]
+    pages = [(n + 15) // 16 for n in L]
+    blocks = sum(pages) + 3
+    perm = torch.randperm(blocks, generator=g, device=DEV).int()
+    spare = perm[-1]
+    table, at = torch.full((len(new), max(pages) + 2), int(spare), dtype=torch.int32, device=DEV), 0
+    seen = torch.zeros(blocks, 16, dtype=torch.bool, device=DEV)
+    for b, n in enumerate(pages):
+        p = past[b]
+        lo = max(p // chunk * chunk if chunk else 0, p - window + 1 if window else 0)
+        first = lo // 16
+        table[b, first:n] = perm[at + first:at + n]
+        at += n
+        j = torch.arange(lo, L[b], device=DEV)
+        seen[table[b, j // 16].long(), j % 16] = True
+    cache = torch.randn(blocks, 16, 2 * G * d, generator=g, device=DEV).bfloat16()
+    q = torch.randn(sum(new), H, d, generator=g, device=DEV)
+    pos = torch.cat([torch.arange(s, e, device=DEV) for s, e in zip(past, L)])
+    cu = torch.tensor([0] + new, device=DEV).cumsum(0).int()
+    seq = torch.repeat_interleave(torch.arange(len(new), device=DEV, dtype=torch.int32), torch.tensor(new, device=DEV))
+    step = ops_seq.RaggedStep(T=sum(new), B=len(new), position_ids=pos, cu_q=cu, seq_of_token=seq, slot_mapping=pos, block_table=table, state_slots=None)
+
+    def run(c):
+        return ops_seq.talk_attn(q, c, step, kv_heads=G, vdim=d, k_off=0, v_off=G * d, scale=d ** -0.5, chunk=chunk, window=window)
+
+    clean = run(cache)
+    assert bool(clean.isfinite().all())
+    for bad in (math.nan, math.inf):
+        assert torch.equal(run(torch.where(seen[..., None], cache, torch.full_like(cache, bad))), clean)

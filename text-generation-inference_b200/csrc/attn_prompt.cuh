@@ -28,7 +28,9 @@
 // 287: the softmax warps are then compiled for 128 registers).
 // Token-major caches differ in this: a tile is 128 / rep tokens x the rep query heads of a key head (all rows meet the same keys), an item two
 // neighbouring tiles; the softmax warps bring their tile's fp32 queries as bfloat16 themselves; P is bfloat16; key tiles start at the first
-// visible key; and a key or value page is a box [16 tokens x 64 columns] that the copy itself swizzles.
+// visible key; a key or value page is a box [16 tokens x 64 columns] that the copy itself swizzles; and what lies in the cache beside the keys
+// that an item's queries see (slots that were never written, another request's leavings) is zeros to the products: whole pages by copies from
+// outside the cache's rows, the rest of the first and the last visible page by the issuing warp, at most 15 rows each.
 #pragma once
 #include "common.cuh"
 #include "seq_common.cuh"
@@ -88,6 +90,7 @@ struct PfParams {
 struct PfItem {
   int b, q_begin, past, last_page, kv_head;
   int q0[2], rows[2], head[2], k0[2], n_kt[2], j0, n;  // key tiles k0 .. n_kt - 1 of each, j0 .. n - 1 of both
+  int lo, hi;  // token-major: first and last key that a query of the item sees
 };
 
 // first key that the query at position p sees
@@ -112,7 +115,6 @@ __device__ __forceinline__ PfItem pf_item(const PfParams& p, int i) {
     it.q_begin = p.cu_q[it.b];
     const int n_q = p.cu_q[it.b + 1] - it.q_begin;
     it.past = (int)p.position_ids[it.q_begin];
-    it.last_page = (it.past + n_q - 1) / kPageTokens;
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       it.head[u] = it.kv_head * p.rep;
@@ -125,6 +127,8 @@ __device__ __forceinline__ PfItem pf_item(const PfParams& p, int i) {
     }
     it.j0 = it.n_kt[1] > 0 ? min(it.k0[0], it.k0[1]) : it.k0[0];
     it.n = max(it.n_kt[0], it.n_kt[1]);
+    it.lo = pf_first_visible(it.past + it.q0[0], p.chunk, p.window);
+    it.hi = it.past + min(n_q, it.q0[1] + p.tokens) - 1;
     return it;
   }
   // longest query tiles first
@@ -134,6 +138,7 @@ __device__ __forceinline__ PfItem pf_item(const PfParams& p, int i) {
   const int n_q = p.cu_q[it.b + 1] - it.q_begin, L = p.context_lens[it.b];
   it.past = max(L - n_q, 0);  // cached tokens in front of this step's first query
   it.last_page = (L - 1) / kPageTokens;
+  it.lo = it.hi = 0;
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     it.head[u] = p.pair_heads ? 2 * unit + u : unit;
@@ -205,6 +210,14 @@ __device__ __forceinline__ uint64_t umma_desc_mnmajor_sw128(uint32_t smem_addr, 
   d |= (uint64_t)1 << 46;
   d |= (uint64_t)2 << 61;
   return d;
+}
+
+// rows from .. to - 1 (if any) of a K or V tile become zeros; the whole warp calls it, and fences before the tensor cores read them
+template <int SLABS>
+__device__ __forceinline__ void pf_zero_rows(unsigned char* tile, int from, int to, int lane) {
+  for (int i = from * 8 + lane; i < to * 8; i += 32)
+#pragma unroll
+    for (int s = 0; s < SLABS; ++s) *reinterpret_cast<uint4*>(tile + s * kPfSlabBytes + i * 16) = make_uint4(0u, 0u, 0u, 0u);
 }
 
 template <int D, bool TOKEN_MAJOR>
@@ -298,10 +311,16 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         }
         const int32_t* bt = p.block_table + (int64_t)it.b * p.bt_stride;
         for (int j = it.j0; j < it.n; ++j) {
-          // 8 pages of this key tile, a lane each; pages past the sequence's last one repeat it (finite data, masked by the softmax warps)
-          const int page = min(j * (kPfN / kPageTokens) + (lane & 7), it.last_page);
-          // row of the pool viewed as [blocks * n_kv * 16, d], or of the token-major cache viewed as [blocks * 16, row width]
-          const int row = (TOKEN_MAJOR ? bt[page] : bt[page] * p.n_kv + it.kv_head) * kPageTokens;
+          // 8 pages of this key tile, a lane each
+          int page = j * (kPfN / kPageTokens) + (lane & 7), row;
+          if constexpr (TOKEN_MAJOR) {
+            // row of the cache viewed as [blocks * 16, row width]; a page without a visible key is not looked up (its entry may be any value):
+            // the copy then lies in front of the first row and brings zeros
+            row = page >= it.lo / kPageTokens && page <= it.hi / kPageTokens ? bt[page] * kPageTokens : -kPageTokens;
+          } else {
+            // row of the pool viewed as [blocks * n_kv * 16, d]; pages past the sequence's last one repeat it (masked by the softmax warps)
+            row = (bt[min(page, it.last_page)] * p.n_kv + it.kv_head) * kPageTokens;
+          }
           const int k_col = TOKEN_MAJOR ? p.k_off + it.kv_head * D : 0, v_col = TOKEN_MAJOR ? p.v_off + it.kv_head * D : 0;
           mbar_wait_soft(&k_empty[st], ph, ok);
           if (lane == 0) mbar_arrive_expect_tx(&k_full[st], C::kTileBytes);
@@ -370,7 +389,17 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         for (int j = it.j0 - 1; j < it.n; ++j) {  // P V of key tile j, Q K^T of key tile j + 1
           const bool more = j + 1 < it.n;
           if (more) mbar_wait_soft(&k_full[kst], kph, ok);
-          if (j >= it.j0) mbar_wait_soft(&v_full[vst], vph, ok);
+          if (j >= it.j0) {
+            mbar_wait_soft(&v_full[vst], vph, ok);
+            if constexpr (TOKEN_MAJOR) {
+              // value rows of the first and the last visible page that no query of the item sees: their weight is 0, but 0 x NaN is NaN
+              const int key0 = j * kPfN;
+              pf_zero_rows<C::kSlabs>(sV + vst * C::kTileBytes, max((it.lo & -kPageTokens) - key0, 0), min(it.lo - key0, kPfN), lane);
+              pf_zero_rows<C::kSlabs>(sV + vst * C::kTileBytes, max(it.hi + 1 - key0, 0), min((it.hi | (kPageTokens - 1)) + 1 - key0, kPfN), lane);
+              fence_proxy_async_smem();
+              __syncwarp();
+            }
+          }
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
             if (j >= it.k0[u] && j < it.n_kt[u]) {
