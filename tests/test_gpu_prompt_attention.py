@@ -74,3 +74,32 @@ def test_maxima_that_move(grow):
 @pytest.mark.parametrize("scale", [0.0, -0.1])
 def test_scales_that_are_not_positive(scale):
     _run([300, 20], 50, 4, 2, 64, scale, seed=5)
+
+
+def test_scores_of_minus_infinity():
+    """keys that a query must not weigh at all: a first key tile of nothing else, single ones among others; a query that sees no other key gives zeros"""
+    import tgis_b200  # noqa: F401
+    from tgis_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(6)
+    H, G, d, L = 4, 2, 64, 400
+    kp, vp = torch.randn(26, G, 16, d, generator=g, device=DEV).half(), torch.randn(26, G, 16, d, generator=g, device=DEV).half()
+    t, c = torch.arange(16, device=DEV)[:, None], torch.arange(d // 8, device=DEV)[None, :]
+    table = torch.randperm(26, generator=g, device=DEV).int()[None, :25].contiguous()
+    dead = torch.zeros(25 * 16, dtype=torch.bool, device=DEV)
+    dead[:150], dead[200], dead[300:310] = True, True, True
+    K = torch.randn(25 * 16, G, d, generator=g, device=DEV).half()
+    K[dead, :, 0] = -math.inf
+    kp[table[0].long()] = K.unflatten(0, (25, 16)).transpose(1, 2).unflatten(-1, (-1, 8))[..., t, c ^ (t & 7), :].flatten(-2)   # the swizzle is its own inverse
+    V = vp[table[0].long()].unflatten(-1, (-1, 8))[..., t, c ^ (t & 7), :].flatten(-2).transpose(1, 2).flatten(0, 1).double()
+    q = torch.randn(L, H, d, generator=g, device=DEV).half()
+    q[..., 0] = q[..., 0].abs() + 0.5
+    out = ops.attn_prefill_paged(q, kp, vp, table, torch.tensor([L], dtype=torch.int32, device=DEV), torch.tensor([0, L], dtype=torch.int32, device=DEV), L, 0.125)
+    assert bool((out[:150] == 0).all())
+    ok = (torch.arange(L, device=DEV)[None] <= torch.arange(L, device=DEV)[:, None]) & ~dead[None]
+    for h in range(H):
+        s = q[:, h].double() @ K[:, h * G // H].double().nan_to_num(neginf=0.0).T * 0.125
+        w = torch.softmax(s.masked_fill(~ok, -math.inf), 1)[150:]
+        ref, spread = w @ V[:, h * G // H], w @ V[:, h * G // H].abs()
+        top = s.abs().amax(1, keepdim=True)[150:]
+        tol = 2.0 ** -11 * ref.abs() + (2 * 2.0 ** -11 + 2 * d * 2.0 ** -24 * (1 + top)) * spread + 1e-6
+        assert bool(((out[150:, h].double() - ref).abs() <= tol).all())

@@ -528,7 +528,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         for (int k = 0; k < 4; ++k) mx4[k] = fmaxf(mx4[k], s[kPfN - 4 + k]);
         const float mx = fmaxf(max3(mx4[0], mx4[1], mx4[2]), mx4[3]) * scale;
         if (j == k0) {
-          m = TOKEN_MAJOR ? fmaxf(mx, -1.0e30f) : mx;  // (a row may meet its first visible key in a later tile)
+          m = fmaxf(mx, -1.0e30f);  // finite: a row may meet its first visible key, or its first score above -infinity, in a later tile
           if (TOKEN_MAJOR && p.sink) {  // one more logit of the denominator
             const float sk = p.sink[head + row % p.rep] * 1.4426950408889634f;
             m = fmaxf(m, sk);
