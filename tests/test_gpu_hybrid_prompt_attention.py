@@ -130,3 +130,51 @@ def test_what_no_query_sees_does_not_matter(d, H, G, new, past, chunk, window):
     assert bool(clean.isfinite().all())
     for bad in (math.nan, math.inf):
         assert torch.equal(run(torch.where(seen[..., None], cache, torch.full_like(cache, bad))), clean)
+
+
+def _fp32_case(H, G, d, new, seed):
+    """queries that bfloat16 does not hold; -> call, largest difference to float64, the same relative to the weighted mean of |v|"""
+    from tgis_b200 import ops_seq
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    pages = [(n + 15) // 16 for n in new]
+    table, at = torch.zeros(len(new), max(pages), dtype=torch.int32, device=DEV), 0
+    for b, n in enumerate(pages):
+        table[b, :n] = torch.arange(at, at + n, device=DEV, dtype=torch.int32)
+        at += n
+    cache = torch.randn(at, 16, 2 * G * d, generator=g, device=DEV).bfloat16()
+    q = torch.randn(sum(new), H, d, generator=g, device=DEV)
+    pos = torch.cat([torch.arange(n, device=DEV) for n in new])
+    seq = torch.repeat_interleave(torch.arange(len(new), device=DEV, dtype=torch.int32), torch.tensor(new, device=DEV))
+    step = ops_seq.RaggedStep(T=sum(new), B=len(new), position_ids=pos, cu_q=torch.tensor([0] + new, device=DEV).cumsum(0).int(), seq_of_token=seq,
+                              slot_mapping=pos, block_table=table, state_slots=None)
+    out = ops_seq.talk_attn(q, cache, step, kv_heads=G, vdim=d, k_off=0, v_off=G * d, scale=d ** -0.5).double()
+    worst, row = 0.0, 0
+    for b, n in enumerate(new):
+        rows = cache[table[b, :pages[b]].long()].flatten(0, 1)[:n].double()
+        K, V = rows[:, :G * d].unflatten(1, (G, d)).repeat_interleave(H // G, 1), rows[:, G * d:].unflatten(1, (G, d)).repeat_interleave(H // G, 1)
+        s = torch.einsum("nhd,lhd->hnl", q[row:row + n].double(), K) * d ** -0.5
+        w = torch.softmax(s.masked_fill(torch.arange(n, device=DEV)[None] > torch.arange(n, device=DEV)[:, None], -math.inf), -1)
+        ref, spread = torch.einsum("hnl,lhd->nhd", w, V), torch.einsum("hnl,lhd->nhd", w, V.abs())
+        worst = max(worst, float(((out[row:row + n] - ref).abs() / spread).max()))
+        row += n
+    return worst
+
+
+@pytest.mark.parametrize("H,G,d", [(16, 16, 128), (32, 16, 128), (24, 24, 64), (64, 16, 128), (32, 32, 64)])
+def test_shapes_that_are_computed_in_fp32(H, G, d):
+    """shapes that the m16n8k16 kernel does not take keep fp32 queries, weights and sums on the general kernel.  Bound: d 2^-24 of a score of size
+    up to ~6 (its error is the weight's relative one), and the sums over 150 keys"""
+    import tgis_b200  # noqa: F401
+    assert _fp32_case(H, G, d, [150, 40], H + d) < (6 * d + 150) * 2.0 ** -24 * 2
+
+
+def test_the_switch_for_fp32():
+    """B200_SEQ_ATTN_MMA=0 selects the fp32 form for prompts as well (read once per process: a process of its own)"""
+    import os
+    import subprocess
+    import sys
+    code = "import torch, tests.test_gpu_hybrid_prompt_attention as t; import tgis_b200; print(t._fp32_case(16, 4, 128, [150, 40], 1))"
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    worst = [float(subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, B200_SEQ_ATTN_MMA=v), check=True, capture_output=True, text=True).stdout)
+             for v in ("0", "1")]
+    assert worst[0] < (6 * 128 + 150) * 2.0 ** -24 * 2 < worst[1]

@@ -724,12 +724,15 @@ extern "C" int b200_seq_talk_attn_splits(int dt, int64_t T, int B, int H, int G,
 // Prompts without a mix take the tcgen05 kernel: tiles of 128 (token, head) rows, so it wants steps of enough tokens per sequence to fill them.
 // Measured on B200 (us, the m16n8k16 kernel / this one; 16 / 4 heads, d = 128): 2118 + 1882 tokens in chunks of 2048 387 / 94, 4 x 512 84 / 25, 300 after
 // 800 cached 51 / 35, 4 x 40 after 500 38 / 26, 4 x 24 after 1900 56 / 43, 24 after 20 24.5 / 14.3; 4 x 16 after 1900 55 / 53, 4 x 8 48 / 50.
-// What it needs beside that: heads of 64 or 128 columns, whole 128-row tiles (128 % (heads / kv_heads) == 0), pages of 16 tokens, and 16-byte pieces.
+// What it needs beside that: heads of 64 or 128 columns, whole 128-row tiles (128 % (heads / kv_heads) == 0), pages of 16 tokens, and 16-byte pieces; and a
+// shape that talk_mma_plan accepts: those rounded queries and weights to bfloat16 before, the others (at d = 128: 16 / 16, 32 / 32, 32 / 16, 64 / 16 ... heads,
+// and everything under B200_SEQ_ATTN_MMA=0) are computed in fp32 and stay so.
 constexpr int kTalkPromptTokens = 24;  // average tokens per sequence from which on
 
 static bool talk_prompt_route(const void* q, const void* cache, int dt, int64_t RW, int k_off, int v_off, const int32_t* cu_q, const float* talk,
                               const void* out, int64_t T, int B, int H, int G, int d, int dv, int page) {
   const int rep = H / G;
+  if (talk_mma_plan(dt, T, B, H, G, d, dv, false).QT == 0) return false;
   return dt == B200_DT_BF16 && talk == nullptr && cu_q != nullptr && B > 0 && T >= (int64_t)kTalkPromptTokens * B && (d == 64 || d == 128) && dv == d &&
          page == b200::kPageTokens && rep <= 128 && 128 % rep == 0 && RW % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0 && T <= (1 << 24) &&
          ((reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
