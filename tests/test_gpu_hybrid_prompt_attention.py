@@ -132,8 +132,8 @@ def test_what_no_query_sees_does_not_matter(d, H, G, new, past, chunk, window):
         assert torch.equal(run(torch.where(seen[..., None], cache, torch.full_like(cache, bad))), clean)
 
 
-def _fp32_case(H, G, d, new, seed):
-    """queries that bfloat16 does not hold; -> call, largest difference to float64, the same relative to the weighted mean of |v|"""
+def _fp32_case(H, G, d, new, seed, held=False):
+    """queries that bfloat16 does not hold (`held`: that it does); -> call, largest difference to float64, the same relative to the weighted mean of |v|"""
     from tgis_b200 import ops_seq
     g = torch.Generator(device=DEV).manual_seed(seed)
     pages = [(n + 15) // 16 for n in new]
@@ -143,6 +143,7 @@ def _fp32_case(H, G, d, new, seed):
         at += n
     cache = torch.randn(at, 16, 2 * G * d, generator=g, device=DEV).bfloat16()
     q = torch.randn(sum(new), H, d, generator=g, device=DEV)
+    q = q.bfloat16().float() if held else q
     pos = torch.cat([torch.arange(n, device=DEV) for n in new])
     seq = torch.repeat_interleave(torch.arange(len(new), device=DEV, dtype=torch.int32), torch.tensor(new, device=DEV))
     step = ops_seq.RaggedStep(T=sum(new), B=len(new), position_ids=pos, cu_q=torch.tensor([0] + new, device=DEV).cumsum(0).int(), seq_of_token=seq,
@@ -166,6 +167,13 @@ def test_shapes_that_are_computed_in_fp32(H, G, d):
     up to ~6 (its error is the weight's relative one), and the sums over 150 keys"""
     import tgis_b200  # noqa: F401
     assert _fp32_case(H, G, d, [150, 40], H + d) < (6 * d + 150) * 2.0 ** -24 * 2
+
+
+@pytest.mark.parametrize("H,G,d", [(16, 4, 128), (8, 2, 64), (32, 8, 128)])
+def test_weights_are_not_rounded_to_bfloat16(H, G, d):
+    """queries that bfloat16 holds leave the weights as the only 16-bit operand: two bfloat16 values each, 2^-17 off, beside the fp32 terms above"""
+    import tgis_b200  # noqa: F401
+    assert _fp32_case(H, G, d, [300, 40], d, held=True) < 2 * 2.0 ** -17 + (6 * d + 300) * 2.0 ** -24 * 2
 
 
 def test_the_switch_for_fp32():

@@ -27,7 +27,9 @@
 // 294 at the first of these.  Tried: four more warps for the output (305 instead of
 // 287: the softmax warps are then compiled for 128 registers).
 // Token-major caches differ in this: a tile is 128 / rep tokens x the rep query heads of a key head (all rows meet the same keys), an item two
-// neighbouring tiles; the softmax warps bring their tile's fp32 queries as bfloat16 themselves; P is bfloat16; key tiles start at the first
+// neighbouring tiles; the softmax warps bring their tile's fp32 queries as bfloat16 themselves; P is the sum of two bfloat16 values (one alone is 2^-9
+// off, and a maximum taken over 128 keys leaves fewer weights at exactly 1 than the 16-key tiles of talk_attn_mma_kernel: prompts of 1882 and 2118 tokens,
+// 16 / 4 heads, d = 128, against float64 1.91e-3 with one value, 1.88e-3 there, 1.47e-3 with two; 90 us, 343 there, 101); key tiles start at the first
 // visible key; a key or value page is a box [16 tokens x 64 columns] that the copy itself swizzles; and what lies in the cache beside the keys
 // that an item's queries see (slots that were never written, another request's leavings) is zeros to the products: whole pages by copies from
 // outside the cache's rows, the rest of the first and the last visible page by the issuing warp, at most 15 rows each.
@@ -410,8 +412,11 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
                 tcgen05_fence_after();
                 if (elect_one()) {
 #pragma unroll
-                  for (int kk = h * 4; kk < h * 4 + 4; ++kk)  // 16 keys = 2 swizzle atoms of 8 key rows = 2048 bytes per step
+                  for (int kk = h * 4; kk < h * 4 + 4; ++kk) {  // 16 keys = 2 swizzle atoms of 8 key rows = 2048 bytes per step
                     umma_f16_ts(tmem_base + 256 + u * D, tmem_base + u * kPfN + kk * 8, b + (uint64_t)((kk * 2048) >> 4), idesc_pv, (j > it.k0[u] || kk > 0) ? 1u : 0u);
+                    if constexpr (TOKEN_MAJOR)  // the weights' second halves
+                      umma_f16_ts(tmem_base + 256 + u * D, tmem_base + u * kPfN + kPfN / 2 + kk * 8, b + (uint64_t)((kk * 2048) >> 4), idesc_pv, 1u);
+                  }
                   if (h == 1 && j == it.n_kt[u] - 1) umma_commit(&o_full[u]);
                 }
                 __syncwarp();
@@ -557,15 +562,18 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         const uint64_t scale2 = f32x2(scale, scale), neg_m = f32x2(-m, -m);
 #pragma unroll
         for (int h = 0; h < kPfN / 32; ++h) {
-          uint32_t pk[16];
+          uint32_t pk[16], rest[TOKEN_MAJOR ? 16 : 1];
 #pragma unroll
           for (int c = 0; c < 32; c += 2) {
             float a, b;
             f32x2_split(fma_f32x2(f32x2(s[h * 32 + c], s[h * 32 + c + 1]), scale2, neg_m), a, b);
             if constexpr (TOKEN_MAJOR) {
-              pk[c / 2] = pack_bf16x2(fast_exp2(a), fast_exp2(b));
-              sum[0] += __uint_as_float(pk[c / 2] << 16);
-              sum[1] += __uint_as_float(pk[c / 2] & 0xffff0000u);
+              a = fast_exp2(a);
+              b = fast_exp2(b);
+              pk[c / 2] = pack_bf16x2(a, b);
+              rest[c / 2] = pack_bf16x2(a - __uint_as_float(pk[c / 2] << 16), b - __uint_as_float(pk[c / 2] & 0xffff0000u));
+              sum[0] += a;
+              sum[1] += b;
             } else {
               pk[c / 2] = pack_half2(fast_exp2(a), fast_exp2(b));
               sum[0] = add_f32_f16(sum[0], (uint16_t)pk[c / 2]);
@@ -573,6 +581,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             }
           }
           tmem_st_32x32b_x16(tmem_s + h * 16, pk);
+          if constexpr (TOKEN_MAJOR) tmem_st_32x32b_x16(tmem_s + kPfN / 2 + h * 16, rest);
           if (h & 1) {  // half of P: its products run under the exponentials of the other half
             tmem_st_wait();
             tcgen05_fence_before();
