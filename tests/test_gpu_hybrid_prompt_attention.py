@@ -186,3 +186,10 @@ def test_the_switch_for_fp32():
     worst = [float(subprocess.run([sys.executable, "-c", code], cwd=root, env=dict(os.environ, B200_SEQ_ATTN_MMA=v), check=True, capture_output=True, text=True).stdout)
              for v in ("0", "1")]
     assert worst[0] < (6 * 128 + 150) * 2.0 ** -24 * 2 < worst[1]
+
+
+@pytest.mark.parametrize("new,H,G", [([600, 500], 16, 4), ([560, 600], 16, 4), ([31, 33, 64, 65, 1, 96], 16, 4), ([40] * 11, 8, 8), ([40] * 9, 8, 8)])
+def test_around_one_tile_per_sm(new, H, G):
+    """steps whose tiles each have an item to themselves, and steps just above that"""
+    _run(new, 0, H, G, 64, seed=10)
+    _run(new, 100, H, G, 64, chunk=256, seed=11)

@@ -103,3 +103,10 @@ def test_scores_of_minus_infinity():
         top = s.abs().amax(1, keepdim=True)[150:]
         tol = 2.0 ** -11 * ref.abs() + (2 * 2.0 ** -11 + 2 * d * 2.0 ** -24 * (1 + top)) * spread + 1e-6
         assert bool(((out[150:, h].double() - ref).abs() <= tol).all())
+
+
+@pytest.mark.parametrize("lens,H,G", [([100] * 4, 37, 37), ([100] * 3, 50, 50), ([100] * 5, 30, 15), ([130, 20], 36, 12), ([130, 20], 38, 38), ([1], 71, 1), ([300], 32, 8)])
+def test_around_one_tile_per_sm(lens, H, G):
+    """up to 148 tiles each has an item to itself; above, items are two tiles: two heads, or two query tiles"""
+    _run(lens, 0, H, G, 64, 0.125, seed=7)
+    _run(lens, 200, H, G, 64, 0.125, seed=8)

@@ -41,10 +41,10 @@ static int launch_prefill_paged(const void* q, int64_t q_stride, int64_t T_q, co
   p.n_kv = n_kv;
   p.B = B;
   // two heads of a key / value head are equally long and share their keys; neighbouring query tiles are not, and a short prompt has no second one
-  p.pair_heads = (n_heads / n_kv) % 2 == 0;
-  p.n_units = p.pair_heads ? n_heads / 2 : n_heads;
   const int tiles = (max_q + kPfM - 1) / kPfM;
-  p.n_groups = p.pair_heads ? tiles : (tiles + 1) / 2;
+  p.pair = (int64_t)B * tiles * n_heads <= pf_num_sms() ? kPfSingle : (n_heads / n_kv) % 2 == 0 ? kPfHeads : kPfTiles;
+  p.n_units = p.pair == kPfHeads ? n_heads / 2 : n_heads;
+  p.n_groups = p.pair == kPfTiles ? (tiles + 1) / 2 : tiles;
   p.scale_log2 = scale * 1.4426950408889634f;
   const int64_t items = (int64_t)p.n_units * p.n_groups * B;
   if (items > (1 << 30)) { b200_set_last_error("attn_prefill_paged: too many query tiles"); return B200_ERR_ARG; }

@@ -6,7 +6,9 @@
 // Design (12 warps, one CTA per SM).  A block takes its own item and then those of blocks that have not started (cluster launch control), longest
 // first: with items dealt out in turn the SMs were busy for 75 % of the time on ragged prompts.  An item is TWO query tiles of 128 rows that meet the same keys, so that the tensor cores work for
 // one while the other is in its soft-max: two query heads of a key / value head when their number is even, else two neighbouring query tiles
-// of a head.
+// of a head.  While every tile can have an SM to itself it does (the second tile of an item is empty): two soft-max warpgroups slow each
+// other down.  Back to back, us, one query tile of one head per CTA / two / this:
+// one prompt of 100 tokens, 32 / 8 heads, d = 128 6.8 / 8.0 / 6.8, of 300 11.2 / 12.3 / 10.7; 32 / 4 heads, d = 64, 129 tokens 7.1 / 8.2 / 6.8.
 //   warp 0      TMA producer.  Q tiles [128 x d] through a 128B-swizzled tensor map; per 128-key tile 8 KV pages x (K, V) x d/64
 //               slabs, each one cp.async.bulk.tensor box [16 tokens x 64 halves] of the pool: the pool stores every token row
 //               with its 16-byte chunks XOR-swizzled by (token & 7), which IS the tcgen05 SWIZZLE_128B image, so
@@ -68,6 +70,9 @@ struct PfCfg {
   static constexpr int kTmemCols = 512;  // S0 [0,128) | S1 [128,256) | O0 [256, 256 + D) | O1 behind it
 };
 
+// two tiles of an item: two query heads, two neighbouring query tiles, or the second one is empty
+enum PfPair { kPfHeads, kPfTiles, kPfSingle };
+
 struct PfParams {
   const int32_t* block_table;
   int64_t bt_stride;
@@ -76,7 +81,7 @@ struct PfParams {
   void* out;
   int64_t out_stride;
   int n_heads, n_kv, B;
-  int pair_heads;        // 1: an item is two heads, 0: two query tiles
+  int pair;              // what an item's two tiles are (PfPair)
   int n_units, n_groups; // head (pair)s, query tile (pair)s of the longest sequence
   int more_blocks;       // the grid is larger than the GPU: blocks take more items
   float scale_log2;
@@ -109,8 +114,9 @@ __device__ __forceinline__ PfItem pf_item(const PfParams& p, int i) {
   if constexpr (TOKEN_MAJOR) {
     // two neighbouring tiles of `tokens` tokens x `rep` heads of a key head; last tiles of the step first
     int tile = p.n_groups - 1 - i / p.n_units;
+    const int span = p.pair == kPfSingle ? p.tokens : 2 * p.tokens;  // tokens of an item
     it.kv_head = i % p.n_units;
-    seq::find_ragged_tile(p.cu_q, p.B, 1, 2 * p.tokens, it.b, tile);
+    seq::find_ragged_tile(p.cu_q, p.B, 1, span, it.b, tile);
     it.n = it.j0 = 0;
     it.n_kt[0] = it.n_kt[1] = it.k0[0] = it.k0[1] = 0;
     if (it.b >= p.B) return it;
@@ -120,8 +126,8 @@ __device__ __forceinline__ PfItem pf_item(const PfParams& p, int i) {
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       it.head[u] = it.kv_head * p.rep;
-      it.q0[u] = (2 * tile + u) * p.tokens;
-      it.rows[u] = min(p.tokens, n_q - it.q0[u]) * p.rep;
+      it.q0[u] = tile * span + u * p.tokens;
+      it.rows[u] = min(min(p.tokens, span - u * p.tokens), n_q - it.q0[u]) * p.rep;
       if (it.rows[u] > 0) {
         it.k0[u] = pf_first_visible(it.past + it.q0[u], p.chunk, p.window) / kPfN;
         it.n_kt[u] = (it.past + it.q0[u] + it.rows[u] / p.rep - 1) / kPfN + 1;
@@ -130,7 +136,7 @@ __device__ __forceinline__ PfItem pf_item(const PfParams& p, int i) {
     it.j0 = it.n_kt[1] > 0 ? min(it.k0[0], it.k0[1]) : it.k0[0];
     it.n = max(it.n_kt[0], it.n_kt[1]);
     it.lo = pf_first_visible(it.past + it.q0[0], p.chunk, p.window);
-    it.hi = it.past + min(n_q, it.q0[1] + p.tokens) - 1;
+    it.hi = it.past + min(n_q, it.q0[0] + span) - 1;
     return it;
   }
   // longest query tiles first
@@ -143,9 +149,9 @@ __device__ __forceinline__ PfItem pf_item(const PfParams& p, int i) {
   it.lo = it.hi = 0;
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
-    it.head[u] = p.pair_heads ? 2 * unit + u : unit;
-    it.q0[u] = (p.pair_heads ? group : 2 * group + u) * kPfM;
-    it.rows[u] = min(kPfM, n_q - it.q0[u]);
+    it.head[u] = p.pair == kPfHeads ? 2 * unit + u : unit;
+    it.q0[u] = (p.pair == kPfTiles ? 2 * group + u : group) * kPfM;
+    it.rows[u] = u == 1 && p.pair == kPfSingle ? 0 : min(kPfM, n_q - it.q0[u]);
     it.k0[u] = 0;
     it.n_kt[u] = it.rows[u] > 0 ? (it.past + it.q0[u] + it.rows[u] - 1) / kPfN + 1 : 0;  // key tiles the last row reaches
   }

@@ -770,7 +770,8 @@ static int launch_talk_prompt(const float* q, const void* cache, int64_t RW, int
   p.rep = H / G;
   p.tokens = 128 / p.rep;
   p.n_units = G;
-  p.n_groups = (int)(T / (2 * p.tokens)) + B;  // upper bound of sum_b ceil(n_b / (2 tokens)); surplus items are passed over
+  p.pair = G * (T / p.tokens + B) <= b200::pf_num_sms() ? b200::kPfSingle : b200::kPfTiles;
+  p.n_groups = (int)(T / (p.pair == b200::kPfSingle ? p.tokens : 2 * p.tokens)) + B;  // upper bound of sum_b ceil(n_b / tokens); surplus items are passed over
   p.scale_log2 = scale * 1.4426950408889634f;
   const int64_t items = (int64_t)p.n_units * p.n_groups;
   p.more_blocks = items > b200::pf_num_sms();
