@@ -110,3 +110,29 @@ def test_around_one_tile_per_sm(lens, H, G):
     """up to 148 tiles each has an item to itself; above, items are two tiles: two heads, or two query tiles"""
     _run(lens, 0, H, G, 64, 0.125, seed=7)
     _run(lens, 200, H, G, 64, 0.125, seed=8)
+
+
+@pytest.mark.parametrize("spread", [0.3, 1.0, 3.0])
+def test_the_largest_weight_is_exact(spread):
+    """behind 1500 keys the result is no further from float64 than weights in fp16 must be: the largest one of a row is exactly 1, all others are
+    rounded once.  The bound is that of the same sums with weights rounded so, and its half percent for fp32 scores, sums and exponentials"""
+    import tgis_b200  # noqa: F401
+    from tgis_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(9)
+    H, G, d, n, L = 16, 4, 128, 200, 1700
+    pages = (L + 15) // 16
+    kp, vp = torch.randn(pages, G, 16, d, generator=g, device=DEV).half(), torch.randn(pages, G, 16, d, generator=g, device=DEV).half()
+    q = (torch.randn(n, H, d, generator=g, device=DEV) * spread).half()
+    table = torch.arange(pages, device=DEV, dtype=torch.int32)[None].contiguous()
+    out = ops.attn_prefill_paged(q, kp, vp, table, torch.tensor([L], dtype=torch.int32, device=DEV), torch.tensor([0, n], dtype=torch.int32, device=DEV), n, d ** -0.5)
+    t, c = torch.arange(16, device=DEV)[:, None], torch.arange(d // 8, device=DEV)[None, :]
+    K, V = (p.unflatten(-1, (-1, 8))[..., t, c ^ (t & 7), :].flatten(-2).transpose(1, 2).flatten(0, 1)[:L].double() for p in (kp, vp))
+    ok = torch.arange(L, device=DEV)[None] <= L - n + torch.arange(n, device=DEV)[:, None]
+    got = must = 0.0
+    for h in range(H):
+        s = (q[:, h].double() @ K[:, h * G // H].T * d ** -0.5).masked_fill(~ok, -math.inf)
+        w = torch.exp(s - s.amax(1, keepdim=True))
+        ref, rounded = w @ V[:, h * G // H] / w.sum(1, keepdim=True), w.half().double()
+        best = (rounded @ V[:, h * G // H] / rounded.sum(1, keepdim=True)).half().double()
+        got, must = got + float((out[:, h].double() - ref).square().sum()), must + float((best - ref).square().sum())
+    assert (got / must) ** 0.5 < 1.005, (got / must) ** 0.5

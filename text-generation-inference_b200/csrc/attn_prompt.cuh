@@ -19,7 +19,9 @@
 //               shared-memory operand (keys are the MMA K dimension, d contiguous), accumulator O in TMEM.
 //   warps 4..7, 8..11   softmax of the first and the second tile: thread = one query row = one TMEM lane (no shuffles).  tcgen05.ld S, causal
 //               mask, fp32 online softmax in the log2 domain, P rounded to fp16 (flash-attn semantics) and stored back to TMEM, O
-//               rescaled in TMEM when a row's reference maximum moves (kPfExactTiles, kPfRescale).  The row's sum adds the rounded P, what the
+//               rescaled in TMEM when a row's maximum moves.  (The reference always is the maximum: one that lags until it is 2^8 behind saves
+//               3 % (272 us where this takes 280, 13 prompts of 300 to 2048 tokens), but a largest weight that is not exactly 1 is rounded, up to 7 % more error behind
+//               1500 cached keys whose scores spread.)  The row's sum adds the rounded P, what the
 //               products weigh.  S of tile j is complete only after P V of tile j - 1 (issue order), so O is quiescent whenever a
 //               softmax warp runs.
 // Causality over absolute positions prunes whole key tiles.  Bound: soft-max exponentials (MUFU, 16 a cycle and SM: 1024 cycles per 128 x 128 tile,
@@ -49,12 +51,6 @@ constexpr int kPfPageSlabBytes = kPageTokens * 128;
 constexpr int kPfCornerBytes = 32 * 128;  // a softmax warp's rows on their way out
 constexpr int kPfStages = 2;
 constexpr int kPfAhead = 2;      // items that are known ahead
-// The reference maximum of a row follows the true one through the first key tiles after the first; later it moves only when the maximum has grown
-// past it by more than 2^8.  A largest weight of exactly 1 is worth some precision (against float64, over prompts of 64 to 2500 keys: 0.993 of
-// the error of following it always with unrounded sums, 1.006 with no exact tiles), following it always costs 323 us where this takes 306.
-// (bfloat16 weights, the token-major caches': always followed.)
-constexpr int kPfExactTiles = 4;
-constexpr float kPfRescale = 8.f;  // log2
 // registers per thread: the launch has 384 x 168; the two softmax warpgroups take 216 each, the other one keeps 72
 constexpr int kPfSoftmaxRegs = 216, kPfServeRegs = 72;
 
@@ -546,7 +542,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             sum[0] = fast_exp2(sk - m);
           }
         } else {
-          const bool grew = mx > m + (TOKEN_MAJOR || j <= kPfExactTiles ? 0.f : kPfRescale);
+          const bool grew = mx > m;
           if (__any_sync(0xffffffffu, grew)) {
             const float alpha = grew ? fast_exp2(m - mx) : 1.f;
             if (grew) m = mx;
