@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-def _run(new, past, H, G, d, chunk=0, window=0, sink=None, page=16, dv=None, pad=0, seed=0, key_scale=1.0):
+def _run(new, past, H, G, d, chunk=0, window=0, sink=None, page=16, dv=None, pad=0, seed=0, key_scale=1.0, width=0):
     import tgis_b200  # noqa: F401
     from tgis_b200 import ops_seq
     g = torch.Generator(device=DEV).manual_seed(seed)
@@ -22,7 +22,7 @@ def _run(new, past, H, G, d, chunk=0, window=0, sink=None, page=16, dv=None, pad
     L = [s + n for s, n in zip(starts, new)]
     pages = [(n + page - 1) // page for n in L]
     perm = torch.randperm(sum(pages) + 2, generator=g, device=DEV).int()
-    table, at = torch.zeros(len(new), max(pages), dtype=torch.int32, device=DEV), 0
+    table, at = torch.zeros(len(new), max(max(pages), width), dtype=torch.int32, device=DEV), 0
     for b, n in enumerate(pages):
         table[b, :n] = perm[at:at + n]
         at += n
@@ -193,3 +193,13 @@ def test_around_one_tile_per_sm(new, H, G):
     """steps whose tiles each have an item to themselves, and steps just above that"""
     _run(new, 0, H, G, 64, seed=10)
     _run(new, 100, H, G, 64, chunk=256, seed=11)
+
+
+@pytest.mark.parametrize("chunk,window,sink", [(0, 0, False), (512, 0, True), (0, 300, False)])
+def test_few_queries_over_a_long_cache(chunk, window, sink):
+    """the same steps on both sides of the rule that leaves few items over many keys to the kernel that cuts the keys into runs (the host takes the
+    block table's width for the number of keys)"""
+    s = torch.linspace(-2, 2, 8, device=DEV) if sink else None
+    for width in (0, 4000):
+        _run([64, 24], [3000, 700], 8, 2, 64, chunk=chunk, window=window, sink=s, seed=12, width=width)
+        _run([30], [5000], 8, 2, 128, chunk=chunk, window=window, sink=s, seed=13, width=width)

@@ -729,13 +729,37 @@ extern "C" int b200_seq_talk_attn_splits(int dt, int64_t T, int B, int H, int G,
 // and everything under B200_SEQ_ATTN_MMA=0) are computed in fp32 and stay so.
 constexpr int kTalkPromptTokens = 24;  // average tokens per sequence from which on
 
+//
+// And few items over many keys are a matter of latency: the m16n8k16 kernel cuts the keys into runs then, this one does not.  `keys`: a bound of
+// the keys that a query sees, as far as the host knows it (the block table's width, a chunk, a window).  Models of both, from 80 steps measured on
+// B200.  Us, m16n8k16 / this one, no chunk, no window: 16 / 4 heads of 128, 24 tokens behind 2000 keys 56 / 51, behind 30 000 454 / 475, 200 behind 8000 181 /
+// 145; 8 / 2 heads of 64, 24 behind 500 36 / 27, 64 behind 8000 77 / 141, 500 behind 8000 103 / 150; 16 / 8 heads of 64, 24 x 16 sequences behind 4000 108 / 127, a
+// prompt of 4000 beside 100 single tokens behind 1500 527 / 248.
+static bool talk_prompt_pays(int64_t T, int B, int H, int G, int d, int dv, int64_t keys, int QT, int nsplit) {
+  const int tokens = 128 / (H / G), sms = b200::pf_num_sms();
+  const int64_t row = 2ll * G * (d + dv), single = G * (T / tokens + B), items = single <= sms ? single : G * (T / (2 * tokens) + B);
+  // us per key of the item that the SM is at; the memory's rate for pieces of 2 d bytes
+  const float per_key = items == single ? (d == 128 ? 0.016f : 0.0125f) : (d == 128 ? 0.020f : 0.0156f);
+  const float chain = per_key * keys * (items > sms ? (float)items / sms : 1.f), memory = (float)B * keys * row / (d * 0.03e6f);
+  const float here = 15.f + fmaxf(chain, memory);
+  const float blocks = (float)((T + QT - 1) / QT) * nsplit / (2 * sms);
+  const float there = 30.f + (0.0007f * d + 0.000016f * row) * keys / nsplit * (blocks > 1.f ? blocks : 1.f);
+  return here <= there;
+}
+
 static bool talk_prompt_route(const void* q, const void* cache, int dt, int64_t RW, int k_off, int v_off, const int32_t* cu_q, const float* talk,
-                              const void* out, int64_t T, int B, int H, int G, int d, int dv, int page) {
+                              const void* out, int64_t T, int B, int H, int G, int d, int dv, int page, int64_t bt_stride, int chunk, int window, int nsplit) {
   const int rep = H / G;
-  if (talk_mma_plan(dt, T, B, H, G, d, dv, false).QT == 0) return false;
-  return dt == B200_DT_BF16 && talk == nullptr && cu_q != nullptr && B > 0 && T >= (int64_t)kTalkPromptTokens * B && (d == 64 || d == 128) && dv == d &&
+  const TalkPlan plan = talk_mma_plan(dt, T, B, H, G, d, dv, false);
+  if (plan.QT == 0) return false;
+  const bool takes = dt == B200_DT_BF16 && talk == nullptr && cu_q != nullptr && B > 0 && T >= (int64_t)kTalkPromptTokens * B && (d == 64 || d == 128) && dv == d &&
          page == b200::kPageTokens && rep <= 128 && 128 % rep == 0 && RW % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0 && T <= (1 << 24) &&
          ((reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  if (!takes) return false;
+  int64_t keys = bt_stride * page;
+  if (chunk > 0 && chunk < keys) keys = chunk;
+  if (window > 0 && window + 128 < keys) keys = window + 128;
+  return talk_prompt_pays(T, B, H, G, d, dv, keys, plan.QT, nsplit);
 }
 
 template <int D>
@@ -793,7 +817,9 @@ extern "C" int b200_seq_talk_attn(const float* q, const void* cache, int dt, int
     return B200_ERR_ARG;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  if (talk_prompt_route(q, cache, dt, row_width, k_off, v_off, cu_q, talk, out, T, B, H, G, d, dv, page)) {
+  if (!partial || nsplit < 1) nsplit = 1;
+  if (nsplit > 8) nsplit = 8;
+  if (talk_prompt_route(q, cache, dt, row_width, k_off, v_off, cu_q, talk, out, T, B, H, G, d, dv, page, bt_stride, chunk, window, nsplit)) {
     if (d == 128)
       return launch_talk_prompt<128>(q, cache, row_width, k_off, v_off, block_table, bt_stride, cu_q, B, position_ids, out, T, H, G, chunk, window, scale, sink, st);
     return launch_talk_prompt<64>(q, cache, row_width, k_off, v_off, block_table, bt_stride, cu_q, B, position_ids, out, T, H, G, chunk, window, scale, sink, st);
@@ -801,8 +827,6 @@ extern "C" int b200_seq_talk_attn(const float* q, const void* cache, int dt, int
   const TalkPlan plan = talk_mma_plan(dt, T, B, H, G, d, dv, talk != nullptr);
   if (plan.QT > 0 && cu_q != nullptr && row_width % 8 == 0 && k_off % 8 == 0 && v_off % 8 == 0 && (reinterpret_cast<uintptr_t>(cache) & 15) == 0) {
     const int64_t tiles = (T + plan.QT - 1) / plan.QT + B;  // upper bound of sum_b ceil(n_b / QT); surplus blocks return at once
-    if (!partial || nsplit < 1) nsplit = 1;
-    if (nsplit > 8) nsplit = 8;
     if (tiles <= 0x7fffffff) {
       dim3 grid((unsigned)tiles, 1, (unsigned)nsplit);
       const unsigned threads = (unsigned)(plan.QT * H / 16 * 32);
