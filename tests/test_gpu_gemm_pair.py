@@ -95,3 +95,22 @@ def test_int4(T, N, K, group, bias):
             # both factors and the product are rounded: |d(silu)/dgate| <= 1.1
             slack = 1.1 * tol[:, :N // 2] * up.abs() + (gate * torch.sigmoid(gate)).abs() * tol[:, N // 2:] + 2 * 2.0 ** -11 * want.abs() + 1e-6
             assert bool(((y.double() - want).abs() <= slack).all()), float(((y.double() - want).abs() - slack).max())
+
+
+@pytest.mark.parametrize("T,N,K", [(100, 520, 20480), (129, 300, 16384), (65, 2048, 1088), (256, 9600, 4096), (250, 40, 600), (96, 19000, 640), (200, 2560, 520)])
+@pytest.mark.parametrize("kind", ["fp16", "bf16", "bf16 relu2"])
+def test_sums_in_pieces(T, N, K, kind):
+    """calls of 65 to 256 tokens add pieces of k in fp32: deep sums, pieces that end unevenly, token tiles of every width, more tiles than pairs"""
+    test_dense(T, N, K, kind)
+
+
+@pytest.mark.parametrize("T,N,K", [(100, 512, 20480), (200, 512, 20480), (256, 4096, 8192)])
+def test_a_deep_sum_is_as_good_as_its_rounding(T, N, K):
+    """against float64 the result is off by the rounding to fp16 and hardly more: the same sum in one tensor-core accumulator is 0.5 % further off at k = 20480"""
+    import tgis_b200  # noqa: F401
+    from tgis_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(K)
+    x, w = torch.randn(T, K, generator=g, device=DEV).half(), (torch.randn(N, K, generator=g, device=DEV) * 0.02).half()
+    ref = x.double() @ w.double().t()
+    off, rounding = (ops.gemm_f16(x, w).double() - ref).norm(), (ref.half().double() - ref).norm()
+    assert float(off / rounding) < 1.002

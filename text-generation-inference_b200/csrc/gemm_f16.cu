@@ -39,12 +39,13 @@ __device__ __forceinline__ void gemm_store(void* y, size_t i, float v) {
 constexpr int kGemmThreads = 192;
 constexpr int kTileM = 128;  // features per tile
 constexpr int kTileK = 64;   // fp16 elements per k-block = one 128-byte swizzle row
-// Calls of more tokens go to the SM pairs (gemm_pair.cuh).  Measured on B200 (us, this kernel / pairs) at 64 tokens: 4096 x 4096 14.8 / 12.9,
-// 4096 -> 22016 37.1 / 40.0, 11008 -> 4096 23.6 / 28.8; at 96: 18.2 / 13.1, 42.9 / 41.3; at 128: 20.5 / 13.4, 45.8 / 42.3, 30.0 / 29.9.
-constexpr int kF16DecodeT = 64;
+// Calls of more than kF16DecodeT tokens may go to the SM pairs (gemm_pair.cuh), calls of more than kF16MostT all do; between the two f16_stream_us
+// says which kernel takes less.  Measured on B200 (us, this kernel / pairs) at 65 tokens: 4096 -> 4096 16.1 / 13.0, 4096 -> 22016 42.2 / 40.0, 5632 -> 2048
+// 16.8 / 15.0, 11008 -> 4096 25 / 29, 16384 -> 2048 25 / 38, 28672 -> 2048 32 / 63, 28672 -> 8192 81 / 93; at 128: 20.8 / 13.5, 45.5 / 41.8, 24.6 / 15.0, 30 / 29,
+// 32 / 38, 39 / 63, 86 / 94; at 256: 33.5 / 15.6, 68 / 50, 44 / 15, 44 / 36, 51 / 38, 61 / 61; at 192 28672 -> 8192 110 / 100.
+constexpr int kF16DecodeT = 64, kF16MostT = 256;
 // fp32 results show how long a sum ran in the tensor cores: cut into stream-K pieces that are added in fp32 it is off by 5e-7 (against float64,
 // k = 2048), in one piece by 2e-6.  So they stay here for as long as this kernel cuts them (one token tile).
-constexpr int kF32OutDecodeT = 256;
 constexpr int64_t kCounterBytes = 64 * 1024;
 
 template <int TN>
@@ -326,6 +327,15 @@ static F16Plan plan_f16(int64_t T, int64_t N, int64_t K, int sms, bool defer = f
   return pl;
 }
 
+// Microseconds of a call of 65 to 256 tokens, a model of what was measured (kF16DecodeT): a 64-wide k-block of a 128-feature tile takes a CTA its own
+// time or the memory's, whichever is longer, and the fix-up of a tile reads a partial of every contributor.
+static float f16_stream_us(const F16Plan& pl, int64_t T) {
+  const int contrib = pl.units_per_cta % pl.nkb == 0 ? 1 : pl.nkb % pl.units_per_cta == 0 ? pl.nkb / pl.units_per_cta : pl.max_contrib;
+  const float straddle = pl.units_per_cta % pl.nkb == 0 || pl.nkb % pl.units_per_cta == 0 ? 1.f : 2.f;
+  const float unit = pl.TN == 128 ? fmaxf(0.29f, 0.0026f * pl.n_ctas) : fmaxf(0.35f, 0.0031f * pl.n_ctas);
+  return unit * pl.units_per_cta + straddle * (4.f + (float)T * (0.0125f * contrib + 0.035f));
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -353,6 +363,23 @@ extern "C" int b200_debug_gemm_plan(int kind, int64_t T, int64_t N, int64_t K, i
   return B200_OK;
 }
 
+// tests (no GPU needed): out[8] = {1 if a launch (with a workspace) takes the SM pairs, token tile, token tiles, feature tiles, SM pairs, k-blocks per
+// stage, pieces of k, stages of a piece}.  kind 0 = fp16 weights (and bfloat16 with results of 16 bits), 1 = int4, 2 = bfloat16 with fp32 results
+static bool f16_takes_pairs(int fmt, int64_t T, int64_t N, int64_t K, bool workspace, int sms);
+static int f16_pieces(int64_t T, int64_t N, int64_t K, int sms);
+extern "C" int b200_debug_pair_plan(int kind, int64_t T, int64_t N, int64_t K, int sms, int32_t* out) {
+  if (!out || T <= 0 || N <= 0 || K <= 0 || sms <= 1 || kind < 0 || kind > 2) {
+    b200_set_last_error("debug_pair_plan: bad arguments");
+    return B200_ERR_ARG;
+  }
+  const int64_t n_kb = kind == 1 ? 2 * ((K + 127) / 128) : (K + kPairK - 1) / kPairK;
+  const PairPlan pl = pair_plan(T, N, n_kb, kind == 1, sms, kind == 1 ? 1 : f16_pieces(T, N, K, sms));
+  const int taken = kind == 1 ? T > kW4DecodeT : f16_takes_pairs(kind == 2 ? 2 : 0, T, N, K, true, sms);
+  const int32_t v[8] = {taken, pl.tn, pl.n_tt, pl.n_m, pl.n_pairs, pl.per_stage, pl.pieces, pl.piece_stages};
+  for (int i = 0; i < 8; ++i) out[i] = v[i];
+  return B200_OK;
+}
+
 extern "C" int64_t b200_gemm_workspace_bytes(int64_t T, int64_t N, int64_t K) {
   const F16Plan pl = plan_f16(T, N, K, 148);
   int64_t f16 = pl.max_contrib > 1 ? (int64_t)pl.n_tiles_t * pl.n_tiles_n * pl.max_contrib * pl.TN * kTileM * 4 : 0;
@@ -373,6 +400,21 @@ extern "C" int64_t b200_gemm_workspace_bytes_max(int64_t N, int64_t K) {
     if (b > best) best = b;
   }
   return best;
+}
+
+// whether a call's kernel is that of gemm_pair.cuh
+static bool f16_takes_pairs(int fmt, int64_t T, int64_t N, int64_t K, bool workspace, int sms) {
+  if (T <= kF16DecodeT || (fmt == 2 && T <= kF16MostT)) return false;
+  if (T > kF16MostT || !workspace) return true;
+  const F16Plan pl = plan_f16(T, N, K, sms);
+  if ((int64_t)pl.n_tiles_n * 4 > kCounterBytes) return true;
+  return pair_plan(T, N, pl.nkb, false, sms).us <= f16_stream_us(pl, T);
+}
+// pieces of k on the pairs: as many as this file's kernel cuts a call of its size into
+static int f16_pieces(int64_t T, int64_t N, int64_t K, int sms) {
+  if (T > kF16MostT) return 1;
+  const F16Plan pl = plan_f16(T, N, K, sms);
+  return (pl.nkb + pl.units_per_cta - 1) / pl.units_per_cta;
 }
 
 template <int TN, int FMT>
@@ -418,14 +460,14 @@ static int gemm_f16_impl(const void* x, const void* w, const void* bias, void* y
     b200_set_last_error("gemm_f16_deferred: needs a workspace, T <= 256 (one token tile) and N % 8 == 0");
     return B200_ERR_UNSUPPORTED;
   }
-  if (!defer && T > (FMT == 2 ? kF32OutDecodeT : kF16DecodeT)) {
+  if (!defer && f16_takes_pairs(FMT, T, N, K, workspace != nullptr, f16_num_sms())) {
     PairParams pp = {};
     pp.y = y;
     pp.bias = bias;
     pp.T = (int)T;
     pp.N = pp.ldy = (int)N;
     pp.n_kb = (int)((K + kPairK - 1) / kPairK);
-    return launch_gemm_pair<FMT>(x, w, K, pp, pair_plan(T, N, pp.n_kb, false, f16_num_sms()), B200_TIME_GEMM_F16, (cudaStream_t)stream);
+    return launch_gemm_pair<FMT>(x, w, K, pp, pair_plan(T, N, pp.n_kb, false, f16_num_sms(), f16_pieces(T, N, K, f16_num_sms())), B200_TIME_GEMM_F16, (cudaStream_t)stream);
   }
   F16Plan pl = plan_f16(T, N, K, f16_num_sms(), defer);
   if (!defer && pl.max_contrib > 1 && (!workspace || (int64_t)pl.n_tiles_n * pl.n_tiles_t * 4 > kCounterBytes)) {

@@ -9,7 +9,10 @@
 //     features and HALF of the tile's tokens: 32 KB per 64-wide k-block for 128 x 256 outputs, two thirds of what a single CTA needs.
 //   * The token tile is any multiple of 32 up to 256, chosen per call so that the tiles fill the pairs (pair_plan), and the last one is cut
 //     to the rows that are left: N is a run-time field of the instruction descriptor.
-//   * Two accumulators in TMEM (2 x 256 columns): the epilogue of one tile runs under the products of the next.
+//   * Two accumulators in TMEM (2 x 256 columns): the epilogue of one tile runs under the products of the next.  Calls of up to 256 tokens cut k into
+//     as many pieces as the weight-streaming kernel would, with an accumulator each (512 columns hold 2 of up to 256 tokens, 4 of 128, 8 of 64; more than
+//     256 columns of them leave no second tile's room), and the epilogue adds them in fp32: one sum of all k in the tensor core is further off (fp16
+//     results, k = 20480, 100 tokens: 2.084e-4 against float64, 2.073e-4 in that kernel's cuts and in pieces).
 //   * int4: four teams of four warps turn 64 k of a record each into the SWIZZLE_128B image of an fp16 A tile (thread = feature row, eight
 //     conflict-free 16-byte stores).  One de-quantised tile serves up to 256 tokens, twice as many as the weight-streaming kernel's, and shared
 //     memory as the operand's place leaves TMEM to the accumulators.
@@ -56,6 +59,7 @@ struct PairCfg {
   static constexpr bool kExperts = KIND >= kPairExpBf16;
   static constexpr bool kOut32 = KIND == kPairBf16F32 || KIND == kPairExpBf16F32;
   static constexpr bool kAct = KIND == kPairW4Silu;
+  static constexpr bool kPieces = !kInt4 && !kExperts;
   static constexpr int kThreads = kInt4 ? 768 : 256;
   static constexpr int kRingBytes = (kInt4 ? 5 : 6) * pair_block_bytes(kPairMaxN);
   static constexpr int kRecs = kInt4 ? 4 : 0;  // ring of int4 records (128 k each)
@@ -77,6 +81,7 @@ struct PairParams {
   int tn, n_tt, n_m;            // token tile, token tiles, feature tiles
   int per_stage, n_stages;      // k-blocks per stage of the ring, stages per tile
   int stages, stage_bytes;      // depth of the ring
+  int pieces, piece_stages, piece_cols;  // pieces of k with an accumulator each, stages and TMEM columns of a piece; one piece: two tiles' accumulators
   const int32_t* offsets;       // experts: first row of each, [E + 1]
   int E;
   int vec;                      // rows of y can be written in 16-byte pieces
@@ -282,22 +287,34 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
         if (!more) break;
         const int nn = tl.nn;
-        const uint32_t idesc = umma_idesc_f16_f32acc(kPairM, nn) | fmt, d = tmem_d + (it & 1) * kPairMaxN;
-        mbar_wait_soft(&tmem_empty[it & 1], ((it >> 1) & 1) ^ 1, ok);
+        const bool one = C::kPieces && p.pieces * p.piece_cols > kPairMaxN;  // accumulators for one tile only
+        const int buf = one ? 0 : it & 1, buf_ph = one ? it & 1 : (it >> 1) & 1;
+        const uint32_t idesc = umma_idesc_f16_f32acc(kPairM, nn) | fmt;
+        uint32_t d = tmem_d + buf * kPairMaxN;
+        mbar_wait_soft(&tmem_empty[buf], buf_ph ^ 1, ok);
+        int left = p.piece_stages;
         for (int kb = 0; kb < p.n_stages; ++kb) {
+          if constexpr (C::kPieces) {
+            if (left == 0) {
+              left = p.piece_stages;
+              d += p.piece_cols;
+            }
+          }
+          const bool first = C::kPieces ? left == p.piece_stages : kb == 0;
+          --left;
           mbar_wait_soft(&full[s], ph, ok);
           tcgen05_fence_after();
           const uint64_t da = desc0 + (uint64_t)((s * p.stage_bytes) >> 4), db = da + (uint64_t)((p.per_stage * kPairABytes) >> 4);
           if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < kPairK / 16; ++k) umma_pair_f16_ss(d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < kPairK / 16; ++k) umma_pair_f16_ss(d, da + (uint64_t)(k * 2), db + (uint64_t)(k * 2), idesc, (!first || k > 0) ? 1u : 0u);
             if (p.per_stage == 2) {
               const uint64_t da1 = da + (uint64_t)(kPairABytes >> 4), db1 = db + (uint64_t)((p.tn * kPairK) >> 4);
 #pragma unroll
               for (int k = 0; k < kPairK / 16; ++k) umma_pair_f16_ss(d, da1 + (uint64_t)(k * 2), db1 + (uint64_t)(k * 2), idesc, 1u);
             }
             umma_pair_commit(&empty[s]);
-            if (kb == p.n_stages - 1) umma_pair_commit(&tmem_full[it & 1]);
+            if (kb == p.n_stages - 1) umma_pair_commit(&tmem_full[buf]);
           }
           __syncwarp();
           if (++s == p.stages) { s = 0; ph ^= 1; }
@@ -395,16 +412,33 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       const int n_w = C::kAct ? n + (lane >> 4) * p.half : n;  // the weight row behind this lane
       const bool n_ok = n < p.N;
       const float bv = p.bias && n_ok ? pair_bias<KIND>(p.bias, n_w) : 0.f;
-      mbar_wait_soft(&tmem_full[it & 1], (it >> 1) & 1, ok);
+      const bool one = C::kPieces && p.pieces * p.piece_cols > kPairMaxN;
+      const int buf = one ? 0 : it & 1, buf_ph = one ? it & 1 : (it >> 1) & 1;
+      mbar_wait_soft(&tmem_full[buf], buf_ph, ok);
       tcgen05_fence_after();
       for (int c = 0; c < nn; c += 32) {
         uint32_t v[32];
-        tmem_ld_32x32b_x32(tmem_d + lane_base + (it & 1) * kPairMaxN + c, v);
+        const uint32_t acc = tmem_d + lane_base + buf * kPairMaxN;
+        tmem_ld_32x32b_x32(acc + c, v);
         tmem_ld_wait();
+        if constexpr (C::kPieces) {
+          for (int q = 1; q < p.pieces; q += 3) {  // up to three more pieces in flight at once
+            uint32_t w[3][32];
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+              if (q + k < p.pieces) tmem_ld_32x32b_x32(acc + (q + k) * p.piece_cols + c, w[k]);
+            tmem_ld_wait();
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+              if (q + k < p.pieces)
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[k][j]));
+          }
+        }
         if (c + 32 >= nn) {
           tcgen05_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(cluster_map(smem_u32(&tmem_empty[it & 1]), 0));
+          if (lane == 0) mbar_arrive_cluster(cluster_map(smem_u32(&tmem_empty[buf]), 0));
         }
         if (p.vec) {
           // transpose 32 tokens x the warp's features through shared memory: rows of a token's features, written out in 16-byte pieces (one
@@ -457,6 +491,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 struct PairPlan {
   int tn, n_tt, n_m, n_pairs, per_stage;
   float us;  // estimate
+  int pieces, piece_stages, piece_cols;
 };
 
 // Token tile of a call: of all cuts of T into equal tiles of 32-row steps, the one whose waves over the SM pairs cost least.  What a 64-wide
@@ -464,7 +499,8 @@ struct PairPlan {
 // 0.15 at 64, 0.19 at 128, 0.26 at 192, 0.35 at 256; int4 0.22 at 32, 0.25 at 128, 0.29 at 192, 0.37 at 256 (below that, de-quantisation).
 // Small tiles take two k-blocks per stage of the ring: a hand-over costs more than their products (16.2 us instead of 19.6 at 300 x 4096 x
 // 4096 fp16, 21.3 instead of 23.3 int4); large ones need the depth more (97 instead of 98 and 30.3 instead of 31.5 at 4099 and 1000 tokens).
-static PairPlan pair_plan(int64_t T, int64_t N, int64_t n_kb, bool int4, int sms) {
+// `pieces`: how many pieces of k should have an accumulator of their own, as far as the tensor memory holds them.
+static PairPlan pair_plan(int64_t T, int64_t N, int64_t n_kb, bool int4, int sms, int pieces = 1) {
   PairPlan best = {};
   const int pairs = sms / 2, n_m = (int)((N + kPairM - 1) / kPairM);
   for (int tn = 32; tn <= kPairMaxN; tn += 32) {
@@ -474,6 +510,18 @@ static PairPlan pair_plan(int64_t T, int64_t N, int64_t n_kb, bool int4, int sms
     const float us = waves * kb * n_kb + 0.013f * tn;  // the last tile's epilogue is not hidden
     if (best.tn == 0 || us < best.us) best = {tn, n_tt, n_m, (int)(tiles < pairs ? tiles : pairs), per_stage, us};
   }
+  best.pieces = 1;
+  best.piece_stages = (int)((n_kb + best.per_stage - 1) / best.per_stage);
+  best.piece_cols = best.tn <= 64 ? 64 : best.tn <= 128 ? 128 : 256;
+  if (pieces > 1) {
+    const int n_stages = best.piece_stages, most = 512 / best.piece_cols, p = pieces < most ? pieces : most;
+    best.piece_stages = (n_stages + p - 1) / p;
+    best.pieces = (n_stages + best.piece_stages - 1) / best.piece_stages;
+  }
+  // what the cost above leaves out matters where another kernel is to be had: the launch, and the feature tiles' share of the memory's rate (B200,
+  // one wave: 448 k-blocks of 8 tiles 62.6 us, 256 of 16 41.0, 320 of 20 52.6, 448 of 32 92.7)
+  const int64_t tiles = (int64_t)best.n_tt * n_m, waves = (tiles + pairs - 1) / pairs;
+  best.us += 3.f + 0.0016f * (n_m < pairs ? n_m : pairs) * waves * n_kb;
   return best;
 }
 
@@ -498,6 +546,9 @@ static int launch_gemm_pair(const void* x, const void* w, int64_t K, PairParams 
   pp.n_m = pl.n_m;
   pp.per_stage = pl.per_stage;
   pp.n_stages = (pp.n_kb + pl.per_stage - 1) / pl.per_stage;
+  pp.pieces = pl.pieces > 1 ? pl.pieces : 1;
+  pp.piece_stages = pl.pieces > 1 ? pl.piece_stages : pp.n_stages;
+  pp.piece_cols = pl.piece_cols;
   pp.stage_bytes = pl.per_stage * pair_block_bytes(pl.tn);
   pp.stages = C::kRingBytes / pp.stage_bytes < kPairMaxStages ? C::kRingBytes / pp.stage_bytes : kPairMaxStages;
   b200_timing_mark(time_id, 0, st);

@@ -65,10 +65,9 @@ constexpr int kW4Threads = (kW4XProdWarp + 1) * 32;             // 768
 constexpr int kW4AColsPerStage = 64;  // 128 fp16 per row = 64 x 32-bit columns
 constexpr int64_t kW4CounterBytes = 64 * 1024;
 
-// Most tokens of one token tile; more go to the SM pairs (gemm_pair.cuh).  At 128 tokens the pairs would win on wide outputs and short k only
+// kW4DecodeT (w4_format.cuh): most tokens of one token tile; more go to the SM pairs (gemm_pair.cuh).  At 128 tokens the pairs would win on wide outputs and short k only
 // (us, this kernel / pairs: 2048 -> 2560 13.1 / 10.9, 4096 -> 28672 45.2 / 46.3, 4096 -> 4096 15.3 / 19.2, 14336 -> 4096 23.9 / 53.8); at 129 this
 // kernel would need two token tiles (4096 -> 4096 40.1 / 19.6, 14336 -> 4096 107 / 58).
-constexpr int kW4DecodeT = 128;
 constexpr int kW4R = 2;  // feature tiles per super-tile: consecutive units (super-tile, k-block, r = 0..1) share one activation tile
 
 template <int TN>

@@ -5,6 +5,7 @@
 
 namespace b200 {
 
+constexpr int kW4DecodeT = 128;  // calls of up to so many tokens stay with gemm_w4a16.cu's kernel
 constexpr int kW4TileM = 128;
 constexpr int kW4BlockK = 128;
 constexpr int kW4WordBytes = (kW4BlockK / 8) * kW4TileM * 4;  // 8192
