@@ -5,7 +5,7 @@
  * Conventions as in b200_tgis.h: plain device pointers + sizes + a cudaStream_t (void*), status-code return (0 = ok, the
  * message through b200_last_error()), no allocation, enqueue-only.  Element types are passed as codes: 0 = bfloat16,
  * 1 = float32.  Everything called "state", "residual", soft-max and norm statistics is fp32 whatever the element type.
- * The library also exports b200_last_error, b200_cuda_peek_error, b200_launch_count, b200_kv_alloc_* and b200_decode_advance
+ * The library also exports b200_last_error, b200_gave_up, b200_debug_set_gave_up, b200_cuda_peek_error, b200_launch_count, b200_kv_alloc_* and b200_decode_advance
  * with the signatures b200_tgis.h gives them.
  *
  * A ragged step: T token rows of B sequences; sequence b owns rows cu_q[b] .. cu_q[b+1], at consecutive positions
@@ -126,7 +126,7 @@ int32_t* b200_seq_moe_offsets(int32_t* plan, int64_t T, int E, int top);
  * heads: Y[t, z, :N] = W[z] X[t, z, :K]; token strides ldx / ldy and head strides head_x / head_y in elements (Y may be a slice of wider
  * rows), W [Z, N, K] dense; K, ldx, head_x multiples of 8.
  * experts: Y[row] = act(W[expert(row)] X[row]) over a plan's compact rows, X [max_rows, K], Y [max_rows, N] and W [E, N, K] dense; act 0:
- * none, 1: relu(z)^2.  gave_up: blocks that gave up a bounded wait (0 unless something is wrong) */
+ * none, 1: relu(z)^2.  gave_up: as b200_gave_up (0 unless something is wrong) */
 int b200_seq_heads_gemm(const void* x, int64_t ldx, int64_t head_x, const void* w, void* y, int y_dt, int64_t ldy, int64_t head_y, int64_t T,
                         int64_t Z, int64_t N, int64_t K, void* stream);
 int b200_seq_experts_gemm(const void* x, const void* w, void* y, int y_dt, const int32_t* offsets, int64_t max_rows, int E, int64_t N, int64_t K,

@@ -28,6 +28,10 @@ extern "C" {
 
 int b200_abi_version(void);
 const char* b200_last_error(void);
+/* 1: a wait inside a kernel of this library ran out (a fault, never a slow neighbour): results since then are not valid, and the entry points
+ * of such kernels (prompt linears and attention, grouped products) refuse further work.  To be asked once the stream has been waited for */
+int b200_gave_up(void);
+void b200_debug_set_gave_up(int v); /* for tests: as if a wait had run out (1), or not (0) */
 const char* b200_cuda_peek_error(void); /* debug: pending CUDA runtime error string, not cleared */
 void b200_debug_w4_flags(int flags); /* debug timing experiments (results invalid): 1 no x loads, 2 no MMAs, 4 no weight loads, 8 no dequant math */
 void b200_debug_w4_trace(void* device_buffer); /* debug: [n_ctas][64] u64 phase timestamps of int4 GEMM launches; NULL = off */

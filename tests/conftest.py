@@ -12,6 +12,15 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (run on the B200 box with -m gpu)")
 
 
+@pytest.fixture(autouse=True)
+def no_wait_ran_out(request):
+    """after a test on the GPU: no kernel of it gave up a wait"""
+    yield
+    lib = sys.modules.get("tgis_b200._lib")
+    if "gpu" in request.keywords and lib is not None:
+        lib.raise_if_gave_up()
+
+
 def pytest_collection_modifyitems(config, items):
     try:
         import torch

@@ -14,6 +14,8 @@ _P, _I, _L, _F = c_void_p, c_int, c_int64, c_float
 SIGNATURES = {
     "b200_abi_version": (_I, []),
     "b200_last_error": (c_char_p, []),
+    "b200_gave_up": (_I, []),
+    "b200_debug_set_gave_up": (None, [_I]),
     "b200_cuda_peek_error": (c_char_p, []),
     "b200_debug_w4_trace": (None, [_P]),
     "b200_debug_w4_flags": (None, [_I]),
@@ -182,7 +184,7 @@ SEQ_SIGNATURES = {
     "b200_seq_mingru_scan": (_I, [_P, _L, _I, _I, _I, _P, _P, _I, _P, _P, _P, _P, _P, _I, _L, _F, _L, _I, _I, _P]),
     "b200_seq_talk_attn_splits": (_I, [_I, _L, _I, _I, _I, _I, _I, ctypes.POINTER(c_int64)]),
 }
-_SEQ_SHARED = ("b200_last_error", "b200_cuda_peek_error", "b200_launch_count", "b200_kv_alloc_create", "b200_kv_alloc_destroy",
+_SEQ_SHARED = ("b200_last_error", "b200_gave_up", "b200_debug_set_gave_up", "b200_cuda_peek_error", "b200_launch_count", "b200_kv_alloc_create", "b200_kv_alloc_destroy",
                "b200_kv_alloc_num_free", "b200_kv_alloc_take", "b200_kv_alloc_release", "b200_decode_advance", "b200_gemm_bf16",
                "b200_gemm_workspace_bytes_max", "b200_debug_step_trace", "b200_debug_step_trace_begin", "b200_debug_step_trace_names")
 
@@ -192,6 +194,13 @@ _seq_lib = None
 
 class B200Error(RuntimeError):
     pass
+
+
+def raise_if_gave_up() -> None:
+    """After the host has waited for a step: an error if a wait inside one of its kernels ran out, in place of results that mean nothing."""
+    for lib in (_lib, _seq_lib):
+        if lib is not None and lib.b200_gave_up():
+            raise B200Error("a wait inside a kernel ran out: the results of this step are not valid")
 
 
 def load_seq() -> ctypes.CDLL:

@@ -19,6 +19,8 @@ static int launch_prefill_paged(const void* q, int64_t q_stride, int64_t T_q, co
                                 const int32_t* block_table, int64_t bt_stride, const int32_t* context_lens, const int32_t* cu_q, void* out,
                                 int64_t out_stride, int B, int max_q, int n_heads, int n_kv, float scale, cudaStream_t st) {
   using C = PfCfg<D>;
+  unsigned* gave_up = b200_gave_up_word();
+  if (!gave_up) return B200_ERR_CUDA;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(attn_prompt_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
@@ -31,6 +33,7 @@ static int launch_prefill_paged(const void* q, int64_t q_stride, int64_t T_q, co
   const CUtensorMap* mv = get_tmap_2d(v_pool, pool_rows, D, D, kPageTokens, 64, TmapDtype::kF16, TmapSwizzle::kNone);
   if (!mq || !mk || !mv) return B200_ERR_CUDA;
   PfParams p = {};
+  p.gave_up = gave_up;
   p.block_table = block_table;
   p.bt_stride = bt_stride;
   p.context_lens = context_lens;

@@ -54,8 +54,6 @@ constexpr int kPfAhead = 2;      // items that are known ahead
 // registers per thread: the launch has 384 x 168; the two softmax warpgroups take 216 each, the other one keeps 72
 constexpr int kPfSoftmaxRegs = 216, kPfServeRegs = 72;
 
-static __device__ int attn_prompt_gave_up;
-
 template <int D>
 struct PfCfg {
   static constexpr int kSlabs = D / 64;
@@ -81,6 +79,7 @@ struct PfParams {
   int n_units, n_groups; // head (pair)s, query tile (pair)s of the longest sequence
   int more_blocks;       // the grid is larger than the GPU: blocks take more items
   float scale_log2;
+  unsigned* gave_up;     // b200_gave_up_word
   // token-major caches only
   const float* q;        // [tokens][heads][D]
   const int64_t* position_ids;
@@ -650,10 +649,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     }
   }
 
-  if (!ok) {  // gave up: let copies and products in flight end before the block's memory goes
-    atomicAdd(&attn_prompt_gave_up, 1);
-    for (int i = 0; i < 64; ++i) __nanosleep(1000000);
-  }
+  if (!ok) gave_up(p.gave_up);
   tcgen05_fence_before();
   __syncthreads();
   if (warp == 2) tmem_dealloc<C::kTmemCols>(tmem_base);

@@ -25,8 +25,9 @@
 //
 // Warp roles: 0..3 epilogue | (int4: 4..19 de-quantisation) | then W producer / TMEM allocation, x producer, MMA issuer (leader CTA), idle.
 // Barriers: `full` and `tmem_empty` live in the leader (the pair's even CTA) and count both CTAs' work, `empty` and `tmem_full` live in
-// each and are arrived at by multicast commits of the leader's products.  Every wait is bounded: a thread that gives up counts itself in
-// `gemm_pair_gave_up` and goes through the rest without waiting; the block then lets copies in flight land, frees its TMEM and ends.
+// each and are arrived at by multicast commits of the leader's products.  Every wait is bounded (mbar_wait_soft): a thread that gives up goes through
+// the rest without waiting; the block then lets copies in flight land, tells the host, frees its TMEM and ends.  No role waits for what the previous
+// kernel has still to deliver: what can be done ahead of it (the first round of the rings of records and stages) is done, then comes pdl_wait.
 // A team skips phases of `empty` (the teams take turns): products complete in order, so having seen the stage of its last turn freed implies
 // that every earlier one was, and no phase is mistaken for another while the ring is at least as deep as there are teams per stage count
 // (four stages, or two when a stage holds two k-blocks).
@@ -85,9 +86,8 @@ struct PairParams {
   const int32_t* offsets;       // experts: first row of each, [E + 1]
   int E;
   int vec;                      // rows of y can be written in 16-byte pieces
+  unsigned* gave_up;            // b200_gave_up_word
 };
-
-static __device__ int gemm_pair_gave_up;
 
 __device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
   uint32_t r;
@@ -273,6 +273,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
   } else if (warp == C::kServeWarp + 2) {
     // ------------------------------------------------------------------ products, issued by the leader for both CTAs
+    pdl_wait();
     if (rank == 0) {
       constexpr uint32_t fmt = C::kInt4 || KIND == kPairF16 ? 0u : ((1u << 7) | (1u << 10));
       const uint64_t desc0 = umma_desc_kmajor_sw128(smem_u32(smem));
@@ -330,6 +331,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       for (int i = pair; pair_tile<KIND>(p, i, cur, tl); i += n_pairs) {
         const int m = tl.m;
         for (int kb = 0; kb < p.n_kb / 2; ++kb) {
+          if (ph == 0) pdl_wait();
           mbar_wait_soft(&rec_empty[r], ph, ok);
           mbar_arrive_expect_tx(&rec_full[r], p.rec_bytes);
           unsigned char* dst = recs + r * kW4RecMaxBytes;
@@ -362,6 +364,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     int r = team >> 1, rph = 0, s = team / p.per_stage, ph = 1;
     uint32_t wq[8], mrec[2];
     auto fetch = [&]() {
+      if (rph == 1) pdl_wait();
       mbar_wait_soft(&rec_full[r], rph, ok);
       lds_v4(words + r * kW4RecMaxBytes, &wq[0]);
       lds_v4(words + r * kW4RecMaxBytes + 2048, &wq[4]);
@@ -382,6 +385,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         dequant_consts(mrec[c >> 2], scale2, nz1024, nz64);
         dequant_word(wq[c], nz1024, nz64, scale2, &v[c * 4]);
       }
+      if (ph == 0) pdl_wait();
       mbar_wait_soft(&empty[s], ph, ok);
       const uint32_t dst = dst_row + s * p.stage_bytes;
 #pragma unroll
@@ -478,10 +482,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
   }
 
-  if (!ok) {  // gave up: let copies and products in flight end before the pair's memory goes
-    atomicAdd(&gemm_pair_gave_up, 1);
-    for (int i = 0; i < 64; ++i) __nanosleep(1000000);
-  }
+  if (!ok) gave_up(p.gave_up);
   tcgen05_fence_before();
   __syncthreads();
   cluster_sync();  // the leader's products read the other CTA's shared memory and write its TMEM until the epilogues are done
@@ -529,6 +530,8 @@ static PairPlan pair_plan(int64_t T, int64_t N, int64_t n_kb, bool int4, int sms
 template <int KIND>
 static int launch_gemm_pair(const void* x, const void* w, int64_t K, PairParams pp, const PairPlan& pl, int time_id, cudaStream_t st) {
   using C = PairCfg<KIND>;
+  pp.gave_up = b200_gave_up_word();
+  if (!pp.gave_up) return B200_ERR_CUDA;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);

@@ -27,6 +27,50 @@ bool b200_pdl_enabled() {
   return v == 1;
 }
 
+// ---------------------------------------------------------------------------------------------------------
+// Waits that ran out.  A kernel with bounded waits that gives one up goes through the rest without waiting, so what it wrote is worth nothing; it says
+// so in a word of host memory that every device sees.  From then on the library refuses further launches of such kernels, as a CUDA context would after
+// a trap, and a program that has waited for the stream asks b200_gave_up before it uses the results.
+// ---------------------------------------------------------------------------------------------------------
+static std::atomic<unsigned*> g_gave_up_word{nullptr};
+static std::atomic<int> g_gave_up_by_hand{0};
+
+extern "C" int b200_gave_up(void) {
+  const volatile unsigned* w = g_gave_up_word.load(std::memory_order_acquire);
+  return (w && *w) || g_gave_up_by_hand.load(std::memory_order_relaxed) ? 1 : 0;
+}
+// for tests: says that a wait ran out (1), or takes it back (0)
+extern "C" void b200_debug_set_gave_up(int v) {
+  volatile unsigned* w = g_gave_up_word.load(std::memory_order_acquire);
+  if (w) *w = 0;
+  g_gave_up_by_hand.store(v ? 1 : 0, std::memory_order_relaxed);
+}
+// where a kernel reports; NULL (with an error message): one has reported already, or the word could not be allocated
+unsigned* b200_gave_up_word() {
+  if (b200_gave_up()) {
+    b200_set_last_error("a wait inside an earlier kernel ran out: its results are not valid, and no further work is taken");
+    return nullptr;
+  }
+  unsigned* w = g_gave_up_word.load(std::memory_order_acquire);
+  if (w) return w;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  w = g_gave_up_word.load(std::memory_order_acquire);
+  if (w) return w;
+  // the first launch may come while a stream is being captured: an allocation has no part in the capture
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&w), 64, cudaHostAllocPortable | cudaHostAllocMapped);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) {
+    b200_set_last_error(cudaGetErrorString(e));
+    return nullptr;
+  }
+  *w = 0;
+  g_gave_up_word.store(w, std::memory_order_release);
+  return w;
+}
+
 extern "C" const char* b200_last_error(void) { return g_last_error.c_str(); }
 // debug aid: pending CUDA runtime error of this library's runtime instance (does not clear it)
 extern "C" const char* b200_cuda_peek_error(void) { return cudaGetErrorString(cudaPeekAtLastError()); }

@@ -11,7 +11,7 @@
 // that one's epilogue (TMEM -> registers -> HBM) runs under the other's products.
 // Warp roles: 0 = TMA producer, 1 = MMA issuer (one elected thread each), 2..5 = epilogue.
 //
-// Every wait is bounded: a block that gives up counts itself in `group_gemm_gave_up`, waits for its copies in flight, frees its TMEM and ends.
+// Every wait is bounded (mbar_wait_soft): a block that gives up lets its copies land, tells the host, frees its TMEM and ends.
 #include "gemm_pair.cuh"
 #include "seq_common.cuh"
 #include "tmap.cuh"
@@ -20,8 +20,6 @@ namespace b200 {
 namespace seq {
 
 constexpr int kGgThreads = 192, kGgTileM = 128, kGgTileK = 64;
-
-__device__ int group_gemm_gave_up;
 
 template <int TN>
 struct GgCfg {
@@ -37,12 +35,13 @@ struct GgParams {
   int64_t head_x;         // heads: columns between two heads' inputs
   const int32_t* offsets; // experts: first compact row of every expert [E + 1]
   int E, T, N, nkb, out_f32, act;
+  unsigned* gave_up;      // b200_gave_up_word
 };
 
 __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity) {
-  for (uint32_t spins = 0; spins < (1u << 24); ++spins)
-    if (mbar_try_wait(bar, parity)) return true;
-  return false;
+  bool ok = true;
+  mbar_wait_soft(bar, parity, ok);
+  return ok;
 }
 
 template <int TN, int MODE>
@@ -149,6 +148,7 @@ __global__ void __launch_bounds__(kGgThreads, 2) group_gemm_kernel(const __grid_
     __syncwarp();
   } else if (warp == 1) {
     constexpr uint32_t idesc = umma_idesc_f16_f32acc(kGgTileM, TN) | (1u << 7) | (1u << 10);   // a / b format 1 = bf16
+    if constexpr (MODE == 0) pdl_wait();   // the inputs come after it: no wait counts against the kernel before this one
     for (int i = 0; i < p.nkb; ++i) {
       const int s = i % C::kStages;
       if (!mbar_wait_limited(&full_bar[s], (i / C::kStages) & 1)) { ok = false; break; }
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kGgThreads, 2) group_gemm_kernel(const __grid_
       }
     }
   }
-  if (!ok) atomicAdd(&group_gemm_gave_up, 1);
+  if (!ok) gave_up(p.gave_up);
   tcgen05_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc<C::kTmemCols>(tmem_d);
@@ -203,8 +203,10 @@ __global__ void __launch_bounds__(kGgThreads, 2) group_gemm_kernel(const __grid_
 
 template <int TN, int MODE>
 static int launch_group_gemm(const void* w, int64_t w_rows, int64_t K, const void* x, int64_t x_rows, int64_t x_cols, int64_t ldx, dim3 grid,
-                             const GgParams& p, cudaStream_t st) {
+                             GgParams p, cudaStream_t st) {
   using C = GgCfg<TN>;
+  p.gave_up = b200_gave_up_word();
+  if (!p.gave_up) return B200_ERR_CUDA;
   static bool configured = false;
   if (!configured) {
     const cudaError_t e = cudaFuncSetAttribute(group_gemm_kernel<TN, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
@@ -232,11 +234,8 @@ constexpr int64_t kPairRowsPerExpert = 160;
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// blocks of this process's grouped products that gave up a wait (0 unless something is wrong); -1: the count could not be read
-extern "C" int b200_seq_group_gemm_gave_up(void) {
-  int n = 0;
-  return cudaMemcpyFromSymbol(&n, group_gemm_gave_up, sizeof(int)) == cudaSuccess ? n : -1;
-}
+// 1: a kernel of this library gave up a wait (b200_gave_up)
+extern "C" int b200_seq_group_gemm_gave_up(void) { return b200_gave_up(); }
 
 // Y[t, z, :N] = W[z] [N, K] X[t, z, :K] for z < Z, t < T: bfloat16 X (token stride ldx, head stride head_x) and dense W [Z, N, K]; Y of type
 // y_dt (token stride ldy, head stride head_y).  K, ldx and head_x multiples of 8, X and W 16-byte aligned.

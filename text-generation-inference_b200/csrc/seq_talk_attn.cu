@@ -767,6 +767,8 @@ static int launch_talk_prompt(const float* q, const void* cache, int64_t RW, int
                               const int32_t* cu_q, int B, const int64_t* position_ids, float* out, int64_t T, int H, int G, int chunk, int window,
                               float scale, const float* sink, cudaStream_t st) {
   using C = b200::PfCfg<D>;
+  unsigned* gave_up = b200_gave_up_word();
+  if (!gave_up) return B200_ERR_CUDA;
   static bool cfg = false;
   if (!cfg) {
     cudaError_t e = cudaFuncSetAttribute(b200::attn_prompt_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
@@ -777,6 +779,7 @@ static int launch_talk_prompt(const float* q, const void* cache, int64_t RW, int
   const CUtensorMap* m = b200::get_tmap_2d(cache, (uint64_t)1 << 30, (uint64_t)RW, (uint64_t)RW, b200::kPageTokens, 64, b200::TmapDtype::kF16, b200::TmapSwizzle::k128B);
   if (!m) return B200_ERR_CUDA;
   b200::PfParams p = {};
+  p.gave_up = gave_up;
   p.block_table = block_table;
   p.bt_stride = bt_stride;
   p.cu_q = cu_q;

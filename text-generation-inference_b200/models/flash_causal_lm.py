@@ -436,6 +436,7 @@ class FlashCausalLM(Model):
         self._run_fused_step(batch, st)
         forward_time_ns = time.time_ns() - start_time
         ids = st["next_ids"].tolist()  # the step's D2H read
+        _lib.raise_if_gave_up()
         lps = dc.logprobs.tolist() if dc is not None and st["want_logprobs"] else None
         rks = dc.ranks.tolist() if dc is not None and st["want_ranks"] else None
         generated = []
@@ -533,6 +534,7 @@ class FlashCausalLM(Model):
             next_ids = next_ids.clone()
             batch.all_input_ids_tensor.scatter_(dim=1, index=batch.position_ids[:, None], src=next_ids[:, None])
             ids = next_ids.tolist()
+            _lib.raise_if_gave_up()
             lps = lps.tolist() if lps is not None else None
             rks = rks.tolist() if rks is not None else None
             for i, (r, tok) in enumerate(zip(batch.requests, ids)):
@@ -550,11 +552,14 @@ class FlashCausalLM(Model):
                         for r in batch.requests)
         if plain:
             # one D2H copy for the whole batch instead of a .item() sync per request (tokens.py:394)
-            for i, (r, tok) in enumerate(zip(batch.requests, next_ids.tolist())):
+            ids = next_ids.tolist()
+            _lib.raise_if_gave_up()
+            for i, (r, tok) in enumerate(zip(batch.requests, ids)):
                 generated.append(TokenInfo(request_id=r.id, token_id=tok))
                 batch.input_lengths[i] += 1
             return next_ids
         cu = batch.cu_seqlens.tolist()
+        _lib.raise_if_gave_up()
         for i, (r, input_length, next_token, sc, lp, all_ids) in enumerate(
                 zip(batch.requests, batch.input_lengths, next_ids, scores, logprobs, batch.all_input_ids_tensor)):
             try:
