@@ -36,7 +36,7 @@ const char* b200_cuda_peek_error(void); /* debug: pending CUDA runtime error str
 void b200_debug_w4_flags(int flags); /* debug timing experiments (results invalid): 1 no x loads, 2 no MMAs, 4 no weight loads, 8 no dequant math */
 void b200_debug_w4_trace(void* device_buffer); /* debug: [n_ctas][64] u64 phase timestamps of int4 GEMM launches; NULL = off */
 int b200_debug_pair_plan(int kind, int64_t T, int64_t N, int64_t K, int sms, int32_t* out8); /* tests, host only: whether a launch takes the SM pairs, and how; kind 0 fp16, 1 int4, 2 bfloat16 with fp32 results; out = {taken, token tile, token tiles, feature tiles, pairs, k-blocks per stage, pieces of k, stages of a piece} */
-int b200_debug_gemm_plan(int kind, int64_t T, int64_t N, int64_t K, int sms, int32_t* out8); /* tests, host only: stream-K plan of a launch; kind 0 fp16, 1 int4; out = {token tile, k-blocks, feature (super-)tiles, token tiles, units per CTA, CTAs, contributor slots, tiles per unit} */
+int b200_debug_gemm_plan(int kind, int64_t T, int64_t N, int64_t K, int sms, int32_t* out8); /* tests, host only: stream-K plan of a launch of up to 256 (int4: 128) tokens; kind 0 fp16, 1 int4; out = {token tile, k-blocks, feature (super-)tiles, 1, units per CTA, CTAs, contributor slots, tiles per unit} */
 /* debug: per-kernel device timeline of a step.  While a buffer of `capacity` uint64 slots is attached, every kernel this
  * library enqueues is followed by a one-thread kernel storing %globaltimer (ns) into the next slot (slot 0: _begin);
  * _names writes the newline-separated kernel names in launch order and returns the count.  Serialises the stream. */

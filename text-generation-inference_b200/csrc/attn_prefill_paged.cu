@@ -45,13 +45,13 @@ static int launch_prefill_paged(const void* q, int64_t q_stride, int64_t T_q, co
   p.B = B;
   // two heads of a key / value head are equally long and share their keys; neighbouring query tiles are not, and a short prompt has no second one
   const int tiles = (max_q + kPfM - 1) / kPfM;
-  p.pair = (int64_t)B * tiles * n_heads <= pf_num_sms() ? kPfSingle : (n_heads / n_kv) % 2 == 0 ? kPfHeads : kPfTiles;
+  p.pair = (int64_t)B * tiles * n_heads <= b200_num_sms() ? kPfSingle : (n_heads / n_kv) % 2 == 0 ? kPfHeads : kPfTiles;
   p.n_units = p.pair == kPfHeads ? n_heads / 2 : n_heads;
   p.n_groups = p.pair == kPfTiles ? (tiles + 1) / 2 : tiles;
   p.scale_log2 = scale * 1.4426950408889634f;
   const int64_t items = (int64_t)p.n_units * p.n_groups * B;
   if (items > (1 << 30)) { b200_set_last_error("attn_prefill_paged: too many query tiles"); return B200_ERR_ARG; }
-  p.more_blocks = items > pf_num_sms();
+  p.more_blocks = items > b200_num_sms();
   B200_LAUNCH((attn_prompt_kernel<D, false>), dim3((unsigned)items), dim3(kPfThreads), (size_t)C::kSmemBytes, st, *mq, *mk, *mv, p);
   b200_count_launches(1);
   return B200_OK;

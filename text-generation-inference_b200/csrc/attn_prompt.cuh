@@ -655,14 +655,4 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   if (warp == 2) tmem_dealloc<C::kTmemCols>(tmem_base);
 }
 
-static int pf_num_sms() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-  }
-  return n;
-}
-
 }  // namespace b200

@@ -5,7 +5,8 @@
 //
 // Swap-AB: the 128 output features of a weight tile are the UMMA M dimension (A operand, K-major, streamed
 // from HBM once by TMA with 128B swizzle), the step's tokens are the UMMA N dimension (B operand, TN = 16..256),
-// the fp32 accumulator D[128 x TN] lives in TMEM.  Decode (T <= 256) is weight-streaming / HBM-bound: the flattened
+// the fp32 accumulator D[128 x TN] lives in TMEM.  One token tile (T <= 256; larger calls, and those of more than 64 tokens that are faster there, go to
+// gemm_pair.cuh) is weight-streaming / HBM-bound: the flattened
 // (feature tile, 64-wide k-block) unit space is cut into equal contiguous ranges, one per SM (stream-K), so all 148 SMs
 // pull the same number of weight bytes; a tile that straddles CTAs gets its fp32 partials summed in contributor order by
 // the last CTA to finish (deterministic).  PDL: the weight ring is filled before griddepcontrol.wait.
@@ -287,38 +288,24 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
 }
 
 struct F16Plan {
-  int TN, nkb, n_tiles_n, n_tiles_t, units_per_cta, n_ctas, max_contrib;
+  int TN, nkb, n_tiles_n, units_per_cta, n_ctas, max_contrib;
 };
 
-static int f16_num_sms() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-  }
-  return n;
-}
-
+// a call of up to kF16MostT tokens: one token tile
 static F16Plan plan_f16(int64_t T, int64_t N, int64_t K, int sms, bool defer = false) {
   F16Plan pl;
   pl.TN = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : T <= 128 ? 128 : 256;
   pl.nkb = (int)((K + kTileK - 1) / kTileK);
   pl.n_tiles_n = (int)((N + kTileM - 1) / kTileM);
-  pl.n_tiles_t = (int)((T + pl.TN - 1) / pl.TN);
   const int total = pl.n_tiles_n * pl.nkb;
-  if (pl.n_tiles_t > 1) {
-    pl.units_per_cta = pl.nkb;  // whole tiles (prefill: plenty of tiles)
-  } else {
-    const int ctas = total < sms ? total : sms;
-    pl.units_per_cta = (total + ctas - 1) / ctas;
-    if (pl.units_per_cta < 4 && pl.nkb >= 4) pl.units_per_cta = 4;
-    // prefer the largest aligned cut nkb / d (d = 8, 4, 2, 1) that fits the SM count: a CTA that straddles two tiles pays two
-    // fix-ups (measured on B200, round 2: 17.4 -> 14.4 us at 64 x 4096 x 4096, 47.7 -> 33.9 us at T = 256)
-    if (!defer) {
-      for (int d = 8; d >= 1; d >>= 1) {
-        if (pl.nkb % d == 0 && (int64_t)pl.n_tiles_n * d <= sms && pl.nkb / d >= 4) { pl.units_per_cta = pl.nkb / d; break; }
-      }
+  const int ctas = total < sms ? total : sms;
+  pl.units_per_cta = (total + ctas - 1) / ctas;
+  if (pl.units_per_cta < 4 && pl.nkb >= 4) pl.units_per_cta = 4;
+  // prefer the largest aligned cut nkb / d (d = 8, 4, 2, 1) that fits the SM count: a CTA that straddles two tiles pays two
+  // fix-ups (measured on B200: 17.4 -> 14.4 us at 64 x 4096 x 4096, 47.7 -> 33.9 us at T = 256)
+  if (!defer) {
+    for (int d = 8; d >= 1; d >>= 1) {
+      if (pl.nkb % d == 0 && (int64_t)pl.n_tiles_n * d <= sms && pl.nkb / d >= 4) { pl.units_per_cta = pl.nkb / d; break; }
     }
   }
   pl.n_ctas = (total + pl.units_per_cta - 1) / pl.units_per_cta;
@@ -345,10 +332,11 @@ __attribute__((weak)) int64_t b200_w4_partial_bytes(int64_t T, int64_t N, int64_
 __attribute__((weak)) void b200_w4_plan_debug(int64_t T, int64_t N, int64_t K, int sms, int32_t* out);
 
 // tests (no GPU needed): the stream-K plan of one GEMM launch.  kind 0 = fp16 weights, 1 = int4.
-// out[8] = {token tile, k-blocks per tile, feature tiles (int4: super-tiles), token tiles, units per CTA, CTAs,
+// out[8] = {token tile, k-blocks per tile, feature tiles (int4: super-tiles), 1, units per CTA, CTAs,
 //           contributor slots per tile in the workspace, feature tiles per unit (int4: 2)}
+// Calls of more than 256 (int4: 128) tokens have no such plan (b200_debug_pair_plan).
 extern "C" int b200_debug_gemm_plan(int kind, int64_t T, int64_t N, int64_t K, int sms, int32_t* out) {
-  if (!out || T <= 0 || N <= 0 || K <= 0 || sms <= 0 || (kind != 0 && kind != 1)) {
+  if (!out || T <= 0 || T > (kind == 1 ? kW4DecodeT : kF16MostT) || N <= 0 || K <= 0 || sms <= 0 || (kind != 0 && kind != 1)) {
     b200_set_last_error("debug_gemm_plan: bad arguments");
     return B200_ERR_ARG;
   }
@@ -358,7 +346,7 @@ extern "C" int b200_debug_gemm_plan(int kind, int64_t T, int64_t N, int64_t K, i
     return B200_OK;
   }
   const F16Plan pl = plan_f16(T, N, K, sms);
-  const int32_t v[8] = {pl.TN, pl.nkb, pl.n_tiles_n, pl.n_tiles_t, pl.units_per_cta, pl.n_ctas, pl.max_contrib, 1};
+  const int32_t v[8] = {pl.TN, pl.nkb, pl.n_tiles_n, 1, pl.units_per_cta, pl.n_ctas, pl.max_contrib, 1};
   for (int i = 0; i < 8; ++i) out[i] = v[i];
   return B200_OK;
 }
@@ -381,13 +369,13 @@ extern "C" int b200_debug_pair_plan(int kind, int64_t T, int64_t N, int64_t K, i
 }
 
 extern "C" int64_t b200_gemm_workspace_bytes(int64_t T, int64_t N, int64_t K) {
+  if (T > kF16MostT) return kCounterBytes;
   const F16Plan pl = plan_f16(T, N, K, 148);
-  int64_t f16 = pl.max_contrib > 1 ? (int64_t)pl.n_tiles_t * pl.n_tiles_n * pl.max_contrib * pl.TN * kTileM * 4 : 0;
-  if (pl.n_tiles_t == 1) {  // deferred reduction (one token tile) leaves a partial for every tile, even un-split ones
-    const F16Plan pd = plan_f16(T, N, K, 148, true);
-    const int64_t fd = (int64_t)pd.n_tiles_n * pd.max_contrib * pd.TN * kTileM * 4;
-    if (fd > f16) f16 = fd;
-  }
+  int64_t f16 = pl.max_contrib > 1 ? (int64_t)pl.n_tiles_n * pl.max_contrib * pl.TN * kTileM * 4 : 0;
+  // deferred reduction leaves a partial for every tile, even un-split ones
+  const F16Plan pd = plan_f16(T, N, K, 148, true);
+  const int64_t fd = (int64_t)pd.n_tiles_n * pd.max_contrib * pd.TN * kTileM * 4;
+  if (fd > f16) f16 = fd;
   const int64_t w4 = b200_w4_partial_bytes ? b200_w4_partial_bytes(T, N, K) : 0;
   return kCounterBytes + (f16 > w4 ? f16 : w4);
 }
@@ -460,17 +448,17 @@ static int gemm_f16_impl(const void* x, const void* w, const void* bias, void* y
     b200_set_last_error("gemm_f16_deferred: needs a workspace, T <= 256 (one token tile) and N % 8 == 0");
     return B200_ERR_UNSUPPORTED;
   }
-  if (!defer && f16_takes_pairs(FMT, T, N, K, workspace != nullptr, f16_num_sms())) {
+  if (!defer && f16_takes_pairs(FMT, T, N, K, workspace != nullptr, b200_num_sms())) {
     PairParams pp = {};
     pp.y = y;
     pp.bias = bias;
     pp.T = (int)T;
     pp.N = pp.ldy = (int)N;
     pp.n_kb = (int)((K + kPairK - 1) / kPairK);
-    return launch_gemm_pair<FMT>(x, w, K, pp, pair_plan(T, N, pp.n_kb, false, f16_num_sms(), f16_pieces(T, N, K, f16_num_sms())), B200_TIME_GEMM_F16, (cudaStream_t)stream);
+    return launch_gemm_pair<FMT>(x, w, K, pp, pair_plan(T, N, pp.n_kb, false, b200_num_sms(), f16_pieces(T, N, K, b200_num_sms())), B200_TIME_GEMM_F16, (cudaStream_t)stream);
   }
-  F16Plan pl = plan_f16(T, N, K, f16_num_sms(), defer);
-  if (!defer && pl.max_contrib > 1 && (!workspace || (int64_t)pl.n_tiles_n * pl.n_tiles_t * 4 > kCounterBytes)) {
+  F16Plan pl = plan_f16(T, N, K, b200_num_sms(), defer);
+  if (!defer && pl.max_contrib > 1 && (!workspace || (int64_t)pl.n_tiles_n * 4 > kCounterBytes)) {
     pl.units_per_cta = pl.nkb;
     pl.n_ctas = pl.n_tiles_n;
     pl.max_contrib = 1;

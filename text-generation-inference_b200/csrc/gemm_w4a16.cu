@@ -154,7 +154,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
   // Inputs of super-unit j (its activation tile + the 8 team-warp quarters of its two A tiles) are counted in
   // s_ready[j % 8]; the MMA warp polls that word with plain shared-memory loads.  (In the warp that issues tcgen05.mma
-  // every dependent wait costs > 100 cycles during which the tensor pipe drains - tools/ubench/umma_rate.cu - so it gets
+  // every dependent wait costs > 100 cycles during which the tensor pipe drains so it gets
   // exactly one per 16 MMAs.)  Monotonic: super-unit j is ready at 9 * (j / 8 + 1).
   __shared__ uint32_t s_ready[8];
   __shared__ uint32_t s_issued;  // super-units whose MMAs have been issued (hand-over between the two MMA warps)
@@ -280,7 +280,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
   } else if (warp == kW4MmaWarp || warp == kW4MmaWarp + 1) {
     // ------------------------------------------------------------------ MMA issuers.  tcgen05.mma issue is in order and the
     // queue is shallow, so a warp that has just issued 16 MMAs cannot hide its own bookkeeping (barrier polls, commit)
-    // behind them: the tensor pipe would idle ~40 % of the time (tools/ubench/umma_rate.cu).  Two warps take alternate
+    // behind them: the tensor pipe would idle ~40 % of the time.  Two warps take alternate
     // super-units; while one is blocked issuing, the other has already found its inputs ready and only waits for its turn
     // (s_issued), so MMAs reach the pipe back to back and in super-unit order (summation order stays fixed).
     // Warp-uniform loops, one elected thread issues: keeps the tcgen05 operands in uniform registers.
@@ -625,16 +625,6 @@ __global__ void gptq_pack_kernel(const uint32_t* __restrict__ qweight, const uin
 
 static unsigned long long* g_w4_trace = nullptr;
 
-static int num_sms() {
-  static int n = 0;
-  if (n == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-  }
-  return n;
-}
-
 // k-blocks per tile.  Rounded up to a multiple of 8 (empty records; the activation TMA zero-fills past K) when that adds
 // at most 5 % of traffic: it lets a super-tile be cut into 2 / 4 / 8 equal CTA shares (Llama-2 down_proj: 86 -> 88).
 static int w4_nkb(int64_t K) {
@@ -644,13 +634,13 @@ static int w4_nkb(int64_t K) {
 }
 
 struct W4Plan {
-  int TN, nkb, n_super, n_tiles_t, su_per_cta, n_ctas, max_contrib;
+  int TN, nkb, n_super, su_per_cta, n_ctas, max_contrib;
 };
 
-// Decode (one token tile): how many super-units per CTA.  Candidates are the balanced stream-K cut (every SM the same
+// One token tile (T <= kW4DecodeT): how many super-units per CTA.  Candidates are the balanced stream-K cut (every SM the same
 // number of units, but most CTAs then straddle two super-tiles: two fix-ups at the tail) and the aligned cuts nkb / d
 // (a CTA = 1/d of one super-tile: one fix-up with d contributors, or none for d = 1, at the price of idle SMs when
-// n_super * d is not close to a multiple of the SM count).  Costs in microseconds fitted to tools/sweep_w4_su.py on B200
+// n_super * d is not close to a multiple of the SM count).  Costs in microseconds fitted to a sweep of the cut on B200
 // (cold weights): 0.35 per unit in the main loop, ~1 for a direct epilogue, 4.5-6 for one split-K fix-up (partial store,
 // gpu-scope fence, waiting for the slowest contributor, L2-latency-bound slice reduction), ~10 when CTAs straddle.
 static W4Plan plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool defer = false) {
@@ -658,36 +648,31 @@ static W4Plan plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool defer = fal
   pl.TN = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : 128;
   pl.nkb = w4_nkb(K);
   pl.n_super = (int)((N + kW4R * kW4TileM - 1) / (kW4R * kW4TileM));
-  pl.n_tiles_t = (int)((T + pl.TN - 1) / pl.TN);
   const int total = pl.n_super * pl.nkb;
-  if (pl.n_tiles_t > 1) {
-    pl.su_per_cta = pl.nkb;  // whole super-tiles (prefill: plenty of tiles)
-  } else {
-    const int ctas = total < sms ? total : sms;
-    int best = (total + ctas - 1) / ctas;
-    if (best < 2 && pl.nkb >= 2) best = 2;  // one unit per team at least
-    // deferred reduction (the consumer kernel sums the partials): no in-kernel fix-up, a CTA that straddles two super-tiles only
-    // pays a mid-loop accumulator drain (~1 us)
-    auto cost = [&](int su, bool aligned, int d) {
-      const float fix = defer ? (aligned ? 0.f : 1.0f) : (aligned ? (d == 1 ? 1.0f : 4.5f + 0.2f * d) : 10.0f);
-      return 0.35f * kW4R * su + fix;
-    };
-    float best_cost = cost(best, pl.nkb % best == 0, pl.nkb / best);
-    for (int d = 1; d <= 8; d *= 2) {
-      if (pl.nkb % d != 0) break;
-      const int su = pl.nkb / d;
-      if ((int64_t)pl.n_super * d > sms || su < 2) continue;
-      const float c = cost(su, true, d);
-      if (c < best_cost) { best_cost = c; best = su; }
-    }
-    pl.su_per_cta = best;
-    static int env_su = -1;  // experiments: B200_W4_SU forces the cut
-    if (env_su < 0) {
-      const char* e = getenv("B200_W4_SU");
-      env_su = e ? atoi(e) : 0;
-    }
-    if (env_su > 0 && (total + env_su - 1) / env_su <= sms) pl.su_per_cta = env_su;
+  const int ctas = total < sms ? total : sms;
+  int best = (total + ctas - 1) / ctas;
+  if (best < 2 && pl.nkb >= 2) best = 2;  // one unit per team at least
+  // deferred reduction (the consumer kernel sums the partials): no in-kernel fix-up, a CTA that straddles two super-tiles only
+  // pays a mid-loop accumulator drain (~1 us)
+  auto cost = [&](int su, bool aligned, int d) {
+    const float fix = defer ? (aligned ? 0.f : 1.0f) : (aligned ? (d == 1 ? 1.0f : 4.5f + 0.2f * d) : 10.0f);
+    return 0.35f * kW4R * su + fix;
+  };
+  float best_cost = cost(best, pl.nkb % best == 0, pl.nkb / best);
+  for (int d = 1; d <= 8; d *= 2) {
+    if (pl.nkb % d != 0) break;
+    const int su = pl.nkb / d;
+    if ((int64_t)pl.n_super * d > sms || su < 2) continue;
+    const float c = cost(su, true, d);
+    if (c < best_cost) { best_cost = c; best = su; }
   }
+  pl.su_per_cta = best;
+  static int env_su = -1;  // experiments: B200_W4_SU forces the cut
+  if (env_su < 0) {
+    const char* e = getenv("B200_W4_SU");
+    env_su = e ? atoi(e) : 0;
+  }
+  if (env_su > 0 && (total + env_su - 1) / env_su <= sms) pl.su_per_cta = env_su;
   pl.n_ctas = (total + pl.su_per_cta - 1) / pl.su_per_cta;
   pl.max_contrib = (pl.nkb + pl.su_per_cta - 1) / pl.su_per_cta + 1;
   if (pl.su_per_cta % pl.nkb == 0) pl.max_contrib = 1;
@@ -773,7 +758,7 @@ extern "C" int b200_gptq_pack(const void* qweight, const void* qzeros, const voi
 static W4Plan launch_plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool has_workspace, bool defer = false) {
   W4Plan pl = plan_w4(T, N, K, sms, defer);
   if (defer) return pl;  // the caller checked: one token tile, workspace present; no counters, no co-residency requirement
-  if (pl.max_contrib > 1 && (!has_workspace || (int64_t)pl.n_super * pl.n_tiles_t * 8 > kW4CounterBytes || pl.n_ctas > sms)) {
+  if (pl.max_contrib > 1 && (!has_workspace || (int64_t)pl.n_super * 8 > kW4CounterBytes || pl.n_ctas > sms)) {
     pl.su_per_cta = pl.nkb;
     pl.n_ctas = pl.n_super;
     pl.max_contrib = 1;
@@ -781,22 +766,21 @@ static W4Plan launch_plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool has_
   return pl;
 }
 
-// tests (no GPU needed): out = {TN, k-blocks, super-tiles, token tiles, super-units per CTA, CTAs, contributor slots, R}
+// tests (no GPU needed): out = {TN, k-blocks, super-tiles, 1, super-units per CTA, CTAs, contributor slots, R}
 void b200_w4_plan_debug(int64_t T, int64_t N, int64_t K, int sms, int32_t* out) {
   const W4Plan pl = launch_plan_w4(T, N, K, sms, true);
-  const int32_t v[8] = {pl.TN, pl.nkb, pl.n_super, pl.n_tiles_t, pl.su_per_cta, pl.n_ctas, pl.max_contrib, kW4R};
+  const int32_t v[8] = {pl.TN, pl.nkb, pl.n_super, 1, pl.su_per_cta, pl.n_ctas, pl.max_contrib, kW4R};
   for (int i = 0; i < 8; ++i) out[i] = v[i];
 }
 
 int64_t b200_w4_partial_bytes(int64_t T, int64_t N, int64_t K) {
-  const W4Plan pl = plan_w4(T, N, K, num_sms());
-  int64_t need = pl.max_contrib <= 1 ? 0 : (int64_t)pl.n_tiles_t * pl.n_super * pl.max_contrib * kW4R * pl.TN * kW4TileM * 4;
-  if (pl.n_tiles_t == 1) {  // deferred reduction: every super-tile has at least one partial slot
-    const W4Plan pd = plan_w4(T, N, K, num_sms(), true);
-    const int64_t nd = (int64_t)pd.n_super * pd.max_contrib * kW4R * pd.TN * kW4TileM * 4;
-    if (nd > need) need = nd;
-  }
-  return need;
+  if (T > kW4DecodeT) return 0;
+  const W4Plan pl = plan_w4(T, N, K, b200_num_sms());
+  const int64_t need = pl.max_contrib <= 1 ? 0 : (int64_t)pl.n_super * pl.max_contrib * kW4R * pl.TN * kW4TileM * 4;
+  // deferred reduction: every super-tile has at least one partial slot
+  const W4Plan pd = plan_w4(T, N, K, b200_num_sms(), true);
+  const int64_t nd = (int64_t)pd.n_super * pd.max_contrib * kW4R * pd.TN * kW4TileM * 4;
+  return nd > need ? nd : need;
 }
 
 template <int TN, int kGR>
@@ -868,11 +852,11 @@ static int gemm_w4a16_impl(const void* x, const void* packed, const void* bias, 
     pp.rec_bytes = kW4WordBytes + gr * kW4MetaRowBytes;
     pp.group_rows = gr;
     pp.half_tiles = half_tiles;
-    const PairPlan pl = pair_plan(T, N, pp.n_kb, true, num_sms());
+    const PairPlan pl = pair_plan(T, N, pp.n_kb, true, b200_num_sms());
     return act ? launch_gemm_pair<kPairW4Silu>(x, nullptr, K, pp, pl, B200_TIME_GEMM_W4A16, (cudaStream_t)stream)
                : launch_gemm_pair<kPairW4>(x, nullptr, K, pp, pl, B200_TIME_GEMM_W4A16, (cudaStream_t)stream);
   }
-  const W4Plan pl = launch_plan_w4(T, N, K, num_sms(), workspace != nullptr, defer);
+  const W4Plan pl = launch_plan_w4(T, N, K, b200_num_sms(), workspace != nullptr, defer);
   const CUtensorMap* mx = get_tmap_2d(x, T, K, K, pl.TN, 64, TmapDtype::kF16, TmapSwizzle::k128B);
   if (!mx) return B200_ERR_CUDA;
   if (defer) {

@@ -283,7 +283,7 @@ extern "C" int b200_seq_experts_gemm(const void* x, const void* w, void* y, int 
     pp.n_kb = (int)((K + kPairK - 1) / kPairK);
     pp.offsets = offsets;
     pp.E = E;
-    const int n_m = (int)((N + kPairM - 1) / kPairM), pairs = 148 / 2;
+    const int n_m = (int)((N + kPairM - 1) / kPairM), pairs = b200_num_sms() / 2;
     const int64_t most = ((max_rows + kPairMaxN - 1) / kPairMaxN + E) * n_m;
     if (most < (1 << 30)) {
       const PairPlan pl = {kPairMaxN, 0, n_m, (int)(most < pairs ? most : pairs), 1, 0.f};

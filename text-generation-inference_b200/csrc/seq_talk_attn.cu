@@ -736,7 +736,7 @@ constexpr int kTalkPromptTokens = 24;  // average tokens per sequence from which
 // 145; 8 / 2 heads of 64, 24 behind 500 36 / 27, 64 behind 8000 77 / 141, 500 behind 8000 103 / 150; 16 / 8 heads of 64, 24 x 16 sequences behind 4000 108 / 127, a
 // prompt of 4000 beside 100 single tokens behind 1500 527 / 248.
 static bool talk_prompt_pays(int64_t T, int B, int H, int G, int d, int dv, int64_t keys, int QT, int nsplit) {
-  const int tokens = 128 / (H / G), sms = b200::pf_num_sms();
+  const int tokens = 128 / (H / G), sms = b200_num_sms();
   const int64_t row = 2ll * G * (d + dv), single = G * (T / tokens + B), items = single <= sms ? single : G * (T / (2 * tokens) + B);
   // us per key of the item that the SM is at; the memory's rate for pieces of 2 d bytes
   const float per_key = items == single ? (d == 128 ? 0.016f : 0.0125f) : (d == 128 ? 0.020f : 0.0156f);
@@ -797,11 +797,11 @@ static int launch_talk_prompt(const float* q, const void* cache, int64_t RW, int
   p.rep = H / G;
   p.tokens = 128 / p.rep;
   p.n_units = G;
-  p.pair = G * (T / p.tokens + B) <= b200::pf_num_sms() ? b200::kPfSingle : b200::kPfTiles;
+  p.pair = G * (T / p.tokens + B) <= b200_num_sms() ? b200::kPfSingle : b200::kPfTiles;
   p.n_groups = (int)(T / (p.pair == b200::kPfSingle ? p.tokens : 2 * p.tokens)) + B;  // upper bound of sum_b ceil(n_b / tokens); surplus items are passed over
   p.scale_log2 = scale * 1.4426950408889634f;
   const int64_t items = (int64_t)p.n_units * p.n_groups;
-  p.more_blocks = items > b200::pf_num_sms();
+  p.more_blocks = items > b200_num_sms();
   B200_LAUNCH((b200::attn_prompt_kernel<D, true>), dim3((unsigned)items), dim3(b200::kPfThreads), (size_t)C::kSmemBytes, st, *m, *m, *m, p);
   b200_count_launches(1);
   return B200_OK;
