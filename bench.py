@@ -1,12 +1,12 @@
 #!/usr/bin/env python
-"""bench.py — decode throughput of the TGIS continuous-batching hot path on B200 (contract in the task prompt / DESIGN.md).
+"""bench.py — decode throughput of the TGIS continuous-batching hot path on B200.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--workload NAME] [--impl reference] [--no-extra]
 
-Workloads (BASELINE.json):
+Workloads:
   llama3-8b-gptq   the north-star target "batched int4 Llama-8B decode at bs=64": Llama-3-8B (GQA-8) GPTQ int4 g128, bs=64,
                    seq 1024->2048, tensor parallel over N GPUs.  DEFAULT AT EVERY N: it is the one int4 model that shards at
-                   tp = 1/2/4/8 (SURVEY.md §8e), so the driver's 1/2/4/8 curve compares like with like.
+                   tp = 1/2/4/8, so the driver's 1/2/4/8 curve compares like with like.
   llama2-7b-gptq   config[2]: Llama-2-7B GPTQ int4, 1 GPU, bs=64, 1024->2048 (row-sharding stops at tp=2: 11008/tp % 128).
                    Measured in the same run at N=1 and reported under "extra".
   llama2-7b-fp16   config[3]: Llama-2-7B fp16, tensor parallel, bs=64.  Measured in the same run at N>1, under "extra".
@@ -59,7 +59,7 @@ WORKLOADS = {
     "tinyllama-fp16": ("tinyllama-1.1b", None, 32, 512, 1024),
     "tiny-test": ("tiny-test", None, 4, 32, 256),
 }
-# continuous-batching sessions (BASELINE config[4] and a single-GPU sibling): (arch, quantize, max batch, prompt range, output range,
+# continuous-batching sessions (Llama-3-70B over eight GPUs and a single-GPU sibling): (arch, quantize, max batch, prompt range, output range,
 # requests, Poisson arrivals per second)
 MIXED_WORKLOADS = {
     "llama3-70b-gptq-mixed": ("llama-3-70b", "gptq", 128, (256, 1024), (128, 512), 384, 60.0),
@@ -82,7 +82,7 @@ def peaks():
 
 class ClockSampler:
     """nvidia-smi clocks / throttle reasons sampled during the timed region (B200_PROFILING.md recipe).  Started well before
-    the timed region (nvidia-smi needs a second to enumerate an 8-GPU box); only samples between mark() and stop() count."""
+    the timed region (nvidia-smi needs a second to enumerate eight GPUs); only samples between mark() and stop() count."""
 
     FIELDS = ("clocks.sm,clocks.max.sm,clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
               "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
@@ -164,7 +164,7 @@ def run_reference(args, workload):
         "e2e": {"value": r["value"], "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
     if not args.no_extra and workload != "tiny-test":
-        try:  # BASELINE config[0]: gpt2 CausalLM fp32 CPU, bs=4, 128 -> 256 (whole model, really run; random-init: no weights here)
+        try:  # gpt2 CausalLM fp32 CPU, bs=4, 128 -> 256 (whole model, really run; random-init: no weights here)
             from oracle import causal_lm as ocl
             line["extra"] = {"config0_gpt2_cpu": ocl.time_decode_gpt2(4, 192, steps=8, warmup=2)}
         except Exception as e:  # noqa: BLE001
@@ -211,7 +211,7 @@ def make_batch_pb(B, L0, n_new, batch_id=0):
 
 
 def algorithmic_bytes_per_step(cfg, quantize, B, ctx, tp):
-    """SURVEY.md §8d formula, per GPU -> (whole step, attention KV read of one layer, linear weights incl. head)."""
+    """bytes a step cannot do without, per GPU -> (whole step, attention KV read of one layer, linear weights incl. head)."""
     H, I, V, nl = cfg.hidden_size, cfg.intermediate_size, cfg.vocab_size, cfg.num_hidden_layers
     d = H // cfg.num_attention_heads
     h, kv = cfg.num_attention_heads, cfg.num_key_value_heads
@@ -422,7 +422,7 @@ def measure_workload(args, workload, world, rank, full: bool):
 
 
 def run_mixed(args, workload):
-    """continuous batching with add-on prefills, driven through the shard's own Prefill / NextToken messages
+    """Continuous batching with add-on prefills, driven through the shard's own Prefill / NextToken messages
     by tools/router_sim.py (the Rust router's loop restated).  Decode-step and prefill throughput are reported separately."""
     import torch
     import torch.distributed as dist
@@ -621,7 +621,7 @@ def run_gpu(args, workload):
         line["roofline"] = main["roofline"]
     extra = {}
     if not args.no_extra and args.workload is None:
-        other = "llama2-7b-gptq" if world == 1 else "llama2-7b-fp16"  # BASELINE config[2] / config[3]
+        other = "llama2-7b-gptq" if world == 1 else "llama2-7b-fp16"
         try:
             r = measure_workload(args, other, world, rank, full=False)
             extra[other] = {k: r[k] for k in ("value", "ms_per_step", "mean_context_timed", "step_roofline", "prefill", "e2e", "clocks",

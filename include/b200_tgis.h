@@ -1,13 +1,13 @@
 /* b200_tgis.h — C ABI of the B200-native TGIS decode hot path (libb200_tgis.so).
  *
- * Conventions (SURVEY.md §8b "Op / C-ABI"):
+ * Conventions:
  *   - plain pointers and sizes only; every pointer is a DEVICE pointer unless it says "host"
  *   - every call only ENQUEUES work on `stream` (a cudaStream_t passed as void*): no host synchronisation, no
  *     allocation — outputs and workspaces are caller-provided; all entry points are CUDA-graph capturable
  *   - returns 0 (B200_OK) or a negative error code; b200_last_error() gives the message (thread-local)
  *   - fp16 tensors are row-major `__half`; token-major activations [T, features]
  * Each entry point names the reference interface it replaces (paths under
- * /root/reference/server/text_generation_server/).
+ * server/text_generation_server/).
  */
 #ifndef B200_TGIS_H_
 #define B200_TGIS_H_
@@ -70,7 +70,7 @@ int b200_rmsnorm_residual(const void* h, const void* residual, const void* gamma
  * qkv [T, (n_heads + 2 n_kv) * d] is rotated in place (q and k parts); k and v are scattered into the pools at
  * slot_mapping[t] = block * 16 + offset (negative = skip).  cos/sin: fp16 tables [max_pos, d/2] indexed by
  * position_ids (utils/layers.py:453-464).  Pool layout: [num_blocks][n_kv][16][d] fp16, 16-byte chunks XOR-swizzled
- * by (token & 7) (DESIGN.md "KV page layout"). */
+ * by (token & 7) (the layout of utils/paged.py). */
 int b200_rope_kv_write_paged(void* qkv, const void* cos, const void* sin, const int64_t* position_ids,
                              const int64_t* slot_mapping, void* k_pool, void* v_pool, int64_t T, int n_heads, int n_kv_heads,
                              int head_dim, void* stream);
@@ -191,7 +191,7 @@ int b200_gemm_bf16(const void* x, const void* w, const void* bias, void* y, int 
                    void* stream);
 
 /* one-time conversion of the GPTQ checkpoint tensors of one linear into the kernel's streaming layout ("unit records":
- * one contiguous 8 KB + meta block per (128-feature tile, 128-wide k-block), DESIGN.md §2); replaces
+ * one contiguous 8 KB + meta block per (128-feature tile, 128-wide k-block)); replaces
  * exllamav2_kernels.make_q_matrix (utils/gptq/exllamav2.py:23-62), `packed` plays the role of its q_handle.
  * qweight int32 [K/8, N], qzeros int32 [ceil(K/g), N/8], scales fp16 [ceil(K/g), N] in checkpoint layout (read only; the
  * caller may free them afterwards).  groupsize: 32, 64, a multiple of 128, or <= 0 for one group; groups are

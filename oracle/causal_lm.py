@@ -1,14 +1,14 @@
-"""ORACLE / CPU BASELINE (test + measurement infrastructure only — never imported by the product path).
+"""Oracle and CPU baseline (test + measurement infrastructure only — never imported by the product path).
 
 Restates the reference's own CPU path for this workload: `CausalLM.generate_token` on the `hf_transformers` engine
-(/root/reference/server/text_generation_server/models/causal_lm.py:548-739, inference_engine/hf_transformers.py:11-78):
+(server/text_generation_server/models/causal_lm.py:548-739, inference_engine/hf_transformers.py:11-78):
 a left-padded rectangular batch, HF `AutoModelForCausalLM.forward` in fp32 with a growing KV cache
 (`past_key_values`, causal_lm.py:612-634), greedy `argmax` on the last position (utils/tokens.py:44-46), wall clock
 around `model.forward` exactly as causal_lm.py:631-633.  The reference pins transformers 4.40.2 (tuple KV cache);
 this image has 5.x, so the cache object is HF's DynamicCache — same arithmetic, same O(KV) growth per step.
 
 Used by bench.py for `cpu_baseline` and for the `--impl reference` arm ("port": the reference's Python cannot be imported
-unmodified here, SURVEY.md §8c).  Bounded sample: a few layers of the named architecture at full width, scaled to
+unmodified here).  Bounded sample: a few layers of the named architecture at full width, scaled to
 the full depth by a two-point fit (1 layer vs 1 + sample_layers).
 """
 from __future__ import annotations
@@ -95,7 +95,7 @@ def time_decode(arch: str, B: int, ctx: int, steps: int, warmup: int, sample_lay
 
 
 def time_decode_gpt2(B: int = 4, ctx: int = 192, steps: int = 8, warmup: int = 2) -> dict:
-    """the reference's CPU CausalLM path on gpt2 (124M: 12 layers, 768 wide, 12 heads, vocab 50257), fp32,
+    """The reference's CPU CausalLM path on gpt2 (124M: 12 layers, 768 wide, 12 heads, vocab 50257), fp32,
     bs = 4, sequence 128 -> 256 (mid context 192), greedy - integration_tests/test_cases_gpt2.yaml runs this model through the
     same path.  The whole model is run (no extrapolation); weights are random-init (no checkpoint in the image), which does not
     change the arithmetic per step."""
@@ -124,5 +124,5 @@ def time_decode_gpt2(B: int = 4, ctx: int = 192, steps: int = 8, warmup: int = 2
                 times.append(dt)
     times.sort()
     t = times[len(times) // 2]
-    return {"workload": "gpt2 CausalLM fp32 CPU, bs=4, seq 128->256 (BASELINE config[0])", "value": B / t, "unit": "tokens/s",
+    return {"workload": "gpt2 CausalLM fp32 CPU, bs=4, seq 128->256", "value": B / t, "unit": "tokens/s",
             "ms_per_step": t * 1e3, "steps_timed": steps, "cores": cores, "extrapolated": False, "weights": "random-init"}

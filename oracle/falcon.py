@@ -1,6 +1,6 @@
 """CPU oracle (test infrastructure only) for the flash Falcon / RefinedWeb graph (multi-query and grouped-query attention).
 
-Restates /root/reference/server/text_generation_server/models/custom_modeling/flash_rw_modeling.py with the fp16 rounding
+Restates server/text_generation_server/models/custom_modeling/flash_rw_modeling.py with the fp16 rounding
 points of its fused ops, in its three layer forms:
   * "RefinedWebModel" with parallel_attn (Falcon-7B, FlashRWLayer :339-356): ONE LayerNorm feeds attention and MLP, their
     outputs are added in fp16 and re-enter the residual stream through the next layer's fused residual add;

@@ -95,7 +95,7 @@ def gemm_half_q_half(x: torch.Tensor, qweight, qzeros, scales, g_idx=None, group
 
 
 def quantize_rtn(weight_nk: torch.Tensor, groupsize: int = 128, seed: int | None = None):
-    """Synthetic-checkpoint helper (SURVEY.md §8d): round-to-nearest group quantization of an
+    """Synthetic-checkpoint helper: round-to-nearest group quantization of an
     fp W[N,K] (nn.Linear layout) into reference-format tensors
     (qweight [K/8,N], qzeros [K/g,N/8], scales [K/g,N] fp16, g_idx [K]).
     Packing identical to QuantLinear.pack (quant_linear.py:290-345)."""
@@ -123,7 +123,7 @@ def _np(t):
 
 
 # --------------------------------------------------------------------------------------
-# The product's packed weight stream (DESIGN.md §2), restated with plain numpy so that tests can
+# The product's packed weight stream, restated with plain numpy so that tests can
 # (a) compare what b200_gptq_pack writes and (b) check, on a CPU, that the kernel's register
 # arithmetic on those records is bit-identical to `dequantize` above.
 # --------------------------------------------------------------------------------------

@@ -2,10 +2,10 @@
 
 CPU restatement (PyTorch, fp32 arithmetic with fp16 rounding exactly where the reference rounds)
 of the reference's FlashLlama decode/prefill hot path.  Each function cites the reference lines
-it follows (paths relative to /root/reference/server/text_generation_server/).
+it follows (paths relative to server/text_generation_server/).
 
 The GPU kernels that the reference calls here are third-party and un-vendored (flash-attn 2.5.6
-`flash_attn_2_cuda`, `dropout_layer_norm`, `rotary_emb`; SURVEY.md §8c), and no reference test pins
+`flash_attn_2_cuda`, `dropout_layer_norm`, `rotary_emb`), and no reference test pins
 their results: for those ops the status is "PARITY UNPINNED" — the arithmetic below restates their
 published behaviour (fp32 statistics / fp32 softmax, fp16 I/O) and is anchored on
   (a) the reference's own call sites, and
@@ -349,11 +349,11 @@ class LlamaOracle:
 
 
 # --------------------------------------------------------------------------------------
-# synthetic checkpoints (SURVEY.md §8d) and TP slicing (utils/weights.py:79-201)
+# synthetic checkpoints and TP slicing (utils/weights.py:79-201)
 # --------------------------------------------------------------------------------------
 def make_state_dict(cfg: LlamaConfig, seed: int = 1234, quantize: Optional[str] = None,
                     groupsize: int = 128, std: float = 0.02, act_order: bool = False) -> Dict[str, torch.Tensor]:
-    """HF-named tensors (SURVEY.md Appendix D). quantize='gptq' -> reference-format int4 tensors.
+    """HF-named tensors. quantize='gptq' -> reference-format int4 tensors.
     act_order: every linear gets a shuffled g_idx (rows assigned to groups at random, `groupsize` rows each); projections
     that the loader fuses (q/k/v, gate/up) share one, as utils/weights.py:131-135 requires."""
     g = torch.Generator().manual_seed(seed)

@@ -1,6 +1,6 @@
 """CPU oracle (test infrastructure only) for the flash GPT-NeoX graph.
 
-Restates /root/reference/server/text_generation_server/models/custom_modeling/flash_neox_modeling.py with the fp16
+Restates server/text_generation_server/models/custom_modeling/flash_neox_modeling.py with the fp16
 rounding points of its fused ops: FastLayerNorm = residual add + LayerNorm with fp32 statistics (utils/layers.py:360-392 ->
 dropout_layer_norm), QKV re-layout [h, 3, d] -> [3, h, d] (:57-80), partial half-split rotary with fp16 tables
 (utils/layers.py:436-472; rotary_dim = cos.shape[-1] * 2), varlen causal / decode attention (utils/flash_attn.py:43-127),
@@ -69,7 +69,7 @@ def linear(x, w, b):
 
 
 def make_state_dict(cfg: NeoXConfig, seed: int = 1234, std: float = 0.02) -> Dict[str, torch.Tensor]:
-    """HF-named GPT-NeoX tensors (SURVEY.md Appendix D), QKV rows head-interleaved [h, 3, d] as in the checkpoints."""
+    """HF-named GPT-NeoX tensors, QKV rows head-interleaved [h, 3, d] as in the checkpoints."""
     g = torch.Generator().manual_seed(seed)
 
     def rnd(*shape, s=std):

@@ -1,6 +1,6 @@
 """CPU oracle (test infrastructure only) for the flash Santacoder / StarCoder (gpt_bigcode, multi-query attention) graph.
 
-Restates /root/reference/server/text_generation_server/models/custom_modeling/flash_santacoder_modeling.py with the fp16
+Restates server/text_generation_server/models/custom_modeling/flash_santacoder_modeling.py with the fp16
 rounding points of its fused ops: token + learned position embedding added in fp16 (:383-386), FastLayerNorm = residual add
 + LayerNorm with fp32 statistics (utils/layers.py:360-392), the fused `c_attn` projection [q heads | k | v] with ONE key /
 value head shared by every query head (:214-224), varlen causal / decode attention (utils/flash_attn.py:43-127), GELU

@@ -2,9 +2,9 @@
 //
 // Replaces: utils/flash_attn.py:43-127 `attention(...)` in its decode form (flash_llama_modeling.py:285-295,
 // flash_attn_2_cuda.varlen_fwd with max_s_q = 1, causal = False) and fms-extras `paged_attention_v1/v2`
-// (paged_llama_modeling.py:267) of /root/reference/server/text_generation_server.
+// (paged_llama_modeling.py:267) of server/text_generation_server.
 //
-// Design (DESIGN.md §kernels/attn_decode):
+// Design:
 //   * work item = (sequence b, kv head, 512-token chunk): split-KV so B*h_kv*chunks >> 148 SMs, 2 CTAs/SM
 //   * KV pages [16 tokens][d] fp16 are stored in HBM already XOR-swizzled; a producer warp streams them with
 //     cp.async.bulk (TMA, one 2-4 KB copy per page-head tile for K and V) into a 3/4-stage ring, mbarrier-tracked

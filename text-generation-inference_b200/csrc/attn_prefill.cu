@@ -1,11 +1,11 @@
 // Varlen causal prefill attention over the fresh (un-paged) q/k/v of the step.
 //
 // Replaces: utils/flash_attn.py:43-127 `attention(q, k, v, cu_seqlens, max_s, softmax_scale)` in its prefill form
-// (flash_llama_modeling.py:271-278; flash_attn_2_cuda.varlen_fwd, causal) of /root/reference/server/text_generation_server.
+// (flash_llama_modeling.py:271-278; flash_attn_2_cuda.varlen_fwd, causal) of server/text_generation_server.
 //
 // 64 query rows per CTA (4 warps x 16 rows), 64-key tiles double-buffered with cp.async into XOR-swizzled shared
 // memory, m16n8k16 HMMA with fp32 accumulators, fp32 online softmax, P rounded to fp16 before P.V (flash-attn semantics).
-// Round-1 kernel: correct and tensor-core based; the tcgen05/TMEM version is the planned successor.
+// m16n8k16 products; prompts over the paged pool take the tcgen05 kernel of attn_prompt.cuh.
 #include "common.cuh"
 
 namespace b200 {

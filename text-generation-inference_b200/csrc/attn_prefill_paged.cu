@@ -1,11 +1,11 @@
 // Prefill / chunked-prefill attention over the PAGED KV pool on the 5th-generation tensor cores.
 //
 // Replaces: utils/flash_attn.py:43-127 `attention(q, k, v, cu_seqlens, max_s, softmax_scale)` in its prefill form
-// (flash_llama_modeling.py:271-278; flash_attn_2_cuda.varlen_fwd, causal) of /root/reference/server/text_generation_server, and
+// (flash_llama_modeling.py:271-278; flash_attn_2_cuda.varlen_fwd, causal) of server/text_generation_server, and
 // the prefill half of the paged twin (paged_llama_modeling.py:253-264).  Unlike the reference's prefill it reads K and V from the
 // block pool (the step's own tokens have just been appended by b200_rope_kv_write_paged), so the queries of a step may follow a
 // CACHED context: query i of sequence b sits at absolute position context_lens[b] - n_q(b) + i and attends keys 0 .. that position.
-// That is what an add-on prefill over a prompt prefix, a chunked prefill and a mixed prefill + decode step need (SURVEY.md §8 f1).
+// That is what an add-on prefill over a prompt prefix, a chunked prefill and a mixed prefill + decode step need.
 //
 // The kernel and its design: attn_prompt.cuh.
 #include "attn_prompt.cuh"

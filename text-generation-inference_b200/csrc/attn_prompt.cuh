@@ -3,15 +3,16 @@
 //   token-major pages of bfloat16 rows [... keys of all key heads ... | ... values ...], queries and results fp32, a chunked mask and / or a
 //   sliding window, sink logits (seq_talk_attn.cu).
 //
-// Design (12 warps, one CTA per SM).  A block takes its own item and then those of blocks that have not started (cluster launch control), longest
-// first: with items dealt out in turn the SMs were busy for 75 % of the time on ragged prompts.  An item is TWO query tiles of 128 rows that meet the same keys, so that the tensor cores work for
+// Design (12 warps, one CTA per SM).  A block takes its own item and then those of blocks that have not started (cluster launch control): with items
+// dealt out in turn the SMs were busy for 75 % of the time on ragged prompts.  Head-major items come longest first; token-major ones from the step's
+// last tile backwards, which is longest first within a sequence (and within a chunk).  An item is TWO query tiles of 128 rows that meet the same keys, so that the tensor cores work for
 // one while the other is in its soft-max: two query heads of a key / value head when their number is even, else two neighbouring query tiles
 // of a head.  While every tile can have an SM to itself it does (the second tile of an item is empty): two soft-max warpgroups slow each
 // other down.  Back to back, us, one query tile of one head per CTA / two / this:
 // one prompt of 100 tokens, 32 / 8 heads, d = 128 6.8 / 8.0 / 6.8, of 300 11.2 / 12.3 / 10.7; 32 / 4 heads, d = 64, 129 tokens 7.1 / 8.2 / 6.8.
 //   warp 0      TMA producer.  Q tiles [128 x d] through a 128B-swizzled tensor map; per 128-key tile 8 KV pages x (K, V) x d/64
 //               slabs, each one cp.async.bulk.tensor box [16 tokens x 64 halves] of the pool: the pool stores every token row
-//               with its 16-byte chunks XOR-swizzled by (token & 7) (DESIGN.md §2), which IS the tcgen05 SWIZZLE_128B image, so
+//               with its 16-byte chunks XOR-swizzled by (token & 7), which IS the tcgen05 SWIZZLE_128B image, so
 //               pages land in shared memory ready for the tensor core without any software swizzle.  2-stage rings of K and V.
 //   warp 1      MMA issuer (one elected thread): P0 V, Q0 K of the next key tile, P1 V, Q1 K of the next key tile, and so on.
 //               S = Q K^T: tcgen05.mma kind::f16, both operands K-major from shared memory, fp32 accumulator in TMEM.

@@ -2,7 +2,7 @@
 // applying per-request parameters.
 //
 // Replaces, for one step of a batch, the torch op chain of HeterogeneousNextTokenChooser.__call__
-// (/root/reference/server/text_generation_server/utils/tokens.py:238-271): the min_new_tokens EOS mask (:242-246) and the length
+// (server/text_generation_server/utils/tokens.py:238-271): the min_new_tokens EOS mask (:242-246) and the length
 // penalty (:247-252), HeterogeneousRepetitionPenaltyLogitsProcessor (utils/logits_process.py:93-143), the temperature, top-k and
 // top-p warpers (:146-176, :241-317, :179-238), Greedy / per-request Sampling (tokens.py:30-46, 49-78) and the log_softmax /
 // rank of get_token_info (:388-425).  Rows with typical-p or top-n details stay on the host-side torch path.

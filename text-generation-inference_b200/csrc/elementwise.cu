@@ -1,7 +1,7 @@
 // HBM-bound row kernels of the decode step: fused residual-add + RMSNorm, RoPE + paged KV write,
 // SiLU*mul, vocabulary-parallel embedding gather, greedy arg-max.
 //
-// Reference ops replaced (paths under /root/reference/server/text_generation_server/):
+// Reference ops replaced (paths under server/text_generation_server/):
 //   rmsnorm_residual ......... dropout_layer_norm.dropout_add_ln_fwd, models/custom_modeling/flash_llama_modeling.py:132-148
 //   rope_kv_write_paged ...... rotary_emb.apply_rotary (utils/layers.py:466-472) + KV append
 //                              (flash_llama_modeling.py:268,282) / fms-extras reshape_and_cache (paged_llama_modeling.py:250)
@@ -17,7 +17,7 @@ namespace b200 {
 
 // ------------------------------------------------------------------------------------------------
 // residual-add + RMSNorm.  One CTA per token row; 8 halves (16 B) per thread per iteration.
-// fp32 statistics on the un-rounded sum (SURVEY.md Appendix A.2).
+// fp32 statistics on the un-rounded sum.
 // Optional split-K input: `h` may be `n_parts` fp32 partial matrices [n_parts][T][H] (gemm split-K
 // workspace); they are summed and rounded to fp16 first, which is exactly the GEMM's fp16 output.
 // ------------------------------------------------------------------------------------------------

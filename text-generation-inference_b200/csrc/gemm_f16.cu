@@ -1,7 +1,7 @@
 // fp16 linear  Y[T,N] = X[T,K] . W[N,K]^T  (fp32 accumulate, fp16 out) on tcgen05 tensor cores.
 //
 // Replaces the cuBLAS HGEMM behind `FastLinear.forward` / `TensorParallelHead.forward`
-// (/root/reference/server/text_generation_server/utils/layers.py:110-111, 257-262).
+// (server/text_generation_server/utils/layers.py:110-111, 257-262).
 //
 // Swap-AB: the 128 output features of a weight tile are the UMMA M dimension (A operand, K-major, streamed
 // from HBM once by TMA with 128B swizzle), the step's tokens are the UMMA N dimension (B operand, TN = 16..256),

@@ -2,7 +2,8 @@
 // accumulator tile, persistent over the tiles of the output.
 //
 // Used by gemm_f16.cu (fp16 / bfloat16 weights) and gemm_w4a16.cu (GPTQ int4 weights, de-quantised into shared memory) for calls of more
-// tokens than their weight-streaming kernels are good at.  Bound: the tensor pipe (an m256 n256 k16 product takes the pair 128 cycles) and,
+// tokens than their weight-streaming kernels are good at, and by seq_group_gemm.cu for routed experts with many rows each (row tiles of one expert,
+// found from the plan's offsets).  Bound: the tensor pipe (an m256 n256 k16 product takes the pair 128 cycles) and,
 // close behind it, the L2 -> shared-memory path.
 //
 //   * Swap-AB: features are the UMMA M dimension (each CTA of the pair holds 128 of the 256), tokens its N dimension.  A CTA stages its own

@@ -2,7 +2,7 @@
 // straight into TMEM (no fp16 scratch matrix, for any T).  This kernel takes calls of up to 128 tokens (kW4DecodeT), gemm_pair.cuh larger ones.
 //
 // Replaces `exllamav2_kernels.make_q_matrix` / `gemm_half_q_half`
-// (/root/reference/server/text_generation_server/utils/gptq/exllamav2.py:14-62,139-144), including its M > 50
+// (server/text_generation_server/utils/gptq/exllamav2.py:14-62,139-144), including its M > 50
 // "dequantise everything to temp_dq, then cuBLAS" branch (:87), and follows the dequant formula of record
 // utils/gptq/quant_linear.py:184-192:  W[k,n] = fp16( scales[g,n] * (q[k,n] - (qzeros[g,n] + 1)) ).
 //

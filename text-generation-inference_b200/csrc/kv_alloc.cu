@@ -1,7 +1,7 @@
 // Paged KV block allocator (host side, C++) and the device-side per-step bookkeeping kernel.
 //
 // Replaces the un-vendored fms-extras `PagedKVCacheManager` block bookkeeping used by
-// /root/reference/server/text_generation_server/models/paged_causal_lm.py:338-353 and utils/paged.py:92-134
+// server/text_generation_server/models/paged_causal_lm.py:338-353 and utils/paged.py:92-134
 // (allocate_tokens / free_sequences; block size 16).  The allocator is a LIFO free list of block ids; the
 // per-sequence block lists live in the Python manager (utils/paged.py of this package).
 #include "common.cuh"

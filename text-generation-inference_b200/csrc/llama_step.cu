@@ -2,7 +2,7 @@
 // Python host pays one FFI call per step and the sequence is CUDA-graph capturable.
 //
 // Restates the op order of FlashLlamaModel.forward / FlashLlamaLayer.forward / FlashLlamaAttention.forward / LlamaMLP.forward
-// (/root/reference/server/text_generation_server/models/custom_modeling/flash_llama_modeling.py:425-497, 356-389, 240-297,
+// (server/text_generation_server/models/custom_modeling/flash_llama_modeling.py:425-497, 356-389, 240-297,
 // 332-335) and FlashLlamaForCausalLM.forward (:514-540) over the kernels of this library.
 //
 // Two things move between kernels at decode sizes (T <= 128), without changing any result bit:

@@ -1,11 +1,11 @@
 // One-shot all-reduce over NVLink peer memory for the tensor-parallel layer boundary.
 //
 // Replaces (default for decode-sized messages; B200_P2P_ALLREDUCE=0 keeps NCCL): torch.distributed.all_reduce after the row-parallel o_proj / down_proj and the
-// vocab-parallel embedding (/root/reference/server/text_generation_server/utils/layers.py:303-306 TensorParallelRowLinear,
+// vocab-parallel embedding (server/text_generation_server/utils/layers.py:303-306 TensorParallelRowLinear,
 // :343-345 TensorParallelEmbedding; flash_llama_modeling.py:296, :335) for the decode-sized messages of the step
 // (bs 64 x hidden 4096 fp16 = 512 KB): NCCL costs 10-15 us per call there, twice per layer.
 //
-// Validated on a 2-GPU B200 box in round 2 (tests/test_gpu_p2p.py, tests/test_gpu_tp.py; profiles/r2_tp2_and_splitk_validation.txt).
+// Validated on two B200 (tests/test_gpu_p2p.py, tests/test_gpu_tp.py; profiles/r2_tp2_and_splitk_validation.txt).
 //
 // Design.  Every rank owns a *window* in its own HBM, allocated here with cudaMalloc and exported over CUDA IPC:
 //     [kBlocks][kMaxWorld] u32 arrival flags | [kBlocks] u32 epochs | pad to 4 KB | 2 slots x max_bytes of fp16 data
@@ -352,7 +352,7 @@ __global__ void p2p_fill_kernel(uint4* p, int64_t n, uint32_t word) {
 }
 
 // ------------------------------------------------------------------------------------------------------------------
-// Tensor-parallel greedy head without the logits all-gather (SURVEY.md §5; replaces TensorParallelHead's
+// Tensor-parallel greedy head without the logits all-gather (replaces TensorParallelHead's
 // all_gather_into_tensor of [T, V/tp] fp16 per rank, utils/layers.py:249-269, followed by Greedy's argmax, utils/tokens.py:44-46,
 // for all-greedy batches): every rank takes the arg-max of its own vocabulary shard, the (value, index) pairs cross NVLink
 // (8 bytes per row and rank instead of V/tp logits), and every rank picks the same winner: the largest value, ties to the

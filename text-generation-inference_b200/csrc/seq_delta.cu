@@ -303,7 +303,8 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
 
 // The memory's rows lie over kRowLanes lanes, NR each (dk <= kRowLanes NR).  Sixteen lanes and eight columns per warp take fewer instructions; 32 lanes
 // and four columns put twice as many warps on a small grid and shorten the chain from four tokens to the next four, which is what bounds it
-// then.  Measured on B200 (us, 16 / 32 lanes, heads of 128 x 128): 16 heads, 690 tokens 251 / 180, 4 sequences of 256 to 768 281 / 257, 2 of 125 55 / 46;
+// then.  (A sequence's sums are added in another order on either side of the line, so its result depends on how many others share the step, by
+// rounding.)  Measured on B200 (us, 16 / 32 lanes, heads of 128 x 128): 16 heads, 690 tokens 251 / 180, 4 sequences of 256 to 768 281 / 257, 2 of 125 55 / 46;
 // 32 heads, 400 tokens 164 / 134, 8 x 500 557 / 707, 6 of 400 to 800 681 / 775; 16 heads, 16 x 250 305 / 401.
 template <int NR, int kRowLanes>
 __global__ void __launch_bounds__(256, NR * kRowLanes <= 128 ? 2 : 1) delta_chunk_kernel(
@@ -781,7 +782,9 @@ extern "C" int b200_seq_delta_rows_scan(const float* pre, int channels, float* S
 #undef DST
   }
   const int vec = (dk % 4 == 0 && dv % 4 == 0 && aligned) ? 1 : 0;
-  // 64 columns per block share each staged vector among more of the memory; a small grid is spread over 32 columns and 32 lanes
+  // 64 columns per block share each staged vector among more of the memory; a small grid is spread over 32 columns and 32 lanes.  The line lies where
+  // ragged prompts gain by it still (4 of 256 to 768 tokens, 256 blocks, 281 -> 257 us); between 149 and 296 blocks equal ones lose (2 x 500 tokens, 32
+  // heads, 197 -> 209, 3 x 150 of 16 heads 68 -> 70), and the host does not know the lengths.
   const bool small = (int64_t)B * H * ((dv + 31) / 32) <= 2 * 148;
   const int most = small ? 32 : 64;
   const int blocks = (dv + most - 1) / most;

@@ -3,7 +3,7 @@
 Only the hot-path branch exists: a flash decoder family served by `FlashCausalLM` over the paged KV pool.  FLASH_ATTENTION /
 PAGED_ATTENTION (models/__init__.py:15-16) both select it - the KV cache here is always paged -, `deployment_framework` is
 forced to `tgis_native` as the reference does for those modes (:48-54, :95-101), and anything else (seq2seq, the non-flash
-`CausalLM` path, other engines) raises: that code is outside the scope of this library (DESIGN.md §1).
+`CausalLM` path, other engines) raises: that code is outside the scope of this library.
 """
 import os
 from typing import Optional

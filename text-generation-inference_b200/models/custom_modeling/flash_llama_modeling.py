@@ -1,6 +1,6 @@
 """FlashLlama on the B200 step runtime.
 
-Mirrors /root/reference/server/text_generation_server/models/custom_modeling/flash_llama_modeling.py: same module
+Mirrors server/text_generation_server/models/custom_modeling/flash_llama_modeling.py: same module
 tree and constructor contract `FlashLlamaForCausalLM(config, weights)` (:499-512), same `forward` positional
 signature (:514-540) and op order (:240-297, 332-335, 356-389, 425-497).  Differences, all storage-only:
   * `past_key_values` is a `PagedKVState` over the model's block pool (utils/paged.py) instead of a contiguous

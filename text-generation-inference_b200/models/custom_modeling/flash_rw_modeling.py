@@ -1,7 +1,7 @@
 """Flash Falcon / RefinedWeb on the B200 kernels: multi-query (Falcon-7B) and grouped-query (Falcon-40B) attention, full-head
 rotary embedding, LayerNorm, exact GELU, attention and MLP in parallel off one or two LayerNorms.
 
-Mirrors /root/reference/server/text_generation_server/models/custom_modeling/flash_rw_modeling.py: `load_row` (:20-33),
+Mirrors server/text_generation_server/models/custom_modeling/flash_rw_modeling.py: `load_row` (:20-33),
 `RWConfig` (:36-118), `FlashRWAttention` (:121-214), `FlashRWLargeAttention` (:217-323), `FlashMLP` (:326-345), `FlashRWLayer`
 (:348-433), `FlashRWLargeLayer` (:436-492), `FlashRWModel` (:499-603), `FlashRWForCausalLM` (:606-648) — same class names,
 constructor arguments and `forward` signature.  Differences, as for the other flash families here: `past_key_values` is the

@@ -1,7 +1,7 @@
 """Flash Santacoder / StarCoder (gpt_bigcode) on the B200 kernels: multi-query attention — ONE key / value head shared by
 every query head and replicated on every tensor-parallel rank —, learned position embeddings, LayerNorm, GELU, tied head.
 
-Mirrors /root/reference/server/text_generation_server/models/custom_modeling/flash_santacoder_modeling.py: `load_multi_mqa`
+Mirrors server/text_generation_server/models/custom_modeling/flash_santacoder_modeling.py: `load_multi_mqa`
 (:19-159: this rank's block of query rows followed by the shared 2 * head_size key / value rows, for fp16 and GPTQ
 checkpoints), `load_col` / `load_row` (:162-190), `FlashMQAttention` (:193-268), `MLP` (:271-300), `Block` (:303-347),
 `FlashSantacoderModel` (:350-432), `FlashSantacoderForCausalLM` (:435-478) — same class names, constructor arguments and

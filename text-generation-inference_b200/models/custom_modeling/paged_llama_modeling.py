@@ -1,6 +1,6 @@
 """The paged calling convention of the Llama graph.
 
-Mirrors /root/reference/server/text_generation_server/models/custom_modeling/paged_llama_modeling.py:427-462
+Mirrors server/text_generation_server/models/custom_modeling/paged_llama_modeling.py:427-462
 (`PagedLlamaForCausalLM`: `forward(input_ids, position_ids, cache_data, inputs_embeds=None, return_embeds=False)`,
 `get_kv_cache_block_size`, `get_input_embeddings`) on top of the same C++ step runtime and kernels as the flash
 convention (flash_llama_modeling.py of this package): the two conventions differ only in how the per-step indices arrive.

@@ -9,7 +9,7 @@
    batch the whole step is replayed as a CUDA graph.  FlashLlama implements the protocol with the C++ step runtime
    (csrc/llama_step.cu); `PythonFusedGreedy` implements it by enqueuing the family's ordinary decode forward, whose torch
    temporaries then come from the graph's private pool.  On by default on a single rank (validated on B200 for GPT-NeoX and
-   Santacoder, round 2); sharded models take it with B200_PY_FUSED_STEP=1 only (NCCL inside the captured graph), and
+   Santacoder); sharded models take it with B200_PY_FUSED_STEP=1 only (NCCL inside the captured graph), and
    B200_PY_FUSED_STEP=0 turns it off.
 """
 from __future__ import annotations

@@ -1,6 +1,6 @@
 """Ragged (un-padded) continuous-batching model runtime over the paged KV cache.
 
-Mirrors /root/reference/server/text_generation_server/models/flash_causal_lm.py: `FlashCausalLMBatch`
+Mirrors server/text_generation_server/models/flash_causal_lm.py: `FlashCausalLMBatch`
 (:28-62) with `from_pb` (:68-194), `concatenate` (:197-285), `prune` (:291-353); `FlashCausalLM.generate_token`
 (:405-460) and the token post-processing (:462-588) — same signatures, same in-place batch mutation, same results.
 What changes is storage only: KV lives in the model's block pool (`kv_cache_manager`, like the reference's

@@ -1,10 +1,10 @@
 """`Model` ABC: what the shard server drives.
 
-Mirrors /root/reference/server/text_generation_server/models/model.py:34-221 for the attributes the server reads
+Mirrors server/text_generation_server/models/model.py:34-221 for the attributes the server reads
 (`batch_type`, `tokenizer`, `dtype`, `device`, `word_embeddings`, `prefix_cache`, `use_position_ids`,
 `context_manager`, `engine`, `config`, `model`; server.py:82,106,131-139,326-332) and `generate_token` /
 `get_indices_to_keep` (:169-188).  PT2 compile wrappers (:97-157) and the prompt-prefix cache (:47-90) are out of
-scope (SURVEY.md §2.1 rows 22-23): `prefix_cache` is None and requests with a prefix_id get a GenerateError.
+scope: `prefix_cache` is None and requests with a prefix_id get a GenerateError.
 """
 from __future__ import annotations
 

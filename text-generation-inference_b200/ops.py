@@ -247,7 +247,7 @@ def permute_columns(x: torch.Tensor, perm: torch.Tensor) -> torch.Tensor:
 
 def gptq_pack(qweight: torch.Tensor, qzeros: torch.Tensor, scales: torch.Tensor, groupsize: int,
               layout: int = W4_LAYOUT_PLAIN, row_perm: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """Checkpoint GPTQ tensors of one linear -> the kernel's unit-record stream (uint8 tensor).
+    """Checkpoint GPTQ tensors of one linear -> the kernel's unit-record stream (uint8 tensor; format in csrc/gemm_w4a16.cu).
     layout = W4_LAYOUT_GATE_UP pairs gate tile s with up tile s (fused [gate; up] projection, N = 2 I, I % 128 == 0)."""
     _req(qweight, torch.int32, "qweight")
     _req(qzeros, torch.int32, "qzeros")
@@ -372,7 +372,7 @@ def splitk_silu_mul(parts: SplitK) -> torch.Tensor:
 
 
 # ------------------------------------------------------------------------------------------------------
-# KV pool helpers (layout documented in DESIGN.md; used by tests and the block manager)
+# KV pool helpers (layout: utils/paged.py; used by tests and the block manager)
 # ------------------------------------------------------------------------------------------------------
 def kv_pool_alloc(num_blocks: int, n_kv_heads: int, head_dim: int, device) -> Tuple[torch.Tensor, torch.Tensor]:
     shape = (num_blocks, n_kv_heads, PAGE, head_dim)

@@ -1,6 +1,6 @@
 """`generate.v1` protobuf messages and the TextGenerationService gRPC surface, built at run time.
 
-The reference generates `text_generation_server/pb/generate_pb2(_grpc).py` from /root/reference/proto/generate.proto
+The reference generates `text_generation_server/pb/generate_pb2(_grpc).py` from proto/generate.proto
 with grpc_tools at install time (server/Makefile:7-17); neither protoc nor grpc_tools exists in this image, so the same
 descriptors are constructed here programmatically.  Field names, numbers, types, labels and proto3 `optional`
 presence are identical to proto/generate.proto:5-224 (pinned by tests/test_pb.py against a fixture extracted from

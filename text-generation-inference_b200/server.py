@@ -1,11 +1,11 @@
 """Shard server: the router-facing `generate.v1.TextGenerationService` over `unix://{uds_path}-{rank}`.
 
-Thin re-host of /root/reference/server/text_generation_server/server.py:58-249 (servicer: batch cache keyed by batch id,
+Thin re-host of server/text_generation_server/server.py:58-249 (servicer: batch cache keyed by batch id,
 prune -> concatenate -> `generate_token`, health batch id 2^64-1 never cached, OOM -> RESOURCE_EXHAUSTED) and :251-441
 (`serve`: one process per GPU, rank 0 answers ServiceDiscovery with every shard's URL), plus `cache.py:8-33`.
 Same message semantics, so the unchanged Rust router (`router/client/src/sharded_client.rs`) drives it.  Model loading
 is `FlashCausalLM` only (the hot-path model class); `ModelInfo.batch_padding` is false (ragged batches, server.py:83) and the
-memory-scaling coefficients are analytic bytes-per-token of the paged KV pool (SURVEY.md §8 f3).
+memory-scaling coefficients are analytic bytes-per-token of the paged KV pool.
 """
 from __future__ import annotations
 

@@ -1,6 +1,6 @@
 """The attention op boundary of the flash models.
 
-Mirrors /root/reference/server/text_generation_server/utils/flash_attn.py:43-127: same positional signature
+Mirrors server/text_generation_server/utils/flash_attn.py:43-127: same positional signature
 `attention(q, k, v, cu_seqlens, max_s, softmax_scale, cu_seqlens_q=None, max_s_q=None, causal=True)`.
 Prefill (cu_seqlens_q is None): varlen causal attention over fresh q/k/v.  Decode: q holds one token per sequence and
 `k` is a `PagedKVLayer` view of the block pool (block table + context lengths) instead of a contiguous cache slice.
@@ -18,7 +18,7 @@ from . import _ops
 
 @dataclass
 class PagedKVLayer:
-    k_pool: torch.Tensor  # [num_blocks, n_kv, 16, d] swizzled
+    k_pool: torch.Tensor  # [num_blocks, n_kv, 16, d] swizzled (utils/paged.py)
     v_pool: torch.Tensor
     block_table: torch.Tensor  # [B, max_blocks] int32
     context_lens: torch.Tensor  # [B] int32

@@ -1,6 +1,6 @@
 """GPTQ int4 linear on the tcgen05 in-kernel-dequant GEMM.
 
-Mirrors /root/reference/server/text_generation_server/utils/gptq/exllamav2.py:100-144 (`Ex4bitLinearV2`: same
+Mirrors server/text_generation_server/utils/gptq/exllamav2.py:100-144 (`Ex4bitLinearV2`: same
 constructor arguments, `post_init()` one-time repack, `forward`), with `exllamav2_kernels.make_q_matrix` /
 `gemm_half_q_half` replaced by `b200_gptq_pack` / `b200_gemm_w4a16`: `post_init()` converts the checkpoint tensors once
 into the kernel's streaming layout (`q_handle` = the packed buffer) and drops them.  No scratch `temp_dq`: the kernel

@@ -1,6 +1,6 @@
 """Linear / embedding / rotary building blocks over the B200 kernels.
 
-Mirrors /root/reference/server/text_generation_server/utils/layers.py: `FastLinear` (:88-111), `get_linear` (:172-203),
+Mirrors server/text_generation_server/utils/layers.py: `FastLinear` (:88-111), `get_linear` (:172-203),
 `TensorParallelHead` (:215-277), `TensorParallelColumnLinear` / `TensorParallelRowLinear` (:280-322),
 `TensorParallelEmbedding` (:325-357), `FastLayerNorm` (:360-396), `PositionRotaryEmbedding` (:406-481).  Same names, constructor arguments and
 sharding behaviour; the CUDA work goes through the C ABI (ops.py), collectives through torch.distributed (NCCL).

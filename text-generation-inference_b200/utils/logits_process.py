@@ -1,9 +1,9 @@
 """Per-request (heterogeneous) logit processors applied in one vectorised pass over the [B, V] scores.
 
-Behavioural mirror of /root/reference/server/text_generation_server/utils/logits_process.py:93-402
+Behavioural mirror of server/text_generation_server/utils/logits_process.py:93-402
 (repetition penalty :93-143, temperature :146-176, top-p :179-238, top-k :241-317, typical-p :320-402): same
 constructor arguments, in-place semantics, `filter(indices)` contract (returns None when the processor becomes a no-op).
-These are caller-side of the hot path (SURVEY.md §8 a13 / f2); they run as torch ops on the GPU.
+These are caller-side of the hot path; they run as torch ops on the GPU.
 """
 from __future__ import annotations
 

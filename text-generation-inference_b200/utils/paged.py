@@ -1,11 +1,11 @@
 """Paged KV cache manager: block-16 pools per layer, per-sequence block lists, device-resident step state.
 
 Stands in for the un-vendored fms-extras `PagedKVCacheManager` that the reference's paged path uses
-(/root/reference/server/text_generation_server/models/paged_causal_lm.py:338-353 constructor arguments,
+(server/text_generation_server/models/paged_causal_lm.py:338-353 constructor arguments,
 utils/paged.py:92-159 `allocate_tokens`, server.py:233-249 `free_sequences`).  Block bookkeeping is the C++
 allocator behind the C ABI (csrc/kv_alloc.cu); this class owns the pools and the per-sequence lists.
 
-HBM layout (DESIGN.md "KV page layout"): one tensor [n_layers, 2, num_blocks, n_kv_heads/tp, 16, head_dim] fp16;
+HBM layout: one tensor [n_layers, 2, num_blocks, n_kv_heads/tp, 16, head_dim] fp16;
 a (block, kv head) tile is 16*d*2 contiguous bytes, its 16-byte chunks XOR-swizzled by (token & 7).
 """
 from __future__ import annotations
@@ -71,7 +71,7 @@ class PagedKVCacheManager:
         self.head_dim = emb_dim // num_heads
         kv_heads = kv_heads or num_heads
         if kv_heads < tensor_parallel_size or kv_heads % tensor_parallel_size:
-            # flash_llama_modeling.py:220-222 silently floors; guard it (SURVEY.md §8e)
+            # flash_llama_modeling.py:220-222 silently floors; guard it
             raise ValueError(f"num_key_value_heads {kv_heads} not divisible by tensor parallel size {tensor_parallel_size}")
         self.kv_heads = kv_heads // tensor_parallel_size
         self.device = torch.device(device)

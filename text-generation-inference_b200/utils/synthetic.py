@@ -1,6 +1,6 @@
-"""Synthetic checkpoints and tokenizer for benchmarks and tests (SURVEY.md §8d): seeded random weights of a named
+"""Synthetic checkpoints and tokenizer for benchmarks and tests: seeded random weights of a named
 architecture generated directly in device memory, served through the `Weights` interface so the model code loads them
-exactly like a safetensors checkpoint (same tensor names — SURVEY.md Appendix D — and the same TP slicing rules).
+exactly like a safetensors checkpoint (same tensor names and the same TP slicing rules).
 There is no network and no real checkpoint in the image; `data: synthetic` in bench lines refers to this.
 """
 from __future__ import annotations

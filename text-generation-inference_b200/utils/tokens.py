@@ -1,6 +1,6 @@
 """Next-token choosing and token-info extraction (caller side of the logits).
 
-Behavioural mirror of /root/reference/server/text_generation_server/utils/tokens.py: `Sampling` (:32-41), `Greedy`
+Behavioural mirror of server/text_generation_server/utils/tokens.py: `Sampling` (:32-41), `Greedy`
 (:44-46), `HeterogeneousNextTokenChooser` (:161-333), `HeterogeneousSampling` (:336-384), `get_token_info` (:388-425),
 `get_input_tokens_info` (:429-506).  Greedy batches build no warpers and arg-max the fp16 logits (:197-219) — here with
 the library's arg-max kernel when the scores live on the GPU.

@@ -1,7 +1,7 @@
 """Micro-benchmark of the attention kernels (CUDA events over graph-replayed launches):
   prefill: b200_attn_prefill_varlen (HMMA, fresh q/k/v) vs b200_attn_prefill_paged (tcgen05 + TMA through the block pool)
   decode : b200_attn_decode_paged at the served shapes
-  python tools/bench_attn.py [--out gpurun_out/bench_attn.txt]
+  python tools/bench_attn.py [--out bench_attn.txt]
 """
 import argparse
 import os

@@ -58,7 +58,7 @@ def main():
         w = [torch.randn(N, K, device=dev).half() for _ in range(nbuf)]
         us = timeit(lambda i: ops.gemm_f16(x, w[i % nbuf], out=out))
         bytes_ = N * K * 2 + T * K * 2 + T * N * 2
-        # cuBLAS on the same shapes, same graph-replayed rotation over > L2 of weights (the library kernel to beat)
+        # cuBLAS on the same shapes, same graph-replayed rotation over > L2 of weights: the library kernel to beat
         us_cublas = timeit(lambda i: torch.matmul(x, w[i % nbuf].t(), out=out))
         print(f"f16   T={T:4d} N={N:6d} K={K:6d}: {us:8.1f} us  {bytes_ / us / 1e3:8.1f} GB/s   cuBLAS {us_cublas:8.1f} us  "
               f"{bytes_ / us_cublas / 1e3:8.1f} GB/s   ratio {us_cublas / us:5.2f}x")

@@ -1,4 +1,4 @@
-"""Long-trajectory greedy parity report (SURVEY.md §8c): B sequences generated through FlashCausalLM.generate_token for n_new
+"""Long-trajectory greedy parity report: B sequences generated through FlashCausalLM.generate_token for n_new
 tokens each (prefill, then the CUDA-graph-replayed fused step at contexts L0 .. L0 + n_new), checked token by token against the
 CPU oracle run teacher-forced on the generated ids.  A token counts when the oracle's top-1 / top-2 logit gap exceeds 2 fp16 ulp
 at that magnitude (the tie band); it must then equal the oracle's arg-max.  Writes a JSON report.
@@ -102,7 +102,7 @@ def main():
     t1 = time.time()
     oracle.generate_greedy(prompts, a.new, banned_token=eos, forced=got, keep_logits=False, on_step=on_step)
     report = {
-        "what": "greedy ids of FlashCausalLM.generate_token vs the CPU oracle run teacher-forced on them (SURVEY.md §8c exactness rule)",
+        "what": "greedy ids of FlashCausalLM.generate_token vs the CPU oracle run teacher-forced on them",
         "model": f"{a.arch} widths, {a.layers} layers, vocab {a.vocab}, {quantize or 'fp16'}", "batch": a.batch, "prompt_len": a.prompt,
         "new_tokens_per_sequence": a.new, "generated_tokens": a.batch * a.new, "contexts": [a.prompt, a.prompt + a.new - 1],
         "decode_steps_through_cuda_graph_replay": graph_steps,

@@ -1,8 +1,8 @@
-"""Profiling driver (run under ncu on the GPU box): builds a synthetic model of the named workload with a few layers,
+"""Profiling driver (to be run under ncu): builds a synthetic model of the named workload with a few layers,
 prefills B prompts of `--ctx` tokens through the public API and runs `--steps` eager (un-graphed) decode steps so that
 every kernel of a decode step appears as an individual launch.
 
-  ncu --metrics gpu__time_duration.sum --clock-control none -c 2000 --csv --log-file gpurun_out/launches.csv \
+  ncu --metrics gpu__time_duration.sum --clock-control none -c 2000 --csv --log-file launches.csv \
       python tools/profile_decode.py --workload llama2-7b-gptq --layers 2 --ctx 1536 --steps 3
 """
 import argparse

@@ -6,7 +6,7 @@ does over gRPC: while requests are waiting and the running batch has room, an ad
 `to_prune` field carries the completed ids of cached batches, server.py:105-122), then `NextToken` naming every cached batch
 id with its `completed_ids` - the shard prunes and concatenates (server.py:183-231).  Requests arrive by a Poisson process
 in measured time (the clock advances by the wall time of each RPC; idle gaps are skipped), prompt and output lengths are
-uniform in the given ranges, seeded (SURVEY.md §8d config 5).
+uniform in the given ranges, seeded.
 
 `run_session` returns per-request token ids plus timing / traffic totals for decode steps and prefills separately.
 """

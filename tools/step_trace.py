@@ -2,7 +2,7 @@
 launch).  The stamps serialise the stream, so PDL overlap between kernels is lost: read the table as "device time of each
 kernel including its launch gap, warm L2 state as in the served step", and compare its sum with the untraced step time.
 
-  python tools/step_trace.py [--workload llama3-8b-gptq] [--context 1536] [--layers N] [--out gpurun_out/step_trace.txt]
+  python tools/step_trace.py [--workload llama3-8b-gptq] [--context 1536] [--layers N] [--out step_trace.txt]
   torchrun --nproc-per-node 8 ... tools/step_trace.py ...   (tensor parallel: the launch list of rank 0's step)
 """
 import argparse

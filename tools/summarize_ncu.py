@@ -1,4 +1,4 @@
-"""Turns the ncu outputs brought back in gpurun_out/ into the small text/CSV/JSON summaries committed under profiles/.
+"""Turns ncu's outputs into the small text/CSV/JSON summaries committed under profiles/.
 
   python tools/summarize_ncu.py <launches.csv> <full.ncu-rep> <tag> [workload]
 """
@@ -41,7 +41,7 @@ for k, (c, v) in sorted(agg.items(), key=lambda x: -x[1][1]):
     lines.append(f"{k:45s} n={c:3d} total={v / 1e3:8.1f} us  avg={v / c / 1e3:7.1f} us  share={v / tot * 100:5.1f}%")
 
 # ---- full report: headline metrics per captured kernel
-# `rep` is the .ncu-rep, or the CSV of its raw page produced on the GPU box (`ncu -i x.ncu-rep --page raw --csv > x_raw.csv`: the
+# `rep` is the .ncu-rep, or the CSV of its raw page produced where it was captured (`ncu -i x.ncu-rep --page raw --csv > x_raw.csv`: the
 # reports themselves are too large to bring back)
 raw = open(rep).read() if rep.endswith(".csv") else subprocess.run(["ncu", "-i", rep, "--page", "raw", "--csv"], capture_output=True, text=True).stdout
 r = list(csv.reader(raw.splitlines()))
