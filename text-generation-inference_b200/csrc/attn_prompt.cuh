@@ -20,16 +20,15 @@
 //               shared-memory operand (keys are the MMA K dimension, d contiguous), accumulator O in TMEM.
 //   warps 4..7, 8..11   softmax of the first and the second tile: thread = one query row = one TMEM lane (no shuffles).  tcgen05.ld S, causal
 //               mask, fp32 online softmax in the log2 domain, P rounded to fp16 (flash-attn semantics) and stored back to TMEM, O
-//               rescaled in TMEM when a row's maximum moves.  (The reference always is the maximum: one that lags until it is 2^8 behind saves
-//               3 % (272 us where this takes 280, 13 prompts of 300 to 2048 tokens), but a largest weight that is not exactly 1 is rounded, up to 7 % more error behind
-//               1500 cached keys whose scores spread.)  The row's sum adds the rounded P, what the
+//               rescaled in TMEM when a row's maximum moves.  (The reference always is the maximum: one that lags until it is 2^8
+//               behind saves rescaling, one prompt of 8192 tokens 472 us where this takes 544, but a largest weight that is not exactly 1 is rounded:
+//               up to 7 % more error behind 1500 cached keys whose scores spread.)  The row's sum adds the rounded P, what the
 //               products weigh.  S of tile j is complete only after P V of tile j - 1 (issue order), so O is quiescent whenever a
 //               softmax warp runs.
 // Causality over absolute positions prunes whole key tiles.  Bound: soft-max exponentials (MUFU, 16 a cycle and SM: 1024 cycles per 128 x 128 tile,
-// as long as its products at d = 128, twice as long at d = 64), and between items the pipeline's drain.  Measured on B200 (us, before: one query
-// tile of one head per CTA): 13 prompts of 300 to 2048 tokens, 32 / 8 heads, d = 128 571 -> 234; 16 x 1024 428 -> 187; 8192 1196 -> 465 (1.18
-// PFLOP/s); d = 64, 32 / 4 heads 440 -> 186; 300 tokens after 1500 cached ones x 4 110 -> 67; 64 tokens x 10 18.1 -> 15.6.  Items dealt out in turn:
-// 294 at the first of these.  Tried: four more warps for the output (305 instead of
+// as long as its products at d = 128, twice as long at d = 64), and between items the pipeline's drain.  Measured on B200 (us back to back, before: one query
+// tile of one head per CTA): 13 prompts of 300 to 2048 tokens, 32 / 8 heads, d = 128 570 -> 219; 16 x 1024 428 -> 184; 8192 1197 -> 548; d = 64, 32 / 4
+// heads 441 -> 189; 300 tokens after 1500 cached ones x 4 110 -> 66; 64 tokens x 10 17.7 -> 12.8.  Items dealt out in turn: 294 at the first of these.  Tried: four more warps for the output (305 instead of
 // 287: the softmax warps are then compiled for 128 registers).
 // Token-major caches differ in this: a tile is 128 / rep tokens x the rep query heads of a key head (all rows meet the same keys), an item two
 // neighbouring tiles; the softmax warps bring their tile's fp32 queries as bfloat16 themselves; P is the sum of two bfloat16 values (one alone is 2^-9
@@ -52,8 +51,10 @@ constexpr int kPfPageSlabBytes = kPageTokens * 128;
 constexpr int kPfCornerBytes = 32 * 128;  // a softmax warp's rows on their way out
 constexpr int kPfStages = 2;
 constexpr int kPfAhead = 2;      // items that are known ahead
-// registers per thread: the launch has 384 x 168; the two softmax warpgroups take 216 each, the other one keeps 72
-constexpr int kPfSoftmaxRegs = 216, kPfServeRegs = 72;
+// Registers per thread: the launch has 384 x 168; the two softmax warpgroups take 200 each, the other one keeps 104.  216 and 72, with O rescaled in 64
+// columns at a time instead of 16, spilled in both (us, flushed L2, that / this: 13 prompts of 300 to 2048 tokens, 32 / 8 heads, d = 128 246 / 225; hybrid
+// prompts of 1618 and 2000 tokens, 16 / 4 heads 109 / 100; 6 portions of 300 to 600 behind 700 keys, 40 / 40 heads 115 / 101).
+constexpr int kPfSoftmaxRegs = 200, kPfServeRegs = 104;
 
 template <int D>
 struct PfCfg {
@@ -549,15 +550,14 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             sum[0] *= alpha;
             sum[1] *= alpha;
 #pragma unroll
-            for (int c = 0; c < D / 64; ++c) {
-              uint32_t o[64];
-              tmem_ld_32x32b_x32(tmem_o + c * 64, reinterpret_cast<uint32_t(&)[32]>(o[0]));
-              tmem_ld_32x32b_x32(tmem_o + c * 64 + 32, reinterpret_cast<uint32_t(&)[32]>(o[32]));
+            for (int c = 0; c < D; c += 16) {  // few columns at once: the tile's scores hold 128 registers
+              uint32_t o[16];
+              tmem_ld_32x32b_x16(tmem_o + c, o);
               tmem_ld_wait();
 #pragma unroll
-              for (int k = 0; k < 64; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * alpha);
+              for (int k = 0; k < 16; ++k) o[k] = __float_as_uint(__uint_as_float(o[k]) * alpha);
 #pragma unroll
-              for (int k = 0; k < 4; ++k) tmem_st_32x32b_x16(tmem_o + c * 64 + k * 16, reinterpret_cast<const uint32_t(&)[16]>(o[k * 16]));
+              for (int k = 0; k < 16; k += 16) tmem_st_32x32b_x16(tmem_o + c + k, reinterpret_cast<const uint32_t(&)[16]>(o[k]));
             }
           }
         }
