@@ -26,13 +26,14 @@
 //               products weigh.  S of tile j is complete only after P V of tile j - 1 (issue order), so O is quiescent whenever a
 //               softmax warp runs.
 // Causality over absolute positions prunes whole key tiles.  Bound: soft-max exponentials (MUFU, 16 a cycle and SM: 1024 cycles per 128 x 128 tile,
-// as long as its products at d = 128, twice as long at d = 64), and between items the pipeline's drain.  Measured on B200 (us back to back, before: one query
-// tile of one head per CTA): 13 prompts of 300 to 2048 tokens, 32 / 8 heads, d = 128 570 -> 219; 16 x 1024 428 -> 184; 8192 1197 -> 548; d = 64, 32 / 4
-// heads 441 -> 189; 300 tokens after 1500 cached ones x 4 110 -> 66; 64 tokens x 10 17.7 -> 12.8.  Items dealt out in turn: 294 at the first of these.  Tried: four more warps for the output (305 instead of
-// 287: the softmax warps are then compiled for 128 registers).
+// as long as its products at d = 128, twice as long at d = 64), and between items the pipeline's drain.  Measured on B200 (us back to back, before: one
+// query tile of one head per CTA): 13 prompts of 300 to 2048 tokens, 32 / 8 heads, d = 128 570 -> 219; 16 x 1024 428 -> 184; 8192 1197 -> 548; d = 64, 32 / 4
+// heads 441 -> 189; 300 tokens after 1500 cached ones x 4 110 -> 66; 64 tokens x 10 17.7 -> 12.8.  An earlier form with
+// items dealt out in turn took 294 at the first of these; four more warps for the output 305 instead of 287 (the softmax warps are then compiled for 128
+// registers).
 // Token-major caches differ in this: a tile is 128 / rep tokens x the rep query heads of a key head (all rows meet the same keys), an item two
 // neighbouring tiles; the softmax warps bring their tile's fp32 queries as bfloat16 themselves; P is the sum of two bfloat16 values (one alone is 2^-9
-// off, and a maximum taken over 128 keys leaves fewer weights at exactly 1 than the 16-key tiles of talk_attn_mma_kernel: prompts of 1882 and 2118 tokens,
+// off, and a maximum taken over 128 keys leaves fewer weights at exactly 1 than the 16-key tiles of talk_attn_mma_kernel: prompts of 1618 and 2000 tokens,
 // 16 / 4 heads, d = 128, against float64 1.91e-3 with one value, 1.88e-3 there, 1.47e-3 with two; 90 us, 343 there, 101); key tiles start at the first
 // visible key; a key or value page is a box [16 tokens x 64 columns] that the copy itself swizzles; and what lies in the cache beside the keys
 // that an item's queries see (slots that were never written, another request's leavings) is zeros to the products: whole pages by copies from

@@ -21,8 +21,9 @@
 //     warp, so that both factors of an output sit in one warp, sixteen lanes apart.
 //   * Lane = feature in the epilogue, transposed through shared memory into 16-byte stores; rows that those do not fit are stored by value.
 //
-// Measured on B200 (us, cold weights; before = one CTA per tile): fp16 4099 x 4096 x 4096 134 -> 98, 300 x 4096 x 4096 31.4 -> 16.2, 3001 x 5120 x
-// 20480 670 -> 421 (1.50 PFLOP/s; cuBLAS 442); int4 4099 x 14336 x 4096 451 -> 360 (1.34 PFLOP/s), gate|up 1000 x 4096 x 28672 294 -> 201.
+// Measured on B200 (us, launches back to back over weights larger than L2; before = one CTA per tile): fp16 4099 x 4096 x 4096 133 -> 98, 300 x 4096 x
+// 4096 31.2 -> 16.0, 3001 x 5120 x 20480 668 -> 425 (1.48 PFLOP/s; cuBLAS 442; a call by itself with flushed L2 785 -> 501); int4 4099 x 14336 x 4096 451
+// -> 365 (1.32 PFLOP/s; by itself 514 -> 428), gate|up 1000 x 4096 x 28672 295 -> 199.
 //
 // Warp roles: 0..3 epilogue | (int4: 4..19 de-quantisation) | then W producer / TMEM allocation, x producer, MMA issuer (leader CTA), idle.
 // Barriers: `full` and `tmem_empty` live in the leader (the pair's even CTA) and count both CTAs' work, `empty` and `tmem_full` live in

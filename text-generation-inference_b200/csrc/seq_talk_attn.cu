@@ -722,15 +722,14 @@ extern "C" int b200_seq_talk_attn_splits(int dt, int64_t T, int B, int H, int G,
 }
 
 // Prompts without a mix take the tcgen05 kernel: tiles of 128 (token, head) rows, so it wants steps of enough tokens per sequence to fill them.
-// Measured on B200 (us, the m16n8k16 kernel / this one; 16 / 4 heads, d = 128): 2118 + 1882 tokens in chunks of 2048 387 / 94, 4 x 512 84 / 25, 300 after
-// 800 cached 51 / 35, 4 x 40 after 500 38 / 26, 4 x 24 after 1900 56 / 43, 24 after 20 24.5 / 14.3; 4 x 16 after 1900 55 / 53, 4 x 8 48 / 50.
+// Measured on B200 (us, the m16n8k16 kernel / this one; 16 / 4 heads, d = 128): 1618 + 2000 tokens in chunks of 2048 343 / 101, 1000 108 / 39, 16 x 24 after
+// 4000 cached 134 / 90, 2 x 40 after 100 32 / 25, 24 after 500 38 / 32; with one bfloat16 value per weight 4 x 16 after 1900 55 / 53, 4 x 8 48 / 50.
 // What it needs beside that: heads of 64 or 128 columns, whole 128-row tiles (128 % (heads / kv_heads) == 0), pages of 16 tokens, and 16-byte pieces; and a
 // shape that talk_mma_plan accepts: those rounded queries and weights to bfloat16 before, the others (at d = 128: 16 / 16, 32 / 32, 32 / 16, 64 / 16 ... heads,
 // and everything under B200_SEQ_ATTN_MMA=0) are computed in fp32 and stay so.
 constexpr int kTalkPromptTokens = 24;  // average tokens per sequence from which on
 
-//
-// And few items over many keys are a matter of latency: the m16n8k16 kernel cuts the keys into runs then, this one does not.  `keys`: a bound of
+// Few items over many keys are a matter of latency: the m16n8k16 kernel cuts the keys into runs then, this one does not.  `keys`: a bound of
 // the keys that a query sees, as far as the host knows it (the block table's width, a chunk, a window).  Models of both, from 80 steps measured on
 // B200.  Us, m16n8k16 / this one, no chunk, no window: 16 / 4 heads of 128, 24 tokens behind 2000 keys 56 / 51, behind 30 000 454 / 475, 200 behind 8000 181 /
 // 145; 8 / 2 heads of 64, 24 behind 500 36 / 27, 64 behind 8000 77 / 141, 500 behind 8000 103 / 150; 16 / 8 heads of 64, 24 x 16 sequences behind 4000 108 / 127, a
