@@ -114,3 +114,36 @@ def test_a_deep_sum_is_as_good_as_its_rounding(T, N, K):
     ref = x.double() @ w.double().t()
     off, rounding = (ops.gemm_f16(x, w).double() - ref).norm(), (ref.half().double() - ref).norm()
     assert float(off / rounding) < 1.002
+
+
+def test_first_calls_inside_a_capture():
+    """a process whose first prompt linear and first prompt attention are captured into a graph (where a kernel reports a wait that ran out is set up
+    then): replays give what a call gives"""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch, tgis_b200
+from tgis_b200 import ops
+D = 'cuda:0'
+x, w = torch.randn(300, 256, device=D).half(), torch.randn(384, 256, device=D).half()
+q, kp, vp = torch.randn(300, 4, 64, device=D).half(), torch.randn(20, 2, 16, 64, device=D).half(), torch.randn(20, 2, 16, 64, device=D).half()
+table, lens, cu = torch.arange(20, device=D, dtype=torch.int32)[None].contiguous(), torch.tensor([300], dtype=torch.int32, device=D), torch.tensor([0, 300], dtype=torch.int32, device=D)
+ws = ops.gemm_workspace(x.device, 300, 384, 256)
+call = lambda: (ops.gemm_f16(x, w), ops.attn_prefill_paged(q, kp, vp, table, lens, cu, 300, 0.125))
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    a = call()
+for _ in range(2):
+    for t in a:
+        t.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    b = call()
+    assert all(torch.equal(s, t) and bool(s.abs().sum() > 0) for s, t in zip(a, b))
+print('ok')
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stderr[-2000:]
