@@ -6,8 +6,9 @@
 //   delta_prepare_kernel : everything of a token that does not depend on S, once per token: short depth-wise causal convolution + SiLU
 //                          of the q / k / v columns (earlier inputs from the sequence's convolution state), unit vectors, decays,
 //                          write strengths -> one row [q | k | v | g | beta] per token.  When every sequence brings one token it also
-//                          advances the convolution state (otherwise delta_conv_state_kernel does, after it).
-//   delta_chunk_kernel   : prompts and portions.  A block owns (sequence, head, up to 64 value columns) and takes four tokens at a
+//                          advances the convolution state (otherwise delta_conv_state_kernel does, after it; over runs, each sequence's first).
+//   delta_spans.cuh      : prompts of some length, sixteen tokens at a time, what happens among them solved ahead of the memory.
+//   delta_chunk_kernel   : shorter prompts and portions, and shapes that the spans don't take.  A block owns (sequence, head, up to 64 value columns) and takes four tokens at a
 //                          time: their predictions and read-outs against the OLD memory are one pass over the state registers, the
 //                          dependence among the four goes through 4 x 4 matrices of decayed inner products, and the memory is
 //                          rewritten once.  With G_j = g_1 .. g_j and D_i = g_(i+1) .. g_4 (products per key channel, no division):
@@ -18,7 +19,7 @@
 //                          between global memory and registers in whole rows; tokens in order, one at a time.
 //
 // A sequence whose first token of the step is at position 0 starts from a zero state and never reads its (possibly reused) slot.
-// All arithmetic is fp32; the two scan forms (and delta_scan_kernel of seq_recurrent.cu, which keeps one order of operations for any cut of
+// All arithmetic is fp32; the three scan forms (and delta_scan_kernel of seq_recurrent.cu, which keeps one order of operations for any cut of
 // a sequence and knows decays per head only) differ by rounding.
 #include "seq_common.cuh"
 
@@ -141,7 +142,7 @@ constexpr int kRunTok = 16, kRunMinTokens = 384;
 
 template <typename TP>
 __global__ void __launch_bounds__(256) delta_prepare_run_kernel(
-    const float* __restrict__ u, int64_t ld, int col0, int taps, const TP* __restrict__ w, const float* __restrict__ conv_state,
+    const float* __restrict__ u, int64_t ld, int col0, int taps, const TP* __restrict__ w, float* conv_state,
     const int32_t* __restrict__ state_slots, const int32_t* __restrict__ cu_q, int B, const int64_t* __restrict__ position_ids,
     const float* __restrict__ raw, int64_t ldr, int col_b, const float* __restrict__ dec, int64_t ldd, int col_a, int channels,
     const TP* __restrict__ A_log, const TP* __restrict__ dt_bias, float q_scale, float* __restrict__ out, int H, int G, int dk, int dv) {
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(256) delta_prepare_run_kernel(
   const int lane = lane_id(), row0 = cu_q[b], t0 = row0 + tile * kRunTok, n_tok = min(kRunTok, cu_q[b + 1] - t0);
   const int64_t s = position_ids[row0], p0 = s + tile * kRunTok;
   const int C = 2 * G * dk + H * dv;
-  const float* st = conv_state + (int64_t)state_slots[b] * (taps > 1 ? taps - 1 : 1) * C;
+  float* st = conv_state + (int64_t)state_slots[b] * (taps > 1 ? taps - 1 : 1) * C;
   const DeltaRow lay = delta_row(H, G, dk, dv, channels != 0);
   const int spans = (C + 127) / 128, n_dec = channels ? H * dk : 0, g_spans = (n_dec + 127) / 128;
   const int task = blockIdx.y * 8 + warp_id(), c = (task < spans ? task : task - spans) * 128 + lane * 4;
@@ -171,6 +172,16 @@ __global__ void __launch_bounds__(256) delta_prepare_run_kernel(
       if (j < 3 && live && jj >= 0 && pp >= 0) v = pp >= s ? *reinterpret_cast<const float4*>(u + (row0 + (pp - s)) * ld + col0 + c)
                                                            : *reinterpret_cast<const float4*>(st + (pp - s + taps - 1) * C + c);
       x[j][0] = v.x; x[j][1] = v.y; x[j][2] = v.z; x[j][3] = v.w;
+    }
+    if (tile == 0 && live) {   // only a sequence's first run reads its state, so it can advance it too (as delta_conv_state_kernel)
+      const int64_t e = s + cu_q[b + 1] - row0;
+      for (int j = 0; j < taps - 1; ++j) {
+        const int64_t pp = e - (taps - 1) + j;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (pp >= s) v = *reinterpret_cast<const float4*>(u + (row0 + (pp - s)) * ld + col0 + c);
+        else if (pp >= 0) v = *reinterpret_cast<const float4*>(st + (pp - s + taps - 1) * C + c);
+        *reinterpret_cast<float4*>(st + (int64_t)j * C + c) = v;
+      }
     }
     const bool unit = c < 2 * G * dk;                        // (a span never holds both kinds: 2 G dk is a multiple of 128 or the spans' lanes differ)
     const float unit_scale = c < G * dk ? q_scale : 1.f;
@@ -556,6 +567,14 @@ __global__ void __launch_bounds__(256, NR * kRowLanes <= 128 ? 2 : 1) delta_chun
   }
 }
 
+}  // namespace seq
+}  // namespace b200
+
+#include "delta_spans.cuh"
+
+namespace b200 {
+namespace seq {
+
 constexpr int kStepThreads = 256, kStepWarps = kStepThreads / 32;
 
 // CL lanes side by side hold VEC columns each, the 256 / CL groups of them take every so many-th state row: NR rows per thread
@@ -702,10 +721,7 @@ extern "C" int b200_seq_delta_prepare(const float* u, int64_t ld, int col0, int 
     B200_SEQ_DISPATCH(dt, E, B200_LAUNCH((delta_prepare_run_kernel<E>), dim3((unsigned)(T / kRunTok + B), (unsigned)((run_tasks + 7) / 8)), dim3(256), 0, st, u, ld, col0,
                                          taps, (const E*)w, conv_state, state_slots, cu_q, B, position_ids, raw, ldr, col_b, dec, ldd, col_a, channels,
                                          (const E*)A_log, (const E*)dt_bias, q_scale, out, H, kv_heads, dk, dv));
-    if (taps > 1)
-      B200_LAUNCH(delta_conv_state_kernel, dim3((unsigned)B, (unsigned)((C + 255) / 256)), dim3(256), 0, st, u, ld, col0, C, taps, conv_state, state_slots, cu_q,
-                  position_ids);
-    b200_count_launches(taps > 1 ? 2 : 1);
+    b200_count_launches(1);
     return B200_OK;
   }
   const int tasks = 2 * kv_heads + (H * dv + kPrepSpan - 1) / kPrepSpan + ((channels ? H * dk : H) + kPrepSpan - 1) / kPrepSpan +
@@ -750,11 +766,64 @@ static int launch_delta_step(const float* pre, float* S_state, const int32_t* st
   return B200_OK;
 }
 
+// Spans of a step that one pair of launches may leave records of: all of them, or those of the next `cap` tokens of every sequence where the records of
+// all would take more than kSpanRoom bytes (`cap` == 0: too many sequences for that, or a shape that the spans don't take).
+// kSpanMean: tokens per sequence from which spans are faster than the chain over four tokens; on grids that fill the chip the chain hides its waits better.
+// Measured on B200 (us with the preparation, chain / spans, heads of 128): 16 heads: 1 x 40 tokens 26 / 32, 2 x 125 67 / 54, 6 x 96 - 120 95 / 79, 1 x 690
+// 201 / 135, 4 x 256 - 768 292 / 210; 32 heads: 6 x 30 - 60 83 / 93, 1 x 96 52 / 45, 3 x 100 - 200 126 / 109, 6 x 128 - 140 165 / 171, 1 x 450 208 / 125,
+// 6 x 400 - 800 797 / 656.
+constexpr int64_t kSpanRoom = (int64_t)2 << 30, kSpanMean = 96, kSpanMeanFull = 192;
+struct SpanPlan {
+  int64_t spans, bytes;
+  int cap;
+};
+static SpanPlan delta_span_plan(int64_t T, int B, int H, int dk, int dv) {
+  SpanPlan pl = {0, 0, 0};
+  const bool full = (int64_t)B * H * (dv / kSpanCols) > 4 * 148;   // more blocks than can be on the chip at once
+  if ((dk != 64 && dk != 128) || dv % kSpanCols != 0 || T < (full ? kSpanMeanFull : kSpanMean) * B) return pl;
+  const int64_t rec = (int64_t)span_record_floats(dk, dv) * 4 * H;
+  pl.spans = T / kSpan + B;
+  pl.cap = 1 << 30;
+  if (pl.spans * rec > kSpanRoom) {
+    const int64_t each = kSpanRoom / (rec * B);   // spans per sequence
+    pl.cap = each >= 64 ? (int)(each * kSpan) : 0;
+    pl.spans = each * B;
+  }
+  pl.bytes = pl.cap ? pl.spans * rec : 0;
+  return pl;
+}
+
+// bytes of workspace with which b200_seq_delta_rows_scan takes a step in spans of sixteen tokens (0: it does not)
+extern "C" int64_t b200_seq_delta_rows_scan_bytes(int64_t T, int B, int H, int dk, int dv) { return B > 0 && H > 0 ? delta_span_plan(T, B, H, dk, dv).bytes : 0; }
+
+template <int DK>
+static int launch_delta_spans(const float* pre, const DeltaRow& lay, int channels, float* S_state, const int32_t* state_slots, const int32_t* cu_q,
+                              const int64_t* position_ids, float* y, int64_t ld_y, int64_t T, int B, int H, int G, int dv, const SpanPlan& pl, float* records,
+                              cudaStream_t st) {
+  using Scan = SpanScan<DK>;
+  static const cudaError_t configured[2] = {
+      cudaFuncSetAttribute(delta_span_scan_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, Scan::kBytes),
+      cudaFuncSetAttribute(delta_span_prepare_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, SpanPrep<DK>::kBytes)};
+  for (const cudaError_t e : configured)
+    if (e != cudaSuccess) { b200_set_last_error(cudaGetErrorString(e)); return B200_ERR_CUDA; }
+  unsigned* word = b200_gave_up_word();
+  if (!word) return B200_ERR_CUDA;
+  for (int64_t off = 0; off < T; off += pl.cap) {   // (the host does not know how long the longest sequence is: T at most)
+    B200_LAUNCH((delta_span_prepare_kernel<DK>), dim3((unsigned)pl.spans, (unsigned)((H + kSpanPrepHeads - 1) / kSpanPrepHeads)), dim3(kSpanPrepHeads * 64),
+                (size_t)SpanPrep<DK>::kBytes, st, pre, lay.width, lay.k, lay.v, lay.g, lay.b, cu_q, B, (int)off, pl.cap, H, H / G, channels, dv, records, y, ld_y);
+    B200_LAUNCH((delta_span_scan_kernel<DK>), dim3((unsigned)(B * H * (dv / kSpanCols))), dim3(Scan::kWarps * 32), (size_t)Scan::kBytes, st, records,
+                S_state, state_slots, cu_q, position_ids, y, ld_y, (int)off, pl.cap, B, H, dv, word);
+    b200_count_launches(2);
+  }
+  return B200_OK;
+}
+
 // pre fp32 [T, b200_seq_delta_row_width]: rows as b200_seq_delta_prepare leaves them; S_state fp32 [slots, H, dk, dv] advanced in place
-// -> y fp32 [T, H * dv].  T: token rows of the step (steps with few rows per sequence take the form that is bound by the state's traffic)
+// -> y fp32 [T, H * dv].  T: token rows of the step (steps with few rows per sequence take the form that is bound by the state's traffic).
+// workspace: b200_seq_delta_rows_scan_bytes bytes, 16-byte aligned, or NULL (the step then goes four tokens at a time)
 extern "C" int b200_seq_delta_rows_scan(const float* pre, int channels, float* S_state, const int32_t* state_slots, const int32_t* cu_q,
                                    const int64_t* position_ids, float* y, int64_t ld_y, int64_t T, int B, int H, int kv_heads, int dk, int dv,
-                                   void* stream) {
+                                   void* workspace, void* stream) {
   if (T == 0 || B == 0) return B200_OK;
   if (kv_heads <= 0 || H % kv_heads != 0 || dk <= 0 || dk > 256 || dv <= 0) {
     b200_set_last_error("seq_delta_rows_scan: need heads % kv_heads == 0 and 0 < key size <= 256");
@@ -780,6 +849,12 @@ extern "C" int b200_seq_delta_rows_scan(const float* pre, int channels, float* S
     if (rows <= 16) DST(16, 1);
     DST(32, 1);
 #undef DST
+  }
+  const SpanPlan pl = delta_span_plan(T, B, H, dk, dv);
+  if (workspace && pl.cap && aligned) {
+    const DeltaRow lay = delta_row(H, kv_heads, dk, dv, channels != 0);
+    return dk == 64 ? launch_delta_spans<64>(pre, lay, channels, S_state, state_slots, cu_q, position_ids, y, ld_y, T, B, H, kv_heads, dv, pl, (float*)workspace, st)
+                    : launch_delta_spans<128>(pre, lay, channels, S_state, state_slots, cu_q, position_ids, y, ld_y, T, B, H, kv_heads, dv, pl, (float*)workspace, st);
   }
   const int vec = (dk % 4 == 0 && dv % 4 == 0 && aligned) ? 1 : 0;
   // 64 columns per block share each staged vector among more of the memory; a small grid is spread over 32 columns and 32 lanes.  The line lies where

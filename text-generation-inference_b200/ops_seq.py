@@ -579,9 +579,12 @@ def delta_rows_scan(rows: torch.Tensor, S: torch.Tensor, step: RaggedStep, H: in
     _cuda(rows, S)
     assert rows.dtype == torch.float32 and rows.is_contiguous() and S.dtype == torch.float32 and S.is_contiguous() and S.shape[1:] == (H, dk, dv)
     y = torch.empty(step.T, H * dv, dtype=torch.float32, device=rows.device)
-    _lib.check_seq(_lib.load_seq().b200_seq_delta_rows_scan(_ptr(rows), int(channels), _ptr(S), _ptr(step.state_slots), _ptr(step.cu_q),
-                                                       _ptr(step.position_ids), _ptr(y), y.stride(0), step.T, step.B, H, kv_heads, dk, dv,
-                                                       _stream()), "seq_delta_rows_scan")
+    lib = _lib.load_seq()
+    need = lib.b200_seq_delta_rows_scan_bytes(step.T, step.B, H, dk, dv)
+    ws = torch.empty(need, dtype=torch.uint8, device=rows.device) if need else None
+    _lib.check_seq(lib.b200_seq_delta_rows_scan(_ptr(rows), int(channels), _ptr(S), _ptr(step.state_slots), _ptr(step.cu_q),
+                                                _ptr(step.position_ids), _ptr(y), y.stride(0), step.T, step.B, H, kv_heads, dk, dv, _ptr(ws), _stream()),
+                    "seq_delta_rows_scan")
     return y
 
 
