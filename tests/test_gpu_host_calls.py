@@ -1,0 +1,126 @@
+"""The native per-call host side (csrc/host/host_calls.cpp): the calls that it serves give what the Python path gives, and calls that it leaves to
+Python end as they would without it - the same results for the unusual ones, the same errors for the wrong ones."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+class _Nothing:
+    """a native side that serves no call"""
+
+    def __getattr__(self, name):
+        return lambda *a: None
+
+
+@pytest.fixture(params=["ops", "ops_seq"])
+def both(request, monkeypatch):
+    """runs a call with the native side and without it"""
+    import tgis_b200
+    from tgis_b200 import ops, ops_seq
+
+    mod = {"ops": ops, "ops_seq": ops_seq}[request.param]
+    native = mod._native()
+
+    def run(call):
+        got = []
+        for side in (native, _Nothing()):
+            monkeypatch.setattr(mod, "_host", side)
+            try:
+                got.append(call(mod))
+            except Exception as e:
+                got.append((type(e), str(e)))
+        monkeypatch.setattr(mod, "_host", native)
+        a, b = got
+        assert type(a) is type(b) and (torch.equal(a, b) and a.dtype == b.dtype and a.stride() == b.stride() if isinstance(a, torch.Tensor) else a == b), (a, b)
+        return a
+    run.name = request.param
+    return run
+
+
+def _r(*shape, dtype=torch.float16):
+    return torch.randn(*shape, device=DEV, dtype=torch.float32).to(dtype)
+
+
+def test_linears(both):
+    x, w, b = _r(5, 256), _r(96, 256), _r(96)
+    if both.name == "ops_seq":
+        x, w, b = (t.bfloat16() for t in (x, w, b))
+        for dt in (None, torch.bfloat16, torch.float32):
+            assert both(lambda m: m.linear(x, w, b, out_dtype=dt)).dtype == (dt or torch.bfloat16)
+            both(lambda m: m.linear(x, w, None, out_dtype=dt))
+        both(lambda m: m.linear(x.float(), w.float(), b.float()))                      # a true 32-bit product
+        wide = _r(5, 300).bfloat16()
+        both(lambda m: m.linear(wide[:, :256], w))                                     # row-strided
+        both(lambda m: m.linear(x[:, :40].contiguous(), w[:, :40].contiguous()))       # small k
+        both(lambda m: m.linear(x, w, act=m.ACT_RELU2))
+        both(lambda m: m.linear(x[:0], w))
+        assert both(lambda m: m.linear(x.cpu(), w))[0].__name__ == "B200Error"
+        assert both(lambda m: m.linear(x, w[:, :128]))[0] is AssertionError
+        return
+    out, ws = torch.empty(5, 96, dtype=torch.float16, device=DEV), torch.zeros(1 << 24, dtype=torch.uint8, device=DEV)
+    both(lambda m: m.gemm_f16(x, w, b))
+    both(lambda m: m.gemm_f16(x, torch.nn.Parameter(w, requires_grad=False)))
+    assert both(lambda m: m.gemm_f16(x, w, b, out)).data_ptr() == out.data_ptr()
+    both(lambda m: m.gemm_f16(x, w, workspace=ws))
+    both(lambda m: m.gemm_f16(x[:0], w))
+    assert both(lambda m: m.gemm_f16(x.float(), w))[0].__name__ == "B200Error"
+    assert both(lambda m: m.gemm_f16(x.cpu(), w))[0].__name__ == "B200Error"
+    assert both(lambda m: m.gemm_f16(x.t(), w))[0] is AssertionError
+    assert both(lambda m: m.gemm_f16(x[0], w))[0] is ValueError
+    assert both(lambda m: m.gemm_f16(_r(5, 100), _r(96, 100)))[0].__name__ == "B200Error"   # refused by the entry
+
+
+def test_int4(both):
+    if both.name != "ops":
+        return
+    from tgis_b200 import ops
+    g = torch.Generator(device=DEV).manual_seed(1)
+    K, N = 256, 512
+    qweight = torch.randint(-2 ** 31, 2 ** 31, (K // 8, N), generator=g, device=DEV).int()
+    qzeros, scales = torch.full((K // 128, N // 8), 0x77777777, device=DEV).int(), torch.rand(K // 128, N, device=DEV).half() * 0.01
+    plain, pairs = ops.gptq_pack(qweight, qzeros, scales, 128), ops.gptq_pack(qweight, qzeros, scales, 128, ops.W4_LAYOUT_GATE_UP)
+    x, b = _r(3, K), _r(N)
+    both(lambda m: m.gemm_w4a16(x, plain, N, 128))
+    both(lambda m: m.gemm_w4a16(x, plain, N, 128, b, torch.empty(3, N, dtype=torch.float16, device=DEV)))
+    assert both(lambda m: m.gemm_w4a16(x, pairs, N, 128, layout=1, silu_mul=True)).shape == (3, N // 2)
+    assert both(lambda m: m.gemm_w4a16(x, plain, N, 128, silu_mul=True))[0].__name__ == "B200Error"   # needs the other layout
+    assert both(lambda m: m.gemm_w4a16(x.bfloat16(), plain, N, 128))[0].__name__ == "B200Error"
+
+
+def test_attention(both):
+    if both.name != "ops":
+        return
+    lens = torch.tensor([20, 3], dtype=torch.int32, device=DEV)
+    table = torch.tensor([[0, 2], [1, 0]], dtype=torch.int32, device=DEV)
+    k, v = _r(3, 2, 16, 64), _r(3, 2, 16, 64)
+    qkv = _r(2, 8 * 64)
+    q = qkv[:, :4 * 64].unflatten(1, (4, 64))
+    both(lambda m: m.attn_decode_paged(q, k, v, table, lens, 20, 0.125, 2))
+    both(lambda m: m.attn_decode_paged(q, k, v, table, lens, 20, 0.125, 2, torch.empty(2, 4, 64, dtype=torch.float16, device=DEV)))
+    assert both(lambda m: m.attn_decode_paged(q, k, v, table, lens, 4000, 0.125, 2, workspace=lens))[0].__name__ == "B200Error"
+    assert both(lambda m: m.attn_decode_paged(q, k, v, table.long(), lens, 20, 0.125, 2))[0].__name__ == "B200Error"
+    assert both(lambda m: m.attn_decode_paged(q.transpose(0, 1), k, v, table, lens, 20, 0.125, 2))[0] is AssertionError
+    cu = torch.tensor([0, 1, 2], dtype=torch.int32, device=DEV)
+    both(lambda m: m.attn_prefill_paged(q, k, v, table, lens, cu, 1, 0.125))
+    assert both(lambda m: m.attn_prefill_paged(q, k[:, :, ::2], v, table, lens, cu, 1, 0.125))[0] is AssertionError
+    assert both(lambda m: m.attn_prefill_paged(q, k, v, table, lens, cu.long(), 1, 0.125))[0].__name__ == "B200Error"
+
+
+def test_first_calls_inside_a_capture(both):
+    """a workspace that has to grow while a stream is captured comes from the capture's pool, as the Python path's does"""
+    x = _r(4, 512) if both.name == "ops" else _r(4, 512, dtype=torch.bfloat16)
+    w = _r(40960, 512, dtype=x.dtype)
+
+    def call(m):
+        f = m.gemm_f16 if both.name == "ops" else m.linear
+        f(x, w)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            y = f(x, w)
+        graph.replay()
+        torch.cuda.synchronize()
+        return y.clone()
+    both(call)

@@ -189,8 +189,11 @@ _SEQ_SHARED = ("b200_last_error", "b200_gave_up", "b200_debug_set_gave_up", "b20
                "b200_kv_alloc_num_free", "b200_kv_alloc_take", "b200_kv_alloc_release", "b200_decode_advance", "b200_gemm_bf16",
                "b200_gemm_workspace_bytes_max", "b200_debug_step_trace", "b200_debug_step_trace_begin", "b200_debug_step_trace_names")
 
+HOST_PATH = os.path.join(_HERE, "_b200_host.so")
+
 _lib = None
 _seq_lib = None
+_host = None
 
 
 class B200Error(RuntimeError):
@@ -247,6 +250,25 @@ def load() -> ctypes.CDLL:
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+def load_host(which: int, lib: ctypes.CDLL, gemm_workspace, attn_workspace):
+    """The native per-call host side (csrc/host/host_calls.cpp), bound to a loaded library (which: 0 libb200_tgis.so, 1 libb200_seq.so) and to the callables
+    that hand out its workspaces.  Its functions return None for a call that they leave to Python."""
+    global _host
+    if _host is None:
+        import importlib.machinery
+        import importlib.util
+        if not os.path.exists(HOST_PATH):
+            raise B200Error(f"{HOST_PATH} is missing: build it with `python text-generation-inference_b200/build.py`")
+        loader = importlib.machinery.ExtensionFileLoader("_b200_host", HOST_PATH)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_b200_host", loader))
+        loader.exec_module(mod)
+        _host = mod
+    entries = [n for n in ("b200_gemm_workspace_bytes_max", "b200_gemm_w4a16_ex", "b200_gemm_f16", "b200_gemm_bf16", "b200_attn_decode_workspace_bytes",
+                           "b200_attn_decode_paged", "b200_attn_prefill_paged") if hasattr(lib, n)]
+    _host.bind(which, {n: ctypes.cast(getattr(lib, n), c_void_p).value for n in entries}, gemm_workspace, attn_workspace)
+    return _host
 
 
 def check(status: int, what: str) -> None:

@@ -4,21 +4,26 @@
   libb200_tgis.so  every source: the whole C ABI of include/b200_tgis.h
   libb200_seq.so   the sources the hybrid decoder families need (seq_*.cu + the block allocator and the runtime pieces); a
                    process that serves only such a model builds and loads this one (`--seq`, `build(target="seq")`)
-Objects are shared between the two.  The libraries are git-ignored; they are built in the tree at first use.
+  _b200_host.so    csrc/host/host_calls.cpp: the operators' per-call host work as a CPython extension over torch's C++ headers
+Objects are shared between the first two.  The libraries are git-ignored; they are built in the tree at first use.
 """
 from __future__ import annotations
 
 import concurrent.futures
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(CSRC, "_obj")
 LIB = os.path.join(HERE, "libb200_tgis.so")
 SEQ_LIB = os.path.join(HERE, "libb200_seq.so")
+HOST_SRC = os.path.join(CSRC, "host", "host_calls.cpp")
+HOST_LIB = os.path.join(HERE, "_b200_host.so")
 SEQ_EXTRA_SOURCES = ("runtime.cu", "kv_alloc.cu", "gemm_f16.cu")
 
 NVCC_FLAGS = [
@@ -48,6 +53,23 @@ def _stale(target: str, deps) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_host(force: bool = False) -> None:
+    if not force and not _stale(HOST_LIB, [HOST_SRC]):
+        return
+    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    part = f"{HOST_LIB}.{os.getpid()}.part"
+    includes = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
+                os.path.join(cuda, "include")]
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-D_GLIBCXX_USE_CXX11_ABI=1", *(f"-I{d}" for d in includes), HOST_SRC, "-o", part,
+           f"-L{os.path.join(torch_dir, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("g++ failed on host_calls.cpp")
+    os.replace(part, HOST_LIB)
+
+
 def build(force: bool = False, verbose: bool = False, target: str = "all") -> str:
     """target "all": both libraries; "seq": libb200_seq.so only (compiles nothing else)."""
     os.makedirs(OBJ, exist_ok=True)
@@ -67,7 +89,8 @@ def build(force: bool = False, verbose: bool = False, target: str = "all") -> st
         r = subprocess.run(cmd, capture_output=True, text=True)
         return src, r
 
-    with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
+    with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, 1 + len(jobs))) as ex:
+        host = ex.submit(build_host, force)
         for src, r in ex.map(compile_one, jobs):
             if r.returncode != 0:
                 sys.stderr.write(r.stdout + r.stderr)
@@ -76,6 +99,7 @@ def build(force: bool = False, verbose: bool = False, target: str = "all") -> st
                 sys.stderr.write(f"== {src}\n{r.stderr}\n")
             with open(os.path.join(OBJ, src[:-3] + ".ptxas.txt"), "w") as f:
                 f.write(r.stderr)
+        host.result()
     for lib, which in ((LIB, "all"), (SEQ_LIB, "seq")):
         if target == "seq" and which == "all":
             continue

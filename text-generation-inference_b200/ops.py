@@ -131,12 +131,33 @@ def argmax(logits: torch.Tensor, banned_ids: Optional[torch.Tensor] = None, out:
 
 
 _attn_ws = {}
+_host = None
+
+
+def _native():
+    """the native side of the calls below; what it does not serve comes back as None and takes the Python path, which also raises the errors"""
+    global _host
+    if _host is None:
+        _host = _lib.load_host(0, _lib.load(), lambda x, N, K: gemm_workspace(x.device, 0, N, K), lambda q, need: _attn_workspace(q.device, need))
+    return _host
+
+
+def _attn_workspace(device, need: int) -> torch.Tensor:
+    """per-device grow-only workspace"""
+    workspace = _attn_ws.get(device)
+    if workspace is None or workspace.numel() < need:
+        workspace = torch.zeros(max(need, 1 << 22), dtype=torch.uint8, device=device)
+        _attn_ws[device] = workspace
+    return workspace
 
 
 def attn_decode_paged(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor, block_table: torch.Tensor,
                       context_lens: torch.Tensor, max_context_len: int, softmax_scale: float, n_kv_heads: int,
                       out: Optional[torch.Tensor] = None, workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
     """q [B, n_heads, d] (may be a strided view of the fused qkv activation: stride(0) arbitrary, inner contiguous)."""
+    done = (_host or _native()).attn_decode_paged(q, k_pool, v_pool, block_table, context_lens, max_context_len, softmax_scale, n_kv_heads, out, workspace)
+    if done is not None:
+        return done
     _req(q, torch.float16, "q")
     _req(block_table, torch.int32, "block_table")
     _req(context_lens, torch.int32, "context_lens")
@@ -146,11 +167,8 @@ def attn_decode_paged(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tenso
         out = torch.empty(B, h, d, dtype=torch.float16, device=q.device)
     lib = _lib.load()
     need = lib.b200_attn_decode_workspace_bytes(B, h, d, max_context_len)
-    if workspace is None:  # per-device grow-only workspace
-        workspace = _attn_ws.get(q.device)
-        if workspace is None or workspace.numel() < need:
-            workspace = torch.zeros(max(need, 1 << 22), dtype=torch.uint8, device=q.device)
-            _attn_ws[q.device] = workspace
+    if workspace is None:
+        workspace = _attn_workspace(q.device, need)
     elif workspace.numel() * workspace.element_size() < need:
         raise _lib.B200Error("attn_decode_paged: workspace too small")
     _lib.check(lib.b200_attn_decode_paged(_ptr(q), q.stride(0), _ptr(k_pool), _ptr(v_pool), _ptr(block_table),
@@ -183,6 +201,9 @@ def attn_prefill_paged(q: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tens
                        out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """q [T_q, h, d] (a strided view of the fused qkv activation is fine); pools [num_blocks, n_kv, 16, d] already holding this
     step's K / V; context_lens [B] include them.  Causal over absolute positions (queries may follow a cached context)."""
+    done = (_host or _native()).attn_prefill_paged(q, k_pool, v_pool, block_table, context_lens, cu_seqlens_q, max_q, softmax_scale, out)
+    if done is not None:
+        return done
     _req(q, torch.float16, "q")
     _req(block_table, torch.int32, "block_table")
     _req(context_lens, torch.int32, "context_lens")
@@ -219,6 +240,9 @@ def gemm_workspace(device, T: int, N: int, K: int) -> torch.Tensor:
 def gemm_f16(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
              workspace: Optional[torch.Tensor] = None) -> torch.Tensor:
     """x [T,K] @ w[N,K]^T -> [T,N] fp16."""
+    done = (_host or _native()).gemm_f16(x, w, bias, out, workspace)
+    if done is not None:
+        return done
     _req(x, torch.float16, "x")
     _req(w, torch.float16, "w")
     assert x.is_contiguous() and w.is_contiguous()
@@ -273,6 +297,9 @@ def gemm_w4a16(x: torch.Tensor, packed: torch.Tensor, N: int, groupsize: int, bi
                silu_mul: bool = False) -> torch.Tensor:
     """x [T,K] fp16 @ dequant(packed) -> [T,N] fp16; `packed` from gptq_pack for the same (K, N, groupsize, layout).
     silu_mul (gate|up layout only): returns [T, N/2] = SiLU(x Wgate) * (x Wup)."""
+    done = (_host or _native()).gemm_w4a16(x, packed, N, groupsize, bias, out, workspace, layout, silu_mul)
+    if done is not None:
+        return done
     _req(x, torch.float16, "x")
     _req(packed, torch.uint8, "packed")
     assert x.is_contiguous() and packed.is_contiguous()

@@ -82,6 +82,17 @@ def _gemm_workspace(device, N: int, K: int, side: Optional[bool] = None) -> torc
     return ws
 
 
+_host = None
+
+
+def _native():
+    """the native side of `linear`; what it does not serve comes back as None and takes the Python path, which also raises the errors"""
+    global _host
+    if _host is None:
+        _host = _lib.load_host(1, _lib.load_seq(), lambda x, N, K: _gemm_workspace(x.device, N, K, side=False), None)
+    return _host
+
+
 class beside:
     """`with beside(device) as s:` queues what is inside on a second stream, behind everything queued so far; `s.join()` makes the current
     stream wait for it.  Only while a CUDA graph is captured: there the two branches become parallel parts of the graph, so that the
@@ -131,6 +142,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
     """act(x [M, K] @ w [N, K]^T) -> [M, N], fp32 accumulation (act: ACT_NONE or ACT_RELU2).  bfloat16 operands go to the tcgen05 product
     (csrc/gemm_f16.cu, output bfloat16 or fp32) when they are dense and K is a multiple of 8 of at least 64; everything else - float32 operands
     (a true 32-bit product), row-strided slices, small or odd K - to the plain product with ascending-k accumulation."""
+    if out is None and act == ACT_NONE and _TC_GEMM and not _on_side and (out_dtype is None or out_dtype in (torch.bfloat16, torch.float32)):
+        done = (_host or _native()).linear_bf16(x, w, bias, int(out_dtype == torch.float32))
+        if done is not None:
+            return done
     _cuda(x, w, bias)
     assert x.dim() == 2 and w.dim() == 2 and x.stride(1) == 1 and w.stride(1) == 1 and x.shape[1] == w.shape[1]
     M, K = x.shape
