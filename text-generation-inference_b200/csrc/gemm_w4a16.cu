@@ -1,5 +1,6 @@
 // GPTQ int4 linear  Y[T,N] = X[T,K] . dequant(Wq)[K,N]  on tcgen05 tensor cores, weights de-quantised in-kernel
-// straight into TMEM (no fp16 scratch matrix, for any T).  This kernel takes calls of up to 128 tokens (kW4DecodeT), gemm_pair.cuh larger ones.
+// straight into TMEM (no fp16 scratch matrix, for any T).  This kernel takes calls of up to 128 tokens (kW4DecodeT) but for
+// those of gemm_w4_few.cuh, gemm_pair.cuh larger ones.
 //
 // Replaces `exllamav2_kernels.make_q_matrix` / `gemm_half_q_half`
 // (server/text_generation_server/utils/gptq/exllamav2.py:14-62,139-144), including its M > 50
@@ -43,6 +44,7 @@
 // later use test_wait: try_wait may suspend the thread until a time-out while the phase is pending.
 #include "common.cuh"
 #include "gemm_pair.cuh"
+#include "gemm_w4_few.cuh"
 #include "tmap.cuh"
 #include "w4_format.cuh"
 #include "../../include/b200_tgis.h"
@@ -855,6 +857,39 @@ static int gemm_w4a16_impl(const void* x, const void* packed, const void* bias, 
     const PairPlan pl = pair_plan(T, N, pp.n_kb, true, b200_num_sms());
     return act ? launch_gemm_pair<kPairW4Silu>(x, nullptr, K, pp, pl, B200_TIME_GEMM_W4A16, (cudaStream_t)stream)
                : launch_gemm_pair<kPairW4>(x, nullptr, K, pp, pl, B200_TIME_GEMM_W4A16, (cudaStream_t)stream);
+  }
+  const W4FewPlan few = T <= kFewMostT ? few_plan(N, K, few_clusters()) : W4FewPlan{0, 0};
+  if (few.d && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+    W4FewParams fp = {};
+    fp.x = (const __half*)x;
+    fp.y = (__half*)y;
+    fp.partial = defer ? (float*)((char*)workspace + kW4CounterBytes) : nullptr;
+    fp.bias = (const __half*)bias;
+    fp.packed = (const unsigned char*)packed;
+    fp.T = (int)T;
+    fp.N = (int)N;
+    fp.K = (int)K;
+    fp.nkb = (int)((K + kW4BlockK - 1) / kW4BlockK);
+    fp.rec_per_tile = w4_nkb(K);
+    fp.half_tiles = half_tiles;
+    fp.act = act;
+    fp.ldy = (int)(act ? N / 2 : N);
+    fp.tn = kFewMostT;
+    fp.x_blocks = few.blocks;
+    fp.gave_up = b200_gave_up_word();
+    if (!fp.gave_up) return B200_ERR_CUDA;
+    if (defer) {
+      splitk->partial = fp.partial;
+      splitk->bias = bias;
+      splitk->tiles_per_unit = kW4R;
+      splitk->tn = fp.tn;
+      splitk->nkb = splitk->units_per_cta = fp.nkb;   // one contributor
+      splitk->max_contrib = 1;
+      splitk->half_tiles = half_tiles;
+      splitk->N = (int32_t)N;
+      splitk->T = (int32_t)T;
+    }
+    return launch_w4_few_plan(fp, gr, (int)((N + kW4R * kW4TileM - 1) / (kW4R * kW4TileM)), few, (cudaStream_t)stream);
   }
   const W4Plan pl = launch_plan_w4(T, N, K, b200_num_sms(), workspace != nullptr, defer);
   const CUtensorMap* mx = get_tmap_2d(x, T, K, K, pl.TN, 64, TmapDtype::kF16, TmapSwizzle::k128B);
