@@ -44,7 +44,10 @@ constexpr int kTileK = 64;   // fp16 elements per k-block = one 128-byte swizzle
 // says which kernel takes less.  Measured on B200 (us, this kernel / pairs) at 65 tokens: 4096 -> 4096 16.1 / 13.0, 4096 -> 22016 42.2 / 40.0, 5632 -> 2048
 // 16.8 / 15.0, 11008 -> 4096 25 / 29, 16384 -> 2048 25 / 38, 28672 -> 2048 32 / 63, 28672 -> 8192 81 / 93; at 128: 20.8 / 13.5, 45.5 / 41.8, 24.6 / 15.0, 30 / 29,
 // 32 / 38, 39 / 63, 86 / 94; at 256: 33.5 / 15.6, 68 / 50, 44 / 15, 44 / 36, 51 / 38, 61 / 61; at 192 28672 -> 8192 110 / 100.
-constexpr int kF16DecodeT = 64, kF16MostT = 256;
+// Up to 64 tokens the pairs take wide outputs only (feature tiles that no wave of clusters holds), from kF16PairT tokens on; us, this kernel / pairs, at 16
+// and 64 tokens: 2048 -> 11264 10.9 / 10.6 and 13.0 / 11.7, 2048 -> 32000 24.1 / 22.8 and 29.0 / 24.3, 4096 -> 12288 18.9 / 18.9 and 21.1 / 20.4, 5120 ->
+// 15360 25.8 / 26.6 and 28.4 / 28.4, 4096 -> 22016 (a wave and a sixth) 31.4 / 34.7 and 37.0 / 38.5.
+constexpr int kF16PairT = 16, kF16DecodeT = 64, kF16MostT = 256;
 // fp32 results show how long a sum ran in the tensor cores: cut into stream-K pieces that are added in fp32 it is off by 5e-7 (against float64,
 // k = 2048), in one piece by 2e-6.  So they stay here for as long as this kernel cuts them (one token tile).
 constexpr int64_t kCounterBytes = 64 * 1024;
@@ -55,8 +58,9 @@ struct GemmF16Cfg {
   static constexpr int kBBytes = TN * kTileK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kStages = TN <= 64 ? 8 : (TN == 128 ? 6 : 4);
-  static constexpr int kTmemCols = TN < 32 ? 32 : TN;
+  static constexpr int kTmemCols = 2 * TN;   // clusters: an accumulator for either half of a CTA's k
   static constexpr int kSmemBytes = kStages * kStageBytes + (2 * kStages + 2) * 8 + 16 + 1024;
+  static_assert(TN * (kTileM + 4) * 4 <= kStages * kStageBytes, "a cluster's sums lie where the ring was");
 };
 
 struct F16Params {
@@ -69,8 +73,59 @@ struct F16Params {
   int units_per_cta;  // contiguous (tile, k-block) units per CTA
   int total_units;
   int max_contrib;    // partial slots per tile
+  int cluster;        // > 0: a cluster of so many CTAs has one feature tile, each a part of k
   int defer;          // 1: leave every tile segment as an fp32 partial for the consumer kernel (B200SplitK), no fix-up
 };
+
+constexpr int kF16SumPitch = kTileM + 4;   // floats of a token's sums in shared memory
+
+// The end of a feature tile that a cluster shares: every CTA has fp32 sums of its part of k in shared memory ([token][kF16SumPitch]); CTA r adds its share of
+// the outputs over all of them in their order.  Against partial sums in global memory that the last CTA to arrive adds by itself (us in a replayed graph,
+// 8 / 32 / 64 tokens): 2048 -> 2048 5.1 / 8.2 / 13.0 -> 5.3 / 5.8 / 6.9, 4096 -> 4096 9.0 / 11.5 / 14.5 -> 9.4 / 10.2 / 10.9, 11008 -> 4096 16.5 / 18.9 / 21.9 ->
+// 17.0 / 17.8 / 18.6, 20480 -> 5120 42.3 / 44.9 / 49.5 -> 35.2 / 36.1 / 40.7 (three CTAs to a tile instead of tiles that straddle CTAs).
+template <int FMT>
+__device__ __forceinline__ void f16_cluster_sum(const F16Params& p, const float* sums, int tile, int rank) {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const uint32_t base = smem_u32(sums);
+  const int d = p.cluster, items = p.T * (kTileM / 4), share = (items + d - 1) / d, hi = min(items, (rank + 1) * share);
+  for (int i = rank * share + (int)threadIdx.x; i < hi; i += kGemmThreads) {
+    const int tok = i / (kTileM / 4), m = (i % (kTileM / 4)) * 4, n = tile * kTileM + m;
+    const uint32_t at = base + (tok * kF16SumPitch + m) * 4;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int c = 0; c < d; c += 4) {
+      float v[4][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (c + j < d) {
+          const uint32_t a = cluster_map(at, c + j);
+          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[j][0]), "=f"(v[j][1]), "=f"(v[j][2]), "=f"(v[j][3]) : "r"(a) : "memory");
+        } else {
+          v[j][0] = v[j][1] = v[j][2] = v[j][3] = 0.f;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[e] += v[j][e];
+    }
+    if (p.bias)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[e] += n + e < p.N ? gemm_load_bias<FMT>(p.bias, n + e) : 0.f;
+    const size_t o = (size_t)tok * p.N + n;
+    if (FMT == 0 && n + 3 < p.N && (p.N & 3) == 0) {
+      *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(p.y) + o) = make_uint2(pack_half2(s[0], s[1]), pack_half2(s[2], s[3]));
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (n + e < p.N) gemm_store<FMT>(p.y, o + e, s[e]);
+    }
+  }
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // nobody leaves while its sums are read
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 template <int TN, int FMT>
 __global__ void __launch_bounds__(kGemmThreads, 1)
@@ -87,8 +142,9 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
 
   pdl_launch_dependents();
   const int warp = warp_id(), lane = lane_id();
-  const int u0 = blockIdx.x * p.units_per_cta;
-  const int u1 = min(p.total_units, u0 + p.units_per_cta);
+  const int c_tile = p.cluster ? (int)blockIdx.x / p.cluster : 0, c_rank = p.cluster ? (int)blockIdx.x - c_tile * p.cluster : 0;
+  const int u0 = p.cluster ? c_tile * p.nkb + c_rank * p.nkb / p.cluster : blockIdx.x * p.units_per_cta;
+  const int u1 = p.cluster ? c_tile * p.nkb + (c_rank + 1) * p.nkb / p.cluster : min(p.total_units, u0 + p.units_per_cta);
   const int n_units = u1 - u0;
   const int tile0 = u0 / p.nkb, kb0 = u0 - tile0 * p.nkb;
 
@@ -141,9 +197,12 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     constexpr uint32_t idesc = umma_idesc_f16_f32acc(kTileM, TN) | (FMT != 0 ? ((1u << 7) | (1u << 10)) : 0u);  // a/b format 1 = bf16
+    const int half = p.cluster ? (n_units + 1) / 2 : n_units;   // clusters: the second half of the part of k has an accumulator of its own
+    uint32_t d = tmem_d;
     int seg = 0, kb = kb0;
     for (int i = 0; i < n_units; ++i) {
-      const bool seg_first = (i == 0) || kb == 0;
+      if (i == half) d += TN;
+      const bool seg_first = (i == 0) || kb == 0 || i == half;
       const bool seg_last = (i == n_units - 1) || kb == p.nkb - 1;
       const int s = i % C::kStages;
       if (seg_first && seg > 0) mbar_wait(tmem_empty, (seg - 1) & 1);  // epilogue drained the previous segment's D
@@ -155,7 +214,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
         const uint64_t bdesc = umma_desc_kmajor_sw128(a_addr + C::kABytes);
 #pragma unroll
         for (int k = 0; k < kTileK / 16; ++k)
-          umma_f16_ss(tmem_d, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, (!seg_first || k > 0) ? 1u : 0u);
+          umma_f16_ss(d, adesc + (uint64_t)(k * 2), bdesc + (uint64_t)(k * 2), idesc, (!seg_first || k > 0) ? 1u : 0u);
         umma_commit(&empty_bar[s]);
         if (seg_last) umma_commit(tmem_full);
       }
@@ -181,6 +240,19 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
       const int my_contrib = (int)blockIdx.x - c_first;
       mbar_wait(tmem_full, seg & 1);
       tcgen05_fence_after();
+      if (p.cluster) {   // one segment; the ring has been used up: every product is done
+        float* sums = reinterpret_cast<float*>(smem);
+#pragma unroll 1
+        for (int c = 0; c < TN; c += 16) {
+          uint32_t d0[16], d1[16];
+          tmem_ld_32x32b_x16(tmem_d + lane_base + c, d0);
+          tmem_ld_32x32b_x16(tmem_d + lane_base + TN + c, d1);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) sums[(c + j) * kF16SumPitch + m] = n_units > 1 ? __uint_as_float(d0[j]) + __uint_as_float(d1[j]) : __uint_as_float(d0[j]);
+        }
+        break;
+      }
       const float bv = (p.bias && n_ok) ? gemm_load_bias<FMT>(p.bias, n) : 0.f;
       float* part = p.partial + ((size_t)tile * p.max_contrib + my_contrib) * (TN * kTileM);
 #pragma unroll 1
@@ -285,11 +357,51 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
   tcgen05_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc<C::kTmemCols>(tmem_d);
+  if (p.cluster) {
+    pdl_wait();
+    f16_cluster_sum<FMT>(p, reinterpret_cast<const float*>(smem), c_tile, c_rank);
+  }
 }
 
 struct F16Plan {
   int TN, nkb, n_tiles_n, units_per_cta, n_ctas, max_contrib;
 };
+
+// CTAs of a cluster -> clusters that the chip holds at one CTA per SM (148 SMs in GPCs of unlike size: 15 clusters of eight, 22 of six, 26 of five, 33 of
+// four, 45 of three, 74 of two).  More would be a second wave, which takes a launch twice as long.
+static const int* f16_clusters() {
+  static const struct Table {
+    int n[9];
+    Table() : n{0, 0, 74, 45, 33, 26, 22, 15, 15} {   // (plans made without a device)
+      constexpr auto kernel = gemm_f16_kernel<64, 0>;
+      constexpr int smem = GemmF16Cfg<64>::kSmemBytes;
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      for (int d = 2; d <= 8; ++d) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(d * 16));
+        cfg.blockDim = dim3(kGemmThreads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)d;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int v;
+        if (cudaOccupancyMaxActiveClusters(&v, kernel, &cfg) == cudaSuccess) n[d] = v;
+      }
+      cudaGetLastError();
+    }
+  } table;
+  return table.n;
+}
+// CTAs per feature tile: the most that one wave of clusters allows, of at least four k-blocks; 0: not two
+static int f16_cluster(int64_t N, int64_t K, const int* clusters) {
+  const int64_t tiles = (N + kTileM - 1) / kTileM, nkb = (K + kTileK - 1) / kTileK;
+  for (int d = 8; d >= 2; --d)
+    if (clusters[d] >= tiles && nkb / d >= 4) return d;
+  return 0;
+}
 
 // a call of up to kF16MostT tokens: one token tile
 static F16Plan plan_f16(int64_t T, int64_t N, int64_t K, int sms, bool defer = false) {
@@ -392,9 +504,15 @@ extern "C" int64_t b200_gemm_workspace_bytes_max(int64_t N, int64_t K) {
 
 // whether a call's kernel is that of gemm_pair.cuh
 static bool f16_takes_pairs(int fmt, int64_t T, int64_t N, int64_t K, bool workspace, int sms) {
-  if (T <= kF16DecodeT || (fmt == 2 && T <= kF16MostT)) return false;
-  if (T > kF16MostT || !workspace) return true;
+  if (T <= kF16PairT || (fmt == 2 && T <= kF16MostT)) return false;
+  if (T > kF16MostT || (!workspace && T > kF16DecodeT)) return true;
   const F16Plan pl = plan_f16(T, N, K, sms);
+  if (T <= kF16DecodeT) {
+    // Wide outputs: both stream the weights at the memory's rate, the pairs without fix-ups; but the pairs' last wave has to be a full one, and over
+    // three waves and more the fix-ups no longer show (4096 -> 128256 at 64 tokens 168 us, 96 % of the memory's rate).
+    const int64_t n_m = (N + kPairM - 1) / kPairM, pairs = sms / 2, waves = (n_m + pairs - 1) / pairs;
+    return f16_cluster(N, K, f16_clusters()) == 0 && workspace && waves <= 2 && (waves == 1 || n_m * 5 >= waves * pairs * 4);
+  }
   if ((int64_t)pl.n_tiles_n * 4 > kCounterBytes) return true;
   return pair_plan(T, N, pl.nkb, false, sms).us <= f16_stream_us(pl, T);
 }
@@ -407,7 +525,7 @@ static int f16_pieces(int64_t T, int64_t N, int64_t K, int sms) {
 
 template <int TN, int FMT>
 static int launch_gemm_f16(const CUtensorMap* mw, const CUtensorMap* mx, void* y, void* workspace, const void* bias, int T, int N,
-                           const F16Plan& pl, int defer, cudaStream_t st) {
+                           const F16Plan& pl, int cluster, int defer, cudaStream_t st) {
   using C = GemmF16Cfg<TN>;
   static bool configured = false;
   if (!configured) {
@@ -426,10 +544,14 @@ static int launch_gemm_f16(const CUtensorMap* mw, const CUtensorMap* mx, void* y
   p.units_per_cta = pl.units_per_cta;
   p.total_units = pl.n_tiles_n * pl.nkb;
   p.max_contrib = pl.max_contrib;
+  p.cluster = cluster;
   p.defer = defer;
-  const dim3 grid(pl.n_ctas);
+  const dim3 grid(cluster ? pl.n_tiles_n * cluster : pl.n_ctas);
   b200_timing_mark(B200_TIME_GEMM_F16, 0, st);
-  B200_LAUNCH((gemm_f16_kernel<TN, FMT>), grid, dim3(kGemmThreads), (size_t)C::kSmemBytes, st, *mw, *mx, p);
+  constexpr auto kernel = gemm_f16_kernel<TN, FMT>;
+  const cudaError_t le = b200_launch_cluster(kernel, grid, dim3(kGemmThreads), (size_t)C::kSmemBytes, st, (unsigned)cluster, *mw, *mx, p);
+  if (le != cudaSuccess) { b200_set_last_error(cudaGetErrorString(le)); return B200_ERR_CUDA; }
+  b200_step_trace_stamp("gemm_f16_kernel", st);
   b200_timing_mark(B200_TIME_GEMM_F16, 1, st);
   b200_count_launches(1);
   return B200_OK;
@@ -480,12 +602,16 @@ static int gemm_f16_impl(const void* x, const void* w, const void* bias, void* y
   }
   cudaStream_t st = (cudaStream_t)stream;
   const int df = defer ? 1 : 0;
+  int cluster = defer ? 0 : f16_cluster(N, K, f16_clusters());
+  // Few tokens leave partial sums of a few KB, and equal parts of a tile may be more CTAs than clusters allow (us, this kernel without / with clusters,
+  // eight tokens: 5632 -> 2048 6.9 / 7.5, 4096 -> 4096 9.0 / 9.3, 2048 -> 2048 5.1 / 5.2; fewer CTAs, 2048 -> 2560 5.6 / 5.5, 20480 -> 5120 42.3 / 35.2).
+  if (T <= 8 && workspace && pl.nkb % pl.units_per_cta == 0 && pl.n_ctas >= pl.n_tiles_n * cluster) cluster = 0;
   switch (pl.TN) {
-    case 16: return launch_gemm_f16<16, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, df, st);
-    case 32: return launch_gemm_f16<32, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, df, st);
-    case 64: return launch_gemm_f16<64, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, df, st);
-    case 128: return launch_gemm_f16<128, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, df, st);
-    default: return launch_gemm_f16<256, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, df, st);
+    case 16: return launch_gemm_f16<16, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, df, st);
+    case 32: return launch_gemm_f16<32, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, df, st);
+    case 64: return launch_gemm_f16<64, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, df, st);
+    case 128: return launch_gemm_f16<128, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, df, st);
+    default: return launch_gemm_f16<256, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, df, st);
   }
 }
 extern "C" int b200_gemm_f16(const void* x, const void* w, const void* bias, void* y, int64_t T, int64_t N, int64_t K,

@@ -255,21 +255,8 @@ static W4FewPlan few_plan(int64_t N, int64_t K, const int* clusters) {
 
 template <int kGR>
 static int launch_w4_few(const W4FewParams& p, int n_super, int d, cudaStream_t st) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(n_super * d));
-  cfg.blockDim = dim3(kFewThreads);
-  cfg.dynamicSmemBytes = (size_t)few_smem(p.x_blocks);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)d;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = b200_pdl_enabled() ? 2 : 1;
   b200_timing_mark(B200_TIME_GEMM_W4A16, 0, st);
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_w4_few_kernel<kGR>, p);
+  const cudaError_t e = b200_launch_cluster(gemm_w4_few_kernel<kGR>, dim3((unsigned)(n_super * d)), dim3(kFewThreads), (size_t)few_smem(p.x_blocks), st, (unsigned)d, p);
   if (e != cudaSuccess) { b200_set_last_error(cudaGetErrorString(e)); return B200_ERR_CUDA; }
   b200_step_trace_stamp("gemm_w4_few_kernel", st);
   b200_timing_mark(B200_TIME_GEMM_W4A16, 1, st);
