@@ -10,8 +10,12 @@
 //     cp.async.bulk (TMA, one 2-4 KB copy per page-head tile for K and V) into a 3/4-stage ring, mbarrier-tracked
 //   * the GQA group's G query heads form the (padded) 16-row A operand of m16n8k16 HMMA so every K/V byte is read
 //     once per group; fp32 online softmax with quad shuffles; P rounded to fp16 before P.V like flash-attn
-//   * per-chunk (m, l, O) partials -> fp32 workspace, merged by attn_decode_combine_kernel
+//   * up to eight chunks: a cluster has a (sequence, kv head); its CTAs cut the sequence's own pages into equal runs, leave (m, l, O) in shared memory and
+//     each merge a share of the outputs through distributed shared memory.  More chunks: partials -> fp32 workspace, merged by attn_decode_combine_kernel
 // The kernel is bandwidth-bound: algorithmic bytes = 2 * L * d * 2 B per (sequence, kv head).
+// Measured on B200, us in a replayed graph, 32 / 8 heads of 128 (a second kernel merges always / as here): 1 x 16 tokens 3.9 / 2.65, 64 x 16 - 32 8.3 / 5.9, 64 x
+// 256 - 512 (one run each) 24.5 / 22.0, 1 x 1024 6.4 / 5.2, 8 x 256 - 512 7.2 / 5.7, 4 x 2048 - 4096 13.7 / 12.5; 64 x 1024 - 2048, where it still does, 72.1 -> 70.0
+// since all its loads are in flight at once.
 #include "common.cuh"
 
 #include <cstdlib>
@@ -24,6 +28,7 @@ constexpr int kPagesPerStage = 4;
 constexpr int kConsumerWarps = 4;
 constexpr int kDecodeThreads = (kConsumerWarps + 1) * 32;
 constexpr float kNegBig = -1.0e30f;
+constexpr int kMaxCluster = 8;        // runs of a sequence that a cluster merges
 
 template <int D>
 struct DecodeSmem {
@@ -34,12 +39,22 @@ struct DecodeSmem {
   static constexpr int kBytes = kStages * kStageBytes + 2 * kStages * 8 + 16;
 };
 
-template <int D>
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, uint32_t rank) {
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// kMerge: gridDim.x CTAs are one cluster and write `out`; otherwise chunks of chunk_tokens leave partials
+template <int D, bool kMerge>
 __global__ void __launch_bounds__(kDecodeThreads, 2)
 attn_decode_paged_kernel(const __half* __restrict__ q, int64_t q_token_stride, const __half* __restrict__ k_pool,
                          const __half* __restrict__ v_pool, const int32_t* __restrict__ block_table, int64_t bt_stride,
                          const int32_t* __restrict__ context_lens, float* __restrict__ part_o, float* __restrict__ part_ml,
-                         int n_heads, int n_kv, int n_chunks_max, int chunk_tokens, float scale_log2) {
+                         __half* __restrict__ out, int64_t out_token_stride, int n_heads, int n_kv, int n_chunks_max, int chunk_tokens,
+                         float scale_log2) {
   using S = DecodeSmem<D>;
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* stages = smem;
@@ -49,13 +64,17 @@ attn_decode_paged_kernel(const __half* __restrict__ q, int64_t q_token_stride, c
   pdl_launch_dependents();
   pdl_wait();
   const int chunk = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
-  const int L = context_lens[b];
+  const int L = context_lens[b], G = n_heads / n_kv;
+  if (kMerge) {   // the sequence's own pages, cut evenly
+    chunk_tokens = max(1, ((L + n_chunks_max - 1) / n_chunks_max + kPageTokens - 1) / kPageTokens) * kPageTokens;
+    if (L <= 0 && chunk == 0)
+      for (int i = threadIdx.x; i < G * D; i += kDecodeThreads) out[(int64_t)b * out_token_stride + hk * G * D + i] = __float2half_rn(0.f);
+  }
   const int tok0 = chunk * chunk_tokens;
-  if (tok0 >= L) return;
+  if (tok0 >= L) return;   // (a cluster's barrier waits for threads that are still there)
   const int n_tok = min(chunk_tokens, L - tok0);
   const int n_pages = (n_tok + kPageTokens - 1) / kPageTokens;
   const int n_iters = (n_pages + kPagesPerStage - 1) / kPagesPerStage;
-  const int G = n_heads / n_kv;
   const int warp = warp_id(), lane = lane_id();
 
   if (threadIdx.x == 0) {
@@ -210,6 +229,8 @@ attn_decode_paged_kernel(const __half* __restrict__ q, int64_t q_token_stride, c
     if (tig == 0) { mml[(warp * 16 + g + 8) * 2] = m1; mml[(warp * 16 + g + 8) * 2 + 1] = l1; }
   }
   asm volatile("bar.sync 1, %0;" ::"n"(kConsumerWarps * 32));
+  float* run_o = mml + kConsumerWarps * 16 * 2;   // kMerge: this run's [G][D], then its [G][m, l]
+  float* run_ml = run_o + 16 * D;
   for (int idx = threadIdx.x; idx < G * D; idx += kConsumerWarps * 32) {
     const int r = idx / D, d = idx % D;
     float M = kNegBig;
@@ -222,29 +243,88 @@ attn_decode_paged_kernel(const __half* __restrict__ q, int64_t q_token_stride, c
       acc += f * mo[(w * 16 + r) * S::kMergeStride + d];
       lsum += f * mml[(w * 16 + r) * 2 + 1];
     }
-    const int64_t slot = ((int64_t)b * n_heads + hk * G + r) * n_chunks_max + chunk;
-    part_o[slot * D + d] = acc;
-    if (d == 0) { part_ml[slot * 2] = M; part_ml[slot * 2 + 1] = lsum; }
+    if (kMerge && n_chunks_max == 1) {
+      out[(int64_t)b * out_token_stride + hk * G * D + idx] = __float2half_rn(acc / lsum);
+    } else if constexpr (kMerge) {
+      run_o[idx] = acc;
+      if (d == 0) { run_ml[r * 2] = M; run_ml[r * 2 + 1] = lsum; }
+    } else {
+      const int64_t slot = ((int64_t)b * n_heads + hk * G + r) * n_chunks_max + chunk;
+      part_o[slot * D + d] = acc;
+      if (d == 0) { part_ml[slot * 2] = M; part_ml[slot * 2 + 1] = lsum; }
+    }
+  }
+  if constexpr (kMerge) {
+    if (n_chunks_max == 1) return;
+    const int runs = (L + chunk_tokens - 1) / chunk_tokens, share = (G * D + runs - 1) / runs, hi = min(G * D, (chunk + 1) * share);
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const uint32_t o_at = smem_u32(run_o), ml_at = smem_u32(run_ml);
+    for (int idx = chunk * share + (int)threadIdx.x; idx < hi; idx += kConsumerWarps * 32) {
+      const int r = idx / D;
+      float m[kMaxCluster], l[kMaxCluster], v[kMaxCluster], M = kNegBig, acc = 0.f, lsum = 0.f;
+#pragma unroll
+      for (int c = 0; c < kMaxCluster; ++c) {
+        m[c] = c < runs ? ld_cluster_f32(ml_at + r * 8, c) : kNegBig;
+        l[c] = c < runs ? ld_cluster_f32(ml_at + r * 8 + 4, c) : 0.f;
+        v[c] = c < runs ? ld_cluster_f32(o_at + idx * 4, c) : 0.f;
+      }
+#pragma unroll
+      for (int c = 0; c < kMaxCluster; ++c) M = fmaxf(M, m[c]);
+#pragma unroll
+      for (int c = 0; c < kMaxCluster; ++c) {
+        if (c < runs) {
+          const float f = fast_exp2(m[c] - M);
+          acc += f * v[c];
+          lsum += f * l[c];
+        }
+      }
+      out[(int64_t)b * out_token_stride + hk * G * D + idx] = __float2half_rn(acc / lsum);
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");   // nobody leaves while its run is read
   }
 }
 
 template <int D>
-__global__ void attn_decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+__global__ void __launch_bounds__(D) attn_decode_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                            const int32_t* __restrict__ context_lens, __half* __restrict__ out,
                                            int64_t out_token_stride, int n_heads, int n_chunks_max, int chunk_tokens) {
   pdl_launch_dependents();
   pdl_wait();
   const int head = blockIdx.x, b = blockIdx.y, d = threadIdx.x;
-  const int L = context_lens[b];
-  const int nc = (L + chunk_tokens - 1) / chunk_tokens;
   const int64_t base = ((int64_t)b * n_heads + head) * n_chunks_max;
-  float M = kNegBig;
-  for (int c = 0; c < nc; ++c) M = fmaxf(M, part_ml[(base + c) * 2]);
-  float acc = 0.f, l = 0.f;
-  for (int c = 0; c < nc; ++c) {
-    const float f = fast_exp2(part_ml[(base + c) * 2] - M);
-    acc += f * part_o[(base + c) * D + d];
-    l += f * part_ml[(base + c) * 2 + 1];
+  float M = kNegBig, acc = 0.f, l = 0.f;
+  int nc;
+  if (n_chunks_max <= 8) {   // everything that may count is under way at once: the length is one of several loads in flight, not ahead of them
+    float m8[8], l8[8], o8[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const bool in = c < n_chunks_max;
+      m8[c] = in ? part_ml[(base + c) * 2] : 0.f;
+      l8[c] = in ? part_ml[(base + c) * 2 + 1] : 0.f;
+      o8[c] = in ? part_o[(base + c) * D + d] : 0.f;
+    }
+    nc = (context_lens[b] + chunk_tokens - 1) / chunk_tokens;
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      if (c < nc) M = fmaxf(M, m8[c]);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      if (c < nc) {   // (beyond them lies whatever an earlier call has left)
+        const float f = fast_exp2(m8[c] - M);
+        acc += f * o8[c];
+        l += f * l8[c];
+      }
+    }
+  } else {
+    nc = (context_lens[b] + chunk_tokens - 1) / chunk_tokens;
+    for (int c = 0; c < nc; ++c) M = fmaxf(M, part_ml[(base + c) * 2]);
+    for (int c = 0; c < nc; ++c) {
+      const float f = fast_exp2(part_ml[(base + c) * 2] - M);
+      acc += f * part_o[(base + c) * D + d];
+      l += f * part_ml[(base + c) * 2 + 1];
+    }
   }
   out[(int64_t)b * out_token_stride + head * D + d] = __float2half_rn(nc > 0 ? acc / l : 0.f);
 }
@@ -273,18 +353,29 @@ static int launch_decode(const void* q, int64_t q_token_stride, const void* k_po
                          int64_t bt_stride, const int32_t* context_lens, void* out, int64_t out_token_stride, void* workspace,
                          int B, int n_heads, int n_kv, int n_chunks, int chunk_tokens, float scale, cudaStream_t st) {
   using S = DecodeSmem<D>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_paged_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes);
+  static const cudaError_t configured[2] = {cudaFuncSetAttribute(attn_decode_paged_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes),
+                                            cudaFuncSetAttribute(attn_decode_paged_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes)};
+  for (const cudaError_t e : configured)
     if (e != cudaSuccess) { b200_set_last_error(cudaGetErrorString(e)); return B200_ERR_CUDA; }
-    configured = true;
-  }
   float* part_o = (float*)workspace;
   float* part_ml = part_o + (int64_t)B * n_heads * n_chunks * D;
   dim3 grid(n_chunks, n_kv, B);
   b200_timing_mark(B200_TIME_ATTN_DECODE, 0, st);
-  B200_LAUNCH(attn_decode_paged_kernel<D>, grid, dim3(kDecodeThreads), (size_t)S::kBytes, st, (const __half*)q, q_token_stride,
-              (const __half*)k_pool, (const __half*)v_pool, block_table, bt_stride, context_lens, part_o, part_ml, n_heads, n_kv,
+  // One run needs no merging.  Clusters only while all CTAs are on the chip at once (two per SM): in a longer grid a CTA that waits for its cluster keeps the
+  // next one's loads from starting (64 x 1024 - 2048 tokens, 2048 CTAs: 72.1 us with the second kernel, 85.9 in clusters).
+  if (n_chunks == 1 || (n_chunks <= kMaxCluster && (int64_t)B * n_kv * n_chunks <= 2 * decode_num_sms())) {
+    constexpr auto kernel = attn_decode_paged_kernel<D, true>;
+    const cudaError_t e = b200_launch_cluster(kernel, grid, dim3(kDecodeThreads), (size_t)S::kBytes, st, n_chunks == 1 ? 0u : (unsigned)n_chunks, (const __half*)q, q_token_stride,
+                                              (const __half*)k_pool, (const __half*)v_pool, block_table, bt_stride, context_lens, part_o, part_ml, (__half*)out,
+                                              out_token_stride, n_heads, n_kv, n_chunks, chunk_tokens, scale * 1.4426950408889634f);
+    if (e != cudaSuccess) { b200_set_last_error(cudaGetErrorString(e)); return B200_ERR_CUDA; }
+    b200_step_trace_stamp("attn_decode_paged_kernel", st);
+    b200_timing_mark(B200_TIME_ATTN_DECODE, 1, st);
+    b200_count_launches(1);
+    return B200_OK;
+  }
+  B200_LAUNCH((attn_decode_paged_kernel<D, false>), grid, dim3(kDecodeThreads), (size_t)S::kBytes, st, (const __half*)q, q_token_stride,
+              (const __half*)k_pool, (const __half*)v_pool, block_table, bt_stride, context_lens, part_o, part_ml, (__half*)out, out_token_stride, n_heads, n_kv,
                 n_chunks, chunk_tokens, scale * 1.4426950408889634f);
   b200_timing_mark(B200_TIME_ATTN_DECODE, 1, st);
   b200_count_launches(1);

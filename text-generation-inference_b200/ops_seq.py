@@ -595,7 +595,7 @@ def delta_rows_scan(rows: torch.Tensor, S: torch.Tensor, step: RaggedStep, H: in
     assert rows.dtype == torch.float32 and rows.is_contiguous() and S.dtype == torch.float32 and S.is_contiguous() and S.shape[1:] == (H, dk, dv)
     y = torch.empty(step.T, H * dv, dtype=torch.float32, device=rows.device)
     lib = _lib.load_seq()
-    need = lib.b200_seq_delta_rows_scan_bytes(step.T, step.B, H, dk, dv)
+    need = lib.b200_seq_delta_rows_scan_bytes(step.T, step.B, H, dk, dv) if step.T >= 96 * step.B else 0   # (the fewest tokens that have a use for it)
     ws = torch.empty(need, dtype=torch.uint8, device=rows.device) if need else None
     _lib.check_seq(lib.b200_seq_delta_rows_scan(_ptr(rows), int(channels), _ptr(S), _ptr(step.state_slots), _ptr(step.cu_q),
                                                 _ptr(step.position_ids), _ptr(y), y.stride(0), step.T, step.B, H, kv_heads, dk, dv, _ptr(ws), _stream()),
