@@ -50,7 +50,7 @@ def test_few_tokens(N, K, gs, T):
     for _ in range(2):   # the workspace is left as it was found
         got = ops.gemm_w4a16(x, packed, N, gs, bias)
         _near(got, x, w, bias)
-        assert torch.equal(ops.splitk_reduce(ops.gemm_w4a16_deferred(x, packed, N, gs, bias=bias)), got) or T > 8
+        _near(ops.splitk_reduce(ops.gemm_w4a16_deferred(x, packed, N, gs, bias=bias)), x, w, bias)   # (goes the other way)
 
 
 @pytest.mark.parametrize("I,K", [(256, 512), (2048, 2048), (128, 96)])

@@ -27,10 +27,9 @@ constexpr int kFewMostT = 8, kFewMostBlocks = 8;   // tokens; k-blocks of a CTA
 struct W4FewParams {
   const __half* x;
   __half* y;
-  float* partial;   // != NULL: fp32 sums [super-tile][2][tn][128] for the next kernel instead of y (no bias, no activation)
   const __half* bias;
   const unsigned char* packed;
-  int T, N, K, nkb, rec_per_tile, half_tiles, act, ldy, tn, x_blocks;   // x_blocks: k-blocks a CTA has at most
+  int T, N, K, nkb, rec_per_tile, half_tiles, act, ldy, x_blocks;   // x_blocks: k-blocks a CTA has at most
   unsigned* gave_up;   // b200_gave_up_word
 };
 
@@ -197,8 +196,6 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemm_w4_few_kernel(const W4Few
       add_bias(u, col + p.half_tiles * kW4TileM);
       const __half o[4] = {silu_mul_f16(s.x, u.x), silu_mul_f16(s.y, u.y), silu_mul_f16(s.z, u.z), silu_mul_f16(s.w, u.w)};
       *reinterpret_cast<uint2*>(&p.y[(size_t)tok * p.ldy + col]) = *reinterpret_cast<const uint2*>(o);
-    } else if (p.partial) {
-      *reinterpret_cast<float4*>(&p.partial[(((size_t)sup * 2 + r) * p.tn + tok) * kW4TileM + m]) = s;
     } else {
       const int col = (p.half_tiles ? sup + r * p.half_tiles : sup * 2 + r) * kW4TileM + m;
       if (col < p.N) {   // N % 32 == 0: four columns never straddle it
