@@ -54,6 +54,31 @@ __device__ __forceinline__ float4 splitk_sum4(const B200SplitK& d, int t, int n)
   return acc;
 }
 
+// Two groups of four columns at once, all their loads in flight together; `bias_a`, `bias_b`: their first columns.  (The references are index arithmetic on
+// launch parameters: a kernel forms them ahead of pdl_wait.)
+__device__ __forceinline__ void splitk_sum4_pair(const B200SplitK& d, const SplitKRef& ra, const SplitKRef& rb, int bias_a, int bias_b, float4& a, float4& b) {
+  a = b = make_float4(0.f, 0.f, 0.f, 0.f);
+  const int n = max(ra.n_contrib, rb.n_contrib);
+  for (int c0 = 0; c0 < n; c0 += 8) {
+    float4 la[8], lb[8];
+#pragma unroll
+    for (int cc = 0; cc < 8; ++cc) {
+      la[cc] = c0 + cc < ra.n_contrib ? __ldcg(reinterpret_cast<const float4*>(ra.base + (size_t)(c0 + cc) * ra.stride)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      lb[cc] = c0 + cc < rb.n_contrib ? __ldcg(reinterpret_cast<const float4*>(rb.base + (size_t)(c0 + cc) * rb.stride)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int cc = 0; cc < 8; ++cc) {
+      if (c0 + cc < ra.n_contrib) { a.x += la[cc].x; a.y += la[cc].y; a.z += la[cc].z; a.w += la[cc].w; }
+      if (c0 + cc < rb.n_contrib) { b.x += lb[cc].x; b.y += lb[cc].y; b.z += lb[cc].z; b.w += lb[cc].w; }
+    }
+  }
+  if (d.bias) {
+    const __half *pa = reinterpret_cast<const __half*>(d.bias) + bias_a, *pb = reinterpret_cast<const __half*>(d.bias) + bias_b;
+    a.x += __half2float(pa[0]); a.y += __half2float(pa[1]); a.z += __half2float(pa[2]); a.w += __half2float(pa[3]);
+    b.x += __half2float(pb[0]); b.y += __half2float(pb[1]); b.z += __half2float(pb[2]); b.w += __half2float(pb[3]);
+  }
+}
+
 __device__ __forceinline__ float splitk_sum1(const B200SplitK& d, int t, int n) {
   const SplitKRef ref = splitk_ref(d, t, n);
   float acc = 0.f;
@@ -67,6 +92,29 @@ __device__ __forceinline__ float splitk_sum1(const B200SplitK& d, int t, int n) 
   }
   if (d.bias) acc += __half2float(reinterpret_cast<const __half*>(d.bias)[n]);
   return acc;
+}
+
+// two single columns at once
+__device__ __forceinline__ void splitk_sum1_pair(const B200SplitK& d, const SplitKRef& ra, const SplitKRef& rb, int bias_a, int bias_b, float& a, float& b) {
+  a = b = 0.f;
+  const int n = max(ra.n_contrib, rb.n_contrib);
+  for (int c0 = 0; c0 < n; c0 += 8) {
+    float la[8], lb[8];
+#pragma unroll
+    for (int cc = 0; cc < 8; ++cc) {
+      la[cc] = c0 + cc < ra.n_contrib ? __ldcg(ra.base + (size_t)(c0 + cc) * ra.stride) : 0.f;
+      lb[cc] = c0 + cc < rb.n_contrib ? __ldcg(rb.base + (size_t)(c0 + cc) * rb.stride) : 0.f;
+    }
+#pragma unroll
+    for (int cc = 0; cc < 8; ++cc) {
+      if (c0 + cc < ra.n_contrib) a += la[cc];
+      if (c0 + cc < rb.n_contrib) b += lb[cc];
+    }
+  }
+  if (d.bias) {
+    a += __half2float(reinterpret_cast<const __half*>(d.bias)[bias_a]);
+    b += __half2float(reinterpret_cast<const __half*>(d.bias)[bias_b]);
+  }
 }
 
 }  // namespace b200
