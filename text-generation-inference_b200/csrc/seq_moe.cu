@@ -303,13 +303,15 @@ __global__ void __launch_bounds__(256) moe_linear_kernel(const TA* __restrict__ 
   }
 }
 
-// Tensor-core form of moe_linear_kernel for bfloat16 operands: 64 x 64 output tile per block of four warps (each 32 x 32), k in
-// steps of 64 through a three-stage cp.async pipeline, m16n8k16 products with fp32 accumulation in ascending k.  With the few
-// rows per expert of a decoding step the work is streaming each picked expert's weights once; the tiles of the plan keep that
-// to the experts that were picked.  Needs K % 8 == 0 and 16-byte aligned rows.
-constexpr int kMmaBK = 64, kMmaStages = 3, kMmaLd = kMmaBK + 8;
+// Tensor-core form of moe_linear_kernel for bfloat16 operands: a 64 x 64 output tile per block of four warps (each 16 features by as many groups of 16 rows
+// as the tile has), k in steps of 64 through a cp.async pipeline of three or six stages, m16n8k16 products with fp32 accumulation in ascending k.  With
+// the few rows per expert of a decoding step the work is streaming each picked expert's weights once; the tiles of the plan keep that to the experts
+// that were picked, so what counts is bytes in flight, and nothing is loaded or multiplied for rows that a tile lacks.  Needs K % 8 == 0 and 16-byte aligned rows.
+// Measured on B200, us of a routed feed-forward of 16 experts (three stages and 64 rows always / three / six): width 2048, 1 token 38.5 / 37.5 / 21.5, 4
+// tokens 73 / 67 / 40, 64 tokens 81 / 75 / 77, 400 tokens 98 / 100 / 104; width 4096, 16 tokens 221 / 219 / 200, 64 tokens 283 / 243 / 251, 128 tokens 292 / 254 / 268.
+constexpr int kMmaBK = 64, kMmaLd = kMmaBK + 8;
 
-template <typename TC>
+template <typename TC, int kMmaStages>
 __global__ void __launch_bounds__(128) moe_linear_mma_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, int gather,
                                                              const __nv_bfloat16* __restrict__ W, TC* __restrict__ C, int64_t ldc, MoePlan p, int N,
                                                              int K, int act) {
@@ -320,7 +322,7 @@ __global__ void __launch_bounds__(128) moe_linear_mma_kernel(const __nv_bfloat16
   __nv_bfloat16* Ws = As + kMmaStages * kMoeTile * kMmaLd;             // [stages][64][kMmaLd]
   const int tile = blockIdx.y;
   if (tile >= *p.n_tiles) return;
-  const int e = p.tile_expert[tile], m0 = p.tile_row0[tile], m_end = p.offsets[e + 1];
+  const int e = p.tile_expert[tile], m0 = p.tile_row0[tile], rows = min(kMoeTile, p.offsets[e + 1] - m0), groups = (rows + 15) >> 4;
   W += (int64_t)e * N * K;
   const int n0 = blockIdx.x * kMoeTile;
   const int tid = threadIdx.x, w = warp_id(), lane = lane_id();
@@ -330,62 +332,65 @@ __global__ void __launch_bounds__(128) moe_linear_mma_kernel(const __nv_bfloat16
   const __nv_bfloat16* w_src[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int row = (tid >> 3) + i * 16;
-    const int m = m0 + row, n = n0 + row;
-    a_src[i] = m < m_end ? A + (gather ? (int64_t)p.token_of_row[m] : (int64_t)m) * lda : nullptr;
+    const int row = (tid >> 3) + i * 16, n = n0 + row;
+    a_src[i] = row < rows ? A + (gather ? (int64_t)p.token_of_row[m0 + row] : (int64_t)(m0 + row)) * lda : nullptr;
     w_src[i] = n < N ? W + (int64_t)n * K : nullptr;
   }
-  auto load = [&](int stage, int kt) {
-    const int k = kt * kMmaBK + kc;
+  auto load = [&](int kt) {
+    const int k = kt * kMmaBK + kc, stage = kt % kMmaStages;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int row = (tid >> 3) + i * 16;
-      const bool pa = a_src[i] != nullptr && k < K, pw = w_src[i] != nullptr && k < K;
-      cp_async_16(As + (stage * kMoeTile + row) * kMmaLd + kc, pa ? a_src[i] + k : A, pa);
+      const bool pw = w_src[i] != nullptr && k < K;
       cp_async_16(Ws + (stage * kMoeTile + row) * kMmaLd + kc, pw ? w_src[i] + k : W, pw);
+      if (i < groups) {
+        const bool pa = a_src[i] != nullptr && k < K;
+        cp_async_16(As + (stage * kMoeTile + row) * kMmaLd + kc, pa ? a_src[i] + k : A, pa);
+      }
     }
-    cp_async_commit();
   };
   const int nk = (K + kMmaBK - 1) / kMmaBK;
-  load(0, 0);
-  if (nk > 1) load(1, 1);
-  float acc[2][4][4] = {};
-  const int wm = w >> 1, wn = w & 1, lm = lane >> 3, lr = lane & 7;
+#pragma unroll
+  for (int kt = 0; kt < kMmaStages - 1; ++kt) {   // (a group per step, empty ones too: the wait below counts groups)
+    if (kt < nk) load(kt);
+    cp_async_commit();
+  }
+  float acc[4][2][4] = {};
+  const int lm = lane >> 3, lr = lane & 7;
   const uint32_t as_addr = smem_u32(As), ws_addr = smem_u32(Ws);
   for (int kt = 0; kt < nk; ++kt) {
     const int stage = kt % kMmaStages;
-    if (kt + 1 < nk) cp_async_wait<1>();
-    else cp_async_wait<0>();
+    cp_async_wait<kMmaStages - 2>();
     __syncthreads();  // stage kt has landed; everyone is done with the stage that the next load overwrites
-    if (kt + 2 < nk) load((kt + 2) % kMmaStages, kt + 2);
-    const uint32_t a_lane = as_addr + (uint32_t)(((stage * kMoeTile + wm * 32 + (lm & 1) * 8 + lr) * kMmaLd + (lm >> 1) * 8) * 2);
-    const uint32_t b_lane = ws_addr + (uint32_t)(((stage * kMoeTile + wn * 32 + (lm >> 1) * 8 + lr) * kMmaLd + (lm & 1) * 8) * 2);
+    if (kt + kMmaStages - 1 < nk) load(kt + kMmaStages - 1);
+    cp_async_commit();
+    const uint32_t a_lane = as_addr + (uint32_t)(((stage * kMoeTile + (lm & 1) * 8 + lr) * kMmaLd + (lm >> 1) * 8) * 2);
+    const uint32_t b_lane = ws_addr + (uint32_t)(((stage * kMoeTile + w * 16 + (lm >> 1) * 8 + lr) * kMmaLd + (lm & 1) * 8) * 2);
 #pragma unroll
     for (int kk = 0; kk < kMmaBK; kk += 16) {
-      uint32_t a[2][4], b[2][4];
+      uint32_t b[4];
+      ldmatrix_x4(b[0], b[1], b[2], b[3], b_lane + (uint32_t)(kk * 2));
 #pragma unroll
-      for (int mt = 0; mt < 2; ++mt) ldmatrix_x4(a[mt][0], a[mt][1], a[mt][2], a[mt][3], a_lane + (uint32_t)((mt * 16 * kMmaLd + kk) * 2));
-#pragma unroll
-      for (int np = 0; np < 2; ++np) ldmatrix_x4(b[np][0], b[np][1], b[np][2], b[np][3], b_lane + (uint32_t)((np * 16 * kMmaLd + kk) * 2));
-#pragma unroll
-      for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int np = 0; np < 2; ++np) {
-          mma_m16n8k16_bf16f32(acc[mt][2 * np], a[mt], b[np][0], b[np][1]);
-          mma_m16n8k16_bf16f32(acc[mt][2 * np + 1], a[mt], b[np][2], b[np][3]);
+      for (int mt = 0; mt < 4; ++mt) {
+        if (mt < groups) {
+          uint32_t a[4];
+          ldmatrix_x4(a[0], a[1], a[2], a[3], a_lane + (uint32_t)((mt * 16 * kMmaLd + kk) * 2));
+          mma_m16n8k16_bf16f32(acc[mt][0], a, b[0], b[1]);
+          mma_m16n8k16_bf16f32(acc[mt][1], a, b[2], b[3]);
         }
+      }
     }
   }
   const int cq = (lane & 3) * 2;
 #pragma unroll
-  for (int mt = 0; mt < 2; ++mt)
+  for (int mt = 0; mt < 4; ++mt)
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
+    for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
       for (int el = 0; el < 4; ++el) {
-        const int m = m0 + wm * 32 + mt * 16 + (lane >> 2) + (el >> 1) * 8;
-        const int n = n0 + wn * 32 + nt * 8 + cq + (el & 1);
-        if (m < m_end && n < N) stf(C + (int64_t)m * ldc + n, moe_act(acc[mt][nt][el], act));
+        const int row = mt * 16 + (lane >> 2) + (el >> 1) * 8;
+        const int n = n0 + w * 16 + nt * 8 + cq + (el & 1);
+        if (row < rows && n < N) stf(C + (int64_t)(m0 + row) * ldc + n, moe_act(acc[mt][nt][el], act));
       }
 }
 
@@ -492,19 +497,25 @@ extern "C" int b200_seq_moe_linear(const void* A, int a_dt, int64_t lda, int gat
   static const bool use_mma = []() { const char* e = getenv("B200_SEQ_MOE_MMA"); return !(e && e[0] == '0'); }();
   if (use_mma && a_dt == B200_DT_BF16 && w_dt == B200_DT_BF16 && K % 8 == 0 && lda % 8 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 &&
       (reinterpret_cast<uintptr_t>(W) & 15) == 0) {
-    const size_t smem = (size_t)2 * kMmaStages * kMoeTile * kMmaLd * 2;
     dim3 grid((unsigned)((N + kMoeTile - 1) / kMoeTile), (unsigned)p.max_tiles);
-#define MMA_LAUNCH(TC)                                                                                                                  \
+#define MMA_LAUNCH(TC, STAGES)                                                                                                                  \
   do {                                                                                                                                  \
-    static bool cfg = false;                                                                                                            \
-    if (!cfg) { cudaFuncSetAttribute(moe_linear_mma_kernel<TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); cfg = true; }   \
-    B200_LAUNCH((moe_linear_mma_kernel<TC>), grid, dim3(128), smem, st, (const __nv_bfloat16*)A, lda, gather, (const __nv_bfloat16*)W,   \
+    constexpr size_t smem = (size_t)2 * (STAGES) * kMoeTile * kMmaLd * 2;                                                               \
+    static const cudaError_t cfg = cudaFuncSetAttribute(moe_linear_mma_kernel<TC, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    if (cfg != cudaSuccess) { b200_set_last_error(cudaGetErrorString(cfg)); return B200_ERR_CUDA; }                                     \
+    B200_LAUNCH((moe_linear_mma_kernel<TC, STAGES>), grid, dim3(128), smem, st, (const __nv_bfloat16*)A, lda, gather, (const __nv_bfloat16*)W,   \
                 (TC*)C, ldc, p, (int)N, (int)K, act);                                                                                   \
     b200_count_launches(1);                                                                                                             \
     return B200_OK;                                                                                                                     \
   } while (0)
-    if (c_dt == B200_DT_F32) MMA_LAUNCH(float);
-    else MMA_LAUNCH(__nv_bfloat16);
+    // Few rows are few blocks: two per SM with six stages each keep more bytes in flight than four with three; from a few rows per expert on the grid has
+    // several waves, whose starts and ends four blocks per SM hide better (us, both products, three / six stages: note above the kernel).
+    if (T * top < 64) {
+      if (c_dt == B200_DT_F32) MMA_LAUNCH(float, 6);
+      MMA_LAUNCH(__nv_bfloat16, 6);
+    }
+    if (c_dt == B200_DT_F32) MMA_LAUNCH(float, 3);
+    MMA_LAUNCH(__nv_bfloat16, 3);
 #undef MMA_LAUNCH
   }
   const int key = a_dt * 4 + w_dt * 2 + c_dt;

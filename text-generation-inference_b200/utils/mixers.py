@@ -329,7 +329,10 @@ class RoutedExperts(nn.Module):
     products of the same input that run with the router's; `route` returns their fp32 results after the routing.
     Tensors under `prefix`: router, [correction,] [e<j>.gate,] e<j>.up, e<j>.down."""
 
-    group_rows_per_expert = 64   # average rows per expert from which a step takes the tcgen05 groups
+    # Average rows per router output from which a step takes the tcgen05 groups, whose bulk copies keep the weights' stream fuller than the blocks of warp-level
+    # products.  B200, us of a step of 16 experts beside 4 identity outputs, two picks a token (warp-level / groups), width 2048: 8 tokens 45 / 63, 14 72 / 75, 16
+    # 72 / 52, 128 82 / 67, 600 139 / 75; width 4096: 4 tokens 118 / 130, 14 197 / 164, 20 202 / 173, 128 247 / 209, 600 435 / 230.
+    group_rows_per_expert = 1.6
 
     def __init__(self, prefix: str, weights, *, experts: int, top: int, limit: Optional[float], alpha: float = 1.702,
                  sigmoid_scores: bool = False, correction: bool = False, weight_scale: float = 1.0, softmax_scores: bool = False,
@@ -372,7 +375,7 @@ class RoutedExperts(nn.Module):
         act1 = ops.ACT_RELU2 if self.plain else ops.ACT_NONE
         rows = h.shape[0] * self.top
         if h.dtype == torch.bfloat16 and rows >= self.group_rows_per_expert * self.n_route and h.shape[1] % 8 == 0 and self.w_down.shape[2] % 8 == 0:
-            # prompts: enough rows per expert for the tcgen05 products, one launch each over the compact rows of all experts
+            # enough rows per expert for the tcgen05 products, one launch each over the compact rows of all experts
             gu = ops.experts_linear(ops.moe_gather_rows(h, routing), self.w_gate_up, routing, h.dtype, act=act1)
             return ops.experts_linear(self._act(gu), self.w_down, routing, torch.float32)
         gu = ops.moe_linear(h, self.w_gate_up, routing, gather=True, out_dtype=h.dtype, act=act1)
