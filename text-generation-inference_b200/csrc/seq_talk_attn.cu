@@ -326,16 +326,13 @@ __global__ void __launch_bounds__(512) talk_attn_mma_kernel(
   const int per_split = (n_ktiles + gridDim.z - 1) / gridDim.z;
   const int j_start = j_first + (int)blockIdx.z * per_split * KT;
   const int j_end = min(p_last, j_start + per_split * KT - 1);   // last key of this block's run
+  if (gridDim.z > 1 && j_start > j_end) {   // no keys are left for this run: it says so and takes no time
+    float* base = partial + (((int64_t)blockIdx.x * gridDim.z + blockIdx.z) * R) * (dv + 2) + dv;
+    for (int r = threadIdx.x; r < R; r += nthreads) base[(int64_t)r * (dv + 2)] = -INFINITY;
+    return;
+  }
   const int w = warp_id(), lane = lane_id();
   const int32_t* table = block_table + (int64_t)b * bt_stride;
-  for (int r = w; r < R; r += nthreads / 32) {
-    const int c = r / rows_g, rr = r % rows_g, tok = rr / rep, hh = rr % rep;
-    const float* src = q + ((int64_t)(row0 + tok) * H + c * rep + hh) * d;
-    const bool live = tok < ntok;
-    for (int i = lane; i < d; i += 32) Qs[r * DP + i] = __float2bfloat16_rn(live ? src[i] : 0.f);
-  }
-  if (talk)
-    for (int i = threadIdx.x; i < H * H; i += nthreads) Ts[i] = talk[i];
   const int kchunks = KD / 8, vchunks = VD / 8;
   const int page_shift = (page & (page - 1)) == 0 ? 31 - __clz(page) : -1;
   // one block-table lookup per thread and row, then the row's 16-byte pieces go round eight threads
@@ -354,6 +351,31 @@ __global__ void __launch_bounds__(512) talk_attn_mma_kernel(
     }
     cp_async_commit();
   };
+  if (j_start <= j_end) load_rows(Ks, KP, k_off, kchunks, j_start);
+  {   // queries, while the first keys are under way: four pieces of four columns per thread in flight
+    const int d4 = d >> 2, pieces = R * d4;
+    const bool vec = (reinterpret_cast<uintptr_t>(q) & 15) == 0;
+    for (int at = threadIdx.x; at < pieces; at += 4 * nthreads) {
+      float4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = at + u * nthreads, r = i / d4, c = r / rows_g, rr = r % rows_g, tok = rr / rep;
+        const float* src = q + ((int64_t)(row0 + tok) * H + c * rep + rr % rep) * d + (i - r * d4) * 4;
+        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < pieces && tok < ntok) v[u] = vec ? *reinterpret_cast<const float4*>(src) : make_float4(src[0], src[1], src[2], src[3]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = at + u * nthreads, r = i / d4;
+        if (i < pieces) {
+          __nv_bfloat162 lo = __floats2bfloat162_rn(v[u].x, v[u].y), hi = __floats2bfloat162_rn(v[u].z, v[u].w);
+          *reinterpret_cast<uint2*>(Qs + r * DP + (i - r * d4) * 4) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+        }
+      }
+    }
+  }
+  if (talk)
+    for (int i = threadIdx.x; i < H * H; i += nthreads) Ts[i] = talk[i];
   // this thread's two accumulator rows
   const int cq = (lane & 3) * 2;
   const int c_w = (w * 16) / rows_g;   // the warp's key / value head group
@@ -384,7 +406,6 @@ __global__ void __launch_bounds__(512) talk_attn_mma_kernel(
   const uint32_t qs_addr = smem_u32(Qs), ks_addr = smem_u32(Ks), vs_addr = smem_u32(Vs);
   const int lm = lane >> 3, lr = lane & 7;
   const uint32_t a_lane = qs_addr + (uint32_t)(((w * 16 + (lm & 1) * 8 + lr) * DP + (lm >> 1) * 8) * 2);
-  if (j_start <= j_end) load_rows(Ks, KP, k_off, kchunks, j_start);
   for (int j0 = j_start; j0 <= j_end; j0 += KT) {
     load_rows(Vs, VP, v_off, vchunks, j0);   // the value buffer is free: the previous tile ended with a barrier
     cp_async_wait<1>();                      // this tile's keys have landed (its values may still be in flight)
@@ -576,7 +597,9 @@ __global__ void __launch_bounds__(512) talk_attn_mma_kernel(
   }
 }
 
-// out[row] = sum_z e^(m_z - M) O_z / sum_z e^(m_z - M) l_z over the key runs of talk_attn_mma_kernel; one warp per row, blocks (query tile, 8 rows)
+// out[row] = sum_z e^(m_z - M) O_z / sum_z e^(m_z - M) l_z over the key runs of talk_attn_mma_kernel; one warp per row, a lane per run for the maxima and
+// sums, blocks (query tile, 8 rows)
+constexpr int kTalkMaxSplit = 32;
 __global__ void __launch_bounds__(256) talk_attn_merge_kernel(const float* __restrict__ partial, float* __restrict__ out, const int32_t* __restrict__ cu_q,
                                                              int B, int H, int G, int QT, int dv, int nsplit) {
   pdl_launch_dependents();
@@ -585,32 +608,36 @@ __global__ void __launch_bounds__(256) talk_attn_merge_kernel(const float* __res
   talk_find_tile(cu_q, B, QT, blockIdx.x, b, row0, ntok);
   if (b >= B) return;
   const int rep = H / G, R = QT * H, rows_g = QT * rep, lane = lane_id();
-  constexpr int kMaxSplit = 8;
   for (int r = blockIdx.y * 8 + warp_id(); r < R; r += 8 * gridDim.y) {
     const int c = r / rows_g, rr = r % rows_g, tok = rr / rep;
     if (tok >= ntok) continue;
     const float* base = partial + (((int64_t)blockIdx.x * nsplit) * R + r) * (dv + 2);
     const int64_t zs = (int64_t)R * (dv + 2);
-    float M = -INFINITY, wz[kMaxSplit];
-#pragma unroll
-    for (int z = 0; z < kMaxSplit; ++z) {
-      wz[z] = z < nsplit ? base[z * zs + dv] : -INFINITY;
-      M = fmaxf(M, wz[z]);
-    }
-    float den = 0.f;
-#pragma unroll
-    for (int z = 0; z < kMaxSplit; ++z) {
-      wz[z] = wz[z] > -INFINITY ? expf(wz[z] - M) : 0.f;  // an empty run carries no weight
-      if (z < nsplit) den += wz[z] * base[z * zs + dv + 1];
-    }
-    const float inv = 1.f / den;
+    const float m = lane < nsplit ? base[lane * zs + dv] : -INFINITY, l = lane < nsplit ? base[lane * zs + dv + 1] : 0.f;
+    const float M = warp_max(m), weight = m > -INFINITY ? expf(m - M) : 0.f;
+    const unsigned some = __ballot_sync(0xffffffffu, m > -INFINITY);           // an empty run carries no weight and has left nothing else
+    const float inv = 1.f / warp_sum(m > -INFINITY ? weight * l : 0.f);
     float* dst = out + ((int64_t)(row0 + tok) * H + c * rep + rr % rep) * dv;
-    for (int col = lane; col < dv; col += 32) {
-      float acc = 0.f;
+    for (int c0 = 0; c0 < dv; c0 += 64) {   // two columns of eight runs in flight
+      const int col = c0 + lane, col2 = col + 32;
+      float acc = 0.f, acc2 = 0.f;
+      for (int z0 = 0; z0 < nsplit; z0 += 8) {
+        float v[8], v2[8];
 #pragma unroll
-      for (int z = 0; z < kMaxSplit; ++z)
-        if (z < nsplit) acc = fmaf(wz[z], base[z * zs + col], acc);
-      dst[col] = acc * inv;
+        for (int i = 0; i < 8; ++i) {
+          const bool in = some >> (z0 + i) & 1;
+          v[i] = in && col < dv ? base[(z0 + i) * zs + col] : 0.f;
+          v2[i] = in && col2 < dv ? base[(z0 + i) * zs + col2] : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float wz = __shfl_sync(0xffffffffu, weight, z0 + i);
+          acc = fmaf(wz, v[i], acc);
+          acc2 = fmaf(wz, v2[i], acc2);
+        }
+      }
+      if (col < dv) dst[col] = acc * inv;
+      if (col2 < dv) dst[col2] = acc2 * inv;
     }
   }
 }
@@ -705,7 +732,9 @@ static TalkPlan talk_mma_plan(int dt, int64_t T, int B, int H, int G, int d, int
 }
 
 // Over how many blocks the tensor-core kernel should split each query tile's keys in this step (1: no split; 0: the plain kernel runs)
-// and the fp32 workspace (`partial`) that takes
+// and the fp32 workspace (`partial`) that takes.  A block goes from tile to tile of keys in several microseconds, so few query tiles are cut into up to 32 runs
+// (us on B200, at most 8 / 32 runs, 16 / 4 heads of 128: a token behind 1000 keys 23.2 / 17.6, 4 x 3 - 6 behind 1500 44.2 / 29.7; 32 / 8 heads 3 x 10 -
+// 20 behind 900 46.8 / 42.8; with the queries brought in four pieces at a time behind the first keys 14.9, 27.4 and 37.2).
 extern "C" int b200_seq_talk_attn_splits(int dt, int64_t T, int B, int H, int G, int d, int dv, int64_t* workspace_floats) {
   if (workspace_floats) *workspace_floats = 0;
   const TalkPlan p = talk_mma_plan(dt, T, B, H, G, d, dv, true);
@@ -716,7 +745,7 @@ extern "C" int b200_seq_talk_attn_splits(int dt, int64_t T, int B, int H, int G,
   int64_t per_sm = (int64_t)233472 / (int64_t)(p.smem + 1024);   // 228 KB per SM, 1 KB reserved per block
   per_sm = per_sm < 1 ? 1 : per_sm;
   int64_t n = (148 * per_sm) / (busy > 0 ? busy : 1);
-  n = n < 1 ? 1 : (n > 8 ? 8 : n);
+  n = n < 1 ? 1 : (n > kTalkMaxSplit ? kTalkMaxSplit : n);
   if (n > 1 && workspace_floats) *workspace_floats = tiles * n * p.QT * H * (dv + 2);
   return (int)n;
 }
@@ -820,8 +849,9 @@ extern "C" int b200_seq_talk_attn(const float* q, const void* cache, int dt, int
   }
   cudaStream_t st = (cudaStream_t)stream;
   if (!partial || nsplit < 1) nsplit = 1;
-  if (nsplit > 8) nsplit = 8;
-  if (talk_prompt_route(q, cache, dt, row_width, k_off, v_off, cu_q, talk, out, T, B, H, G, d, dv, page, bt_stride, chunk, window, nsplit)) {
+  if (nsplit > kTalkMaxSplit) nsplit = kTalkMaxSplit;
+  if (talk_prompt_route(q, cache, dt, row_width, k_off, v_off, cu_q, talk, out, T, B, H, G, d, dv, page, bt_stride, chunk, window,
+                        nsplit < 8 ? nsplit : 8)) {
     if (d == 128)
       return launch_talk_prompt<128>(q, cache, row_width, k_off, v_off, block_table, bt_stride, cu_q, B, position_ids, out, T, H, G, chunk, window, scale, sink, st);
     return launch_talk_prompt<64>(q, cache, row_width, k_off, v_off, block_table, bt_stride, cu_q, B, position_ids, out, T, H, G, chunk, window, scale, sink, st);
