@@ -72,6 +72,8 @@ constexpr int64_t kW4CounterBytes = 64 * 1024;
 // kernel would need two token tiles (4096 -> 4096 40.1 / 19.6, 14336 -> 4096 107 / 58).
 constexpr int kW4R = 2;  // feature tiles per super-tile: consecutive units (super-tile, k-block, r = 0..1) share one activation tile
 
+constexpr int kW4SumPitch = kW4R * kW4TileM + 4;  // floats of a token's sums in shared memory
+
 template <int TN>
 struct GemmW4Cfg {
   static constexpr int kSuRing = TN >= 128 ? 2 : 3;            // super-units whose A tiles fit in TMEM at once
@@ -92,6 +94,7 @@ struct GemmW4Cfg {
   // a team at super-unit j has seen super-unit j - 2 - kSuRing complete, which implies j - 2 kSuRing did (no phase aliasing)
   static_assert(kSuRing >= 2, "A ring depth");
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
+  static_assert(TN * kW4SumPitch * 4 <= kXStages * kXStageBytes + kWStages * kW4RecMaxBytes, "the last super-tile's sums lie where the rings were");
 };
 
 __device__ __forceinline__ uint32_t lds_acquire_cta(const uint32_t* p) {
@@ -138,8 +141,46 @@ struct W4Params {
   unsigned long long* trace;  // debug: per-CTA phase timestamps (globaltimer ns), NULL in production
 };
 
+// The end of a CTA's last super-tile when nobody shares it: the epilogue warps leave its fp32 sums in shared memory ([token][kW4SumPitch]) and all 24 warps
+// write the outputs, four features of a token each.  By the four epilogue warps alone, a feature per thread, the SiLU's divisions (a branch each, so one
+// after the other) took 1.9 us at 16 tokens, 7.9 at 64 and 15 at 128 behind the last product (4096 -> 28672: 26.8 us of which 7.9 -> 21.5 with 2.4; 128 tokens 42.6 -> 32).
+// kWhole: from 17 tokens on, and with the SiLU from 9 if no super-tile is shared; otherwise the outputs are too few to pay for the barrier, or for the code
+// alone (14336 -> 4096 at one token 12.6 us without and 13.0 with it, 4096 -> 22016 with the SiLU at 16 tokens 18.0 and 18.2; 4096 -> 28672 with the SiLU 18.4 and
+// 18.5 at one token, 19.7 and 18.7 at 16).
+__device__ __forceinline__ void w4_finish(const W4Params& p, const float* sums, int sup) {
+  const int per_tok = p.act ? kW4TileM / 4 : kW4R * kW4TileM / 4;
+  for (int i = threadIdx.x; i < p.T * per_tok; i += kW4Threads) {
+    const int tok = i / per_tok, f = (i % per_tok) * 4, r = f / kW4TileM, m = f % kW4TileM;
+    float4 s = *reinterpret_cast<const float4*>(&sums[tok * kW4SumPitch + f]);
+    const int col = p.act ? sup * kW4TileM + f : (p.half_tiles ? sup + r * p.half_tiles : sup * kW4R + r) * kW4TileM + m;
+    if (!p.act && col >= p.N) continue;   // N % 32 == 0: four columns never straddle it
+    if (p.bias) {
+      s.x += __half2float(p.bias[col]); s.y += __half2float(p.bias[col + 1]); s.z += __half2float(p.bias[col + 2]); s.w += __half2float(p.bias[col + 3]);
+    }
+    uint2 o;
+    if (p.act) {
+      float4 u = *reinterpret_cast<const float4*>(&sums[tok * kW4SumPitch + kW4TileM + f]);
+      if (p.bias) {
+        const __half* b = p.bias + col + p.half_tiles * kW4TileM;
+        u.x += __half2float(b[0]); u.y += __half2float(b[1]); u.z += __half2float(b[2]); u.w += __half2float(b[3]);
+      }
+      const __half h[4] = {silu_mul_f16(s.x, u.x), silu_mul_f16(s.y, u.y), silu_mul_f16(s.z, u.z), silu_mul_f16(s.w, u.w)};
+      o = *reinterpret_cast<const uint2*>(h);
+    } else {
+      o = make_uint2(pack_half2(s.x, s.y), pack_half2(s.z, s.w));
+    }
+    __half* y = &p.y[(size_t)tok * p.ldy + col];
+    if ((reinterpret_cast<uintptr_t>(p.y) & 7) == 0) {
+      *reinterpret_cast<uint2*>(y) = o;
+    } else {
+      const __half* h = reinterpret_cast<const __half*>(&o);
+      for (int j = 0; j < 4; ++j) y[j] = h[j];
+    }
+  }
+}
+
 // kGR = meta rows per unit record (1, 2 or 4 = 128 / groupsize, 1 for groupsize >= 128).
-template <int TN, int kGR>
+template <int TN, int kGR, bool kWhole>
 __global__ void __launch_bounds__(kW4Threads, 1)
 gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) {
   using C = GemmW4Cfg<TN>;
@@ -162,6 +203,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
   __shared__ uint32_t s_issued;  // super-units whose MMAs have been issued (hand-over between the two MMA warps)
   __shared__ int s_fix[2][3];  // super-tiles this CTA shares with others: {super-tile, contributors, my index}
   __shared__ int s_nfix;
+  __shared__ int s_whole;      // the last super-tile if this CTA has it alone: all threads finish it; -1: none
 
   pdl_launch_dependents();
   const int warp = warp_id(), lane = lane_id();
@@ -213,6 +255,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
     for (int i = 0; i < 8; ++i) s_ready[i] = 0;
     s_issued = 0;
     s_nfix = 0;
+    s_whole = -1;
     mbar_fence_init();
   }
   if (warp == 0) tmem_alloc<C::kTmemCols>(tmem_slot);
@@ -412,10 +455,10 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
         const int n0 = (p.half_tiles ? sup : sup * kW4R) * kW4TileM + m;
         const int n1 = (p.half_tiles ? sup + p.half_tiles : sup * kW4R + 1) * kW4TileM + m;
         const bool ok0 = n0 < p.N, ok1 = n1 < p.N;
-        const bool direct = n_contrib == 1 && !p.defer;
+        const bool direct = n_contrib == 1 && !p.defer, whole = kWhole && direct && seg_end == su1;
         const float bv0 = (p.bias && ok0 && direct) ? __half2float(p.bias[n0]) : 0.f;
         const float bv1 = (p.bias && ok1 && direct) ? __half2float(p.bias[n1]) : 0.f;
-        constexpr int kCh = TN < 32 ? TN : 32;  // columns fetched per tcgen05.wait::ld
+        constexpr int kCh = 16;  // columns fetched per tcgen05.wait::ld (32 spill)
 #pragma unroll 1
         for (int c = 0; c < TN; c += kCh) {
           uint32_t d0[kCh], d1[kCh];
@@ -425,7 +468,14 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
             tmem_ld_32x32b_x16(tmem_d + lane_base + (buf * kW4R + 1) * TN + c + q * 16, reinterpret_cast<uint32_t(&)[16]>(d1[q * 16]));
           }
           tmem_ld_wait();
-          if (!direct) {
+          if (whole) {   // the rings have been used up: every product is done
+            float* sums = reinterpret_cast<float*>(smem);
+#pragma unroll
+            for (int j = 0; j < kCh; ++j) {
+              sums[(c + j) * kW4SumPitch + m] = __uint_as_float(d0[j]);
+              sums[(c + j) * kW4SumPitch + kW4TileM + m] = __uint_as_float(d1[j]);
+            }
+          } else if (!direct) {
 #pragma unroll
             for (int j = 0; j < kCh; ++j) {
               if (c + j < p.T) {
@@ -453,6 +503,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
           }
         }
       }
+      if (kWhole && threadIdx.x == 0 && n_contrib == 1 && !p.defer && seg_end == su1) s_whole = sup;
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[buf]);
@@ -573,6 +624,10 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
         __threadfence();
       }
     }
+  }
+  if (kWhole && s_whole >= 0) {
+    if (nfix == 0) pdl_wait();
+    w4_finish(p, reinterpret_cast<const float*>(smem), s_whole);
   }
   W4_TRACE(63, 0);
 }
@@ -785,13 +840,13 @@ int64_t b200_w4_partial_bytes(int64_t T, int64_t N, int64_t K) {
   return nd > need ? nd : need;
 }
 
-template <int TN, int kGR>
+template <int TN, int kGR, bool kWhole>
 static int launch_gemm_w4(const CUtensorMap* mx, const void* packed, void* y, void* workspace, const void* bias, int T, int N,
                           const W4Plan& pl, int half_tiles, int act, int defer, cudaStream_t st) {
   using C = GemmW4Cfg<TN>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_w4a16_kernel<TN, kGR>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(gemm_w4a16_kernel<TN, kGR, kWhole>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) { b200_set_last_error(cudaGetErrorString(e)); return B200_ERR_CUDA; }
     configured = true;
   }
@@ -816,7 +871,7 @@ static int launch_gemm_w4(const CUtensorMap* mx, const void* packed, void* y, vo
   p.trace = g_w4_trace;
   const dim3 grid(pl.n_ctas);
   b200_timing_mark(B200_TIME_GEMM_W4A16, 0, st);
-  constexpr auto kernel = gemm_w4a16_kernel<TN, kGR>;
+  constexpr auto kernel = gemm_w4a16_kernel<TN, kGR, kWhole>;
   B200_LAUNCH_AS("gemm_w4a16_kernel", kernel, grid, dim3(kW4Threads), (size_t)C::kSmemBytes, st, *mx, p);
   b200_timing_mark(B200_TIME_GEMM_W4A16, 1, st);
   b200_count_launches(1);
@@ -860,7 +915,7 @@ static int gemm_w4a16_impl(const void* x, const void* packed, const void* bias, 
   }
   // (A deferred result has no fix-up to save: the step of Llama-3-8B stays 1 % faster with its partials left in global memory.)
   const W4FewPlan few = T <= kFewMostT && !defer ? few_plan(N, K, few_clusters()) : W4FewPlan{0, 0};
-  if (few.d && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+  if (few.d && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(y) & 7) == 0) {
     W4FewParams fp = {};
     fp.x = (const __half*)x;
     fp.y = (__half*)y;
@@ -895,15 +950,16 @@ static int gemm_w4a16_impl(const void* x, const void* packed, const void* bias, 
     splitk->T = (int32_t)T;
   }
   cudaStream_t st = (cudaStream_t)stream;
-#define W4_DISPATCH(TNV)                                                                                                           \
-  (gr == 1 ? launch_gemm_w4<TNV, 1>(mx, packed, y, workspace, bias, (int)T, (int)N, pl, half_tiles, act, defer ? 1 : 0, st)          \
-           : gr == 2 ? launch_gemm_w4<TNV, 2>(mx, packed, y, workspace, bias, (int)T, (int)N, pl, half_tiles, act, defer ? 1 : 0, st) \
-                     : launch_gemm_w4<TNV, 4>(mx, packed, y, workspace, bias, (int)T, (int)N, pl, half_tiles, act, defer ? 1 : 0, st))
+  const int df = defer ? 1 : 0;
+#define W4_DISPATCH(TNV, W)                                                                                                  \
+  (gr == 1   ? launch_gemm_w4<TNV, 1, W>(mx, packed, y, workspace, bias, (int)T, (int)N, pl, half_tiles, act, df, st)         \
+   : gr == 2 ? launch_gemm_w4<TNV, 2, W>(mx, packed, y, workspace, bias, (int)T, (int)N, pl, half_tiles, act, df, st)         \
+             : launch_gemm_w4<TNV, 4, W>(mx, packed, y, workspace, bias, (int)T, (int)N, pl, half_tiles, act, df, st))
   switch (pl.TN) {
-    case 16: return W4_DISPATCH(16);
-    case 32: return W4_DISPATCH(32);
-    case 64: return W4_DISPATCH(64);
-    default: return W4_DISPATCH(128);
+    case 16: return act && T > 8 && pl.max_contrib == 1 ? W4_DISPATCH(16, true) : W4_DISPATCH(16, false);
+    case 32: return W4_DISPATCH(32, true);
+    case 64: return W4_DISPATCH(64, true);
+    default: return W4_DISPATCH(128, true);
   }
 #undef W4_DISPATCH
 }

@@ -79,21 +79,6 @@ __device__ __forceinline__ void splitk_sum4_pair(const B200SplitK& d, const Spli
   }
 }
 
-__device__ __forceinline__ float splitk_sum1(const B200SplitK& d, int t, int n) {
-  const SplitKRef ref = splitk_ref(d, t, n);
-  float acc = 0.f;
-  for (int c0 = 0; c0 < ref.n_contrib; c0 += 8) {
-    float ld[8];
-#pragma unroll
-    for (int cc = 0; cc < 8; ++cc) ld[cc] = c0 + cc < ref.n_contrib ? __ldcg(ref.base + (size_t)(c0 + cc) * ref.stride) : 0.f;
-#pragma unroll
-    for (int cc = 0; cc < 8; ++cc)
-      if (c0 + cc < ref.n_contrib) acc += ld[cc];
-  }
-  if (d.bias) acc += __half2float(reinterpret_cast<const __half*>(d.bias)[n]);
-  return acc;
-}
-
 // two single columns at once
 __device__ __forceinline__ void splitk_sum1_pair(const B200SplitK& d, const SplitKRef& ra, const SplitKRef& rb, int bias_a, int bias_b, float& a, float& b) {
   a = b = 0.f;
