@@ -79,3 +79,19 @@ def test_without_workspace():
         y = torch.empty(T, N, dtype=torch.float16, device=DEV)
         _lib.check(_lib.load().b200_gemm_f16(x.data_ptr(), w.data_ptr(), bias.data_ptr(), y.data_ptr(), T, N, K, None, ops._stream()), "gemm_f16")
         _near(y, x, w, bias, 2 ** -11)
+
+
+@pytest.mark.parametrize("T", [8, 24, 64])
+def test_a_result_off_any_eight_bytes(T):
+    """a result that starts one element into its memory: equal to the aligned one, and nothing beside it is touched"""
+    import tgis_b200  # noqa: F401
+    from tgis_b200 import _lib, ops
+    N, K = 2560, 2048
+    x, w, bias = _data(T, N, K, torch.float16)
+    got = []
+    for off in (0, 1):
+        room = torch.full((T * N + 2,), 7.0, dtype=torch.float16, device=DEV)
+        _lib.check(_lib.load().b200_gemm_f16(x.data_ptr(), w.data_ptr(), bias.data_ptr(), room[off:].data_ptr(), T, N, K, None, ops._stream()), "gemm_f16")
+        got.append(room[off:off + T * N].clone())
+        assert all(float(v) == 7.0 for v in torch.cat([room[:off], room[off + T * N:]]))
+    assert torch.equal(*got)

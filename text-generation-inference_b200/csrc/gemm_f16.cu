@@ -114,7 +114,7 @@ __device__ __forceinline__ void f16_cluster_sum(const F16Params& p, const float*
 #pragma unroll
       for (int e = 0; e < 4; ++e) s[e] += n + e < p.N ? gemm_load_bias<FMT>(p.bias, n + e) : 0.f;
     const size_t o = (size_t)tok * p.N + n;
-    if (FMT == 0 && n + 3 < p.N && (p.N & 3) == 0) {
+    if (FMT == 0 && n + 3 < p.N && (p.N & 3) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0) {
       *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(p.y) + o) = make_uint2(pack_half2(s[0], s[1]), pack_half2(s[2], s[3]));
     } else {
 #pragma unroll

@@ -851,7 +851,7 @@ extern "C" int b200_seq_delta_rows_scan(const float* pre, int channels, float* S
 #undef DST
   }
   const SpanPlan pl = delta_span_plan(T, B, H, dk, dv);
-  if (workspace && pl.cap && aligned) {
+  if (workspace && pl.cap && aligned && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0) {
     const DeltaRow lay = delta_row(H, kv_heads, dk, dv, channels != 0);
     return dk == 64 ? launch_delta_spans<64>(pre, lay, channels, S_state, state_slots, cu_q, position_ids, y, ld_y, T, B, H, kv_heads, dv, pl, (float*)workspace, st)
                     : launch_delta_spans<128>(pre, lay, channels, S_state, state_slots, cu_q, position_ids, y, ld_y, T, B, H, kv_heads, dv, pl, (float*)workspace, st);
