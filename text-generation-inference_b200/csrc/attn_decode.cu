@@ -204,6 +204,7 @@ attn_decode_paged_kernel(const __half* __restrict__ q, int64_t q_token_stride, c
         mma_m16n8k16_f16f32(o[2 * dc + 1], pa, v2, v3);
       }
     }
+    fence_proxy_async_smem();  // the page has been read before another one may take its place
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty_bar[s]);
   }

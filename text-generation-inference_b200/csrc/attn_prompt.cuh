@@ -162,6 +162,7 @@ __device__ __forceinline__ PfItem pf_item(const PfParams& p, int i) {
 // Asks for a block of the grid that has not started: its index in x, or -1 when there is none left (no further request may follow then).
 // One thread; `resp` 16 bytes of shared memory, `bar` an mbarrier of one arrival.
 __device__ __forceinline__ int take_block(uint32_t* resp, uint64_t* bar, uint32_t parity, bool& ok) {
+  fence_proxy_async_smem();  // the previous answer has been read
   mbar_arrive_expect_tx(bar, 16);
   asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(smem_u32(resp)), "r"(smem_u32(bar)) : "memory");
   mbar_wait_soft(bar, parity, ok);

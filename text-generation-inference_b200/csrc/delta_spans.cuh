@@ -439,7 +439,10 @@ __global__ void __launch_bounds__(SpanScan<DK>::kWarps * 32, 3) delta_span_scan_
     __syncwarp();
   };
   for (int s = 0; s < spans; ++s) {
-    if (s > 0) __syncthreads();   // the other stage is used up
+    if (s > 0) {   // the other stage is used up
+      fence_proxy_async_smem();
+      __syncthreads();
+    }
     if (threadIdx.x == 0 && s + 1 < spans) load(s + 1);
     const float* st = sm + (s & 1) * L::kStage;
     mbar_wait_soft(&full[s & 1], (s >> 1) & 1, ok);

@@ -373,6 +373,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       // the 64 k of a half lie in one group row, or in two when a group is 32 wide
       mrec[0] = lds_u32(meta + r * kW4RecMaxBytes + (h * p.group_rows / 2) * kW4MetaRowBytes);
       mrec[1] = p.group_rows == 4 ? lds_u32(meta + r * kW4RecMaxBytes + (h * 2 + 1) * kW4MetaRowBytes) : mrec[0];
+      fence_proxy_async_smem();  // the words are in registers before a bulk copy may take their place
       __syncwarp();
       if (lane == 0) mbar_arrive(&rec_empty[r]);
       r += 2;

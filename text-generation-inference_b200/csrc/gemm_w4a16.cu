@@ -383,6 +383,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
     const uint32_t meta_thread = smem_u32(w_ring) + kW4WordBytes + m * 4;
     uint32_t wq[16], mrec[kGR];
     int ws = team, wph = 0;   // weight-ring stage / parity of the unit being loaded
+    int held = 0;             // stage whose words are on their way to registers: given back behind fence_proxy_async_smem
     // unit i (super-unit j = i / 2) lives in A stage i % kAStages and may be written once the MMAs of super-unit
     // j - kSuRing have completed: barrier su_done[j % kSuRing], phase j / kSuRing - 1
     auto load_unit = [&](bool landed) {
@@ -392,12 +393,16 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
       for (int c = 0; c < 4; ++c) lds_v4(w_thread + st + c * (kW4TileM * 16), &wq[c * 4]);
 #pragma unroll
       for (int r = 0; r < kGR; ++r) mrec[r] = lds_u32(meta_thread + st + r * kW4MetaRowBytes);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty_w[ws]);
+      held = ws;
       ws += kW4Teams;
       if (ws >= C::kWStages) { ws -= C::kWStages; wph ^= 1; }
     };
-    if (team < n_units) load_unit(false);
+    if (team < n_units) {
+      load_unit(false);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty_w[held]);
+    }
     if (team == 0) W4_TRACE(2, kW4FirstDqWarp * 32);
     int n = 0;
     for (int i = team; i < n_units; i += kW4Teams, ++n) {
@@ -426,8 +431,12 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
       if (more) load_unit(w_landed);  // next unit's words: the shared-memory reads overlap the TMEM store latency
       tmem_st_wait();
       tcgen05_fence_before();
+      fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) red_release_cta_shared_inc(&s_ready[(i >> 1) & 7]);
+      if (lane == 0) {
+        red_release_cta_shared_inc(&s_ready[(i >> 1) & 7]);
+        if (more) mbar_arrive(&empty_w[held]);
+      }
     }
     if (team == 0) W4_TRACE(4, kW4FirstDqWarp * 32);
   } else {
