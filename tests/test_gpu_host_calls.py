@@ -124,3 +124,64 @@ def test_first_calls_inside_a_capture(both):
         torch.cuda.synchronize()
         return y.clone()
     both(call)
+
+
+@pytest.mark.parametrize("entry", ["gemm_f16", "gemm_w4a16", "linear_bf16", "attn_decode_paged"])
+def test_workspace_lives_until_the_entry_returns(entry):
+    """While an entry runs, other threads may make a call that needs a larger workspace, which replaces the first: its memory is not given to
+    anybody else before the entry has returned.  The entries are functions of this test, which launch nothing."""
+    import ctypes
+
+    import tgis_b200  # noqa: F401
+    from tgis_b200 import _lib, ops, ops_seq
+    which = int(entry == "linear_bf16")
+    seen = []
+    need = [1 << 20]
+
+    def run(*a):
+        ws = {"gemm_f16": 7, "gemm_w4a16": 10, "linear_bf16": 8, "attn_decode_paged": 9}[entry]
+        if need[0] == 1 << 20:
+            need[0] = 1 << 21
+            call()                                                                       # as another thread's larger call
+            others = [torch.empty(1 << 20, dtype=torch.uint8, device=DEV) for _ in range(64)]   # who asks now must not get the first one's memory
+            seen.append((a[ws], [t.data_ptr() for t in others]))
+        return 0
+
+    P, L, I, F = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, ctypes.c_float
+    types = {"gemm_f16": [P, P, P, P, L, L, L, P, P], "gemm_w4a16": [P, P, P, P, L, L, L, I, I, I, P, P], "linear_bf16": [P, P, P, P, I, L, L, L, P, P],
+             "attn_decode_paged": [P, L, P, P, P, L, P, P, L, P, L, I, I, I, I, I, F, P]}[entry]
+    fns = [ctypes.CFUNCTYPE(I, *types)(run), ctypes.CFUNCTYPE(L, L, L)(lambda n, k: 1 << 20 if n == 64 else 1 << 21),
+           ctypes.CFUNCTYPE(L, I, I, I, I)(lambda b, h, d, most: need[0])]
+    names = [{"gemm_f16": "b200_gemm_f16", "gemm_w4a16": "b200_gemm_w4a16_ex", "linear_bf16": "b200_gemm_bf16", "attn_decode_paged": "b200_attn_decode_paged"}[entry],
+             "b200_gemm_workspace_bytes_max", "b200_attn_decode_workspace_bytes"]
+    host = (ops_seq if which else ops)._native()
+    held = {}
+
+    def make(like, *a):
+        held["ws"] = torch.zeros(a[0] if len(a) == 1 else 1 << 20 if a[0] == 64 else 1 << 21, dtype=torch.uint8, device=DEV)
+        return held["ws"]
+
+    x, q = _r(2, 64), _r(2, 4, 64)
+    pool, table, lens = _r(3, 2, 16, 64), torch.zeros(2, 2, dtype=torch.int32, device=DEV), torch.ones(2, dtype=torch.int32, device=DEV)
+
+    def call():
+        N = 64 if need[0] == 1 << 20 else 128
+        w = _r(N, 64)
+        if entry == "gemm_f16":
+            return host.gemm_f16(x, w, None, None, None)
+        if entry == "gemm_w4a16":
+            return host.gemm_w4a16(x, torch.empty(64, dtype=torch.uint8, device=DEV), N, 64, None, None, None, 0, False)
+        if entry == "linear_bf16":
+            return host.linear_bf16(x.bfloat16(), w.bfloat16(), None, 0)
+        return host.attn_decode_paged(q, pool, pool, table, lens, 20, 0.125, 2, None, None)
+
+    try:
+        torch.cuda.empty_cache()
+        host.bind(which, {n: ctypes.cast(f, P).value for n, f in zip(names, fns)}, make, make)
+        assert call() is not None
+    finally:
+        for m in (ops, ops_seq):
+            m._host = None
+            m._native()
+    (used, taken), = seen
+    assert used not in taken

@@ -63,8 +63,9 @@ bool real(PyObject* o, double& v) {
 }
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
-// the device's workspace of at least `need` bytes, from Python when there is none yet or it is too small
-const at::Tensor* workspace(std::vector<at::Tensor>& have, PyObject* make, PyObject* like, const at::Tensor& t, int64_t need, PyObject* a, PyObject* b) {
+// The device's workspace of at least `need` bytes, from Python when there is none yet or it is too small; undefined where there is none to be had.  The caller
+// holds it until its entry has returned: other threads run meanwhile, and one that needs more replaces it here and in Python.
+at::Tensor workspace(std::vector<at::Tensor>& have, PyObject* make, PyObject* like, const at::Tensor& t, int64_t need, PyObject* a, PyObject* b) {
   const size_t dev = (size_t)t.get_device();
   if (have.size() <= dev) have.resize(dev + 1);
   if (!have[dev].defined() || have[dev].numel() < need) {
@@ -72,23 +73,25 @@ const at::Tensor* workspace(std::vector<at::Tensor>& have, PyObject* make, PyObj
     const at::Tensor* w = nullptr;
     if (!got || !tensor(got, w) || w->numel() < need) {
       Py_XDECREF(got);
-      return nullptr;
+      return {};
     }
     have[dev] = *w;
     Py_DECREF(got);
   }
-  return &have[dev];
+  return have[dev];
 }
-const at::Tensor* gemm_workspace(Library& lib, PyObject* like, const at::Tensor& t, int64_t N, int64_t K) {
+at::Tensor gemm_workspace(Library& lib, PyObject* like, const at::Tensor& t, int64_t N, int64_t K) {
   const uint64_t key = (uint64_t)N << 32 ^ (uint64_t)K;
-  if (N >> 31 || K >> 31) return nullptr;
+  if (N >> 31 || K >> 31) return {};
   auto it = lib.gemm_bytes.find(key);
   if (it == lib.gemm_bytes.end()) {
     if (lib.gemm_bytes.size() >= 4096) lib.gemm_bytes.clear();
     it = lib.gemm_bytes.emplace(key, lib.f.gemm_workspace_bytes_max(N, K)).first;
   }
   PyObject *n = PyLong_FromLongLong(N), *k = PyLong_FromLongLong(K);
-  const at::Tensor* w = n && k ? workspace(lib.gemm_ws, lib.gemm_workspace, like, t, it->second, n, k) : nullptr;
+  const int64_t need = it->second;
+  at::Tensor w;
+  if (n && k) w = workspace(lib.gemm_ws, lib.gemm_workspace, like, t, need, n, k);
   Py_XDECREF(n);
   Py_XDECREF(k);
   return w;
@@ -134,8 +137,12 @@ PyObject* gemm_w4a16(PyObject*, PyObject* const* a, Py_ssize_t n) {
       return nullptr;
     if (x->scalar_type() != at::kHalf || packed->scalar_type() != at::kByte || x->dim() != 2 || !x->is_contiguous() || !packed->is_contiguous() || N <= 0) return nullptr;
     const int64_t T = x->size(0), K = x->size(1);
-    if (!ws && !(ws = gemm_workspace(g_tgis, a[0], *x, N, K))) return nullptr;
-    at::Tensor made;
+    at::Tensor made, held;
+    if (!ws) {
+      held = gemm_workspace(g_tgis, a[0], *x, N, K);
+      if (!held.defined()) return nullptr;
+      ws = &held;
+    }
     if (!out) made = at::empty({T, silu ? N / 2 : N}, x->options());
     const at::Tensor& y = out ? *out : made;
     void *px = x->data_ptr(), *pp = packed->data_ptr(), *pb = ptr(bias), *py = y.data_ptr(), *pw = ws->data_ptr(), *st = stream();
@@ -151,8 +158,12 @@ PyObject* gemm_f16(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (n != 5 || !tensor(a[0], x) || !tensor(a[1], w) || !maybe_tensor(a[2], bias) || !maybe_tensor(a[3], out) || !maybe_tensor(a[4], ws)) return nullptr;
     if (x->scalar_type() != at::kHalf || w->scalar_type() != at::kHalf || x->dim() != 2 || w->dim() != 2 || !x->is_contiguous() || !w->is_contiguous()) return nullptr;
     const int64_t T = x->size(0), K = x->size(1), N = w->size(0);
-    if (!ws && !(ws = gemm_workspace(g_tgis, a[0], *x, N, K))) return nullptr;
-    at::Tensor made;
+    at::Tensor made, held;
+    if (!ws) {
+      held = gemm_workspace(g_tgis, a[0], *x, N, K);
+      if (!held.defined()) return nullptr;
+      ws = &held;
+    }
     if (!out) made = at::empty({T, N}, x->options());
     const at::Tensor& y = out ? *out : made;
     void *px = x->data_ptr(), *pm = w->data_ptr(), *pb = ptr(bias), *py = y.data_ptr(), *pw = ws->data_ptr(), *st = stream();
@@ -164,7 +175,7 @@ PyObject* gemm_f16(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // x, w, bias, out in fp32: bfloat16 operands, new result in bfloat16 or fp32, no activation
 PyObject* linear_bf16(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return serve([&]() -> PyObject* {
-    const at::Tensor *x, *w, *bias, *ws;
+    const at::Tensor *x, *w, *bias;
     int64_t f32;
     if (n != 4 || !tensor(a[0], x) || !tensor(a[1], w) || !maybe_tensor(a[2], bias) || !integer(a[3], f32)) return nullptr;
     if (x->scalar_type() != at::kBFloat16 || w->scalar_type() != at::kBFloat16 || (bias && bias->scalar_type() != at::kBFloat16) || x->dim() != 2 || w->dim() != 2 ||
@@ -172,9 +183,10 @@ PyObject* linear_bf16(PyObject*, PyObject* const* a, Py_ssize_t n) {
       return nullptr;
     const int64_t M = x->size(0), K = x->size(1), N = w->size(0);
     if (w->size(1) != K || K % 8 != 0 || K < 64 || M == 0 || N == 0 || ((uintptr_t)x->data_ptr() | (uintptr_t)w->data_ptr()) % 16 != 0) return nullptr;
-    if (!(ws = gemm_workspace(g_seq, a[0], *x, N, K))) return nullptr;
+    const at::Tensor ws = gemm_workspace(g_seq, a[0], *x, N, K);
+    if (!ws.defined()) return nullptr;
     at::Tensor y = at::empty({M, N}, x->options().dtype(f32 ? at::kFloat : at::kBFloat16));
-    void *px = x->data_ptr(), *pm = w->data_ptr(), *pb = ptr(bias), *py = y.data_ptr(), *pw = ws->data_ptr(), *st = stream();
+    void *px = x->data_ptr(), *pm = w->data_ptr(), *pb = ptr(bias), *py = y.data_ptr(), *pw = ws.data_ptr(), *st = stream();
     if (!enqueue([&] { return g_seq.f.gemm_bf16(px, pm, pb, py, f32 != 0, M, N, K, pw, st); })) return nullptr;
     return THPVariable_Wrap(y);
   });
@@ -195,15 +207,16 @@ PyObject* attn_decode_paged(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (!heads_rows(*q) || table->scalar_type() != at::kInt || lens->scalar_type() != at::kInt || table->dim() < 1 || (out && out->dim() < 1)) return nullptr;
     const int64_t B = q->size(0), h = q->size(1), d = q->size(2);
     const int64_t need = g_tgis.f.attn_decode_workspace_bytes((int)B, (int)h, (int)d, (int)most);
+    at::Tensor made, held;
     if (ws) {
       if ((int64_t)(ws->numel() * ws->element_size()) < need) return nullptr;
     } else {
       PyObject* bytes = PyLong_FromLongLong(need);
-      ws = bytes ? workspace(g_tgis.attn_ws, g_tgis.attn_workspace, a[0], *q, need, bytes, nullptr) : nullptr;
+      if (bytes) held = workspace(g_tgis.attn_ws, g_tgis.attn_workspace, a[0], *q, need, bytes, nullptr);
       Py_XDECREF(bytes);
-      if (!ws) return nullptr;
+      if (!held.defined()) return nullptr;
+      ws = &held;
     }
-    at::Tensor made;
     if (!out) made = at::empty({B, h, d}, q->options());
     const at::Tensor& y = out ? *out : made;
     void *pq = q->data_ptr(), *pk = k->data_ptr(), *pv = v->data_ptr(), *py = y.data_ptr(), *pw = ws->data_ptr(), *st = stream();
@@ -265,6 +278,9 @@ PyObject* bind(PyObject*, PyObject* args) {
   Py_INCREF(attn);
   lib.gemm_workspace = gemm;
   lib.attn_workspace = attn;
+  lib.gemm_bytes.clear();
+  lib.gemm_ws.clear();   // what earlier callables handed out is theirs
+  lib.attn_ws.clear();
   Py_RETURN_NONE;
 }
 
