@@ -207,16 +207,27 @@ def raise_if_gave_up() -> None:
             raise B200Error("a wait inside a kernel ran out: the results of this step are not valid")
 
 
+def _build_module():
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("_b200_build", os.path.join(_HERE, "build.py"))
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod
+
+
+class _NoHost:
+    """in the place of the native host side: leaves every call to Python"""
+
+    def __getattr__(self, name):
+        return lambda *a: None
+
+
 def load_seq() -> ctypes.CDLL:
     """Loads libb200_seq.so, compiling it in the tree first when it is absent or older than its sources (nvcc needs no GPU)."""
     global _seq_lib
     if _seq_lib is None:
-        import importlib.util
-        spec = importlib.util.spec_from_file_location("_b200_build", os.path.join(_HERE, "build.py"))
-        mod = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(mod)
         try:
-            mod.build(target="seq")
+            _build_module().build(target="seq")
         except Exception as e:
             if not os.path.exists(SEQ_LIB_PATH):
                 raise B200Error(f"{SEQ_LIB_PATH} could not be built: {e}")
@@ -254,16 +265,22 @@ def load() -> ctypes.CDLL:
 
 def load_host(which: int, lib: ctypes.CDLL, gemm_workspace, attn_workspace):
     """The native per-call host side (csrc/host/host_calls.cpp), bound to a loaded library (which: 0 libb200_tgis.so, 1 libb200_seq.so) and to the callables
-    that hand out its workspaces.  Its functions return None for a call that they leave to Python."""
+    that hand out its workspaces.  Its functions return None for a call that they leave to Python; where there is none that fits this Python and torch, all calls
+    go that way."""
     global _host
     if _host is None:
         import importlib.machinery
         import importlib.util
-        if not os.path.exists(HOST_PATH):
-            raise B200Error(f"{HOST_PATH} is missing: build it with `python text-generation-inference_b200/build.py`")
-        loader = importlib.machinery.ExtensionFileLoader("_b200_host", HOST_PATH)
-        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_b200_host", loader))
-        loader.exec_module(mod)
+        import warnings
+        try:
+            if not _build_module().host_fits():
+                raise ImportError("it is missing, or built for another Python or torch")
+            loader = importlib.machinery.ExtensionFileLoader("_b200_host", HOST_PATH)
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_b200_host", loader))
+            loader.exec_module(mod)
+        except ImportError as e:
+            warnings.warn(f"{HOST_PATH} is not used ({e}): operators take some microseconds more a call; `python text-generation-inference_b200/build.py` builds it")
+            mod = _NoHost()
         _host = mod
     entries = [n for n in ("b200_gemm_workspace_bytes_max", "b200_gemm_w4a16_ex", "b200_gemm_f16", "b200_gemm_bf16", "b200_attn_decode_workspace_bytes",
                            "b200_attn_decode_paged", "b200_attn_prefill_paged") if hasattr(lib, n)]

@@ -4,12 +4,14 @@
   libb200_tgis.so  every source: the whole C ABI of include/b200_tgis.h
   libb200_seq.so   the sources the hybrid decoder families need (seq_*.cu + the block allocator and the runtime pieces); a
                    process that serves only such a model builds and loads this one (`--seq`, `build(target="seq")`)
-  _b200_host.so    csrc/host/host_calls.cpp: the operators' per-call host work as a CPython extension over torch's C++ headers
+  _b200_host.so    csrc/host/host_calls.cpp: the operators' per-call host work as a CPython extension over torch's C++ headers.  It saves time only:
+                   where it cannot be built (no headers of Python's or torch's) or is another Python's or torch's, the same calls go through Python
 Objects are shared between the first two.  The libraries are git-ignored; they are built in the tree at first use.
 """
 from __future__ import annotations
 
 import concurrent.futures
+import importlib.metadata
 import importlib.util
 import os
 import shutil
@@ -53,16 +55,29 @@ def _stale(target: str, deps) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def host_tag() -> str:
+    """what a built _b200_host.so names itself: it fits one Python and one torch only"""
+    return "b200_host for python %d.%d, torch %s;" % (*sys.version_info[:2], importlib.metadata.version("torch"))
+
+
+def host_fits() -> bool:
+    try:
+        with open(HOST_LIB, "rb") as f:
+            return host_tag().encode() in f.read()
+    except (OSError, importlib.metadata.PackageNotFoundError):
+        return False
+
+
 def build_host(force: bool = False) -> None:
-    if not force and not _stale(HOST_LIB, [HOST_SRC]):
+    if not force and not _stale(HOST_LIB, [HOST_SRC]) and host_fits():
         return
     torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     part = f"{HOST_LIB}.{os.getpid()}.part"
     includes = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
                 os.path.join(cuda, "include")]
-    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-D_GLIBCXX_USE_CXX11_ABI=1", *(f"-I{d}" for d in includes), HOST_SRC, "-o", part,
-           f"-L{os.path.join(torch_dir, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-D_GLIBCXX_USE_CXX11_ABI=1", f'-DB200_HOST_TAG="{host_tag()}"', *(f"-I{d}" for d in includes), HOST_SRC,
+           "-o", part, f"-L{os.path.join(torch_dir, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)
@@ -99,7 +114,10 @@ def build(force: bool = False, verbose: bool = False, target: str = "all") -> st
                 sys.stderr.write(f"== {src}\n{r.stderr}\n")
             with open(os.path.join(OBJ, src[:-3] + ".ptxas.txt"), "w") as f:
                 f.write(r.stderr)
-        host.result()
+        try:
+            host.result()
+        except Exception as e:
+            sys.stderr.write(f"{HOST_LIB} could not be built ({e}): calls go through Python\n")
     for lib, which in ((LIB, "all"), (SEQ_LIB, "seq")):
         if target == "seq" and which == "all":
             continue

@@ -18,6 +18,9 @@
 #include <unordered_map>
 #include <vector>
 
+// which Python and torch this file is built for (build.py looks for it in the built file)
+extern "C" __attribute__((used, visibility("default"))) const char b200_host_tag[] = B200_HOST_TAG;
+
 namespace {
 
 struct Entries {   // the C ABI (include/b200_tgis.h, include/b200_seq.h)
