@@ -153,8 +153,9 @@ int b200_seq_delta_scan(const float* c, int64_t ldc, int col_q, int col_k, int c
  * steps) and SiLU; q and k become unit vectors, q times q_scale; beta = sigmoid(raw[col_b + h]); decay per head,
  * g = exp(-exp(A_log[h]) softplus(dec[col_a + h] + dt_bias[h])), or (channels != 0) per head and key channel n, acting on row n of S,
  * g = exp(-exp(A_log[h]) softplus(dec[col_a + h dk + n] + dt_bias[h dk + n])) -> out fp32 [T, b200_seq_delta_row_width].
- * b200_seq_delta_rows_scan: advances S over the prepared rows -> y fp32 [T, H * dv] (q / k shared by H / kv_heads heads); with a
- * workspace of b200_seq_delta_rows_scan_bytes (0: the shape has no use for one; NULL is fine) sixteen tokens at a time */
+ * b200_seq_delta_rows_scan: advances S over the prepared rows -> y fp32 [T, H * dv] (q / k shared by H / kv_heads heads)
+ * b200_seq_delta_rows_scan_in: the same, sixteen tokens at a time where there is room for their records: b200_seq_delta_rows_scan_bytes (0: the
+ * step has no use for any) take as few parts as they should, less takes more parts, less than 64 spans' (or NULL) is as without */
 int b200_seq_delta_row_width(int H, int kv_heads, int dk, int dv, int channels);
 int b200_seq_delta_prepare(const float* u, int64_t ld, int col0, int taps, const void* w, float* conv_state, const int32_t* state_slots,
                            const int32_t* seq_of_token, const int32_t* cu_q, const int64_t* position_ids, const float* raw, int64_t ldr,
@@ -163,7 +164,10 @@ int b200_seq_delta_prepare(const float* u, int64_t ld, int col0, int taps, const
 int64_t b200_seq_delta_rows_scan_bytes(int64_t T, int B, int H, int dk, int dv);
 int b200_seq_delta_rows_scan(const float* pre, int channels, float* S_state, const int32_t* state_slots, const int32_t* cu_q,
                         const int64_t* position_ids, float* y, int64_t ld_y, int64_t T, int B, int H, int kv_heads, int dk, int dv,
-                        void* workspace, void* stream);
+                        void* stream);
+int b200_seq_delta_rows_scan_in(const float* pre, int channels, float* S_state, const int32_t* state_slots, const int32_t* cu_q,
+                                const int64_t* position_ids, float* y, int64_t ld_y, int64_t T, int B, int H, int kv_heads, int dk, int dv,
+                                void* workspace, int64_t workspace_bytes, void* stream);
 /* per token: RMS norm over the whole q projection (H * d columns) and the whole k projection (G * d) when whole_norm != 0 (weights per
  * column, may be NULL), rotation of the first `rot` columns of every head, column i paired with i + rot / 2 (cos / sin fp32
  * [positions, rot / 2]); keys and values to the token-major cache row [k_off: G * d | v_off: G * dv], queries to q_out fp32 [T, H * d].

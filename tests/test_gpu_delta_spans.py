@@ -114,3 +114,60 @@ def test_records_in_parts():
     y = _scan(x, S, _step([0], lens, [0]), H, G, dk, dv, False)
     want, S_want = _exact(*x, torch.zeros(1, H, dk, dv, device=DEV), lens)
     assert _close(y, want) and _close(S.double(), S_want)
+
+
+def _scan_in(x, S, st, H, G, dk, dv, channels, spans):
+    """with room for so many spans' records"""
+    import ctypes
+    from tgis_b200 import _lib
+    lib, rows = _lib.load_seq(), _rows(*x)
+    room = spans * (lib.b200_seq_delta_rows_scan_bytes(500, 1, H, dk, dv) // (500 // 16 + 1))
+    ws, y = torch.empty(room, dtype=torch.uint8, device=DEV), torch.full((st.T, H * dv), 9.0, device=DEV)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    _lib.check_seq(lib.b200_seq_delta_rows_scan_in(p(rows), int(channels), p(S), p(st.state_slots), p(st.cu_q), p(st.position_ids), p(y), H * dv, st.T, st.B, H, G, dk,
+                                                   dv, p(ws), room, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)), "rows_scan_in")
+    return y
+
+
+@pytest.mark.parametrize("lens", [[1, 1030, 16, 0, 2100, 17, 1020, 500], [5, 33, 900, 16, 0] * 9, [3000, 1], [1, 1, 1, 1700]])
+@pytest.mark.parametrize("H,G,dk,dv,channels", [(3, 1, 64, 32, True), (2, 1, 128, 64, False)])
+def test_parts_of_several_sequences(lens, H, G, dk, dv, channels):
+    """sequences that end in an earlier part, go over from one to the next, or begin in the last: the same bits as in one part, states included"""
+    import tgis_b200  # noqa: F401
+    g = torch.Generator(device=DEV).manual_seed(len(lens))
+    x, B = _inputs(g, lens, H, G, dk, dv, channels), len(lens)
+    S0 = torch.randn(B, H, dk, dv, generator=g, device=DEV)
+    starts = [0 if i % 3 == 1 else 16 + i for i in range(B)]
+    st = _step(starts, lens, list(range(B)))
+    whole = S0.clone()
+    want = _scan_in(x, whole, st, H, G, dk, dv, channels, sum(lens) // 16 + B)
+    assert _close(want.unflatten(1, (H, dv)).double(), _exact(*x, torch.where(torch.tensor([s == 0 for s in starts], device=DEV)[:, None, None, None], 0.0, S0), lens)[0])
+    for spans in (64, 65, 100, sum(lens) // 16 + B - 1):
+        S = S0.clone()
+        assert torch.equal(_scan_in(x, S, st, H, G, dk, dv, channels, spans), want) and torch.equal(S, whole)
+    S = S0.clone()   # too little room: four tokens at a time
+    assert _close(_scan_in(x, S, st, H, G, dk, dv, channels, 63).double(), want.double()) and _close(S.double(), whole.double())
+
+
+def test_no_room_at_all(monkeypatch):
+    """a step whose records cannot be had goes four tokens at a time, as it did before there were any"""
+    import tgis_b200  # noqa: F401
+    from tgis_b200 import ops_seq
+    H, G, dk, dv, lens = 2, 1, 128, 64, [250, 130]
+    g = torch.Generator(device=DEV).manual_seed(5)
+    x, S0 = _inputs(g, lens, H, G, dk, dv, True), torch.randn(2, H, dk, dv, generator=g, device=DEV)
+    st, got, empty, asked = _step([16, 0], lens, [0, 1]), [], torch.empty, []
+    for most in (1 << 40, 0):
+        def some(*a, **k):
+            if k.get("dtype") == torch.uint8:
+                asked.append(a[0])
+                if a[0] > most:
+                    raise torch.cuda.OutOfMemoryError("out of memory")
+            return empty(*a, **k)
+        monkeypatch.setattr(ops_seq.torch, "empty", some)
+        S = S0.clone()
+        got.append((_scan(x, S, st, H, G, dk, dv, True), S.double()))
+        monkeypatch.undo()
+    assert len(asked) == 3 and asked[0] == asked[1] == 8 * asked[2]
+    (a, Sa), (b, Sb) = got
+    assert _close(b, a) and _close(Sb, Sa)

@@ -171,7 +171,8 @@ SEQ_SIGNATURES = {
     "b200_seq_delta_prepare": (_I, [_P, _L, _I, _I, _P, _P, _P, _P, _P, _P, _P, _L, _I, _P, _L, _I, _I, _P, _P, _I, _F, _P, _L, _I, _I, _I, _I, _I,
                                     _P]),
     "b200_seq_delta_rows_scan_bytes": (_L, [_L, _I, _I, _I, _I]),
-    "b200_seq_delta_rows_scan": (_I, [_P, _I, _P, _P, _P, _P, _P, _L, _L, _I, _I, _I, _I, _I, _P, _P]),
+    "b200_seq_delta_rows_scan": (_I, [_P, _I, _P, _P, _P, _P, _P, _L, _L, _I, _I, _I, _I, _I, _P]),
+    "b200_seq_delta_rows_scan_in": (_I, [_P, _I, _P, _P, _P, _P, _P, _L, _L, _I, _I, _I, _I, _I, _P, _L, _P]),
     "b200_seq_qk_rot_prepare": (_I, [_P, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P, _I, _F, _P, _P, _I, _P, _P, _P, _I, _L, _I, _I, _P, _L, _P, _P, _I,
                                      _I, _I, _P]),
     "b200_seq_talk_attn": (_I, [_P, _P, _I, _L, _I, _I, _P, _L, _P, _P, _I, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _F, _I, _P, _I, _P, _P]),

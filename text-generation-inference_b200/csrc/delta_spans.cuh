@@ -34,8 +34,8 @@ struct SpanRecord {
 };
 __host__ __device__ constexpr int span_record_floats(int dk, int dv) { return 3 * kSpan * dk + dk + kSpan * dv; }
 
-// tokens of sequence b inside the part [off, off + cap) of every sequence that one pair of launches covers
-__device__ __forceinline__ int span_tokens(const int32_t* cu_q, int b, int off, int cap) { return max(0, min(cu_q[b + 1] - cu_q[b] - off, cap)); }
+// The spans of a step count from its first sequence on; a pair of launches covers those numbered from .. from + cap - 1.
+__device__ __forceinline__ int spans_of(const int32_t* cu_q, int b) { return (cu_q[b + 1] - cu_q[b] + kSpan - 1) / kSpan; }
 
 __device__ __forceinline__ uint64_t span_fma2(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t r;
@@ -100,16 +100,16 @@ struct SpanPrep {
 };
 template <int DK>
 __global__ void __launch_bounds__(kSpanPrepHeads * 64, 3) delta_span_prepare_kernel(const float* __restrict__ pre, int width, int k_col, int v_col, int g_col, int b_col,
-                                                                                    const int32_t* __restrict__ cu_q, int B, int off, int cap, int H, int group,
-                                                                                    int channels, int dv, float* __restrict__ out, float* __restrict__ y, int64_t ld_y) {
+                                                                                    const int32_t* __restrict__ cu_q, int B, int from, int H, int group, int channels,
+                                                                                    int dv, float* __restrict__ out, float* __restrict__ y, int64_t ld_y) {
   using R = SpanRecord<DK>;
   pdl_wait();
   extern __shared__ __align__(16) float sm[];
   const int lane = lane_id(), part = warp_id() & 1, slot = warp_id() >> 1, h = blockIdx.y * kSpanPrepHeads + slot;
-  // which span: the part's spans in the order of the sequences
-  int b = -1, tile = blockIdx.x;
+  // which sequence's which span
+  int b = -1, tile = from + blockIdx.x;
   for (int b0 = 0; b0 < B && b < 0; b0 += 32) {
-    const int nt = b0 + lane < B ? (span_tokens(cu_q, b0 + lane, off, cap) + kSpan - 1) / kSpan : 0;
+    const int nt = b0 + lane < B ? spans_of(cu_q, b0 + lane) : 0;
     int upto = nt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kSpanPrepHeads * 64, 3) delta_span_prepare_ker
   }
   if (b >= 0 && h < H) {
     auto sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(slot + 1) : "memory"); };   // the two warps
-    const int t0 = cu_q[b] + off + tile * kSpan, n_tok = min(kSpan, span_tokens(cu_q, b, off, cap) - tile * kSpan);
+    const int t0 = cu_q[b] + tile * kSpan, n_tok = min(kSpan, cu_q[b + 1] - t0);
     const float* row = pre + (int64_t)t0 * width;
     float* rec = out + ((int64_t)blockIdx.x * H + h) * span_record_floats(DK, dv);
     float* in = sm + slot * SpanPrep<DK>::kHead;
@@ -304,7 +304,7 @@ template <int DK>
 __global__ void __launch_bounds__(SpanScan<DK>::kWarps * 32, 3) delta_span_scan_kernel(const float* __restrict__ rec, float* __restrict__ S_state,
                                                                                        const int32_t* __restrict__ state_slots, const int32_t* __restrict__ cu_q,
                                                                                        const int64_t* __restrict__ position_ids, float* __restrict__ y, int64_t ld_y,
-                                                                                       int off, int cap, int B, int H, int dv, unsigned* gave_up_word) {
+                                                                                       int from, int cap, int B, int H, int dv, unsigned* gave_up_word) {
   using R = SpanRecord<DK>;
   using L = SpanScan<DK>;
   constexpr int NP = DK / 32;   // pairs of channels
@@ -317,24 +317,32 @@ __global__ void __launch_bounds__(SpanScan<DK>::kWarps * 32, 3) delta_span_scan_
   // blocks start in the order of their numbers: the longest sequences first, so that short ones fill what is left (up to 32 of them; more even out by themselves)
   int b = blockIdx.x / (H * parts);
   if (B <= 32) {
-    const int mine = lane < B ? span_tokens(cu_q, lane, off, cap) : -1;
-    int rank = 0;
+    const int nt = lane < B ? spans_of(cu_q, lane) : 0;
+    int upto = nt, rank = 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    // spans inside the part; of as many, tokens decide
+    const int inside = max(0, min(upto, from + cap) - max(upto - nt, from));
+    const int mine = lane < B ? inside * kSpan - (inside > 0 && upto <= from + cap ? nt * kSpan - (cu_q[lane + 1] - cu_q[lane]) : 0) : -1;
     for (int i = 0; i < B; ++i) {
       const int other = __shfl_sync(0xffffffffu, mine, i);
       rank += other > mine || (other == mine && i < lane);
     }
     b = __ffs(__ballot_sync(0xffffffffu, lane < B && rank == b)) - 1;
   }
-  const int n_all = span_tokens(cu_q, b, off, cap), spans = (n_all + kSpan - 1) / kSpan;
-  if (spans == 0) return;
-  const int t_begin = cu_q[b] + off, v0 = (rest % parts) * kSpanCols;
-  const bool fresh = off == 0 && position_ids[t_begin] == 0;
   int first = 0;   // spans of the sequences ahead
-  for (int i = lane; i < b; i += 32) first += (span_tokens(cu_q, i, off, cap) + kSpan - 1) / kSpan;
+  for (int i = lane; i < b; i += 32) first += spans_of(cu_q, i);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) first += __shfl_xor_sync(0xffffffffu, first, o);
+  const int lo = max(0, from - first), spans = min(spans_of(cu_q, b), from + cap - first) - lo;   // the sequence's spans inside the part
+  if (spans <= 0) return;
+  const int t_begin = cu_q[b] + lo * kSpan, n_all = min(cu_q[b + 1] - t_begin, spans * kSpan), v0 = (rest % parts) * kSpanCols;
+  const bool fresh = lo == 0 && position_ids[t_begin] == 0;
   const int64_t step = (int64_t)H * span_record_floats(DK, dv);
-  const float* src = rec + ((int64_t)first * H + h) * span_record_floats(DK, dv);
+  const float* src = rec + ((int64_t)(first + lo - from) * H + h) * span_record_floats(DK, dv);
   if (threadIdx.x == 0) {
     mbar_init(&full[0], 1);
     mbar_init(&full[1], 1);

@@ -766,39 +766,34 @@ static int launch_delta_step(const float* pre, float* S_state, const int32_t* st
   return B200_OK;
 }
 
-// Spans of a step that one pair of launches may leave records of: all of them, or those of the next `cap` tokens of every sequence where the records of
-// all would take more than kSpanRoom bytes (`cap` == 0: too many sequences for that, or a shape that the spans don't take).
+// Spans of a step (at most; the host knows the number of tokens, not the lengths), and the bytes of their records, up to kSpanRoom (0: a step that the spans
+// don't take).  A smaller workspace takes them in parts, one pair of launches behind the other: sequences one after the other, so a part shouldn't be
+// smaller than what keeps the chip busy for a while (kSpanPart spans).
 // kSpanMean: tokens per sequence from which spans are faster than the chain over four tokens; on grids that fill the chip the chain hides its waits better.
 // Measured on B200 (us with the preparation, chain / spans, heads of 128): 16 heads: 1 x 40 tokens 26 / 32, 2 x 125 67 / 54, 6 x 96 - 120 95 / 79, 1 x 690
 // 201 / 135, 4 x 256 - 768 292 / 210; 32 heads: 6 x 30 - 60 83 / 93, 1 x 96 52 / 45, 3 x 100 - 200 126 / 109, 6 x 128 - 140 165 / 171, 1 x 450 208 / 125,
 // 6 x 400 - 800 797 / 656.
-constexpr int64_t kSpanRoom = (int64_t)2 << 30, kSpanMean = 96, kSpanMeanFull = 192;
+constexpr int64_t kSpanRoom = (int64_t)2 << 30, kSpanMean = 96, kSpanMeanFull = 192, kSpanPart = 64;
 struct SpanPlan {
-  int64_t spans, bytes;
-  int cap;
+  int64_t spans, rec, bytes;   // rec: of one span, all heads
 };
 static SpanPlan delta_span_plan(int64_t T, int B, int H, int dk, int dv) {
   SpanPlan pl = {0, 0, 0};
   const bool full = (int64_t)B * H * (dv / kSpanCols) > 4 * 148;   // more blocks than can be on the chip at once
   if ((dk != 64 && dk != 128) || dv % kSpanCols != 0 || T < (full ? kSpanMeanFull : kSpanMean) * B) return pl;
-  const int64_t rec = (int64_t)span_record_floats(dk, dv) * 4 * H;
+  pl.rec = (int64_t)span_record_floats(dk, dv) * 4 * H;
   pl.spans = T / kSpan + B;
-  pl.cap = 1 << 30;
-  if (pl.spans * rec > kSpanRoom) {
-    const int64_t each = kSpanRoom / (rec * B);   // spans per sequence
-    pl.cap = each >= 64 ? (int)(each * kSpan) : 0;
-    pl.spans = each * B;
-  }
-  pl.bytes = pl.cap ? pl.spans * rec : 0;
+  if (pl.rec * kSpanPart > kSpanRoom) return pl;
+  pl.bytes = pl.spans * pl.rec > kSpanRoom ? kSpanRoom / pl.rec * pl.rec : pl.spans * pl.rec;
   return pl;
 }
 
-// bytes of workspace with which b200_seq_delta_rows_scan takes a step in spans of sixteen tokens (0: it does not)
+// bytes of workspace with which b200_seq_delta_rows_scan_in takes a step in spans of sixteen tokens, as few parts as it should (0: it does not)
 extern "C" int64_t b200_seq_delta_rows_scan_bytes(int64_t T, int B, int H, int dk, int dv) { return B > 0 && H > 0 ? delta_span_plan(T, B, H, dk, dv).bytes : 0; }
 
 template <int DK>
 static int launch_delta_spans(const float* pre, const DeltaRow& lay, int channels, float* S_state, const int32_t* state_slots, const int32_t* cu_q,
-                              const int64_t* position_ids, float* y, int64_t ld_y, int64_t T, int B, int H, int G, int dv, const SpanPlan& pl, float* records,
+                              const int64_t* position_ids, float* y, int64_t ld_y, int B, int H, int G, int dv, int spans, int cap, float* records,
                               cudaStream_t st) {
   using Scan = SpanScan<DK>;
   static const cudaError_t configured[2] = {
@@ -808,11 +803,12 @@ static int launch_delta_spans(const float* pre, const DeltaRow& lay, int channel
     if (e != cudaSuccess) { b200_set_last_error(cudaGetErrorString(e)); return B200_ERR_CUDA; }
   unsigned* word = b200_gave_up_word();
   if (!word) return B200_ERR_CUDA;
-  for (int64_t off = 0; off < T; off += pl.cap) {   // (the host does not know how long the longest sequence is: T at most)
-    B200_LAUNCH((delta_span_prepare_kernel<DK>), dim3((unsigned)pl.spans, (unsigned)((H + kSpanPrepHeads - 1) / kSpanPrepHeads)), dim3(kSpanPrepHeads * 64),
-                (size_t)SpanPrep<DK>::kBytes, st, pre, lay.width, lay.k, lay.v, lay.g, lay.b, cu_q, B, (int)off, pl.cap, H, H / G, channels, dv, records, y, ld_y);
+  for (int from = 0; from < spans; from += cap) {
+    const int n = spans - from < cap ? spans - from : cap;
+    B200_LAUNCH((delta_span_prepare_kernel<DK>), dim3((unsigned)n, (unsigned)((H + kSpanPrepHeads - 1) / kSpanPrepHeads)), dim3(kSpanPrepHeads * 64),
+                (size_t)SpanPrep<DK>::kBytes, st, pre, lay.width, lay.k, lay.v, lay.g, lay.b, cu_q, B, from, H, H / G, channels, dv, records, y, ld_y);
     B200_LAUNCH((delta_span_scan_kernel<DK>), dim3((unsigned)(B * H * (dv / kSpanCols))), dim3(Scan::kWarps * 32), (size_t)Scan::kBytes, st, records,
-                S_state, state_slots, cu_q, position_ids, y, ld_y, (int)off, pl.cap, B, H, dv, word);
+                S_state, state_slots, cu_q, position_ids, y, ld_y, from, n, B, H, dv, word);
     b200_count_launches(2);
   }
   return B200_OK;
@@ -820,10 +816,11 @@ static int launch_delta_spans(const float* pre, const DeltaRow& lay, int channel
 
 // pre fp32 [T, b200_seq_delta_row_width]: rows as b200_seq_delta_prepare leaves them; S_state fp32 [slots, H, dk, dv] advanced in place
 // -> y fp32 [T, H * dv].  T: token rows of the step (steps with few rows per sequence take the form that is bound by the state's traffic).
-// workspace: b200_seq_delta_rows_scan_bytes bytes, 16-byte aligned, or NULL (the step then goes four tokens at a time)
-extern "C" int b200_seq_delta_rows_scan(const float* pre, int channels, float* S_state, const int32_t* state_slots, const int32_t* cu_q,
-                                   const int64_t* position_ids, float* y, int64_t ld_y, int64_t T, int B, int H, int kv_heads, int dk, int dv,
-                                   void* workspace, void* stream) {
+// workspace: room for records, 16-byte aligned; with b200_seq_delta_rows_scan_bytes bytes or less (at least those of kSpanPart spans) the step goes sixteen
+// tokens at a time, otherwise (or NULL) four
+extern "C" int b200_seq_delta_rows_scan_in(const float* pre, int channels, float* S_state, const int32_t* state_slots, const int32_t* cu_q,
+                                           const int64_t* position_ids, float* y, int64_t ld_y, int64_t T, int B, int H, int kv_heads, int dk, int dv,
+                                           void* workspace, int64_t workspace_bytes, void* stream) {
   if (T == 0 || B == 0) return B200_OK;
   if (kv_heads <= 0 || H % kv_heads != 0 || dk <= 0 || dk > 256 || dv <= 0) {
     b200_set_last_error("seq_delta_rows_scan: need heads % kv_heads == 0 and 0 < key size <= 256");
@@ -851,10 +848,11 @@ extern "C" int b200_seq_delta_rows_scan(const float* pre, int channels, float* S
 #undef DST
   }
   const SpanPlan pl = delta_span_plan(T, B, H, dk, dv);
-  if (workspace && pl.cap && aligned && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0) {
+  const int64_t cap = pl.bytes ? (workspace_bytes < pl.bytes ? workspace_bytes : pl.bytes) / pl.rec : 0;
+  if (workspace && (cap >= kSpanPart || (cap > 0 && cap >= pl.spans)) && aligned && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0) {
     const DeltaRow lay = delta_row(H, kv_heads, dk, dv, channels != 0);
-    return dk == 64 ? launch_delta_spans<64>(pre, lay, channels, S_state, state_slots, cu_q, position_ids, y, ld_y, T, B, H, kv_heads, dv, pl, (float*)workspace, st)
-                    : launch_delta_spans<128>(pre, lay, channels, S_state, state_slots, cu_q, position_ids, y, ld_y, T, B, H, kv_heads, dv, pl, (float*)workspace, st);
+    const auto launch = dk == 64 ? launch_delta_spans<64> : launch_delta_spans<128>;
+    return launch(pre, lay, channels, S_state, state_slots, cu_q, position_ids, y, ld_y, B, H, kv_heads, dv, (int)pl.spans, (int)cap, (float*)workspace, st);
   }
   const int vec = (dk % 4 == 0 && dv % 4 == 0 && aligned) ? 1 : 0;
   // 64 columns per block share each staged vector among more of the memory; a small grid is spread over 32 columns and 32 lanes.  The line lies where
@@ -874,4 +872,9 @@ extern "C" int b200_seq_delta_rows_scan(const float* pre, int channels, float* S
   if (dk <= 128) DCH(8, 16);
   DCH(16, 16);
 #undef DCH
+}
+// the same without room for records
+extern "C" int b200_seq_delta_rows_scan(const float* pre, int channels, float* S_state, const int32_t* state_slots, const int32_t* cu_q,
+                                        const int64_t* position_ids, float* y, int64_t ld_y, int64_t T, int B, int H, int kv_heads, int dk, int dv, void* stream) {
+  return b200_seq_delta_rows_scan_in(pre, channels, S_state, state_slots, cu_q, position_ids, y, ld_y, T, B, H, kv_heads, dk, dv, nullptr, 0, stream);
 }

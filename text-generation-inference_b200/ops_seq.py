@@ -595,12 +595,24 @@ def delta_rows_scan(rows: torch.Tensor, S: torch.Tensor, step: RaggedStep, H: in
     assert rows.dtype == torch.float32 and rows.is_contiguous() and S.dtype == torch.float32 and S.is_contiguous() and S.shape[1:] == (H, dk, dv)
     y = torch.empty(step.T, H * dv, dtype=torch.float32, device=rows.device)
     lib = _lib.load_seq()
-    need = lib.b200_seq_delta_rows_scan_bytes(step.T, step.B, H, dk, dv) if step.T >= 96 * step.B else 0   # (the fewest tokens that have a use for it)
-    ws = torch.empty(need, dtype=torch.uint8, device=rows.device) if need else None
-    _lib.check_seq(lib.b200_seq_delta_rows_scan(_ptr(rows), int(channels), _ptr(S), _ptr(step.state_slots), _ptr(step.cu_q),
-                                                _ptr(step.position_ids), _ptr(y), y.stride(0), step.T, step.B, H, kv_heads, dk, dv, _ptr(ws), _stream()),
-                    "seq_delta_rows_scan")
+    ws, need = None, 0
+    if step.T >= 16 * step.B:   # a span each
+        need = min(lib.b200_seq_delta_rows_scan_bytes(step.T, step.B, H, dk, dv), _SPAN_ROOM)
+    for room in (need, need // 8) if need else ():   # what cannot be had makes the step slower, not impossible
+        try:
+            ws = torch.empty(room, dtype=torch.uint8, device=rows.device)
+            break
+        except torch.cuda.OutOfMemoryError:
+            pass
+    _lib.check_seq(lib.b200_seq_delta_rows_scan_in(_ptr(rows), int(channels), _ptr(S), _ptr(step.state_slots), _ptr(step.cu_q),
+                                                   _ptr(step.position_ids), _ptr(y), y.stride(0), step.T, step.B, H, kv_heads, dk, dv, _ptr(ws),
+                                                   0 if ws is None else ws.numel(), _stream()), "seq_delta_rows_scan")
     return y
+
+
+# Bytes that a step's records may take: 33 KB per sixteen tokens and head of 128, 16 k tokens of 16 heads at once; longer steps go in parts.  The cache pool
+# leaves two fifths of the free memory to steps.
+_SPAN_ROOM = 512 << 20
 
 
 def qk_rot_prepare(src: torch.Tensor, *, col_q: int, col_k: int, col_v: int, heads: int, kv_heads: int, dim: int, vdim: int,
