@@ -67,3 +67,29 @@ def test_runs(new, past, chunk, window, with_sink, H, G, d):
         for x in (q, shifted):
             got = ops.talk_attn(x, cache, step, kv_heads=G, vdim=d, k_off=0, v_off=G * d, scale=d ** -0.5, talk=mix, chunk=chunk, window=window, sink=sink).double()
             assert float((got - want).norm()) <= 4e-3 * float(want.norm()) * (1.5 if mix is not None else 1.0)
+
+
+@pytest.mark.parametrize("new,past", [([1], [1000]), ([2, 1], [900, 90])])
+@pytest.mark.parametrize("chunk,window", [(0, 0), (512, 0), (0, 100)])
+@pytest.mark.parametrize("which", ["keys", "one head's keys", "values"])
+def test_what_is_not_a_number_shows(new, past, chunk, window, which):
+    """Keys of four whole pages, which are whole runs, are NaN: every row that sees one of them is NaN, the others are as without."""
+    import tgis_b200  # noqa: F401
+    from tgis_b200 import ops_seq as ops
+    H, G, d = 16, 4, 128
+    g = torch.Generator(device=DEV).manual_seed(7)
+    step, blocks = _step(new, past)
+    cache = torch.randn(blocks, PAGE, 2 * G * d, generator=g, device=DEV).bfloat16()
+    q = torch.randn(sum(new), H, d, generator=g, device=DEV)
+    at = {"keys": slice(0, G * d), "one head's keys": slice(d, 2 * d), "values": slice(G * d, 2 * G * d)}[which]
+    cache[step.block_table[0, 40:44].long(), :, at] = float("nan")   # tokens 640 .. 703 of the first sequence
+    call = lambda mix: ops.talk_attn(q, cache, step, kv_heads=G, vdim=d, k_off=0, v_off=G * d, scale=d ** -0.5, talk=mix, chunk=chunk, window=window).double()  # noqa: E731
+    sees = window == 0   # the window of the first sequence's queries starts behind them
+    for mix in (None, torch.eye(H, device=DEV) + 0.2 * torch.randn(H, H, generator=g, device=DEV)):
+        nan = torch.zeros(sum(new), H, dtype=torch.bool, device=DEV)
+        if sees:
+            nan[:new[0]] = torch.ones(H, dtype=torch.bool, device=DEV) if which != "one head's keys" or mix is not None else torch.arange(H, device=DEV) // (H // G) == 1
+        got = call(mix)
+        assert torch.equal(got.isnan().all(-1), nan) and torch.equal(got.isnan().any(-1), nan)
+        want = _exact(q, cache.nan_to_num(), step, new, past, G, d, d ** -0.5, chunk, window, None, mix)
+        assert float((got - want)[~nan].norm()) <= 6e-3 * float(want[~nan].norm())

@@ -326,9 +326,12 @@ __global__ void __launch_bounds__(512) talk_attn_mma_kernel(
   const int per_split = (n_ktiles + gridDim.z - 1) / gridDim.z;
   const int j_start = j_first + (int)blockIdx.z * per_split * KT;
   const int j_end = min(p_last, j_start + per_split * KT - 1);   // last key of this block's run
-  if (gridDim.z > 1 && j_start > j_end) {   // no keys are left for this run: it says so and takes no time
+  if (gridDim.z > 1 && j_start > j_end) {   // no keys are left for this run: it says so with a sum that no run can have, and takes no time
     float* base = partial + (((int64_t)blockIdx.x * gridDim.z + blockIdx.z) * R) * (dv + 2) + dv;
-    for (int r = threadIdx.x; r < R; r += nthreads) base[(int64_t)r * (dv + 2)] = -INFINITY;
+    for (int r = threadIdx.x; r < R; r += nthreads) {
+      base[(int64_t)r * (dv + 2)] = -INFINITY;
+      base[(int64_t)r * (dv + 2) + 1] = -1.f;
+    }
     return;
   }
   const int w = warp_id(), lane = lane_id();
@@ -615,8 +618,11 @@ __global__ void __launch_bounds__(256) talk_attn_merge_kernel(const float* __res
     const int64_t zs = (int64_t)R * (dv + 2);
     const float m = lane < nsplit ? base[lane * zs + dv] : -INFINITY, l = lane < nsplit ? base[lane * zs + dv + 1] : 0.f;
     const float M = warp_max(m), weight = m > -INFINITY ? expf(m - M) : 0.f;
-    const unsigned some = __ballot_sync(0xffffffffu, m > -INFINITY);           // an empty run carries no weight and has left nothing else
-    const float inv = 1.f / warp_sum(m > -INFINITY ? weight * l : 0.f);
+    // Runs without keys have left nothing.  All others count, also where a row's maximum is -inf: scores that are not a number don't show in it, but in the
+    // sum and the output, and must show in the result.
+    const bool left = lane < nsplit && !(l < 0.f);
+    const unsigned some = __ballot_sync(0xffffffffu, left);
+    const float inv = 1.f / warp_sum(left ? weight * l : 0.f);
     float* dst = out + ((int64_t)(row0 + tok) * H + c * rep + rr % rep) * dv;
     for (int c0 = 0; c0 < dv; c0 += 64) {   // two columns of eight runs in flight
       const int col = c0 + lane, col2 = col + 32;
