@@ -206,6 +206,8 @@ int b200_gptq_pack(const void* qweight, const void* qzeros, const void* scales, 
 #define B200_W4_LAYOUT_GATE_UP 1
 /* row_perm (int32 [K], device) or NULL: act-order checkpoints (non-trivial g_idx; exllamav2.py:31-48 q_perm): a stable
  * arg-sort of g_idx.  Packed row k' = checkpoint row row_perm[k']; feed the GEMM x[:, row_perm] (b200_permute_columns). */
+int b200_settle(void* stream); /* packed weights are read early: after records were written in any other way (a copy of them) than by b200_gptq_pack[_ex],
+                                * which does so itself, this launch has to stand between that and the first linear that reads them */
 int b200_gptq_pack_ex(const void* qweight, const void* qzeros, const void* scales, const int32_t* row_perm, void* packed,
                       int64_t K, int64_t N, int groupsize, int layout, void* stream);
 /* out[t, k'] = x[t, perm[k']], fp16 [T, K] */

@@ -15,6 +15,7 @@ SIGNATURES = {
     "b200_abi_version": (_I, []),
     "b200_last_error": (c_char_p, []),
     "b200_gave_up": (_I, []),
+    "b200_settle": (_I, [_P]),
     "b200_debug_set_gave_up": (None, [_I]),
     "b200_cuda_peek_error": (c_char_p, []),
     "b200_debug_w4_trace": (None, [_P]),

@@ -325,7 +325,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       }
     }
   } else if (C::kInt4 && warp == C::kServeWarp) {
-    // ------------------------------------------------------------------ TMA: int4 records (immutable: no wait for the previous kernel)
+    // ------------------------------------------------------------------ TMA: int4 records (settled when they were packed: no wait for the previous kernel)
     if (elect_one()) {
       int r = 0, ph = 1;
       PairCursor cur;

@@ -65,7 +65,8 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemm_w4_few_kernel(const W4Few
   const int sup = blockIdx.x / d, warp = warp_id(), lane = lane_id(), g = lane >> 2, t = lane & 3, odd = warp >> 3, f0 = (warp & 7) * 16 + g;
   const int kb0 = (int)(rank * p.nkb / d), n = (int)((rank + 1) * p.nkb / d) - kb0;
 
-  // weights do not depend on the kernel before: two k-blocks of the warp are under way before anything else
+  // the CTA's records are on their way to L2 while the kernel before ends (as fast as reading them ahead of it: 4096 -> 6144 at one token 8.0 and 8.0 us)
+  if (threadIdx.x < n) tma_bulk_prefetch(p.packed + ((size_t)sup * p.rec_per_tile + kb0 + threadIdx.x) * 2 * kRec, 2 * kRec);
   struct Block {
     uint4 w[2][2];       // [tile][feature f0, f0 + 8]
     uint32_t meta[2][2];
@@ -88,12 +89,12 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemm_w4_few_kernel(const W4Few
     src += 4 * kRec;
     msrc += 4 * kRec;
   };
-  fetch(blk[0]);
-  fetch(blk[1]);
   if (threadIdx.x < n) mbar_init(&landed[threadIdx.x], kFewThreads);
   mbar_fence_init();
   __syncthreads();
   pdl_wait();
+  fetch(blk[0]);
+  fetch(blk[1]);
   for (int i = 0; i < n; ++i) {
     if (threadIdx.x < p.T * 16) {   // 16-byte pieces of the block; what lies behind K is zero
       const int tok = threadIdx.x >> 4, o = threadIdx.x & 15, k = (kb0 + i) * kW4BlockK + o * 8;

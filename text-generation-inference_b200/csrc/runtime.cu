@@ -220,6 +220,14 @@ extern "C" int b200_debug_step_trace_names(char* out, int64_t cap) {
   }
   return g_trace_n;
 }
+static __global__ void b200_settle_kernel() {}
+// An ordinary launch: it begins when everything ahead of it in the stream is in place, and no launch behind it can begin earlier.
+extern "C" int b200_settle(void* stream) {
+  b200_settle_kernel<<<1, 1, 0, (cudaStream_t)stream>>>();
+  B200_CHECK_LAUNCH();
+  return B200_OK;
+}
+
 void b200_step_trace_stamp(const char* kernel_name, cudaStream_t stream) {
   if (!g_trace_buf || g_trace_n >= g_trace_cap) return;
   b200_stamp_kernel<<<1, 1, 0, stream>>>(g_trace_buf + g_trace_n);

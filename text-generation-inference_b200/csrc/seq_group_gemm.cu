@@ -123,16 +123,9 @@ __global__ void __launch_bounds__(kGgThreads, 2) group_gemm_kernel(const __grid_
     if (elect_one()) {
       const int x_col = MODE == 0 ? (int)(group * p.head_x) : 0, w_row = group * p.N + n0;
       int issued = 0;
-      // weights do not depend on the kernel before this one (heads): the ring is filled with them ahead of the wait for it
-      const int npre = MODE == 0 ? min(p.nkb, C::kStages) : 0;
-      for (; issued < npre; ++issued) {
-        mbar_arrive_expect_tx(&full_bar[issued], C::kStageBytes);
-        tma_load_2d(smem + issued * C::kStageBytes, &tmap_w, issued * kGgTileK, w_row, &full_bar[issued]);
-      }
-      if constexpr (MODE == 0) {
+      if constexpr (MODE == 0) {   // the first ring's weights are on their way to L2 while the kernel before this one ends
+        for (int i = 0; i < min(p.nkb, C::kStages); ++i) tma_prefetch_2d(&tmap_w, i * kGgTileK, w_row);
         pdl_wait();
-        for (int i = 0; i < npre; ++i)
-          tma_load_2d(smem + i * C::kStageBytes + C::kABytes, &tmap_x, x_col + i * kGgTileK, row0, &full_bar[i]);
       }
       for (; issued < p.nkb; ++issued) {
         const int s = issued % C::kStages;

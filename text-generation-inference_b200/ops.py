@@ -303,6 +303,12 @@ def gemm_w4a16(x: torch.Tensor, packed: torch.Tensor, N: int, groupsize: int, bi
     _req(x, torch.float16, "x")
     _req(packed, torch.uint8, "packed")
     assert x.is_contiguous() and packed.is_contiguous()
+def settle() -> None:
+    """Int4 linears read packed weights early.  `gptq_pack` sees to it that they may; after records were written in another way (a copy of them) this has to be
+    called, on the stream that wrote them, before a linear reads them."""
+    _lib.check(_lib.load().b200_settle(_stream()), "settle")
+
+
     T, K = x.shape
     if out is None:
         out = torch.empty(T, N // 2 if silu_mul else N, dtype=torch.float16, device=x.device)
