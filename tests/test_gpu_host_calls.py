@@ -72,9 +72,8 @@ def test_linears(both):
     assert both(lambda m: m.gemm_f16(_r(5, 100), _r(96, 100)))[0].__name__ == "B200Error"   # refused by the entry
 
 
+@pytest.mark.parametrize("both", ["ops"], indirect=True)
 def test_int4(both):
-    if both.name != "ops":
-        return
     from tgis_b200 import ops
     g = torch.Generator(device=DEV).manual_seed(1)
     K, N = 256, 512
@@ -89,9 +88,8 @@ def test_int4(both):
     assert both(lambda m: m.gemm_w4a16(x.bfloat16(), plain, N, 128))[0].__name__ == "B200Error"
 
 
+@pytest.mark.parametrize("both", ["ops"], indirect=True)
 def test_attention(both):
-    if both.name != "ops":
-        return
     lens = torch.tensor([20, 3], dtype=torch.int32, device=DEV)
     table = torch.tensor([[0, 2], [1, 0]], dtype=torch.int32, device=DEV)
     k, v = _r(3, 2, 16, 64), _r(3, 2, 16, 64)
@@ -108,21 +106,82 @@ def test_attention(both):
     assert both(lambda m: m.attn_prefill_paged(q, k, v, table, lens, cu.long(), 1, 0.125))[0].__name__ == "B200Error"
 
 
-def test_first_calls_inside_a_capture(both):
-    """a workspace that has to grow while a stream is captured comes from the capture's pool, as the Python path's does"""
-    x = _r(4, 512) if both.name == "ops" else _r(4, 512, dtype=torch.bfloat16)
-    w = _r(40960, 512, dtype=x.dtype)
+def _forget_workspaces(m, monkeypatch):
+    """as in a process that has made no call yet"""
+    from tgis_b200 import _lib
+    monkeypatch.setattr(m, "_gemm_ws", {})
+    if not isinstance(m._host, _Nothing):
+        m._host = None
+        m._native()
+
+
+def test_first_calls_inside_a_capture(both, monkeypatch):
+    """A workspace that has to be made while a stream is captured belongs to the graph, whose replays zero its counters: a call ahead of the first replay gets
+    another one."""
+    x = _r(4, 2048) if both.name == "ops" else _r(4, 2048, dtype=torch.bfloat16)
+    w = _r(2048, 2048, dtype=x.dtype)
 
     def call(m):
         f = m.gemm_f16 if both.name == "ops" else m.linear
-        f(x, w)
-        torch.cuda.synchronize()
+        _forget_workspaces(m, monkeypatch)
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
-            y = f(x, w)
+            y, z = f(x, w), f(x, w)
+        assert not m._gemm_ws
+        eager = f(x, w)
         graph.replay()
         torch.cuda.synchronize()
+        assert len(m._gemm_ws) == 1 and torch.equal(y, eager) and torch.equal(z, eager)
         return y.clone()
+    both(call)
+
+
+def test_a_workspace_grows(both, monkeypatch):
+    x = _r(4, 2048) if both.name == "ops" else _r(4, 2048, dtype=torch.bfloat16)
+    wide, narrow = _r(20480, 2048, dtype=x.dtype), _r(128, 2048, dtype=x.dtype)
+
+    def call(m):
+        f = m.gemm_f16 if both.name == "ops" else m.linear
+        _forget_workspaces(m, monkeypatch)
+        got, sizes = [], []
+        for w in (narrow, wide, narrow):
+            got.append(f(x, w))
+            sizes.append([t.numel() for t in m._gemm_ws.values()])
+        assert len(sizes[0]) == 1 and sizes[0][0] < sizes[1][0] == sizes[2][0] and torch.equal(got[0], got[2])
+        return torch.cat(got, 1)
+    both(call)
+
+
+def test_calls_from_several_threads(both, monkeypatch):
+    """each thread on a stream of its own, with workspaces of its own, sizes that differ"""
+    import threading
+    dt = torch.float16 if both.name == "ops" else torch.bfloat16
+    xs, ws = [_r(2 + i, 2048, dtype=dt) for i in range(4)], [_r(128 << i, 2048, dtype=dt) for i in range(4)]
+    torch.cuda.synchronize()
+
+    def call(m):
+        got, wrong = [None] * 4, []
+        want = [m.gemm_f16(x, w) if both.name == "ops" else m.linear(x, w) for x, w in zip(xs, ws)]
+        torch.cuda.synchronize()
+
+        def work(i):
+            try:
+                with torch.cuda.stream(torch.cuda.Stream()):
+                    mine = m.gemm_workspace(torch.device(DEV), 8, 1024, 2048).clone() if both.name == "ops" else None
+                    for _ in range(50):
+                        got[i] = m.gemm_f16(xs[i], ws[i], workspace=mine) if both.name == "ops" else m.linear(xs[i].float(), ws[i].float())
+                    torch.cuda.current_stream().synchronize()
+            except Exception as e:
+                wrong.append(e)
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not wrong
+        if both.name == "ops":
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
+        return torch.cat([g.flatten() for g in got])
     both(call)
 
 

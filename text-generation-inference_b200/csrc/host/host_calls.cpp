@@ -11,6 +11,7 @@
 
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -67,7 +68,8 @@ bool real(PyObject* o, double& v) {
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
 // The device's workspace of at least `need` bytes, from Python when there is none yet or it is too small; undefined where there is none to be had.  The caller
-// holds it until its entry has returned: other threads run meanwhile, and one that needs more replaces it here and in Python.
+// holds it until its entry has returned: other threads run meanwhile, and one that needs more replaces it here and in Python.  What is made while
+// the stream is captured belongs to the graph and is not kept.
 at::Tensor workspace(std::vector<at::Tensor>& have, PyObject* make, PyObject* like, const at::Tensor& t, int64_t need, PyObject* a, PyObject* b) {
   const size_t dev = (size_t)t.get_device();
   if (have.size() <= dev) have.resize(dev + 1);
@@ -78,8 +80,10 @@ at::Tensor workspace(std::vector<at::Tensor>& have, PyObject* make, PyObject* li
       Py_XDECREF(got);
       return {};
     }
-    have[dev] = *w;
+    at::Tensor made = *w;
     Py_DECREF(got);
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return made;
+    have[dev] = made;
   }
   return have[dev];
 }

@@ -146,6 +146,8 @@ def _attn_workspace(device, need: int) -> torch.Tensor:
     """per-device grow-only workspace"""
     workspace = _attn_ws.get(device)
     if workspace is None or workspace.numel() < need:
+        if torch.cuda.is_current_stream_capturing():   # it belongs to the graph
+            return torch.empty(max(need, 1 << 22), dtype=torch.uint8, device=device)
         workspace = torch.zeros(max(need, 1 << 22), dtype=torch.uint8, device=device)
         _attn_ws[device] = workspace
     return workspace
@@ -232,8 +234,17 @@ def gemm_workspace(device, T: int, N: int, K: int) -> torch.Tensor:
     need = _gemm_workspace_bytes(N, K)
     ws = _gemm_ws.get(device)
     if ws is None or ws.numel() < need:
+        if torch.cuda.is_current_stream_capturing():
+            return captured_gemm_workspace(device, need)
         ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=device)
         _gemm_ws[device] = ws
+    return ws
+
+
+def captured_gemm_workspace(device, need: int) -> torch.Tensor:
+    """One that has to be made while a stream is captured belongs to the graph, whose replays zero its counters (64 KB); nobody else may have it before."""
+    ws = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=device)
+    ws[:1 << 16].zero_()
     return ws
 
 
@@ -292,6 +303,12 @@ def gptq_pack(qweight: torch.Tensor, qzeros: torch.Tensor, scales: torch.Tensor,
     return packed
 
 
+def settle() -> None:
+    """Int4 linears read packed weights early.  `gptq_pack` sees to it that they may; after records were written in another way (a copy of them) this has to be
+    called, on the stream that wrote them, before a linear reads them."""
+    _lib.check(_lib.load().b200_settle(_stream()), "settle")
+
+
 def gemm_w4a16(x: torch.Tensor, packed: torch.Tensor, N: int, groupsize: int, bias: Optional[torch.Tensor] = None,
                out: Optional[torch.Tensor] = None, workspace: Optional[torch.Tensor] = None, layout: int = W4_LAYOUT_PLAIN,
                silu_mul: bool = False) -> torch.Tensor:
@@ -303,12 +320,6 @@ def gemm_w4a16(x: torch.Tensor, packed: torch.Tensor, N: int, groupsize: int, bi
     _req(x, torch.float16, "x")
     _req(packed, torch.uint8, "packed")
     assert x.is_contiguous() and packed.is_contiguous()
-def settle() -> None:
-    """Int4 linears read packed weights early.  `gptq_pack` sees to it that they may; after records were written in another way (a copy of them) this has to be
-    called, on the stream that wrote them, before a linear reads them."""
-    _lib.check(_lib.load().b200_settle(_stream()), "settle")
-
-
     T, K = x.shape
     if out is None:
         out = torch.empty(T, N // 2 if silu_mul else N, dtype=torch.float16, device=x.device)

@@ -17,6 +17,7 @@ from typing import Optional
 import torch
 
 from . import _lib
+from .ops import captured_gemm_workspace
 
 _DT = {torch.bfloat16: 0, torch.float32: 1}
 
@@ -77,6 +78,8 @@ def _gemm_workspace(device, N: int, K: int, side: Optional[bool] = None) -> torc
     key = (device, _on_side if side is None else side)
     ws = _gemm_ws.get(key)
     if ws is None or ws.numel() < need:
+        if torch.cuda.is_current_stream_capturing():
+            return captured_gemm_workspace(device, need)
         ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=device)
         _gemm_ws[key] = ws
     return ws
