@@ -227,8 +227,8 @@ int b200_gemm_w4a16_ex(const void* x, const void* packed, const void* bias, void
  * Instead of finishing that sum inside the GEMM (a grid-wide wait on the slowest contributor + a second pass, 5-8 us per
  * launch), the *_deferred GEMMs leave the partials in the workspace and describe them with a B200SplitK; the consumer that
  * follows in the stream anyway (residual + RMSNorm, RoPE + KV write, SiLU * up, the tensor-parallel all-reduce) adds them up
- * in contributor order as it reads its input - bit-identical to the in-GEMM fix-up.  A B200SplitK is valid until the next GEMM
- * that uses the same workspace.  Element (t, n), plain layout: tile = n / 128, unit u = tile / tiles_per_unit,
+ * in contributor order as it reads its input.  Deterministic, as the ordinary entries are, and equal to their results up to the order of the
+ * fp32 sums: those may cut k elsewhere.  A B200SplitK is valid until the next GEMM that uses the same workspace.  Element (t, n), plain layout: tile = n / 128, unit u = tile / tiles_per_unit,
  * r = tile % tiles_per_unit, contributors c = 0 .. c_last - c_first with c_first = u nkb / units_per_cta,
  * c_last = ((u + 1) nkb - 1) / units_per_cta:  partial[(((u max_contrib + c) tiles_per_unit + r) tn + t) 128 + n % 128].
  * gate|up layout (half_tiles > 0): unit u holds tiles (u, u + half_tiles) as r = 0, 1. */

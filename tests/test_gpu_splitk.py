@@ -152,3 +152,17 @@ def test_silu_consumes_f16_partials(ops):
     w = (torch.randn(2 * I, K, generator=g) * 0.05).half().to(DEV)
     parts = ops.gemm_f16_deferred(x, w)
     assert torch.equal(ops.splitk_silu_mul(parts), ops.silu_mul(ops.splitk_reduce(parts)))
+
+
+@pytest.mark.parametrize("T,N,K,gs", W4_DEFERRED)
+def test_deferred_and_ordinary_differ_by_rounding_only(ops, T, N, K, gs):
+    """they may cut k elsewhere (up to eight tokens another kernel does): fp32 sums of K products each, off by K 2^-24 of the sum of their absolute values at the
+    most, and a rounding to fp16 each"""
+    x, qw, qz, sc, _, _ = _w4(T, N, K, gs, T + N + K)
+    x, packed, w16 = x.to(DEV), ops.gptq_pack(qw.to(DEV), qz.to(DEV), sc.to(DEV), gs), (torch.randn(N, K, generator=torch.Generator().manual_seed(T)) * 0.05).half().to(DEV)
+    w4 = ogptq.dequantize(qw, qz, sc, None, gs).to(DEV)
+    for a, b, w in ((ops.splitk_reduce(ops.gemm_w4a16_deferred(x, packed, N, gs)), ops.gemm_w4a16(x, packed, N, gs), w4),
+                    (ops.splitk_reduce(ops.gemm_f16_deferred(x, w16)), ops.gemm_f16(x, w16), w16.t())):
+        a, b = a.double(), b.double()
+        size = x.double().abs() @ w.double().abs()
+        assert bool(((a - b).abs() <= 2.0 ** -10 * torch.maximum(a.abs(), b.abs()) + 2 * K * 2.0 ** -24 * size).all())

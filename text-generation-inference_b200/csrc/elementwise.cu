@@ -18,7 +18,7 @@ namespace b200 {
 // ------------------------------------------------------------------------------------------------
 // residual-add + RMSNorm.  One CTA per token row; 8 halves (16 B) per thread per iteration.
 // fp32 statistics on the un-rounded sum.
-// Optional split-K input: a deferred GEMM output arrives as fp32 partials; they are summed and rounded to fp16 first, which is exactly the GEMM's fp16 output.
+// Optional split-K input: a deferred GEMM output arrives as fp32 partials; they are summed and rounded to fp16 first, as splitk_reduce_kernel does.
 // Bound: in a decoding step the latency of loads that wait for one another, so weights, residual and the first
 // partials are in flight at once and the row stays in registers; in a prompt memory, so CTAs are as large as the row needs.  The sums
 // go by thread, warp and warp 0 in the same order for any number of threads (those that a short row lacks would add zeros).

@@ -983,8 +983,8 @@ extern "C" int b200_gemm_w4a16(const void* x, const void* packed, const void* bi
 }
 // Deferred split-K reduction: the GEMM leaves fp32 partials in `workspace` and fills *splitk; the next kernel of the stream
 // (b200_rmsnorm_residual_splitk, b200_rope_kv_write_paged_splitk, b200_splitk_silu_mul, b200_splitk_reduce, the fused all-reduce)
-// sums them in contributor order - bit-identical to b200_gemm_w4a16_ex's own fix-up, without its grid-wide wait.  The bias is
-// applied by the consumer.  T <= 128.
+// sums them in contributor order, without the grid-wide wait of b200_gemm_w4a16_ex's own fix-up and equal to its result up to the order of the fp32 sums
+// (up to eight tokens that has a kernel with other cuts of k).  The bias is applied by the consumer.  T <= 128.
 extern "C" int b200_gemm_w4a16_deferred(const void* x, const void* packed, const void* bias, int64_t T, int64_t N, int64_t K,
                                         int groupsize, int layout, void* workspace, B200SplitK* splitk, void* stream) {
   if (!splitk) { b200_set_last_error("gemm_w4a16_deferred: splitk is NULL"); return B200_ERR_ARG; }

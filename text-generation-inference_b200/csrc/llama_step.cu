@@ -5,7 +5,7 @@
 // (server/text_generation_server/models/custom_modeling/flash_llama_modeling.py:425-497, 356-389, 240-297,
 // 332-335) and FlashLlamaForCausalLM.forward (:514-540) over the kernels of this library.
 //
-// Two things move between kernels at decode sizes (T <= 128), without changing any result bit:
+// Two things move between kernels at decode sizes (T <= 128), without changing a result by more than the order of fp32 sums:
 //   * deferred split-K (s->defer_splitk): a linear leaves its K-slices' fp32 partials in the workspace and the kernel that
 //     consumes its output anyway (residual + RMSNorm, RoPE + KV write, SiLU * up) sums them while it reads - the GEMM no longer
 //     waits for its slowest CTA and re-reads the partials itself (include/b200_tgis.h "B200SplitK");
