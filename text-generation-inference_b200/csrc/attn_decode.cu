@@ -40,10 +40,8 @@ struct DecodeSmem {
 };
 
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr, uint32_t rank) {
-  uint32_t a;
   float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_map(addr, rank)) : "memory");
   return v;
 }
 

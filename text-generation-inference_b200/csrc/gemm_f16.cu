@@ -99,8 +99,8 @@ __device__ __forceinline__ void f16_cluster_sum(const F16Params& p, const float*
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         if (c + j < d) {
-          const uint32_t a = cluster_map(at, c + j);
-          asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[j][0]), "=f"(v[j][1]), "=f"(v[j][2]), "=f"(v[j][3]) : "r"(a) : "memory");
+          const float4 four = ld_cluster_v4(at, c + j);
+          v[j][0] = four.x; v[j][1] = four.y; v[j][2] = four.z; v[j][3] = four.w;
         } else {
           v[j][0] = v[j][1] = v[j][2] = v[j][3] = 0.f;
         }
@@ -372,21 +372,7 @@ static const int* f16_clusters() {
       constexpr auto kernel = gemm_f16_kernel<64, 0>;
       constexpr int smem = GemmF16Cfg<64>::kSmemBytes;
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-      for (int d = 2; d <= 8; ++d) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(d * 16));
-        cfg.blockDim = dim3(kGemmThreads);
-        cfg.dynamicSmemBytes = smem;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)d;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int v;
-        if (cudaOccupancyMaxActiveClusters(&v, kernel, &cfg) == cudaSuccess) n[d] = v;
-      }
-      cudaGetLastError();
+      b200_count_clusters(kernel, kGemmThreads, smem, n);
     }
   } table;
   return table.n;

@@ -91,11 +91,6 @@ struct PairParams {
   unsigned* gave_up;            // b200_gave_up_word
 };
 
-__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));

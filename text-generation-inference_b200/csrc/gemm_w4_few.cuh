@@ -43,13 +43,6 @@ __device__ __forceinline__ void few_ld(uint4& v, const unsigned char* p, uint64_
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p), "l"(policy));
 }
-__device__ __forceinline__ float4 few_ld_cluster(uint32_t addr, uint32_t rank) {
-  uint32_t a;
-  float4 v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
-  return v;
-}
 
 // kGR: meta rows per unit record
 template <int kGR>
@@ -166,7 +159,7 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemm_w4_few_kernel(const W4Few
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int o = 0; o < 2; ++o)
-          v[i][o] = c + i < d ? few_ld_cluster(base + ((o * 8 + tok) * kFewPitch + f) * 4, c + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+          v[i][o] = c + i < d ? ld_cluster_v4(base + ((o * 8 + tok) * kFewPitch + f) * 4, c + i) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -215,22 +208,9 @@ __global__ void __launch_bounds__(kFewThreads, 1) gemm_w4_few_kernel(const W4Few
 static const int* few_clusters() {
   static const struct Table {
     int n[9];
-    Table() {
+    Table() : n{} {
       n[0] = n[1] = b200_num_sms();
-      for (int d = 2; d <= 8; ++d) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(d * 16));
-        cfg.blockDim = dim3(kFewThreads);
-        cfg.dynamicSmemBytes = few_smem(kFewMostBlocks);
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)d;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        if (cudaOccupancyMaxActiveClusters(&n[d], gemm_w4_few_kernel<1>, &cfg) != cudaSuccess) n[d] = 0;
-      }
-      cudaGetLastError();
+      b200_count_clusters(gemm_w4_few_kernel<1>, kFewThreads, few_smem(kFewMostBlocks), n);
     }
   } table;
   return table.n;
