@@ -41,9 +41,11 @@ constexpr int kGemmThreads = 192;
 constexpr int kTileM = 128;  // features per tile
 constexpr int kTileK = 64;   // fp16 elements per k-block = one 128-byte swizzle row
 // Calls of more than kF16DecodeT tokens may go to the SM pairs (gemm_pair.cuh), calls of more than kF16MostT all do; between the two f16_stream_us
-// says which kernel takes less.  Measured on B200 (us, this kernel / pairs) at 65 tokens: 4096 -> 4096 16.1 / 13.0, 4096 -> 22016 42.2 / 40.0, 5632 -> 2048
-// 16.8 / 15.0, 11008 -> 4096 25 / 29, 16384 -> 2048 25 / 38, 28672 -> 2048 32 / 63, 28672 -> 8192 81 / 93; at 128: 20.8 / 13.5, 45.5 / 41.8, 24.6 / 15.0, 30 / 29,
-// 32 / 38, 39 / 63, 86 / 94; at 256: 33.5 / 15.6, 68 / 50, 44 / 15, 44 / 36, 51 / 38, 61 / 61; at 192 28672 -> 8192 110 / 100.
+// says which kernel takes less.  That model is of this kernel with its fix-up through global memory; where clusters share a tile it takes less, so the line lies
+// too far on the pairs' side of the narrower outputs.  Measured on B200 in replayed graphs (us, this kernel / pairs; * the other one is taken) at 65 tokens: 4096 ->
+// 4096 11.1 / 12.7*, 4096 -> 22016 38.8 / 38.8, 5632 -> 2048 11.0 / 16.1*, 11008 -> 4096 19.4 / 27.9, 16384 -> 2048 17.6 / 37.2, 28672 -> 2048 25.9 / 62.5, 28672 ->
+// 8192 78 / 94, 20480 -> 5120 42 / 59*, 2048 -> 2560 8.1 / 7.7; at 128: 12.3 / 12.9*, 45.0 / 41.3, 12.4 / 15.7*, 20.5 / 28.1, 19.0 / 37.5, 27.3 / 62.8, 93 / 111, 40 /
+// 62, 9.3 / 8.1; at 256: 16.0 / 15.1, 74 / 51, 15.8 / 15.8, 26.6 / 34.2*, 25.6 / 37.6*, 37.0 / 62.9, 143 / 129*, 54 / 66*, 12.8 / 9.2.
 // Up to 64 tokens the pairs take wide outputs only (feature tiles that no wave of clusters holds), from kF16PairT tokens on; us, this kernel / pairs, at 16
 // and 64 tokens: 2048 -> 11264 10.9 / 10.6 and 13.0 / 11.7, 2048 -> 32000 24.1 / 22.8 and 29.0 / 24.3, 4096 -> 12288 18.9 / 18.9 and 21.1 / 20.4, 5120 ->
 // 15360 25.8 / 26.6 and 28.4 / 28.4, 4096 -> 22016 (a wave and a sixth) 31.4 / 34.7 and 37.0 / 38.5.
@@ -408,7 +410,7 @@ static F16Plan plan_f16(int64_t T, int64_t N, int64_t K, int sms, bool defer = f
   return pl;
 }
 
-// Microseconds of a call of 65 to 256 tokens, a model of what was measured (kF16DecodeT): a 64-wide k-block of a 128-feature tile takes a CTA its own
+// Microseconds of a call of 65 to 256 tokens without clusters (the note on kF16DecodeT): a 64-wide k-block of a 128-feature tile takes a CTA its own
 // time or the memory's, whichever is longer, and the fix-up of a tile reads a partial of every contributor.
 static float f16_stream_us(const F16Plan& pl, int64_t T) {
   const int contrib = pl.units_per_cta % pl.nkb == 0 ? 1 : pl.nkb % pl.units_per_cta == 0 ? pl.nkb / pl.units_per_cta : pl.max_contrib;
