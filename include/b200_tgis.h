@@ -185,6 +185,9 @@ int64_t b200_gemm_workspace_bytes_max(int64_t N, int64_t K); /* max over all T: 
  * torch.mm in TensorParallelHead.forward (:257-262). */
 int b200_gemm_f16(const void* x, const void* w, const void* bias, void* y, int64_t T, int64_t N, int64_t K, void* workspace,
                   void* stream);
+/* the same for a w that b200_settle has settled and that has not been written since: its first tiles are read while the kernel before ends */
+int b200_gemm_f16_held(const void* x, const void* w, const void* bias, void* y, int64_t T, int64_t N, int64_t K, void* workspace,
+                       void* stream);
 /* bfloat16 operands (x [T, K], w [N, K], bias bfloat16 or NULL); y [T, N], out_kind 0: bfloat16, 1: fp32, 2: bfloat16 after relu(z)^2.  Same kernel
  * (tcgen05 kind::f16 with bfloat16 operand formats), workspace and rules as b200_gemm_f16. */
 int b200_gemm_bf16(const void* x, const void* w, const void* bias, void* y, int out_kind, int64_t T, int64_t N, int64_t K, void* workspace,
@@ -206,8 +209,9 @@ int b200_gptq_pack(const void* qweight, const void* qzeros, const void* scales, 
 #define B200_W4_LAYOUT_GATE_UP 1
 /* row_perm (int32 [K], device) or NULL: act-order checkpoints (non-trivial g_idx; exllamav2.py:31-48 q_perm): a stable
  * arg-sort of g_idx.  Packed row k' = checkpoint row row_perm[k']; feed the GEMM x[:, row_perm] (b200_permute_columns). */
-int b200_settle(void* stream); /* packed weights are read early: after records were written in any other way (a copy of them) than by b200_gptq_pack[_ex],
-                                * which does so itself, this launch has to stand between that and the first linear that reads them */
+/* Some linears read weights while the kernel before them ends: packed records, the w of the *_held entries and the weights of a B200LlamaWeights.  This launch has to
+ * stand between what wrote them and the first such linear; b200_gptq_pack[_ex] makes it itself. */
+int b200_settle(void* stream);
 int b200_gptq_pack_ex(const void* qweight, const void* qzeros, const void* scales, const int32_t* row_perm, void* packed,
                       int64_t K, int64_t N, int groupsize, int layout, void* stream);
 /* out[t, k'] = x[t, perm[k']], fp16 [T, K] */
@@ -241,6 +245,8 @@ int b200_gemm_w4a16_deferred(const void* x, const void* packed, const void* bias
                              int layout, void* workspace, B200SplitK* splitk /* host, out */, void* stream); /* T <= 128 */
 int b200_gemm_f16_deferred(const void* x, const void* w, const void* bias, int64_t T, int64_t N, int64_t K, void* workspace,
                            B200SplitK* splitk /* host, out */, void* stream); /* T <= 256 */
+int b200_gemm_f16_deferred_held(const void* x, const void* w, const void* bias, int64_t T, int64_t N, int64_t K, void* workspace,
+                                B200SplitK* splitk /* host, out */, void* stream); /* w as for b200_gemm_f16_held */
 /* consumers.  y[T, N] fp16 = the GEMM's output (plain layout) */
 int b200_splitk_reduce(const B200SplitK* parts, void* y, void* stream);
 /* b200_rmsnorm_residual with h = the deferred GEMM output [T, H] (o_proj / down_proj, H = parts->N) */

@@ -67,3 +67,28 @@ def test_heads():
         ops_seq.linear_per_head(x, w, out)
         return out
     assert _differs(call, lambda i: torch.mul(a, 0.25 + i, out=w), 100) == 0
+
+
+@pytest.mark.parametrize("T", [1, 16, 64, 200])
+@pytest.mark.parametrize("K,N", [(4096, 4096), (2048, 11264), (512, 384)])
+def test_held_weights(T, K, N):
+    """the entries for weights that were settled: the bits of the plain ones, also right behind the launch that settles"""
+    import ctypes
+    import tgis_b200  # noqa: F401
+    from tgis_b200 import _lib, ops
+    g = torch.Generator(device=DEV).manual_seed(T)
+    a, x = torch.randn(N, K, generator=g, device=DEV).half(), torch.randn(T, K, generator=g, device=DEV).half()
+    w, y, lib = torch.empty_like(a), torch.empty(T, N, dtype=torch.float16, device=DEV), _lib.load()
+    ws = ops.gemm_workspace(w.device, T, N, K)
+
+    def write(i):
+        torch.mul(a, 0.25 + i, out=w)
+        ops.settle()
+
+    def held():
+        _lib.check(lib.b200_gemm_f16_held(x.data_ptr(), w.data_ptr(), None, y.data_ptr(), T, N, K, ws.data_ptr(), ops._stream()), "held")
+        desc = _lib.B200SplitK()
+        _lib.check(lib.b200_gemm_f16_deferred_held(x.data_ptr(), w.data_ptr(), None, T, N, K, ws.data_ptr(), ctypes.byref(desc), ops._stream()), "held")
+        return torch.stack([y, ops.splitk_reduce(ops.SplitK(desc, ws, None))])
+    assert _differs(held, write, 20) == 0
+    assert torch.equal(held(), torch.stack([ops.gemm_f16(x, w), ops.splitk_reduce(ops.gemm_f16_deferred(x, w))]))

@@ -46,6 +46,7 @@ SIGNATURES = {
     "b200_gemm_workspace_bytes": (_L, [_L, _L, _L]),
     "b200_gemm_workspace_bytes_max": (_L, [_L, _L]),
     "b200_gemm_f16": (_I, [_P, _P, _P, _P, _L, _L, _L, _P, _P]),
+    "b200_gemm_f16_held": (_I, [_P, _P, _P, _P, _L, _L, _L, _P, _P]),
     "b200_gemm_bf16": (_I, [_P, _P, _P, _P, _I, _L, _L, _L, _P, _P]),
     "b200_p2p_handle_bytes": (_I, []),
     "b200_p2p_create": (_I, [_L, _I, _I, ctypes.POINTER(_P), _P]),
@@ -110,6 +111,7 @@ SIGNATURES.update({
     "b200_choose_tokens": (_I, [ctypes.POINTER(B200ChooserParams), _P]),
     "b200_gemm_w4a16_deferred": (_I, [_P, _P, _P, _L, _L, _L, _I, _I, _P, _KP, _P]),
     "b200_gemm_f16_deferred": (_I, [_P, _P, _P, _L, _L, _L, _P, _KP, _P]),
+    "b200_gemm_f16_deferred_held": (_I, [_P, _P, _P, _L, _L, _L, _P, _KP, _P]),
     "b200_splitk_reduce": (_I, [_KP, _P, _P]),
     "b200_rmsnorm_residual_splitk": (_I, [_KP, _P, _P, _P, _P, _F, _P]),
     "b200_rope_kv_write_paged_splitk": (_I, [_KP, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _P]),

@@ -76,6 +76,7 @@ struct F16Params {
   int total_units;
   int max_contrib;    // partial slots per tile
   int cluster;        // > 0: a cluster of so many CTAs has one feature tile, each a part of k
+  int held;           // 1: w was settled (b200_settle) and has not been written since
   int defer;          // 1: leave every tile segment as an fp32 partial for the consumer kernel (B200SplitK), no fix-up
 };
 
@@ -171,18 +172,33 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     // ------------------------------------------------------------------ TMA producer
     if (elect_one()) {
       const uint64_t pol_w = policy_evict_first(), pol_x = policy_evict_last();
-      // While the previous kernel ends, the first ring's weight tiles are on their way to L2; nothing of w is read before (it may be that kernel's result).  us in
+      // While the previous kernel ends, the first ring's weight tiles are on their way: held weights to shared memory; others to L2 only, since they
+      // may be that kernel's result.  us in
       // a replayed graph, tiles read ahead / only after the wait / brought to L2 ahead: one token 2048 -> 2560 5.4 / 5.7 / 5.65, 4096 -> 4096 8.65 / 9.6 /
       // 8.95, 11008 -> 4096 17.3 / 18.7 / 16.7, 2048 -> 32000 23.1 / 24.4 / 22.1; 32 tokens 4096 -> 4096 9.6 / 10.3 / 9.7, 4096 -> 22016 33.0 / 33.5 / 31.8.
       int tile = tile0, kb = kb0;
-      for (int i = 0; i < min(n_units, C::kStages); ++i) {
-        tma_prefetch_2d_hint(&tmap_w, kb * kTileK, tile * kTileM, pol_w);
+      const int npre = min(n_units, C::kStages);
+      for (int i = 0; i < npre; ++i) {
+        if (p.held) {
+          mbar_arrive_expect_tx(&full_bar[i], C::kStageBytes);
+          tma_load_2d_hint(smem + i * C::kStageBytes, &tmap_w, kb * kTileK, tile * kTileM, &full_bar[i], pol_w);
+        } else {
+          tma_prefetch_2d_hint(&tmap_w, kb * kTileK, tile * kTileM, pol_w);
+        }
         if (++kb == p.nkb) { kb = 0; ++tile; }
       }
       pdl_wait();
-      tile = tile0;
-      kb = kb0;
-      for (int i = 0; i < n_units; ++i) {
+      int from = 0;
+      if (p.held) {
+        for (int kbx = kb0; from < npre; ++from) {
+          tma_load_2d_hint(smem + from * C::kStageBytes + C::kABytes, &tmap_x, kbx * kTileK, 0, &full_bar[from], pol_x);
+          if (++kbx == p.nkb) kbx = 0;
+        }
+      } else {
+        tile = tile0;
+        kb = kb0;
+      }
+      for (int i = from; i < n_units; ++i) {
         const int s = i % C::kStages;
         mbar_wait(&empty_bar[s], ((i / C::kStages) & 1) ^ 1);
         mbar_arrive_expect_tx(&full_bar[s], C::kStageBytes);
@@ -509,7 +525,7 @@ static int f16_pieces(int64_t T, int64_t N, int64_t K, int sms) {
 
 template <int TN, int FMT>
 static int launch_gemm_f16(const CUtensorMap* mw, const CUtensorMap* mx, void* y, void* workspace, const void* bias, int T, int N,
-                           const F16Plan& pl, int cluster, int defer, cudaStream_t st) {
+                           const F16Plan& pl, int cluster, int held, int defer, cudaStream_t st) {
   using C = GemmF16Cfg<TN>;
   static bool configured = false;
   if (!configured) {
@@ -529,6 +545,7 @@ static int launch_gemm_f16(const CUtensorMap* mw, const CUtensorMap* mx, void* y
   p.total_units = pl.n_tiles_n * pl.nkb;
   p.max_contrib = pl.max_contrib;
   p.cluster = cluster;
+  p.held = held;
   p.defer = defer;
   const dim3 grid(cluster ? pl.n_tiles_n * cluster : pl.n_ctas);
   b200_timing_mark(B200_TIME_GEMM_F16, 0, st);
@@ -546,7 +563,7 @@ static int launch_gemm_f16(const CUtensorMap* mw, const CUtensorMap* mx, void* y
 // splitk != NULL: deferred reduction (see b200_gemm_w4a16_deferred): y is not written.
 template <int FMT>
 static int gemm_f16_impl(const void* x, const void* w, const void* bias, void* y, int64_t T, int64_t N, int64_t K, void* workspace,
-                         B200SplitK* splitk, void* stream) {
+                         B200SplitK* splitk, bool held, void* stream) {
   if (T == 0 || N == 0) return B200_OK;
   if (K % 8 != 0 || K < 64) { b200_set_last_error("gemm_f16: need K % 8 == 0 and K >= 64"); return B200_ERR_ARG; }
   const bool defer = splitk != nullptr;
@@ -591,27 +608,36 @@ static int gemm_f16_impl(const void* x, const void* w, const void* bias, void* y
   // eight tokens: 5632 -> 2048 6.9 / 7.5, 4096 -> 4096 9.0 / 9.3, 2048 -> 2048 5.1 / 5.2; fewer CTAs, 2048 -> 2560 5.6 / 5.5, 20480 -> 5120 42.3 / 35.2).
   if (T <= 8 && workspace && pl.nkb % pl.units_per_cta == 0 && pl.n_ctas >= pl.n_tiles_n * cluster) cluster = 0;
   switch (pl.TN) {
-    case 16: return launch_gemm_f16<16, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, df, st);
-    case 32: return launch_gemm_f16<32, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, df, st);
-    case 64: return launch_gemm_f16<64, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, df, st);
-    case 128: return launch_gemm_f16<128, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, df, st);
-    default: return launch_gemm_f16<256, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, df, st);
+    case 16: return launch_gemm_f16<16, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, held, df, st);
+    case 32: return launch_gemm_f16<32, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, held, df, st);
+    case 64: return launch_gemm_f16<64, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, held, df, st);
+    case 128: return launch_gemm_f16<128, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, held, df, st);
+    default: return launch_gemm_f16<256, FMT>(mw, mx, y, workspace, bias, (int)T, (int)N, pl, cluster, held, df, st);
   }
 }
 extern "C" int b200_gemm_f16(const void* x, const void* w, const void* bias, void* y, int64_t T, int64_t N, int64_t K,
                              void* workspace, void* stream) {
-  return gemm_f16_impl<0>(x, w, bias, y, T, N, K, workspace, nullptr, stream);
+  return gemm_f16_impl<0>(x, w, bias, y, T, N, K, workspace, nullptr, false, stream);
+}
+extern "C" int b200_gemm_f16_held(const void* x, const void* w, const void* bias, void* y, int64_t T, int64_t N, int64_t K,
+                                  void* workspace, void* stream) {
+  return gemm_f16_impl<0>(x, w, bias, y, T, N, K, workspace, nullptr, true, stream);
 }
 // bfloat16 x [T, K] and w [N, K] (bias bfloat16 or NULL) -> y [T, N]; out_kind 0: bfloat16, 1: fp32, 2: bfloat16 after the square of
 // ReLU.  Same kernel, workspace and rules as b200_gemm_f16.
 extern "C" int b200_gemm_bf16(const void* x, const void* w, const void* bias, void* y, int out_kind, int64_t T, int64_t N, int64_t K,
                               void* workspace, void* stream) {
-  if (out_kind == 2) return gemm_f16_impl<3>(x, w, bias, y, T, N, K, workspace, nullptr, stream);
-  if (out_kind == 1) return gemm_f16_impl<2>(x, w, bias, y, T, N, K, workspace, nullptr, stream);
-  return gemm_f16_impl<1>(x, w, bias, y, T, N, K, workspace, nullptr, stream);
+  if (out_kind == 2) return gemm_f16_impl<3>(x, w, bias, y, T, N, K, workspace, nullptr, false, stream);
+  if (out_kind == 1) return gemm_f16_impl<2>(x, w, bias, y, T, N, K, workspace, nullptr, false, stream);
+  return gemm_f16_impl<1>(x, w, bias, y, T, N, K, workspace, nullptr, false, stream);
 }
 extern "C" int b200_gemm_f16_deferred(const void* x, const void* w, const void* bias, int64_t T, int64_t N, int64_t K, void* workspace,
                                       B200SplitK* splitk, void* stream) {
   if (!splitk) { b200_set_last_error("gemm_f16_deferred: splitk is NULL"); return B200_ERR_ARG; }
-  return gemm_f16_impl<0>(x, w, bias, nullptr, T, N, K, workspace, splitk, stream);
+  return gemm_f16_impl<0>(x, w, bias, nullptr, T, N, K, workspace, splitk, false, stream);
+}
+extern "C" int b200_gemm_f16_deferred_held(const void* x, const void* w, const void* bias, int64_t T, int64_t N, int64_t K, void* workspace,
+                                           B200SplitK* splitk, void* stream) {
+  if (!splitk) { b200_set_last_error("gemm_f16_deferred_held: splitk is NULL"); return B200_ERR_ARG; }
+  return gemm_f16_impl<0>(x, w, bias, nullptr, T, N, K, workspace, splitk, true, stream);
 }

@@ -12,6 +12,7 @@
 //   * the tensor-parallel layer boundary (s->p2p_norm): all-reduce over NVLink peer memory + residual + RMSNorm in one
 //     kernel (b200_p2p_allreduce_rmsnorm), fed directly by the row-parallel linear's partials.  The whole sharded step is then
 //     one C call like the single-rank one; without a window the caller all-reduces `hidden` (NCCL) between the block calls.
+// The weights are held: B200LlamaWeights says what its caller has seen to (include/b200_tgis.h).
 #include "common.cuh"
 #include "../../include/b200_tgis.h"
 
@@ -30,7 +31,7 @@ static int linear(const B200Linear* L, const B200LlamaStep* s, const void* x, vo
     if (st != B200_OK) return st;
     return b200_gemm_w4a16_ex(x, L->qweight, L->bias, y, T, L->N, L->K, L->groupsize, L->layout, 0, s->gemm_ws, stream);
   }
-  return b200_gemm_f16(x, L->weight, L->bias, y, T, L->N, L->K, s->gemm_ws, stream);
+  return b200_gemm_f16_held(x, L->weight, L->bias, y, T, L->N, L->K, s->gemm_ws, stream);
 }
 
 // same linear with its split-K reduction left to the consumer of *parts (the next kernel enqueued on the stream)
@@ -40,7 +41,7 @@ static int linear_deferred(const B200Linear* L, const B200LlamaStep* s, const vo
     if (st != B200_OK) return st;
     return b200_gemm_w4a16_deferred(x, L->qweight, L->bias, T, L->N, L->K, L->groupsize, L->layout, s->gemm_ws, parts, stream);
   }
-  return b200_gemm_f16_deferred(x, L->weight, L->bias, T, L->N, L->K, s->gemm_ws, parts, stream);
+  return b200_gemm_f16_deferred_held(x, L->weight, L->bias, T, L->N, L->K, s->gemm_ws, parts, stream);
 }
 
 static bool deferring(const B200LlamaStep* s) { return s->defer_splitk && s->gemm_ws && s->T <= 128 && !s->is_prefill; }

@@ -20,6 +20,7 @@ import torch.distributed
 from torch import nn
 
 from ... import _lib
+from ...utils import _ops
 from ...utils.layers import (
     FastLinear,
     LinearScalingPositionRotaryEmbedding,
@@ -247,6 +248,7 @@ class FlashLlamaForCausalLM(nn.Module):
         w.final_norm = m.norm.weight.data_ptr()
         w.lm_head, w.vocab_rows_head = head.weight.data_ptr(), head.weight.shape[0]
         w.rope_cos, w.rope_sin = cos.data_ptr(), sin.data_ptr()
+        _ops().settle()   # steps read the weights early; whoever writes them in place later does the same
         self._cw_keep = (arr, cos, sin)
         self._cw = w
         return w
