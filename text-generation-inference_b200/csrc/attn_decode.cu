@@ -14,8 +14,8 @@
 //     each merge a share of the outputs through distributed shared memory.  More chunks: partials -> fp32 workspace, merged by attn_decode_combine_kernel
 // The kernel is bandwidth-bound: algorithmic bytes = 2 * L * d * 2 B per (sequence, kv head).
 // Measured on B200, us in a replayed graph, 32 / 8 heads of 128 (a second kernel merges always / as here): 1 x 16 tokens 3.9 / 2.65, 64 x 16 - 32 8.3 / 5.9, 64 x
-// 256 - 512 (one run each) 24.5 / 22.0, 1 x 1024 6.4 / 5.2, 8 x 256 - 512 7.2 / 5.7, 4 x 2048 - 4096 13.7 / 12.5; 64 x 1024 - 2048, where it still does, 72.1 -> 70.0
-// since all its loads are in flight at once.
+// 256 - 512 (one run each) 24.5 / 22.0, 1 x 1024 6.4 / 5.2, 8 x 256 - 512 7.2 / 5.7, 4 x 2048 - 4096 13.7 / 12.5; 64 x 1024 - 2048, where it still does, 71.4 -> 70.5
+// with all its loads in flight at once (runs of one side differ by as much).
 #include "common.cuh"
 
 #include <cstdlib>

@@ -769,6 +769,9 @@ constexpr int kTalkPromptTokens = 24;  // average tokens per sequence from which
 // B200.  Us, m16n8k16 / this one, no chunk, no window: 16 / 4 heads of 128, 24 tokens behind 2000 keys 56 / 51, behind 30 000 454 / 475, 200 behind 8000 181 /
 // 145; 8 / 2 heads of 64, 24 behind 500 36 / 27, 64 behind 8000 77 / 141, 500 behind 8000 103 / 150; 16 / 8 heads of 64, 24 x 16 sequences behind 4000 108 / 127, a
 // prompt of 4000 beside 100 single tokens behind 1500 527 / 248.
+// (The first of each pair was measured in at most kTalkModelRuns runs of keys, with queries ahead of the first keys.  In up to 32 runs that kernel takes less - 32 tokens
+// behind 1000 keys, 16 / 4 heads of 128, 30.4 where this one is taken and takes 33.1 - so the line lies on this one's side.)
+constexpr int kTalkModelRuns = 8;
 static bool talk_prompt_pays(int64_t T, int B, int H, int G, int d, int dv, int64_t keys, int QT, int nsplit) {
   const int tokens = 128 / (H / G), sms = b200_num_sms();
   const int64_t row = 2ll * G * (d + dv), single = G * (T / tokens + B), items = single <= sms ? single : G * (T / (2 * tokens) + B);
@@ -857,7 +860,7 @@ extern "C" int b200_seq_talk_attn(const float* q, const void* cache, int dt, int
   if (!partial || nsplit < 1) nsplit = 1;
   if (nsplit > kTalkMaxSplit) nsplit = kTalkMaxSplit;
   if (talk_prompt_route(q, cache, dt, row_width, k_off, v_off, cu_q, talk, out, T, B, H, G, d, dv, page, bt_stride, chunk, window,
-                        nsplit < 8 ? nsplit : 8)) {
+                        nsplit < kTalkModelRuns ? nsplit : kTalkModelRuns)) {
     if (d == 128)
       return launch_talk_prompt<128>(q, cache, row_width, k_off, v_off, block_table, bt_stride, cu_q, B, position_ids, out, T, H, G, chunk, window, scale, sink, st);
     return launch_talk_prompt<64>(q, cache, row_width, k_off, v_off, block_table, bt_stride, cu_q, B, position_ids, out, T, H, G, chunk, window, scale, sink, st);
