@@ -83,6 +83,11 @@ def test_more_items_than_sms():
     _run([25 + 13 * (i % 7) for i in range(60)], [17 * (i % 5) for i in range(60)], 16, 8, 64, chunk=128, seed=7)
 
 
+def test_long_items_and_short_ones_in_turn():
+    _run([1500, 1, 700, 130, 40, 900], 0, 16, 4, 64, seed=13)   # items of one key tile and of many, several to a block
+    _run([300] * 9 + [1], [0, 900] * 5, 8, 8, 64, chunk=512, seed=14)
+
+
 def test_maxima_that_leap():
     _run([700], 0, 4, 2, 128, key_scale=6.0, seed=8)
 

@@ -51,7 +51,12 @@ constexpr int kPfSlabBytes = 128 * 128;  // 128 rows x 64 halves
 constexpr int kPfPageSlabBytes = kPageTokens * 128;
 constexpr int kPfCornerBytes = 32 * 128;  // a softmax warp's rows on their way out
 constexpr int kPfStages = 2;
-constexpr int kPfAhead = 2;      // items that are known ahead
+// Items that can be known ahead (of short ones the copies are up to two in front of the soft-max).  A block asks for the next one as the copies of its item
+// come to its last kPfAskTiles key tiles: late, so that a long item is not left to a block that still has one while other SMs are idle, and early enough that
+// the answer, and blocks without a tile among the answers, hide behind the products.  Blocks that asked as soon as there was room took three further items
+// each as they started (us, that / this: hybrid prompts of 1618 and 2000 tokens, 16 / 4 heads, SMs busy for 60 % of the time 100 / 76; 6 prompts of 310 to 536, 32 / 32
+// heads 44 / 38; 8 of 100 to 1000, 32 / 4 heads of 64, 64 / 53).
+constexpr int kPfAhead = 2, kPfAskTiles = 2;
 // Registers per thread: the launch has 384 x 168; the two softmax warpgroups take 200 each, the other one keeps 104.  216 and 72, with O rescaled in 64
 // columns at a time instead of 16, spilled in both (us, flushed L2, that / this: 13 prompts of 300 to 2048 tokens, 32 / 8 heads, d = 128 246 / 225; hybrid
 // prompts of 1618 and 2000 tokens, 16 / 4 heads 109 / 100; 6 portions of 300 to 600 behind 700 keys, 40 / 40 heads 115 / 101).
@@ -61,7 +66,7 @@ template <int D>
 struct PfCfg {
   static constexpr int kSlabs = D / 64;
   static constexpr int kTileBytes = kSlabs * kPfSlabBytes;  // a Q, K or V tile
-  static constexpr int kNumBars = 2 + 4 * kPfStages + 8 + 2 * kPfAhead + 1;    // q_full, q_empty | k_full, k_empty, v_full, v_empty | s_full[2], p_ready[2][2 halves], o_full[2]
+  static constexpr int kNumBars = 2 + 4 * kPfStages + 8 + 2 * kPfAhead + 2;    // q_full, q_empty | k_full, k_empty, v_full, v_empty | s_full[2], p_ready[2][2 halves], o_full[2]
   static constexpr int kSmemBytes = (2 + 2 * kPfStages) * kTileBytes + 8 * kPfCornerBytes + kNumBars * 8 + 16 + 1024;
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
   static constexpr int kTmemCols = 512;  // S0 [0,128) | S1 [128,256) | O0 [256, 256 + D) | O1 behind it
@@ -250,7 +255,8 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   uint64_t* next_full = o_full + 2;
   uint64_t* next_empty = next_full + kPfAhead;
   uint64_t* taken = next_empty + kPfAhead;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(taken + 1);
+  uint64_t* ask = taken + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ask + 1);
   __shared__ __align__(16) uint32_t s_resp[4];
   __shared__ int s_next[kPfAhead];
 
@@ -279,6 +285,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       mbar_init(&next_empty[s], 10);  // producer, issuer, eight softmax warps
     }
     mbar_init(taken, 1);
+    mbar_init(ask, 1);
     mbar_fence_init();
   }
   if (warp == 2) tmem_alloc<C::kTmemCols>(tmem_slot);
@@ -306,7 +313,10 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       int st = 0, ph = 1, qph = 1;
       for (int i = blockIdx.x; i >= 0; i = next_item()) {
         const PfItem it = pf_item<TOKEN_MAJOR>(p, i);
-        if (it.n == 0) continue;  // only the block's own item can be empty
+        if (it.n == 0) {  // only the block's own item can be empty
+          if (lane == 0) mbar_arrive(ask);
+          continue;
+        }
         if constexpr (!TOKEN_MAJOR) mbar_wait_soft(q_empty, qph, ok);  // the previous item's last Q K^T
         qph ^= 1;
         if (!TOKEN_MAJOR && lane == 0) {
@@ -318,6 +328,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         }
         const int32_t* bt = p.block_table + (int64_t)it.b * p.bt_stride;
         for (int j = it.j0; j < it.n; ++j) {
+          if (lane == 0 && j == max(it.j0, it.n - kPfAskTiles)) mbar_arrive(ask);
           // 8 pages of this key tile, a lane each
           int page = j * (kPfN / kPageTokens) + (lane & 7), row;
           if constexpr (TOKEN_MAJOR) {
@@ -446,7 +457,7 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     } else if (warp == 3) {
       // ------------------------------------------------------------------ scheduler: after the block's own item those of blocks that have not
       // started, as long as there are any; items without a tile are passed over here
-      int slot = 0, ph = 1, tph = 0;
+      int slot = 0, ph = 1, tph = 0, aph = 0;
       auto publish = [&](int i) {
         mbar_wait_soft(&next_empty[slot], ph, ok);
         if (lane == 0) {
@@ -455,13 +466,15 @@ attn_prompt_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         }
         if (++slot == kPfAhead) { slot = 0; ph ^= 1; }
       };
-      while (p.more_blocks) {
-        int i = -1;
-        if (lane == 0) i = take_block(s_resp, taken, tph, ok);
-        tph ^= 1;
-        i = __shfl_sync(0xffffffffu, i, 0);
-        if (i < 0) break;
-        if (pf_item<TOKEN_MAJOR>(p, i).n > 0) publish(i);
+      for (int i = 0; p.more_blocks && i >= 0;) {
+        mbar_wait_soft(ask, aph, ok);
+        aph ^= 1;
+        do {
+          if (lane == 0) i = take_block(s_resp, taken, tph, ok);
+          tph ^= 1;
+          i = __shfl_sync(0xffffffffu, i, 0);
+        } while (i >= 0 && pf_item<TOKEN_MAJOR>(p, i).n == 0);
+        if (i >= 0) publish(i);
       }
       publish(-1);
     }
