@@ -88,6 +88,12 @@ def test_long_items_and_short_ones_in_turn():
     _run([300] * 9 + [1], [0, 900] * 5, 8, 8, 64, chunk=512, seed=14)
 
 
+@pytest.mark.parametrize("past,window,chunk", [(0, 33, 0), (31, 64, 0), (65, 95, 0), (96, 0, 160), (33, 130, 288)])
+def test_borders_inside_a_key_tile(past, window, chunk):
+    _run([33, 97, 160, 1], past, 8, 2, 64, chunk=chunk, window=window, seed=15)
+    _run([130, 63], past, 16, 1, 128, chunk=chunk, window=window, seed=16)
+
+
 def test_maxima_that_leap():
     _run([700], 0, 4, 2, 128, key_scale=6.0, seed=8)
 

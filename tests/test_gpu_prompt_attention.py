@@ -136,3 +136,10 @@ def test_the_largest_weight_is_exact(spread):
         best = (rounded @ V[:, h * G // H] / rounded.sum(1, keepdim=True)).half().double()
         got, must = got + float((out[:, h].double() - ref).square().sum()), must + float((best - ref).square().sum())
     assert (got / must) ** 0.5 < 1.005, (got / must) ** 0.5
+
+
+@pytest.mark.parametrize("past", [0, 1, 31, 32, 33, 95, 127])
+def test_borders_inside_a_key_tile(past):
+    """the mask is looked at 32 keys at a time"""
+    _run([1, 31, 32, 33, 63, 65, 97, 127, 160], past, 4, 2, 64, 0.125, seed=6 + past)
+    _run([97, 129, 33], past, 4, 2, 128, 128 ** -0.5, seed=6 + past)

@@ -832,6 +832,7 @@ static int launch_talk_prompt(const float* q, const void* cache, int64_t RW, int
   p.chunk = chunk;
   p.window = window;
   p.rep = H / G;
+  p.log2_rep = __builtin_ctz(p.rep);
   p.tokens = 128 / p.rep;
   p.n_units = G;
   p.pair = G * (T / p.tokens + B) <= b200_num_sms() ? b200::kPfSingle : b200::kPfTiles;
