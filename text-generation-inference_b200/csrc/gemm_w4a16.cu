@@ -22,13 +22,13 @@
 //   warp 22       TMA: unit records -> 12..16-deep (8 at TN = 128) weight ring; starts before the CTA set-up barrier.
 //                 Only these bytes come from HBM.
 //   warp 23       TMA: one activation tile [TN x 128] fp16 (two 128B-swizzled sub-tiles) per super-unit -> 6-deep ring
-//                 (L2 hits); also watches the tiles land and counts them into s_ready
+//                 (L2 hits); it lands on the super-unit's own barrier
 //   warps 4..19   dequant: 4 teams x 4 warps; team = unit index mod 4, warp = TMEM lane quarter, thread = one feature row x
 //                 all 128 k of the unit (16 words).  Per 8 weights: 4 LOP3 + SHF (magic-number fp16: 1024 + q / 64 + q),
 //                 4 HADD2 (exact q - zero), 4 HMUL2 (x scale: bit-identical to the formula of record) -> tcgen05.st into a
-//                 ring of A-operand tiles in TMEM (64 columns each), counted into s_ready.  Teams run on their own clocks.
-//   warps 20, 21  MMA issue, alternate super-units: poll s_ready (one shared-memory word per super-unit), wait for the
-//                 turn (s_issued), 16 x tcgen05.mma.kind::f16 (A from TMEM, B from shared memory), ONE tcgen05.commit that
+//                 ring of A-operand tiles in TMEM (64 columns each), an arrival at the super-unit's barrier.  Teams run on their own clocks.
+//   warps 20, 21  MMA issue, alternate super-units: wait for the super-unit's barrier (its activation tile and the 8 team-warp
+//                 quarters of its two A tiles), then for the turn, 16 x tcgen05.mma.kind::f16 (A from TMEM, B from shared memory), ONE tcgen05.commit that
 //                 frees the activation stage and both A stages
 //   warps 0..3    epilogue: tcgen05.ld of a finished super-tile, then fp16 store / fused SiLU(gate) * up store / fp32
 //                 partial store when the super-tile is shared with other CTAs; they sleep while they wait
@@ -86,7 +86,7 @@ struct GemmW4Cfg {
   static constexpr int kXStageBytes = 2 * kXSubBytes;
   static constexpr int kXStages = TN >= 128 ? 4 : 6;           // activation ring (per super-unit = kW4R units)
   static constexpr int kWStages = TN >= 128 ? 8 : (TN == 64 ? 12 : 16);
-  static constexpr int kNumBars = 2 * kWStages + kXStages + kSuRing + 4;
+  static constexpr int kNumBars = 2 * kWStages + 2 * kXStages + kSuRing + 6;
   static constexpr int kSmemBytes = kXStages * kXStageBytes + kWStages * kW4RecMaxBytes + kNumBars * 8 + 16 + 1024;
   static_assert(kABase + kAStages * kW4AColsPerStage <= kTmemCols, "TMEM budget");
   // a team observes every phase of the weight stages it uses only if a stage always belongs to the same team
@@ -97,14 +97,6 @@ struct GemmW4Cfg {
   static_assert(TN * kW4SumPitch * 4 <= kXStages * kXStageBytes + kWStages * kW4RecMaxBytes, "the last super-tile's sums lie where the rings were");
 };
 
-__device__ __forceinline__ uint32_t lds_acquire_cta(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");
-  return v;
-}
-__device__ __forceinline__ void red_release_cta_shared_inc(uint32_t* p) {
-  asm volatile("red.release.cta.shared::cta.add.u32 [%0], 1;" ::"r"(smem_u32(p)) : "memory");
-}
 __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -190,17 +182,13 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
   unsigned char* w_ring = smem + C::kXStages * C::kXStageBytes; // 1024-aligned stages
   uint64_t* full_w = reinterpret_cast<uint64_t*>(w_ring + C::kWStages * kW4RecMaxBytes);
   uint64_t* empty_w = full_w + C::kWStages;
-  uint64_t* full_x = empty_w + C::kWStages;
-  uint64_t* su_done = full_x + C::kXStages;     // [kSuRing] MMA commit of super-unit j -> barrier j % kSuRing: its x stage and its A stages are free
+  uint64_t* su_full = empty_w + C::kWStages;    // [kXStages] super-unit j's inputs are there, its activation tile and the 8 team-warp quarters of its two A tiles
+  uint64_t* x_empty = su_full + C::kXStages;    // [kXStages] the MMAs that read the stage's activation tile have completed
+  uint64_t* su_done = x_empty + C::kXStages;    // [kSuRing] MMA commit of super-unit j -> barrier j % kSuRing: its x stage and its A stages are free
   uint64_t* tmem_full = su_done + C::kSuRing;   // [2]
   uint64_t* tmem_empty = tmem_full + 2;         // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
-  // Inputs of super-unit j (its activation tile + the 8 team-warp quarters of its two A tiles) are counted in
-  // s_ready[j % 8]; the MMA warp polls that word with plain shared-memory loads.  (In the warp that issues tcgen05.mma
-  // every dependent wait costs > 100 cycles during which the tensor pipe drains so it gets
-  // exactly one per 16 MMAs.)  Monotonic: super-unit j is ready at 9 * (j / 8 + 1).
-  __shared__ uint32_t s_ready[8];
-  __shared__ uint32_t s_issued;  // super-units whose MMAs have been issued (hand-over between the two MMA warps)
+  uint64_t* turn = tmem_empty + 2;              // [2] hand-over between the two MMA warps
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(turn + 2);
   __shared__ int s_fix[2][3];  // super-tiles this CTA shares with others: {super-tile, contributors, my index}
   __shared__ int s_nfix;
   __shared__ int s_whole;      // the last super-tile if this CTA has it alone: all threads finish it; -1: none
@@ -247,14 +235,16 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
   }
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmap_x);
-    for (int s = 0; s < C::kXStages; ++s) mbar_init(&full_x[s], 1);
+    for (int s = 0; s < C::kXStages; ++s) {
+      mbar_init(&su_full[s], 1 + 8);
+      mbar_init(&x_empty[s], 1);
+    }
     for (int b = 0; b < C::kSuRing; ++b) mbar_init(&su_done[b], 1);
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tmem_full[b], 1);
       mbar_init(&tmem_empty[b], kW4EpWarps);
+      mbar_init(&turn[b], 1);
     }
-    for (int i = 0; i < 8; ++i) s_ready[i] = 0;
-    s_issued = 0;
     s_nfix = 0;
     s_whole = -1;
     mbar_fence_init();
@@ -283,44 +273,19 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
     }
   } else if (warp == kW4XProdWarp) {
     // ------------------------------------------------------------------ TMA producer: activations (L2 resident),
-    // one [TN x 128] tile per super-unit; the same thread watches the tiles land and counts them into s_ready
+    // one [TN x 128] tile per super-unit; the stage of super-unit j takes the tile of super-unit j + kXStages once the MMAs of j have completed
     if (elect_one()) {
       const uint64_t pol_x = policy_evict_last();
-      int kb = kb0;
-      auto load_x = [&](int s) {
-        mbar_arrive_expect_tx(&full_x[s], C::kXStageBytes);
-        unsigned char* st = x_ring + s * C::kXStageBytes;
-        tma_load_2d_hint(st, &tmap_x, kb * kW4BlockK, 0, &full_x[s], pol_x);
-        tma_load_2d_hint(st + C::kXSubBytes, &tmap_x, kb * kW4BlockK + 64, 0, &full_x[s], pol_x);
-        if (++kb == p.nkb) kb = 0;
-      };
+      int kb = kb0, s = 0, ph = 1;
       pdl_wait();  // x is the previous kernel's output; the weight ring is already streaming
-      for (int j = 0; j < C::kXStages && j < n_su; ++j) load_x(j);
-      // two independent duties, both polled without blocking: count landed tiles into s_ready (in order), and refill the
-      // stage of super-unit j with the tile of super-unit j + kXStages once the MMAs of j have completed
-      int nj = 0, ns = 0, nph = 0;  // next tile to report: index, stage, parity
-      int rj = 0, rs = 0, rb = 0, rph = 0;  // next super-unit whose stage is refilled: index, stage, su_done barrier, parity
-      const int n_refill = n_su - C::kXStages;
-      uint32_t idle = 0;
-      while (nj < n_su) {
-        bool progress = false;
-        if (mbar_test_wait(&full_x[ns], nph)) {
-          red_release_cta_shared_inc(&s_ready[nj & 7]);
-          ++nj;
-          if (++ns == C::kXStages) { ns = 0; nph ^= 1; }
-          progress = true;
-        }
-        if (rj < n_refill && rj < nj && mbar_test_wait(&su_done[rb], rph)) {
-          load_x(rs);
-          ++rj;
-          if (++rs == C::kXStages) rs = 0;
-          if (++rb == C::kSuRing) { rb = 0; rph ^= 1; }
-          progress = true;
-        }
-        if (!progress) {
-          __nanosleep(20);
-          if (++idle > (1u << 26)) __trap();
-        }
+      for (int j = 0; j < n_su; ++j) {
+        mbar_wait(&x_empty[s], ph);
+        mbar_arrive_expect_tx(&su_full[s], C::kXStageBytes);
+        unsigned char* st = x_ring + s * C::kXStageBytes;
+        tma_load_2d_hint(st, &tmap_x, kb * kW4BlockK, 0, &su_full[s], pol_x);
+        tma_load_2d_hint(st + C::kXSubBytes, &tmap_x, kb * kW4BlockK + 64, 0, &su_full[s], pol_x);
+        if (++kb == p.nkb) kb = 0;
+        if (++s == C::kXStages) { s = 0; ph ^= 1; }
       }
     }
   } else if (warp == kW4MmaWarp || warp == kW4MmaWarp + 1) {
@@ -328,7 +293,8 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
     // queue is shallow, so a warp that has just issued 16 MMAs cannot hide its own bookkeeping (barrier polls, commit)
     // behind them: the tensor pipe would idle ~40 % of the time.  Two warps take alternate
     // super-units; while one is blocked issuing, the other has already found its inputs ready and only waits for its turn
-    // (s_issued), so MMAs reach the pipe back to back and in super-unit order (summation order stays fixed).
+    // (a barrier; words in shared memory that both polled took issue slots from the teams: 4096 -> 28672 at 9 tokens 19.7 us, 18.8 so, at 128 tokens 32.6 / 31.0,
+    // 14336 -> 4096 at 64 15.3 / 14.8), so MMAs reach the pipe back to back and in super-unit order (summation order stays fixed).
     // Warp-uniform loops, one elected thread issues: keeps the tcgen05 operands in uniform registers.
     const int me = warp - kW4MmaWarp;
     constexpr uint32_t idesc = umma_idesc_f16_f32acc(kW4TileM, TN);
@@ -340,23 +306,12 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
       const bool seg_last = (j == n_su - 1) || kb == p.nkb - 1;
       const int buf = C::kDBufs == 2 ? (seg & 1) : 0;
       const int sx = j % C::kXStages, sj = j % C::kSuRing;
-      {
-        const uint32_t target = 9u * (uint32_t)((j >> 3) + 1);
-        uint32_t spins = 0;
-        while (lds_acquire_cta(&s_ready[j & 7]) < target) {
-          if (++spins > (1u << 26)) __trap();
-        }
-      }
+      mbar_wait(&su_full[sx], (j / C::kXStages) & 1);
       if (seg_first) {  // the epilogue drained this accumulator set's previous super-tile
         if (C::kDBufs == 2) mbar_wait(&tmem_empty[buf], ((seg >> 1) & 1) ^ 1);
         else mbar_wait(&tmem_empty[0], (seg & 1) ^ 1);
       }
-      {
-        uint32_t spins = 0;
-        while (lds_acquire_cta(&s_issued) < (uint32_t)j) {  // my turn
-          if (++spins > (1u << 26)) __trap();
-        }
-      }
+      if (j > 0) mbar_wait(&turn[me], ((j - 1) >> 1) & 1);  // my turn
       tcgen05_fence_after();
       if (elect_one()) {
         const uint64_t bdesc = bdesc0 + (uint64_t)((sx * C::kXStageBytes) >> 4);
@@ -367,8 +322,9 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
           for (int k = 0; k < kW4BlockK / 16; ++k)
             umma_f16_ts(d, a + k * 8, bdesc + (uint64_t)((k >> 2) * (C::kXSubBytes >> 4) + (k & 3) * 2), idesc, (!seg_first || k > 0) ? 1u : 0u);
         }
-        asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_u32(&s_issued)), "r"((uint32_t)j + 1) : "memory");
+        mbar_arrive(&turn[me ^ 1]);
         umma_commit(&su_done[sj]);
+        umma_commit(&x_empty[sx]);
         if (seg_last) umma_commit(&tmem_full[buf]);
       }
       __syncwarp();
@@ -405,13 +361,14 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
       if (lane == 0) mbar_arrive(&empty_w[held]);
     }
     if (team == 0) W4_TRACE(2, kW4FirstDqWarp * 32);
-    int n = 0;
-    for (int i = team; i < n_units; i += kW4Teams, ++n) {
+    // the team's super-units j are two apart: places in the rings of A tiles and of activation tiles, parity of the A place's last use
+    int jr = (team >> 1) % C::kSuRing, jx = team >> 1;
+    uint32_t done_par = 1;
+    for (int i = team; i < n_units; i += kW4Teams) {
       const bool more = i + kW4Teams < n_units;
       // barrier polls are issued well before their result is needed
-      const int j = i >> 1, jr = j % C::kSuRing;
-      const uint32_t done_par = (uint32_t)(j / C::kSuRing - 1) & 1u;
-      const uint32_t a_dst = a_row + (i % C::kAStages) * kW4AColsPerStage;
+      const int j = i >> 1;
+      const uint32_t a_dst = a_row + (jr * kW4R + (team & 1)) * kW4AColsPerStage;
       const bool a_free = j < C::kSuRing || mbar_test_wait(&su_done[jr], done_par);  // looked at after chunk 0
       const bool w_landed = more && mbar_test_wait(&full_w[ws], wph);                // looked at after chunk 3
       uint32_t scale2, nz1024, nz64;
@@ -435,9 +392,11 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
-        red_release_cta_shared_inc(&s_ready[(i >> 1) & 7]);
+        mbar_arrive(&su_full[jx]);
         if (more) mbar_arrive(&empty_w[held]);
       }
+      if ((jr += 2) >= C::kSuRing) { jr -= C::kSuRing; done_par ^= 1; }
+      if ((jx += 2) >= C::kXStages) jx -= C::kXStages;
     }
     if (team == 0) W4_TRACE(4, kW4FirstDqWarp * 32);
   } else {
