@@ -37,7 +37,8 @@
 // Super-tiles shared by several CTAs are finished after the main loop by ALL their contributors: each sums one slice over
 // the contributors' fp32 partials in contributor order (deterministic, unlike the reference kernel's fp16 atomicAdd across
 // K slices; a reduce-scatter, so the tail costs one partial's worth of L2 reads per CTA however many CTAs share it).
-// The contributors wait for one another: all CTAs of the grid are co-resident (grid <= #SMs, one CTA per SM).
+// The contributors wait for one another: all CTAs of the grid are co-resident (grid <= #SMs, one CTA per SM).  Where that cut would have many contributors
+// or few SMs, the CTAs of a cluster share a super-tile instead and add their parts through shared memory (launch_plan_w4).
 //
 // mbarrier rule used throughout: a thread that waits on a barrier observes every phase of it in order, or an earlier
 // observation implies the skipped phase completed (see the ring-depth static_asserts).  Polls whose result is wanted
@@ -72,6 +73,9 @@ constexpr int64_t kW4CounterBytes = 64 * 1024;
 // kernel would need two token tiles (4096 -> 4096 40.1 / 19.6, 14336 -> 4096 107 / 58).
 constexpr int kW4R = 2;  // feature tiles per super-tile: consecutive units (super-tile, k-block, r = 0..1) share one activation tile
 
+// how a kernel ends: by its four epilogue warps; by all threads where a CTA has its last super-tile alone; super-tiles shared by clusters
+enum W4End { kW4Plain, kW4Whole, kW4Cluster };
+constexpr int kW4MostCluster = 8;   // CTAs that share a super-tile through shared memory
 constexpr int kW4SumPitch = kW4R * kW4TileM + 4;  // floats of a token's sums in shared memory
 
 template <int TN>
@@ -97,9 +101,9 @@ struct GemmW4Cfg {
   static_assert(TN * kW4SumPitch * 4 <= kXStages * kXStageBytes + kWStages * kW4RecMaxBytes, "the last super-tile's sums lie where the rings were");
 };
 
-__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 
@@ -115,7 +119,7 @@ __device__ __forceinline__ void mbar_wait_relaxed(uint64_t* bar, uint32_t parity
 struct W4Params {
   __half* y;
   float* partial;   // [super-tile][contributor][kW4R][TN][128] fp32
-  int* counters;    // [super-tile][2]: partials written / slices reduced
+  unsigned* counters;  // [super-tile]: its n contributors count to n as their partials are written and to 2 n, which is 0 again, as they see n
   const __half* bias;
   const unsigned char* packed;  // unit records, (super-tile, k-block, r) order
   int T, N;
@@ -130,6 +134,7 @@ struct W4Params {
   int ldy;          // output row stride in halves
   int defer;        // 1: every super-tile segment is left as an fp32 partial in the workspace and the NEXT kernel of the stream sums
                     //    them (B200SplitK consumers: rmsnorm / rope / SiLU*up / all-reduce); no counters, no waiting on peer CTAs
+  int cluster;      // > 0: a cluster of so many CTAs has one super-tile, each a part of k
   unsigned long long* trace;  // debug: per-CTA phase timestamps (globaltimer ns), NULL in production
 };
 
@@ -139,11 +144,12 @@ struct W4Params {
 // kWhole: from 17 tokens on, and with the SiLU from 9 if no super-tile is shared; otherwise the outputs are too few to pay for the barrier, or for the code
 // alone (14336 -> 4096 at one token 12.6 us without and 13.0 with it, 4096 -> 22016 with the SiLU at 16 tokens 18.0 and 18.2; 4096 -> 28672 with the SiLU 18.4 and
 // 18.5 at one token, 19.7 and 18.7 at 16).
-__device__ __forceinline__ void w4_finish(const W4Params& p, const float* sums, int sup) {
-  const int per_tok = p.act ? kW4TileM / 4 : kW4R * kW4TileM / 4;
-  for (int i = threadIdx.x; i < p.T * per_tok; i += kW4Threads) {
+// four(at): sums of four features from `at` on, [token][kW4SumPitch]; items lo .. hi - 1 of T * per_tok are this CTA's
+template <class Four>
+__device__ __forceinline__ void w4_finish(const W4Params& p, int sup, int per_tok, int lo, int hi, Four four) {
+  for (int i = lo + threadIdx.x; i < hi; i += kW4Threads) {
     const int tok = i / per_tok, f = (i % per_tok) * 4, r = f / kW4TileM, m = f % kW4TileM;
-    float4 s = *reinterpret_cast<const float4*>(&sums[tok * kW4SumPitch + f]);
+    float4 s = four(tok * kW4SumPitch + f);
     const int col = p.act ? sup * kW4TileM + f : (p.half_tiles ? sup + r * p.half_tiles : sup * kW4R + r) * kW4TileM + m;
     if (!p.act && col >= p.N) continue;   // N % 32 == 0: four columns never straddle it
     if (p.bias) {
@@ -151,7 +157,7 @@ __device__ __forceinline__ void w4_finish(const W4Params& p, const float* sums, 
     }
     uint2 o;
     if (p.act) {
-      float4 u = *reinterpret_cast<const float4*>(&sums[tok * kW4SumPitch + kW4TileM + f]);
+      float4 u = four(tok * kW4SumPitch + kW4TileM + f);
       if (p.bias) {
         const __half* b = p.bias + col + p.half_tiles * kW4TileM;
         u.x += __half2float(b[0]); u.y += __half2float(b[1]); u.z += __half2float(b[2]); u.w += __half2float(b[3]);
@@ -172,10 +178,11 @@ __device__ __forceinline__ void w4_finish(const W4Params& p, const float* sums, 
 }
 
 // kGR = meta rows per unit record (1, 2 or 4 = 128 / groupsize, 1 for groupsize >= 128).
-template <int TN, int kGR, bool kWhole>
+template <int TN, int kGR, int kEnd>
 __global__ void __launch_bounds__(kW4Threads, 1)
 gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) {
   using C = GemmW4Cfg<TN>;
+  constexpr bool kWhole = kEnd == kW4Whole, kCluster = kEnd == kW4Cluster;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   unsigned char* x_ring = smem;                                 // 1024-aligned stages (128B swizzle)
@@ -195,8 +202,10 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
 
   pdl_launch_dependents();
   const int warp = warp_id(), lane = lane_id();
-  const int su0 = blockIdx.x * p.su_per_cta;  // a contiguous range of super-units of the (super-tile, k-block) space
-  const int su1 = min(p.total_su, su0 + p.su_per_cta);
+  // a contiguous range of super-units of the (super-tile, k-block) space
+  const int c_sup = kCluster ? (int)blockIdx.x / p.cluster : 0, c_rank = kCluster ? (int)blockIdx.x % p.cluster : 0;
+  const int su0 = kCluster ? c_sup * p.nkb + c_rank * p.nkb / p.cluster : blockIdx.x * p.su_per_cta;
+  const int su1 = kCluster ? c_sup * p.nkb + (c_rank + 1) * p.nkb / p.cluster : min(p.total_su, su0 + p.su_per_cta);
   const int n_su = su1 - su0;
   const int n_units = n_su * kW4R;
   const int kb0 = su0 % p.nkb;
@@ -413,7 +422,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
       // contributors of this super-tile: CTAs whose range intersects [sup*nkb, (sup+1)*nkb)
       const int c_first = (sup * p.nkb) / p.su_per_cta;
       const int c_last = ((sup + 1) * p.nkb - 1) / p.su_per_cta;
-      const int n_contrib = c_last - c_first + 1;
+      const int n_contrib = kCluster ? 1 : c_last - c_first + 1;
       const int my_contrib = (int)blockIdx.x - c_first;
       float* part = p.partial + ((size_t)sup * p.max_contrib + my_contrib) * (kW4R * TN * kW4TileM);
       mbar_wait_relaxed(&tmem_full[buf], C::kDBufs == 2 ? ((seg >> 1) & 1) : (seg & 1));
@@ -424,7 +433,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
         const int n0 = (p.half_tiles ? sup : sup * kW4R) * kW4TileM + m;
         const int n1 = (p.half_tiles ? sup + p.half_tiles : sup * kW4R + 1) * kW4TileM + m;
         const bool ok0 = n0 < p.N, ok1 = n1 < p.N;
-        const bool direct = n_contrib == 1 && !p.defer, whole = kWhole && direct && seg_end == su1;
+        const bool direct = n_contrib == 1 && !p.defer, whole = kCluster || (kWhole && direct && seg_end == su1);
         const float bv0 = (p.bias && ok0 && direct) ? __half2float(p.bias[n0]) : 0.f;
         const float bv1 = (p.bias && ok1 && direct) ? __half2float(p.bias[n1]) : 0.f;
         constexpr int kCh = 16;  // columns fetched per tcgen05.wait::ld (32 spill)
@@ -482,7 +491,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
         asm volatile("bar.sync 1, %0;" ::"n"(kW4EpWarps * 32) : "memory");
         if (threadIdx.x == 0) {
           __threadfence();
-          atomicAdd(&p.counters[2 * sup], 1);
+          atomicInc(&p.counters[sup], 2 * n_contrib - 1);
           s_fix[nfix][0] = sup;
           s_fix[nfix][1] = n_contrib;
           s_fix[nfix][2] = my_contrib;
@@ -505,11 +514,14 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
   for (int f = 0; f < nfix; ++f) {
     const int sup = s_fix[f][0], n_contrib = s_fix[f][1], my_contrib = s_fix[f][2];
     if (threadIdx.x == 0) {
+      // (one counter that wraps: with a second one for those who had finished, whose last owner re-armed both, a CTA ended 1 us later, behind an answer from L2;
+      // us: 4096 -> 6144 at 9 tokens 9.2 -> 8.7, 4096 -> 22016 at 64 22.6 -> 21.7, 2048 -> 2560 at 16 5.9 -> 5.6)
       uint32_t spins = 0;
-      while (ld_acquire_gpu(&p.counters[2 * sup]) < n_contrib) {  // all contributors are co-resident (grid <= #SMs, 1 CTA/SM)
+      while (ld_acquire_gpu(&p.counters[sup]) < (unsigned)n_contrib) {  // all contributors are co-resident (grid <= #SMs, 1 CTA/SM)
         __nanosleep(64);
         if (++spins > (1u << 24)) __trap();
       }
+      atomicInc(&p.counters[sup], 2 * n_contrib - 1);
     }
     __syncthreads();
     W4_TRACE(41 + f * 3, 0);
@@ -582,21 +594,35 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
       }
     }
     W4_TRACE(42 + f * 3, 0);
-    __syncthreads();
-    W4_TRACE(43 + f * 3, 0);
-    if (threadIdx.x == 0) {
-      // the last contributor to finish its slice re-arms both counters for the next launch (graph replay safe)
-      const int prev = atomicAdd(&p.counters[2 * sup + 1], 1);
-      if (prev == n_contrib - 1) {
-        p.counters[2 * sup] = 0;
-        p.counters[2 * sup + 1] = 0;
-        __threadfence();
-      }
-    }
   }
   if (kWhole && s_whole >= 0) {
     if (nfix == 0) pdl_wait();
-    w4_finish(p, reinterpret_cast<const float*>(smem), s_whole);
+    const float* sums = reinterpret_cast<const float*>(smem);
+    const int per_tok = p.act ? kW4TileM / 4 : kW4R * kW4TileM / 4;
+    w4_finish(p, s_whole, per_tok, 0, p.T * per_tok, [&](int at) { return *reinterpret_cast<const float4*>(sums + at); });
+  }
+  if constexpr (kCluster) {
+    // the cluster's CTAs add their parts of k through one another's shared memory, CTA r its share of the outputs, always in the order of the ranks
+    pdl_wait();
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    W4_TRACE(41, 0);
+    const uint32_t base = smem_u32(smem);
+    const int d = p.cluster, per_tok = p.act ? kW4TileM / 4 : kW4R * kW4TileM / 4, items = p.T * per_tok, share = (items + d - 1) / d;
+    w4_finish(p, c_sup, per_tok, c_rank * share, min(items, (c_rank + 1) * share), [&](int at) {
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 v[kW4MostCluster];
+#pragma unroll
+      for (int i = 0; i < kW4MostCluster; ++i) v[i] = i < d ? ld_cluster_v4(base + at * 4, i) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < kW4MostCluster; ++i) { acc.x += v[i].x; acc.y += v[i].y; acc.z += v[i].z; acc.w += v[i].w; }
+      return acc;
+    });
+    W4_TRACE(42, 0);
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // nobody leaves while its sums are read
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
   W4_TRACE(63, 0);
 }
@@ -661,6 +687,7 @@ static int w4_nkb(int64_t K) {
 
 struct W4Plan {
   int TN, nkb, n_super, su_per_cta, n_ctas, max_contrib;
+  int cluster;   // > 0: so many CTAs share a super-tile and add their sums through shared memory; nothing goes to a workspace
 };
 
 // One token tile (T <= kW4DecodeT): how many super-units per CTA.  Candidates are the balanced stream-K cut (every SM the same
@@ -669,8 +696,9 @@ struct W4Plan {
 // n_super * d is not close to a multiple of the SM count).  Costs in microseconds fitted to a sweep of the cut on B200
 // (cold weights): 0.35 per unit in the main loop, ~1 for a direct epilogue, 4.5-6 for one split-K fix-up (partial store,
 // gpu-scope fence, waiting for the slowest contributor, L2-latency-bound slice reduction), ~10 when CTAs straddle.
-static W4Plan plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool defer = false) {
+static W4Plan plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool defer = false, float* cost_of = nullptr) {
   W4Plan pl;
+  pl.cluster = 0;
   pl.TN = T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : 128;
   pl.nkb = w4_nkb(K);
   pl.n_super = (int)((N + kW4R * kW4TileM - 1) / (kW4R * kW4TileM));
@@ -702,6 +730,7 @@ static W4Plan plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool defer = fal
   pl.n_ctas = (total + pl.su_per_cta - 1) / pl.su_per_cta;
   pl.max_contrib = (pl.nkb + pl.su_per_cta - 1) / pl.su_per_cta + 1;
   if (pl.su_per_cta % pl.nkb == 0) pl.max_contrib = 1;
+  if (cost_of) *cost_of = best_cost;
   return pl;
 }
 
@@ -781,8 +810,28 @@ extern "C" int b200_gptq_pack(const void* qweight, const void* qzeros, const voi
 // bytes of split-K partials the int4 GEMM may write for this shape (the tile counters sit in the first 64 KiB)
 // The plan a launch uses: the stream-K cut needs the workspace (partials + one counter pair per super-tile) and every CTA
 // resident at once (the fix-up spins on its peers); otherwise each CTA takes whole super-tiles.
-static W4Plan launch_plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool has_workspace, bool defer = false) {
-  W4Plan pl = plan_w4(T, N, K, sms, defer);
+// clusters[d]: clusters of d CTAs that the chip holds (NULL: none).  The largest cluster whose super-tiles all fit in one wave, where it costs less: adding up
+// through shared memory takes 2.5 us and 0.8 for each CTA whose sums are read (64 tokens: 64 KB of them).  That is less than a cut that straddles
+// super-tiles, more so the more contributors one has, and about as much as an aligned cut's, which has 8 contributors where the chip holds 15 clusters of
+// 8 or fewer of more CTAs.  us, through global memory / clusters, at 9, 64 and 128 tokens: 5632 -> 2048 (clusters of 8) 9.9 / 7.3, 13.2 / 10.2, 17.8 / 15.5; 4096 ->
+// 12288 (of 2) 12.8 / 12.2, 16.2 / 15.4, 23.0 / 22.1; the other side of the line: 4096 -> 4096 (of 6) 7.4 / 8.1, 9.3 / 11.4, 12.7 / 15.8; 14336 -> 4096 12.6 / 14.3,
+// 14.5 / 17.9, 20.1 / 25.0; 4096 -> 6144 (of 5) 8.7 / 9.4, 11.3 / 12.9, 15.4 / 17.2.
+static W4Plan launch_plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool has_workspace, bool defer = false, const int* clusters = nullptr) {
+  float cost;
+  W4Plan pl = plan_w4(T, N, K, sms, defer, &cost);
+  if (!defer && clusters) {
+    int d = kW4MostCluster;
+    while (d > 1 && (d > pl.nkb || clusters[d] < pl.n_super)) --d;
+    const int su = (pl.nkb + d - 1) / d;
+    if (pl.nkb % pl.su_per_cta != 0) cost += 0.2f * pl.max_contrib;
+    if (d > 1 && 0.35f * kW4R * su + 2.5f + 0.8f * d < cost) {
+      pl.cluster = d;
+      pl.su_per_cta = su;
+      pl.n_ctas = pl.n_super * d;
+      pl.max_contrib = 1;
+      return pl;
+    }
+  }
   if (defer) return pl;  // the caller checked: one token tile, workspace present; no counters, no co-residency requirement
   if (pl.max_contrib > 1 && (!has_workspace || (int64_t)pl.n_super * 8 > kW4CounterBytes || pl.n_ctas > sms)) {
     pl.su_per_cta = pl.nkb;
@@ -809,19 +858,19 @@ int64_t b200_w4_partial_bytes(int64_t T, int64_t N, int64_t K) {
   return nd > need ? nd : need;
 }
 
-template <int TN, int kGR, bool kWhole>
+template <int TN, int kGR, int kEnd>
 static int launch_gemm_w4(const CUtensorMap* mx, const void* packed, void* y, void* workspace, const void* bias, int T, int N,
                           const W4Plan& pl, int half_tiles, int act, int defer, cudaStream_t st) {
   using C = GemmW4Cfg<TN>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_w4a16_kernel<TN, kGR, kWhole>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(gemm_w4a16_kernel<TN, kGR, kEnd>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
     if (e != cudaSuccess) { b200_set_last_error(cudaGetErrorString(e)); return B200_ERR_CUDA; }
     configured = true;
   }
   W4Params p;
   p.y = (__half*)y;
-  p.counters = (int*)workspace;
+  p.counters = (unsigned*)workspace;
   p.partial = workspace ? (float*)((char*)workspace + kW4CounterBytes) : nullptr;
   p.bias = (const __half*)bias;
   p.packed = (const unsigned char*)packed;
@@ -837,14 +886,29 @@ static int launch_gemm_w4(const CUtensorMap* mx, const void* packed, void* y, vo
   p.act = act;
   p.ldy = act ? N / 2 : N;
   p.defer = defer;
+  p.cluster = pl.cluster;
   p.trace = g_w4_trace;
   const dim3 grid(pl.n_ctas);
   b200_timing_mark(B200_TIME_GEMM_W4A16, 0, st);
-  constexpr auto kernel = gemm_w4a16_kernel<TN, kGR, kWhole>;
-  B200_LAUNCH_AS("gemm_w4a16_kernel", kernel, grid, dim3(kW4Threads), (size_t)C::kSmemBytes, st, *mx, p);
+  constexpr auto kernel = gemm_w4a16_kernel<TN, kGR, kEnd>;
+  const cudaError_t e = b200_launch_cluster(kernel, grid, dim3(kW4Threads), (size_t)C::kSmemBytes, st, (unsigned)pl.cluster, *mx, p);
+  if (e != cudaSuccess) { b200_set_last_error(cudaGetErrorString(e)); return B200_ERR_CUDA; }
+  b200_step_trace_stamp("gemm_w4a16_kernel", st);
   b200_timing_mark(B200_TIME_GEMM_W4A16, 1, st);
   b200_count_launches(1);
   return B200_OK;
+}
+
+static const int* w4_clusters() {
+  static const struct Table {
+    int n[kW4MostCluster + 1];
+    Table() : n{} {
+      n[0] = n[1] = b200_num_sms();
+      cudaFuncSetAttribute(gemm_w4a16_kernel<64, 1, kW4Cluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmW4Cfg<64>::kSmemBytes);
+      b200_count_clusters(gemm_w4a16_kernel<64, 1, kW4Cluster>, kW4Threads, (size_t)GemmW4Cfg<64>::kSmemBytes, n);
+    }
+  } table;
+  return table.n;
 }
 
 // packed: output of b200_gptq_pack[_ex] for the same (K, N, groupsize, layout).
@@ -903,7 +967,7 @@ static int gemm_w4a16_impl(const void* x, const void* packed, const void* bias, 
     if (!fp.gave_up) return B200_ERR_CUDA;
     return launch_w4_few_plan(fp, gr, (int)((N + kW4R * kW4TileM - 1) / (kW4R * kW4TileM)), few, (cudaStream_t)stream);
   }
-  const W4Plan pl = launch_plan_w4(T, N, K, b200_num_sms(), workspace != nullptr, defer);
+  const W4Plan pl = launch_plan_w4(T, N, K, b200_num_sms(), workspace != nullptr, defer, w4_clusters());
   const CUtensorMap* mx = get_tmap_2d(x, T, K, K, pl.TN, 64, TmapDtype::kF16, TmapSwizzle::k128B);
   if (!mx) return B200_ERR_CUDA;
   if (defer) {
@@ -924,11 +988,19 @@ static int gemm_w4a16_impl(const void* x, const void* packed, const void* bias, 
   (gr == 1   ? launch_gemm_w4<TNV, 1, W>(mx, packed, y, workspace, bias, (int)T, (int)N, pl, half_tiles, act, df, st)         \
    : gr == 2 ? launch_gemm_w4<TNV, 2, W>(mx, packed, y, workspace, bias, (int)T, (int)N, pl, half_tiles, act, df, st)         \
              : launch_gemm_w4<TNV, 4, W>(mx, packed, y, workspace, bias, (int)T, (int)N, pl, half_tiles, act, df, st))
+  if (pl.cluster) {
+    switch (pl.TN) {
+      case 16: return W4_DISPATCH(16, kW4Cluster);
+      case 32: return W4_DISPATCH(32, kW4Cluster);
+      case 64: return W4_DISPATCH(64, kW4Cluster);
+      default: return W4_DISPATCH(128, kW4Cluster);
+    }
+  }
   switch (pl.TN) {
-    case 16: return act && T > 8 && pl.max_contrib == 1 ? W4_DISPATCH(16, true) : W4_DISPATCH(16, false);
-    case 32: return W4_DISPATCH(32, true);
-    case 64: return W4_DISPATCH(64, true);
-    default: return W4_DISPATCH(128, true);
+    case 16: return act && T > 8 && pl.max_contrib == 1 ? W4_DISPATCH(16, kW4Whole) : W4_DISPATCH(16, kW4Plain);
+    case 32: return W4_DISPATCH(32, kW4Whole);
+    case 64: return W4_DISPATCH(64, kW4Whole);
+    default: return W4_DISPATCH(128, kW4Whole);
   }
 #undef W4_DISPATCH
 }
