@@ -45,6 +45,11 @@ static int linear_deferred(const B200Linear* L, const B200LlamaStep* s, const vo
 }
 
 static bool deferring(const B200LlamaStep* s) { return s->defer_splitk && s->gemm_ws && s->T <= 128 && !s->is_prefill; }
+// int4 linears of more than eight tokens are finished in their own kernel: what the next one saves by it (fp32 partials of up to eight contributors, or gate and
+// up, that it does not read) is more than the fix-up costs.  Llama-3-8B, four layers, us, partials left to the next kernel / finished: 64 tokens behind 1024 -
+// 2048 745 / 707, 64 behind 64 - 128 491 / 461, 16 383 / 376, 9 382 / 373; Llama-2-7B at 20 tokens 320 / 315.  Up to eight tokens, and for fp16 weights, leaving
+// them is faster, and the all-reduce of tensor-parallel ranks takes them in.
+static bool finishes(const B200LlamaWeights* w, const B200LlamaStep* s, const B200Linear* L) { return L->qweight && s->T > 8 && w->tp_size == 1; }
 // the fused NVLink boundary takes steps of up to 2048 token rows (decode, and prefill chunks of continuous batching); anything
 // larger is all-reduced by the caller between the block calls
 static bool fused_boundary(const B200LlamaWeights* w, const B200LlamaStep* s) { return w->tp_size > 1 && s->p2p_norm && s->T <= 2048; }
@@ -85,7 +90,7 @@ static int boundary_norm(const B200LlamaWeights* w, const B200LlamaStep* s, cons
 // A row-parallel linear (o_proj, down_proj): its output is the next boundary's input.  Deferred when that boundary can sum the
 // partials (single rank, or the fused NVLink boundary); materialised into s->hidden otherwise (the caller's NCCL all-reduce).
 static int row_linear(const B200LlamaWeights* w, const B200LlamaStep* s, const B200Linear* L, const void* x, HiddenIn* out, void* stream) {
-  const bool can_defer = deferring(s) && (w->tp_size == 1 || fused_boundary(w, s));
+  const bool can_defer = deferring(s) && !finishes(w, s, L) && (w->tp_size == 1 || fused_boundary(w, s));
   out->deferred = false;
   if (can_defer) {
     RUN(linear_deferred(L, s, x, &out->parts, s->T, stream));
@@ -106,7 +111,7 @@ static int attn_body(const B200LlamaWeights* w, const B200LlamaStep* s, int laye
   const B200LlamaLayer* L = &w->layers[layer];
   char* k_pool = (char*)s->kv_pool + (size_t)layer * s->kv_layer_stride_bytes;
   char* v_pool = k_pool + s->kv_v_offset_bytes;
-  if (deferring(s)) {
+  if (deferring(s) && !finishes(w, s, &L->qkv)) {
     B200SplitK qkv_parts;
     RUN(linear_deferred(&L->qkv, s, s->normed, &qkv_parts, T, stream));
     RUN(b200_rope_kv_write_paged_splitk(&qkv_parts, s->qkv, w->rope_cos, w->rope_sin, s->position_ids, s->slot_mapping, k_pool, v_pool,
@@ -139,12 +144,13 @@ static int attn_body(const B200LlamaWeights* w, const B200LlamaStep* s, int laye
 static int mlp_body(const B200LlamaWeights* w, const B200LlamaStep* s, int layer, HiddenIn* out, void* stream) {
   const int64_t T = s->T;
   const B200LlamaLayer* L = &w->layers[layer];
-  if (deferring(s)) {
+  const bool fused_act = L->gate_up.qweight && L->gate_up.layout == B200_W4_LAYOUT_GATE_UP;
+  if (deferring(s) && !(fused_act && finishes(w, s, &L->gate_up))) {
     // the [T, 2 I] intermediate never exists: SiLU(gate) * up reads the projection's partials (either weight layout)
     B200SplitK gu_parts;
     RUN(linear_deferred(&L->gate_up, s, s->normed, &gu_parts, T, stream));
     RUN(b200_splitk_silu_mul(&gu_parts, s->act, stream));
-  } else if (L->gate_up.qweight && L->gate_up.layout == B200_W4_LAYOUT_GATE_UP) {
+  } else if (fused_act) {
     // int4 gate|up layout: SiLU(gate) * up is the GEMM's epilogue
     const void* x = s->normed;
     RUN(gathered(&L->gate_up, s, &x, T, stream));
