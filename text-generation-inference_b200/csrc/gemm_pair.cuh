@@ -145,7 +145,7 @@ __device__ __forceinline__ __half act_pair(uint32_t first, uint32_t second, floa
   const bool up = lane >= 16;
   const __half other = __ushort_as_half((unsigned short)__shfl_xor_sync(0xffffffffu, (int)__half_as_ushort(up ? a : b), 16));
   const float g = __half2float(up ? other : a);
-  return __hmul(__float2half_rn(g / (1.f + expf(-g))), up ? b : other);
+  return __hmul(__float2half_rn(silu_of_half(g)), up ? b : other);
 }
 template <int KIND>
 __device__ __forceinline__ float pair_bias(const void* bias, int n) {

@@ -139,7 +139,7 @@ struct W4Params {
 };
 
 // The end of a CTA's last super-tile when nobody shares it: the epilogue warps leave its fp32 sums in shared memory ([token][kW4SumPitch]) and all 24 warps
-// write the outputs, four features of a token each.  By the four epilogue warps alone, a feature per thread, the SiLU's divisions (a branch each, so one
+// write the outputs, four features of a token each.  By the four epilogue warps alone, a feature per thread, the SiLU (then with divisions, a branch each, so one
 // after the other) took 1.9 us at 16 tokens, 7.9 at 64 and 15 at 128 behind the last product (4096 -> 28672: 26.8 us of which 7.9 -> 21.5 with 2.4; 128 tokens 42.6 -> 32).
 // kWhole: from 17 tokens on, and with the SiLU from 9 if no super-tile is shared; otherwise the outputs are too few to pay for the barrier, or for the code
 // alone (14336 -> 4096 at one token 12.6 us without and 13.0 with it, 4096 -> 22016 with the SiLU at 16 tokens 18.0 and 18.2; 4096 -> 28672 with the SiLU 18.4 and

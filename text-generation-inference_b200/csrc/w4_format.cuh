@@ -68,7 +68,7 @@ __device__ __forceinline__ void dequant_consts(uint32_t rec, uint32_t& scale2, u
 // by silu_mul_kernel (elementwise.cu; torch fp16 SiLU = fp32 x / (1 + exp(-x)), one rounding, then an fp16 multiply) gives
 __device__ __forceinline__ __half silu_mul_f16(float gate_acc, float up_acc) {
   const float g = __half2float(__float2half_rn(gate_acc));
-  const __half a = __float2half_rn(g / (1.f + expf(-g)));
+  const __half a = __float2half_rn(silu_of_half(g));
   return __hmul(a, __float2half_rn(up_acc));
 }
 
