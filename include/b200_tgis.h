@@ -188,6 +188,9 @@ int b200_gemm_f16(const void* x, const void* w, const void* bias, void* y, int64
 /* the same for a w that b200_settle has settled and that has not been written since: its first tiles are read while the kernel before ends */
 int b200_gemm_f16_held(const void* x, const void* w, const void* bias, void* y, int64_t T, int64_t N, int64_t K, void* workspace,
                        void* stream);
+/* y [T, I] = SiLU(gate) * up of the projection by w = [gate; up] [2 I, K] (bias [2 I] or NULL): what b200_gemm_f16 and b200_silu_mul give, in one kernel.
+ * T > 256, K % 8 == 0, K >= 64, I % 8 == 0, y 16-byte aligned; anything else is B200_ERR_UNSUPPORTED. */
+int b200_gemm_f16_silu(const void* x, const void* w, const void* bias, void* y, int64_t T, int64_t I, int64_t K, void* stream);
 /* bfloat16 operands (x [T, K], w [N, K], bias bfloat16 or NULL); y [T, N], out_kind 0: bfloat16, 1: fp32, 2: bfloat16 after relu(z)^2.  Same kernel
  * (tcgen05 kind::f16 with bfloat16 operand formats), workspace and rules as b200_gemm_f16. */
 int b200_gemm_bf16(const void* x, const void* w, const void* bias, void* y, int out_kind, int64_t T, int64_t N, int64_t K, void* workspace,

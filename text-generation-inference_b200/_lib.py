@@ -47,6 +47,7 @@ SIGNATURES = {
     "b200_gemm_workspace_bytes_max": (_L, [_L, _L]),
     "b200_gemm_f16": (_I, [_P, _P, _P, _P, _L, _L, _L, _P, _P]),
     "b200_gemm_f16_held": (_I, [_P, _P, _P, _P, _L, _L, _L, _P, _P]),
+    "b200_gemm_f16_silu": (_I, [_P, _P, _P, _P, _L, _L, _L, _P]),
     "b200_gemm_bf16": (_I, [_P, _P, _P, _P, _I, _L, _L, _L, _P, _P]),
     "b200_p2p_handle_bytes": (_I, []),
     "b200_p2p_create": (_I, [_L, _I, _I, ctypes.POINTER(_P), _P]),

@@ -623,6 +623,24 @@ extern "C" int b200_gemm_f16_held(const void* x, const void* w, const void* bias
                                   void* workspace, void* stream) {
   return gemm_f16_impl<0>(x, w, bias, y, T, N, K, workspace, nullptr, true, stream);
 }
+// y [T, I] = SiLU(x Wg^T) * (x Wu^T) for w = [Wg; Wu] [2 I, K] (bias [2 I] or NULL), both factors rounded to fp16 first as b200_gemm_f16 and
+// b200_silu_mul do, with the same sums.  Prompts only (T > 256: SM pairs, gemm_pair.cuh): the [T, 2 I] between the two does not go through memory.
+// Measured on B200 (us, b200_gemm_f16 and b200_silu_mul / this, back to back): 2048 -> 2 x 5632 at 300 tokens 23.9 / 17.5, 1000 44.5 / 36.6,
+// 4674 180 / 152 (the product alone 150); 4096 -> 2 x 11008 at 1000 146 / 131, 4674 703 / 629 (582).
+extern "C" int b200_gemm_f16_silu(const void* x, const void* w, const void* bias, void* y, int64_t T, int64_t I, int64_t K, void* stream) {
+  if (I == 0) return B200_OK;
+  if (T <= kF16MostT || K % 8 != 0 || K < 64 || I % 8 != 0 || ((uintptr_t)y & 15)) {
+    b200_set_last_error("gemm_f16_silu: need more than 256 tokens, K % 8 == 0, K >= 64, I % 8 == 0 and a 16-byte aligned y");
+    return B200_ERR_UNSUPPORTED;
+  }
+  PairParams pp = {};
+  pp.y = y;
+  pp.bias = bias;
+  pp.T = (int)T;
+  pp.N = pp.ldy = pp.half = (int)I;
+  pp.n_kb = (int)((K + kPairK - 1) / kPairK);
+  return launch_gemm_pair<kPairF16Silu>(x, w, K, pp, pair_plan(T, 2 * ((I + 127) / 128 * 128), pp.n_kb, false, b200_num_sms()), B200_TIME_GEMM_F16, (cudaStream_t)stream);
+}
 // bfloat16 x [T, K] and w [N, K] (bias bfloat16 or NULL) -> y [T, N]; out_kind 0: bfloat16, 1: fp32, 2: bfloat16 after the square of
 // ReLU.  Same kernel, workspace and rules as b200_gemm_f16.
 extern "C" int b200_gemm_bf16(const void* x, const void* w, const void* bias, void* y, int out_kind, int64_t T, int64_t N, int64_t K,

@@ -156,6 +156,8 @@ static int mlp_body(const B200LlamaWeights* w, const B200LlamaStep* s, int layer
     RUN(gathered(&L->gate_up, s, &x, T, stream));
     RUN(b200_gemm_w4a16_ex(x, L->gate_up.qweight, L->gate_up.bias, s->act, T, L->gate_up.N, L->gate_up.K, L->gate_up.groupsize,
                            B200_W4_LAYOUT_GATE_UP, 1, s->gemm_ws, stream));
+  } else if (!L->gate_up.qweight && T > 256 && L->gate_up.N % 16 == 0 && ((uintptr_t)s->act & 15) == 0) {
+    RUN(b200_gemm_f16_silu(s->normed, L->gate_up.weight, L->gate_up.bias, s->act, T, L->gate_up.N / 2, L->gate_up.K, stream));
   } else {
     RUN(linear(&L->gate_up, s, s->normed, s->gate_up, T, stream));
     RUN(b200_silu_mul(s->gate_up, s->act, T, L->gate_up.N / 2, stream));
