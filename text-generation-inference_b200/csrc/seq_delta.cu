@@ -140,8 +140,12 @@ __global__ void __launch_bounds__(kPrepThreads, TAPS <= 4 ? 4 : 2) delta_prepare
 // 32 heads: 3600 tokens 246 / 108, 400 31.4 / 19.9.
 constexpr int kRunTok = 16, kRunMinTokens = 384;
 
-template <typename TP>
-__global__ void __launch_bounds__(256) delta_prepare_run_kernel(
+// kPerSm: blocks of an SM that registers are left for.  Three (80 registers, a few spilled) from kRunBlocksMany blocks on, where they save a round of blocks; two
+// (116, none spilled) below.  us of a call with the memory's part, two / three: 16 heads 4 x 256 - 768 tokens (854 blocks) 210.8 / 206.4, 16 x 250 353 / 344, 32 heads 6 x
+// 400 - 800 659 / 641; 16 heads 4 x 200 - 250 (420) 110.6 / 112.3, 6 x 96 - 120 (322) 77.1 / 80.8.
+constexpr int kRunBlocksMany = 3 * 148;
+template <typename TP, int kPerSm>
+__global__ void __launch_bounds__(256, kPerSm) delta_prepare_run_kernel(
     const float* __restrict__ u, int64_t ld, int col0, int taps, const TP* __restrict__ w, float* conv_state,
     const int32_t* __restrict__ state_slots, const int32_t* __restrict__ cu_q, int B, const int64_t* __restrict__ position_ids,
     const float* __restrict__ raw, int64_t ldr, int col_b, const float* __restrict__ dec, int64_t ldd, int col_a, int channels,
@@ -718,9 +722,13 @@ extern "C" int b200_seq_delta_prepare(const float* u, int64_t ld, int col0, int 
                     ((ld | col0 | ldd | col_a | (H * dv)) & 3) == 0;
   if (wide && (dk == 64 || dk == 128) && taps <= 4 && T > 4 * (int64_t)B && T >= kRunMinTokens) {
     const int run_tasks = (C + 127) / 128 + (channels ? (H * dk + 127) / 128 : 0) + 1;
-    B200_SEQ_DISPATCH(dt, E, B200_LAUNCH((delta_prepare_run_kernel<E>), dim3((unsigned)(T / kRunTok + B), (unsigned)((run_tasks + 7) / 8)), dim3(256), 0, st, u, ld, col0,
-                                         taps, (const E*)w, conv_state, state_slots, cu_q, B, position_ids, raw, ldr, col_b, dec, ldd, col_a, channels,
-                                         (const E*)A_log, (const E*)dt_bias, q_scale, out, H, kv_heads, dk, dv));
+    const dim3 grid((unsigned)(T / kRunTok + B), (unsigned)((run_tasks + 7) / 8));
+#define DPRUN(N)                                                                                                                                                  \
+  B200_SEQ_DISPATCH(dt, E, B200_LAUNCH((delta_prepare_run_kernel<E, N>), grid, dim3(256), 0, st, u, ld, col0, taps, (const E*)w, conv_state, state_slots, cu_q, B, \
+                                       position_ids, raw, ldr, col_b, dec, ldd, col_a, channels, (const E*)A_log, (const E*)dt_bias, q_scale, out, H, kv_heads, dk, dv))
+    if ((int64_t)grid.x * grid.y > kRunBlocksMany) DPRUN(3);
+    else DPRUN(2);
+#undef DPRUN
     b200_count_launches(1);
     return B200_OK;
   }
