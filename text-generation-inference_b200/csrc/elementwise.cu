@@ -257,7 +257,7 @@ __global__ void rope_kv_write_kernel(__half* __restrict__ qkv, const __half* __r
   }
 }
 
-// Prefill-sized form of the same op (full rotation, plain fp16 input): 16-byte accesses, one (token, head) row per D/16 threads,
+// Form of the same op for many rows (full rotation, plain fp16 input): 16-byte accesses, one (token, head) row per D/16 threads,
 // grid-stride.  The per-(token, head) CTAs above are launch-bound at T = 65 536 (3 M CTAs of 64 threads: 4.9 ms per layer under ncu,
 // as long as the QKV projection); this form moves the same 1.7 GB at HBM speed.
 template <int kHeadDim>
@@ -275,10 +275,10 @@ __global__ void __launch_bounds__(256) rope_kv_write_vec_kernel(__half* __restri
     const int head = (int)(r - t * n_all);
     __half* base = qkv + (size_t)r * kHeadDim;
     const bool is_v = head >= n_heads + n_kv;
+    const int64_t pos = is_v ? 0 : position_ids[t], slot = head >= n_heads ? slot_mapping[t] : -1;   // in flight with the row
     uint4 lo = *reinterpret_cast<const uint4*>(base + lane * 8);
     uint4 hi = *reinterpret_cast<const uint4*>(base + kHeadDim / 2 + lane * 8);
     if (!is_v) {
-      const int64_t pos = position_ids[t];
       const uint4 cv = *reinterpret_cast<const uint4*>(cos_t + pos * (kHeadDim / 2) + lane * 8);
       const uint4 sv = *reinterpret_cast<const uint4*>(sin_t + pos * (kHeadDim / 2) + lane * 8);
       __half* l = reinterpret_cast<__half*>(&lo);
@@ -295,7 +295,6 @@ __global__ void __launch_bounds__(256) rope_kv_write_vec_kernel(__half* __restri
       *reinterpret_cast<uint4*>(base + kHeadDim / 2 + lane * 8) = hi;
     }
     if (head >= n_heads) {
-      const int64_t slot = slot_mapping[t];
       if (slot < 0) continue;  // padding token
       const int64_t blk = slot / kPageTokens;
       const int tok = (int)(slot % kPageTokens);
@@ -620,6 +619,9 @@ extern "C" int b200_splitk_silu_mul(const B200SplitK* parts, void* out, void* st
   return B200_OK;
 }
 
+// (token, head) rows from which the vectorised form is faster in a decoding step, where the other's blocks are one row each: Llama-2-7B int4, four layers, 64 tokens
+// (6144 rows) 446.8 -> 434.5 us a step; Llama-3-8B at 64 (3072) 706.8 / 705.1, at 32 403.6 / 404.3, at 9 373.0 / 375.6.
+constexpr int64_t kRopeVecRows = 4096;
 template <bool kSplitK>
 static int rope_kv_write_impl(void* qkv, const void* cos, const void* sin, const int64_t* position_ids, const int64_t* slot_mapping,
                               void* k_pool, void* v_pool, int64_t T, int n_heads, int n_kv_heads, int head_dim, int rotary_dim,
@@ -631,9 +633,9 @@ static int rope_kv_write_impl(void* qkv, const void* cos, const void* sin, const
   }
   cudaStream_t st = (cudaStream_t)stream;
   if constexpr (!kSplitK) {
-    if (T >= 256 && rotary_dim == head_dim && (head_dim == 128 || head_dim == 64) && ((uintptr_t)qkv & 15) == 0 &&
-        ((uintptr_t)cos & 15) == 0 && ((uintptr_t)sin & 15) == 0) {  // prefill-sized: the vectorised grid-stride form
-      const int64_t n_rows = T * (n_heads + 2 * n_kv_heads);
+    const int64_t n_rows = T * (n_heads + 2 * n_kv_heads);
+    if ((T >= 256 || n_rows >= kRopeVecRows) && rotary_dim == head_dim && (head_dim == 128 || head_dim == 64) && ((uintptr_t)qkv & 15) == 0 &&
+        ((uintptr_t)cos & 15) == 0 && ((uintptr_t)sin & 15) == 0 && (((uintptr_t)k_pool | (uintptr_t)v_pool) & 15) == 0) {  // the vectorised grid-stride form
       const int per_block = 256 / (head_dim / 16);
       int64_t blocks = (n_rows + per_block - 1) / per_block;
       if (blocks > 148 * 32) blocks = 148 * 32;
