@@ -25,16 +25,18 @@
 //               up to 7 % more error behind 1500 cached keys whose scores spread.)  The row's sum adds the rounded P, what the
 //               products weigh.  S of tile j is complete only after P V of tile j - 1 (issue order), so O is quiescent whenever a
 //               softmax warp runs.
-// Causality over absolute positions prunes whole key tiles.  Bound: soft-max exponentials (MUFU, 16 a cycle and SM: 1024 cycles per 128 x 128 tile,
-// as long as its products at d = 128, twice as long at d = 64), and between items the pipeline's drain.  Measured on B200 (us back to back, before: one
-// query tile of one head per CTA): 13 prompts of 300 to 2048 tokens, 32 / 8 heads, d = 128 570 -> 219; 16 x 1024 428 -> 184; 8192 1197 -> 548; d = 64, 32 / 4
-// heads 441 -> 189; 300 tokens after 1500 cached ones x 4 110 -> 66; 64 tokens x 10 17.7 -> 12.8.  An earlier form with
-// items dealt out in turn took 294 at the first of these; four more warps for the output 305 instead of 287 (the softmax warps are then compiled for 128
-// registers).
+// Causality over absolute positions prunes whole key tiles.  Bound: a row's chain.  Of the 3700 cycles between a warp's scores of one 128-key tile and of the next
+// (d = 128, both tiles of an item at work) it waits 1100 for P V and Q K^T, takes 350 for the maximum, 490 to rescale O and 1750 for the exponentials (1024 if MUFU
+// were its own); between items there is the pipeline's drain.  Measured on B200 (us back to back; before: one query tile of one head per CTA): 13 prompts of
+// 300 to 2048 tokens, 32 / 8 heads, d = 128 570 -> 218; 16 x 1024 428 -> 184; 8192 1197 -> 482; d = 64, 32 / 4 heads, 16 x 1024 140; 300 tokens after 1500 cached ones x 4
+// 110 -> 66; 64 tokens x 10 17.7 -> 12.8.  Forms that were no faster (that / this at the time): items dealt out in turn 294 / 219 at the first of these; four more warps for
+// the results 258 / 218 (compiled for 128 registers); two threads a row 245 / 225; scores of 64 keys in two places by turns 276 / 220; O rescaled between the
+// exponentials 241 / 227; a quarter of the exponentials as polynomials on the FMA units 244 / 236; at d = 64, P beside S and the next scores ahead of P V
+// 144 / 140 (16 x 1024).
 // Token-major caches differ in this: a tile is 128 / rep tokens x the rep query heads of a key head (all rows meet the same keys), an item two
 // neighbouring tiles; the softmax warps bring their tile's fp32 queries as bfloat16 themselves; P is the sum of two bfloat16 values (one alone is 2^-9
 // off, and a maximum taken over 128 keys leaves fewer weights at exactly 1 than the 16-key tiles of talk_attn_mma_kernel: prompts of 1618 and 2000 tokens,
-// 16 / 4 heads, d = 128, against float64 1.91e-3 with one value, 1.88e-3 there, 1.47e-3 with two; 90 us, 343 there, 101); key tiles start at the first
+// 16 / 4 heads, d = 128, against float64 1.91e-3 with one value, 1.88e-3 there, 1.47e-3 with two); key tiles start at the first
 // visible key; a key or value page is a box [16 tokens x 64 columns] that the copy itself swizzles; and what lies in the cache beside the keys
 // that an item's queries see (slots that were never written, another request's leavings) is zeros to the products: whole pages by copies from
 // outside the cache's rows, the rest of the first and the last visible page by the issuing warp, at most 15 rows each.
