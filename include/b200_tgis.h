@@ -35,7 +35,9 @@ void b200_debug_set_gave_up(int v); /* for tests: as if a wait had run out (1), 
 const char* b200_cuda_peek_error(void); /* debug: pending CUDA runtime error string, not cleared */
 void b200_debug_w4_flags(int flags); /* debug timing experiments (results invalid): 1 no x loads, 2 no MMAs, 4 no weight loads, 8 no dequant math */
 void b200_debug_w4_trace(void* device_buffer); /* debug: [n_ctas][64] u64 phase timestamps of int4 GEMM launches; NULL = off */
-int b200_debug_pair_plan(int kind, int64_t T, int64_t N, int64_t K, int sms, int32_t* out8); /* tests, host only: whether a launch takes the SM pairs, and how; kind 0 fp16, 1 int4, 2 bfloat16 with fp32 results; out = {taken, token tile, token tiles, feature tiles, pairs, k-blocks per stage, pieces of k, stages of a piece} */
+/* tests, host only: 1 if an fp16 call with a workspace takes the SM pairs where the chip holds clusters[d] clusters of d = 2 .. 8 CTAs, 0 if not */
+int b200_debug_f16_on_pairs(int64_t T, int64_t N, int64_t K, int sms, const int32_t* clusters9);
+int b200_debug_pair_plan(int kind, int64_t T, int64_t N, int64_t K, int sms, int32_t* out8); /* tests, host only: whether a launch takes the SM pairs (of 65 to 256 tokens: where no cluster shares a tile), and how; kind 0 fp16, 1 int4, 2 bfloat16 with fp32 results; out = {taken, token tile, token tiles, feature tiles, pairs, k-blocks per stage, pieces of k, stages of a piece} */
 int b200_debug_gemm_plan(int kind, int64_t T, int64_t N, int64_t K, int sms, int32_t* out8); /* tests, host only: stream-K plan of a launch of up to 256 (int4: 128) tokens; kind 0 fp16, 1 int4; out = {token tile, k-blocks, feature (super-)tiles, 1, units per CTA, CTAs, contributor slots, tiles per unit} */
 /* debug: per-kernel device timeline of a step.  While a buffer of `capacity` uint64 slots is attached, every kernel this
  * library enqueues is followed by a one-thread kernel storing %globaltimer (ns) into the next slot (slot 0: _begin);

@@ -40,12 +40,11 @@ __device__ __forceinline__ void gemm_store(void* y, size_t i, float v) {
 constexpr int kGemmThreads = 192;
 constexpr int kTileM = 128;  // features per tile
 constexpr int kTileK = 64;   // fp16 elements per k-block = one 128-byte swizzle row
-// Calls of more than kF16DecodeT tokens may go to the SM pairs (gemm_pair.cuh), calls of more than kF16MostT all do; between the two f16_stream_us
-// says which kernel takes less.  That model is of this kernel with its fix-up through global memory; where clusters share a tile it takes less, so the line lies
-// too far on the pairs' side of the narrower outputs.  Measured on B200 in replayed graphs (us, this kernel / pairs; * the other one is taken) at 65 tokens: 4096 ->
-// 4096 11.1 / 12.7*, 4096 -> 22016 38.8 / 38.8, 5632 -> 2048 11.0 / 16.1*, 11008 -> 4096 19.4 / 27.9, 16384 -> 2048 17.6 / 37.2, 28672 -> 2048 25.9 / 62.5, 28672 ->
-// 8192 78 / 94, 20480 -> 5120 42 / 59*, 2048 -> 2560 8.1 / 7.7; at 128: 12.3 / 12.9*, 45.0 / 41.3, 12.4 / 15.7*, 20.5 / 28.1, 19.0 / 37.5, 27.3 / 62.8, 93 / 111, 40 /
-// 62, 9.3 / 8.1; at 256: 16.0 / 15.1, 74 / 51, 15.8 / 15.8, 26.6 / 34.2*, 25.6 / 37.6*, 37.0 / 62.9, 143 / 129*, 54 / 66*, 12.8 / 9.2.
+// Calls of more than kF16DecodeT tokens may go to the SM pairs (gemm_pair.cuh), calls of more than kF16MostT all do; between the two f16_cluster_us, or
+// f16_stream_us where no cluster shares a tile, says which kernel takes less.  Measured on B200 in replayed graphs (us, this kernel / pairs) at 65 tokens: 4096 ->
+// 4096 11.1 / 12.7, 4096 -> 22016 38.8 / 38.8, 5632 -> 2048 11.0 / 16.1, 11008 -> 4096 19.4 / 27.9, 16384 -> 2048 17.6 / 37.2, 28672 -> 2048 25.9 / 62.5, 28672 ->
+// 8192 78 / 94, 20480 -> 5120 42 / 59, 2048 -> 2560 8.1 / 7.7; at 128: 12.3 / 12.9, 45.0 / 41.3, 12.4 / 15.7, 20.5 / 28.1, 19.0 / 37.5, 27.3 / 62.8, 93 / 111, 40 /
+// 62, 9.3 / 8.1; at 256: 16.0 / 15.1, 74 / 51, 15.8 / 15.8, 26.6 / 34.2, 25.6 / 37.6, 37.0 / 62.9, 143 / 129, 54 / 66, 12.8 / 9.2.
 // Up to 64 tokens the pairs take wide outputs only (feature tiles that no wave of clusters holds), from kF16PairT tokens on; us, this kernel / pairs, at 16
 // and 64 tokens: 2048 -> 11264 10.9 / 10.6 and 13.0 / 11.7, 2048 -> 32000 24.1 / 22.8 and 29.0 / 24.3, 4096 -> 12288 18.9 / 18.9 and 21.1 / 20.4, 5120 ->
 // 15360 25.8 / 26.6 and 28.4 / 28.4, 4096 -> 22016 (a wave and a sixth) 31.4 / 34.7 and 37.0 / 38.5.
@@ -435,6 +434,15 @@ static float f16_stream_us(const F16Plan& pl, int64_t T) {
   return unit * pl.units_per_cta + straddle * (4.f + (float)T * (0.0125f * contrib + 0.035f));
 }
 
+// The same where clusters of d CTAs share a tile: its own k-blocks, at the rate of a CTA or of the memory, and the end of a tile, which grows with the tokens whose sums go
+// through shared memory.  Fitted to the times at kF16DecodeT: within 9 % of all of them.  (By the model of the fix-up through global memory too many went to the pairs; us, so /
+// now: 5632 -> 2048 at 65 and 200 tokens 15.5 / 10.7, 16.1 / 15.2; 11008 -> 4096 at 200 35.0 / 26.8; 8192 -> 4096 at 128 23.2 / 18.3; 20480 -> 5120 at 65 53.8 / 40.7.)
+static float f16_cluster_us(int64_t T, int64_t N, int64_t K, int d) {
+  const int64_t nkb = (K + kTileK - 1) / kTileK, ctas = (N + kTileM - 1) / kTileM * d;
+  const float unit = T <= 128 ? fmaxf(0.26f, 0.0025f * ctas) : fmaxf(0.355f, 0.0031f * ctas);
+  return unit * ((nkb + d - 1) / d) + 4.8f + 0.0212f * T;
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -465,7 +473,7 @@ extern "C" int b200_debug_gemm_plan(int kind, int64_t T, int64_t N, int64_t K, i
 
 // tests (no GPU needed): out[8] = {1 if a launch (with a workspace) takes the SM pairs, token tile, token tiles, feature tiles, SM pairs, k-blocks per
 // stage, pieces of k, stages of a piece}.  kind 0 = fp16 weights (and bfloat16 with results of 16 bits), 1 = int4, 2 = bfloat16 with fp32 results
-static bool f16_takes_pairs(int fmt, int64_t T, int64_t N, int64_t K, bool workspace, int sms);
+static bool f16_takes_pairs(int fmt, int64_t T, int64_t N, int64_t K, bool workspace, int sms, const int* clusters);
 static int f16_pieces(int64_t T, int64_t N, int64_t K, int sms);
 extern "C" int b200_debug_pair_plan(int kind, int64_t T, int64_t N, int64_t K, int sms, int32_t* out) {
   if (!out || T <= 0 || N <= 0 || K <= 0 || sms <= 1 || kind < 0 || kind > 2) {
@@ -474,10 +482,19 @@ extern "C" int b200_debug_pair_plan(int kind, int64_t T, int64_t N, int64_t K, i
   }
   const int64_t n_kb = kind == 1 ? 2 * ((K + 127) / 128) : (K + kPairK - 1) / kPairK;
   const PairPlan pl = pair_plan(T, N, n_kb, kind == 1, sms, kind == 1 ? 1 : f16_pieces(T, N, K, sms));
-  const int taken = kind == 1 ? T > kW4DecodeT : f16_takes_pairs(kind == 2 ? 2 : 0, T, N, K, true, sms);
+  const int taken = kind == 1 ? T > kW4DecodeT : f16_takes_pairs(kind == 2 ? 2 : 0, T, N, K, true, sms, nullptr);
   const int32_t v[8] = {taken, pl.tn, pl.n_tt, pl.n_m, pl.n_pairs, pl.per_stage, pl.pieces, pl.piece_stages};
   for (int i = 0; i < 8; ++i) out[i] = v[i];
   return B200_OK;
+}
+
+// tests: whether an fp16 call of T tokens with a workspace goes to the SM pairs on a chip that holds clusters[d] clusters of d = 2 .. 8 CTAs
+extern "C" int b200_debug_f16_on_pairs(int64_t T, int64_t N, int64_t K, int sms, const int32_t* clusters) {
+  if (!clusters || T <= 0 || N <= 0 || K <= 0 || sms <= 1) {
+    b200_set_last_error("debug_f16_on_pairs: bad arguments");
+    return B200_ERR_ARG;
+  }
+  return f16_takes_pairs(0, T, N, K, true, sms, clusters) ? 1 : 0;
 }
 
 extern "C" int64_t b200_gemm_workspace_bytes(int64_t T, int64_t N, int64_t K) {
@@ -502,8 +519,8 @@ extern "C" int64_t b200_gemm_workspace_bytes_max(int64_t N, int64_t K) {
   return best;
 }
 
-// whether a call's kernel is that of gemm_pair.cuh
-static bool f16_takes_pairs(int fmt, int64_t T, int64_t N, int64_t K, bool workspace, int sms) {
+// whether a call's kernel is that of gemm_pair.cuh; clusters: as f16_cluster, for calls of more than kF16DecodeT tokens (NULL: none)
+static bool f16_takes_pairs(int fmt, int64_t T, int64_t N, int64_t K, bool workspace, int sms, const int* clusters) {
   if (T <= kF16PairT || (fmt == 2 && T <= kF16MostT)) return false;
   if (T > kF16MostT || (!workspace && T > kF16DecodeT)) return true;
   const F16Plan pl = plan_f16(T, N, K, sms);
@@ -514,7 +531,8 @@ static bool f16_takes_pairs(int fmt, int64_t T, int64_t N, int64_t K, bool works
     return f16_cluster(N, K, f16_clusters()) == 0 && workspace && waves <= 2 && (waves == 1 || n_m * 5 >= waves * pairs * 4);
   }
   if ((int64_t)pl.n_tiles_n * 4 > kCounterBytes) return true;
-  return pair_plan(T, N, pl.nkb, false, sms).us <= f16_stream_us(pl, T);
+  const int d = clusters ? f16_cluster(N, K, clusters) : 0;
+  return pair_plan(T, N, pl.nkb, false, sms).us <= (d ? f16_cluster_us(T, N, K, d) : f16_stream_us(pl, T));
 }
 // pieces of k on the pairs: as many as this file's kernel cuts a call of its size into
 static int f16_pieces(int64_t T, int64_t N, int64_t K, int sms) {
@@ -571,7 +589,7 @@ static int gemm_f16_impl(const void* x, const void* w, const void* bias, void* y
     b200_set_last_error("gemm_f16_deferred: needs a workspace, T <= 256 (one token tile) and N % 8 == 0");
     return B200_ERR_UNSUPPORTED;
   }
-  if (!defer && f16_takes_pairs(FMT, T, N, K, workspace != nullptr, b200_num_sms())) {
+  if (!defer && f16_takes_pairs(FMT, T, N, K, workspace != nullptr, b200_num_sms(), f16_clusters())) {
     PairParams pp = {};
     pp.y = y;
     pp.bias = bias;
