@@ -58,3 +58,36 @@ def test_gate_and_up_with_silu(I, K, T):
     room = torch.full((T * I + 2,), 7.0, dtype=torch.float16, device=DEV)
     assert torch.equal(_whole(x, pairs, room[1:-1].view(T, I), 2 * I, 32, bias, ops.W4_LAYOUT_GATE_UP, 1), one)
     assert float(room[0]) == 7.0 == float(room[-1])
+
+
+# 16 super-tiles of eight CTAs each, 81 that 148 CTAs straddle, and gate and up
+@pytest.mark.parametrize("N,K,act", [(4096, 4096, 0), (20736, 4096, 0), (4096, 4096, 1)])
+@pytest.mark.parametrize("T", [4, 9, 64])
+def test_shared_super_tiles_off_any_four_halves(N, K, act, T):
+    """with a workspace, so that CTAs share super-tiles: a y that starts off any four halves gets the bits of one that does not"""
+    import tgis_b200  # noqa: F401
+    from tgis_b200 import _lib, ops
+    lib, g = _lib.load(), torch.Generator(device=DEV).manual_seed(N + K + T)
+    qweight, qzeros, scales, w = _weights(g, N, K, 128)
+    x, bias = torch.randn(T, K, generator=g, device=DEV).half(), torch.randn(N, generator=g, device=DEV).half()
+    layout = ops.W4_LAYOUT_GATE_UP if act else 0
+    packed = ops.gptq_pack(qweight, qzeros, scales, 128, layout)
+    ws = torch.zeros(lib.b200_gemm_workspace_bytes(T, N, K), dtype=torch.uint8, device=DEV)
+    cols = N // 2 if act else N
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+
+    def call(y, x):
+        st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        assert lib.b200_gemm_w4a16_ex(p(x), p(packed), p(bias), p(y), T, N, K, 128, layout, act, p(ws), st) == 0
+        return y
+    room = torch.full((T * cols + 2,), 7.0, dtype=torch.float16, device=DEV)
+    off = call(room[1:-1].view(T, cols), x)
+    assert float(room[0]) == 7.0 == float(room[-1])
+    if T > 8:   # (up to eight tokens a y on four halves goes to another kernel)
+        assert torch.equal(off, call(torch.empty(T, cols, dtype=torch.float16, device=DEV), x))
+    if not act:
+        return _near(off, x, w, bias)
+    sums, size = x.double() @ w + bias.double(), x.double().abs() @ w.abs()
+    (gate, up), (d_gate, d_up) = sums.chunk(2, 1), (2 ** -11 * sums.abs() + K * 2 ** -24 * size).chunk(2, 1)
+    silu = torch.nn.functional.silu(gate)   # its slope is 1.1 at the most; it and the product round once each
+    assert bool(((off.double() - silu * up).abs() <= 1.1 * d_gate * (up.abs() + d_up) + silu.abs() * d_up + 2 ** -10 * (silu * up).abs() * 1.01 + 2 ** -20).all())

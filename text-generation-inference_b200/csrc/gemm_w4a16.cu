@@ -138,6 +138,16 @@ struct W4Params {
   unsigned long long* trace;  // debug: per-CTA phase timestamps (globaltimer ns), NULL in production
 };
 
+// four features of a token at y; p.y may start off any four halves (rows are a multiple of 32 long, so the first address says it for all)
+__device__ __forceinline__ void w4_store(const W4Params& p, __half* y, uint2 o) {
+  if ((reinterpret_cast<uintptr_t>(p.y) & 7) == 0) {
+    *reinterpret_cast<uint2*>(y) = o;
+  } else {
+    const __half* h = reinterpret_cast<const __half*>(&o);
+    for (int j = 0; j < 4; ++j) y[j] = h[j];
+  }
+}
+
 // The end of a CTA's last super-tile when nobody shares it: the epilogue warps leave its fp32 sums in shared memory ([token][kW4SumPitch]) and all 24 warps
 // write the outputs, four features of a token each.  By the four epilogue warps alone, a feature per thread, the SiLU (then with divisions, a branch each, so one
 // after the other) took 1.9 us at 16 tokens, 7.9 at 64 and 15 at 128 behind the last product (4096 -> 28672: 26.8 us of which 7.9 -> 21.5 with 2.4; 128 tokens 42.6 -> 32).
@@ -167,13 +177,7 @@ __device__ __forceinline__ void w4_finish(const W4Params& p, int sup, int per_to
     } else {
       o = make_uint2(pack_half2(s.x, s.y), pack_half2(s.z, s.w));
     }
-    __half* y = &p.y[(size_t)tok * p.ldy + col];
-    if ((reinterpret_cast<uintptr_t>(p.y) & 7) == 0) {
-      *reinterpret_cast<uint2*>(y) = o;
-    } else {
-      const __half* h = reinterpret_cast<const __half*>(&o);
-      for (int j = 0; j < 4; ++j) y[j] = h[j];
-    }
+    w4_store(p, &p.y[(size_t)tok * p.ldy + col], o);
   }
 }
 
@@ -556,7 +560,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
           uint2 o;
           o.x = pack_half2(acc.x, acc.y);
           o.y = pack_half2(acc.z, acc.w);
-          *reinterpret_cast<uint2*>(&p.y[(size_t)tt * p.ldy + nn]) = o;
+          w4_store(p, &p.y[(size_t)tt * p.ldy + nn], o);
         }
       }
     } else {
@@ -590,7 +594,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
           u.x += __half2float(p.bias[nu]); u.y += __half2float(p.bias[nu + 1]); u.z += __half2float(p.bias[nu + 2]); u.w += __half2float(p.bias[nu + 3]);
         }
         __half o[4] = {silu_mul_f16(g.x, u.x), silu_mul_f16(g.y, u.y), silu_mul_f16(g.z, u.z), silu_mul_f16(g.w, u.w)};
-        *reinterpret_cast<uint2*>(&p.y[(size_t)tt * p.ldy + nn]) = *reinterpret_cast<uint2*>(o);
+        w4_store(p, &p.y[(size_t)tt * p.ldy + nn], *reinterpret_cast<uint2*>(o));
       }
     }
     W4_TRACE(42 + f * 3, 0);
