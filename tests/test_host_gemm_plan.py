@@ -103,9 +103,31 @@ def test_int4_decode_plans_fill_the_gpu(lib):
     assert p["nkb"] % p["units_per_cta"] == 0, p
 
 
+HELD = (0, 0, 74, 45, 33, 26, 22, 15, 15)   # clusters of 2 .. 8 CTAs that B200 holds
+
+
+def _w4_plan(lib, T, N, K, workspace=1, held=HELD):
+    out = (ctypes.c_int32 * 8)()
+    assert lib.b200_debug_w4_plan(T, N, K, SMS, workspace, (ctypes.c_int32 * 9)(*held), out) == 0, lib.b200_last_error()
+    return dict(zip(("TN", "nkb", "tiles", "cluster", "units_per_cta", "ctas", "contrib", "r"), out))
+
+
+@pytest.mark.parametrize("N,K,cluster", [(2048, 5632, 8), (11264, 2048, 3), (12288, 4096, 2), (4096, 4096, 0), (22016, 4096, 0)])
+@pytest.mark.parametrize("T", [9, 64, 128])
+def test_int4_clusters(lib, N, K, cluster, T):
+    """which shapes' super-tiles clusters share; one wave of them holds all, and each CTA has a part of k"""
+    p = _w4_plan(lib, T, N, K)
+    assert p["cluster"] == cluster, p
+    if cluster:
+        assert p["tiles"] <= HELD[cluster] and p["ctas"] == p["tiles"] * cluster and p["contrib"] == 1 and p["units_per_cta"] == -(-p["nkb"] // cluster), p
+    none = _w4_plan(lib, T, N, K, held=(0,) * 9)
+    assert none["cluster"] == 0 and [none[k] for k in ("units_per_cta", "ctas", "contrib")] == [_plan(lib, 1, T, N, K)[k] for k in ("units_per_cta", "ctas", "contrib")]
+
+
 def test_bad_arguments(lib):
     out = (ctypes.c_int32 * 8)()
     assert lib.b200_debug_gemm_plan(2, 1, 128, 128, SMS, out) != 0
     assert lib.b200_debug_gemm_plan(0, 0, 128, 128, SMS, out) != 0
     # no launch of the weight-streaming kernels has so many tokens
     assert lib.b200_debug_gemm_plan(0, 257, 128, 128, SMS, out) != 0 and lib.b200_debug_gemm_plan(1, 129, 128, 128, SMS, out) != 0
+    assert lib.b200_debug_w4_plan(129, 128, 128, SMS, 1, (ctypes.c_int32 * 9)(), out) != 0 and lib.b200_debug_w4_plan(9, 128, 128, SMS, 1, (ctypes.c_int32 * 9)(), None) != 0

@@ -24,6 +24,7 @@ SIGNATURES = {
     "b200_debug_step_trace_begin": (None, [_P]),
     "b200_debug_step_trace_names": (_I, [c_char_p, _L]),
     "b200_debug_gemm_plan": (_I, [_I, _L, _L, _L, _I, _P]),
+    "b200_debug_w4_plan": (_I, [_L, _L, _L, _I, _I, _P, _P]),
     "b200_debug_f16_on_pairs": (_I, [_L, _L, _L, _I, _P]),
     "b200_debug_pair_plan": (_I, [_I, _L, _L, _L, _I, _P]),
     "b200_rmsnorm_residual": (_I, [_P, _P, _P, _P, _P, _L, _L, _F, _P]),

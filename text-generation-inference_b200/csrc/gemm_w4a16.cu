@@ -845,7 +845,8 @@ static W4Plan launch_plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool has_
   return pl;
 }
 
-// tests (no GPU needed): out = {TN, k-blocks, super-tiles, 1, super-units per CTA, CTAs, contributor slots, R}
+// tests (no GPU needed): the cut through a workspace that is taken where no cluster shares super-tiles; out = {TN, k-blocks, super-tiles, 1, super-units per CTA,
+// CTAs, contributor slots, R}
 void b200_w4_plan_debug(int64_t T, int64_t N, int64_t K, int sms, int32_t* out) {
   const W4Plan pl = launch_plan_w4(T, N, K, sms, true);
   const int32_t v[8] = {pl.TN, pl.nkb, pl.n_super, 1, pl.su_per_cta, pl.n_ctas, pl.max_contrib, kW4R};
@@ -913,6 +914,19 @@ static const int* w4_clusters() {
     }
   } table;
   return table.n;
+}
+
+// tests: how an int4 call of up to kW4DecodeT tokens is cut (those that gemm_w4_few.cuh takes too) on a chip that holds clusters[d] clusters of d = 2 .. 8 CTAs; NULL: the
+// present device's
+extern "C" int b200_debug_w4_plan(int64_t T, int64_t N, int64_t K, int sms, int workspace, const int32_t* clusters, int32_t* out) {
+  if (!out || T <= 0 || T > kW4DecodeT || N <= 0 || K <= 0 || sms <= 0) {
+    b200_set_last_error("debug_w4_plan: bad arguments");
+    return B200_ERR_ARG;
+  }
+  const W4Plan pl = launch_plan_w4(T, N, K, sms, workspace != 0, false, clusters ? clusters : w4_clusters());
+  const int32_t v[8] = {pl.TN, pl.nkb, pl.n_super, pl.cluster, pl.su_per_cta, pl.n_ctas, pl.max_contrib, kW4R};
+  for (int i = 0; i < 8; ++i) out[i] = v[i];
+  return B200_OK;
 }
 
 // packed: output of b200_gptq_pack[_ex] for the same (K, N, groupsize, layout).
