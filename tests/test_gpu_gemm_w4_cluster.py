@@ -41,6 +41,20 @@ def test_shared_super_tiles(N, K, gs, cluster, T):
     assert float(room[0]) == 7.0 == float(room[-1])
 
 
+@pytest.mark.parametrize("T", [9, 17, 64, 128])
+def test_without_a_workspace(T):
+    """clusters of six share super-tiles that eight CTAs share through a workspace"""
+    import tgis_b200  # noqa: F401
+    from tgis_b200 import ops
+    N = K = 4096
+    assert (_cluster(T, N, K), _cluster(T, N, K, workspace=0)) == (0, 6)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    qweight, qzeros, scales, w = _weights(g, N, K, 128)
+    x, bias = torch.randn(T, K, generator=g, device=DEV).half(), torch.randn(N, generator=g, device=DEV).half()
+    packed = ops.gptq_pack(qweight, qzeros, scales, 128)
+    _near(_whole(x, packed, torch.empty(T, N, dtype=torch.float16, device=DEV), N, 128, bias), x, w, bias)
+
+
 @pytest.mark.parametrize("I,K", [(1024, 5632), (5632, 2048)])
 @pytest.mark.parametrize("T", [9, 17, 64, 128])
 def test_gate_and_up_with_silu(I, K, T):

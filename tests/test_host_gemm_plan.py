@@ -6,6 +6,9 @@ every (tile, k-block) unit belongs to exactly one CTA, and the workspace the cal
 this path serves (Llama-2/3, TinyLlama, GPT-NeoX) at tensor-parallel degrees 1, 2, 4, 8 and decode batch sizes 1 ... 256.
 """
 import ctypes
+import os
+import subprocess
+import sys
 
 import pytest
 
@@ -122,6 +125,18 @@ def test_int4_clusters(lib, N, K, cluster, T):
         assert p["tiles"] <= HELD[cluster] and p["ctas"] == p["tiles"] * cluster and p["contrib"] == 1 and p["units_per_cta"] == -(-p["nkb"] // cluster), p
     none = _w4_plan(lib, T, N, K, held=(0,) * 9)
     assert none["cluster"] == 0 and [none[k] for k in ("units_per_cta", "ctas", "contrib")] == [_plan(lib, 1, T, N, K)[k] for k in ("units_per_cta", "ctas", "contrib")]
+
+
+def test_int4_clusters_beside_what_else_can_run(lib):
+    """without a workspace the other cut is whole super-tiles, whatever a cut through a workspace would take; a cut that is forced stays"""
+    assert _w4_plan(lib, 64, 4096, 4096)["cluster"] == 0 and _w4_plan(lib, 64, 4096, 4096, workspace=0)["cluster"] == 6
+    few = _w4_plan(lib, 64, 2048, 256, workspace=0)   # two k-blocks: not worth adding up
+    assert few["cluster"] == 0 and few["ctas"] == few["tiles"] == 8
+    code = ("import ctypes, tgis_b200; from tgis_b200 import _lib; out = (ctypes.c_int32 * 8)(); held = (ctypes.c_int32 * 9)(*%r)\n"
+            "assert _lib.load().b200_debug_w4_plan(64, 2048, 5632, %d, 1, held, out) == 0; print(out[3], out[4])" % (HELD, SMS))
+    for su, want in (("0", "8 6"), ("4", "0 4")):
+        r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, env=dict(os.environ, B200_W4_SU=su), cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+        assert r.stdout.strip() == want, r.stdout + r.stderr
 
 
 def test_bad_arguments(lib):

@@ -692,7 +692,11 @@ static int w4_nkb(int64_t K) {
 struct W4Plan {
   int TN, nkb, n_super, su_per_cta, n_ctas, max_contrib;
   int cluster;   // > 0: so many CTAs share a super-tile and add their sums through shared memory; nothing goes to a workspace
+  bool forced;   // B200_W4_SU's cut
 };
+
+constexpr float kW4SuUs = 0.35f * kW4R;   // us that a CTA takes for a super-unit
+static float w4_whole_us(int nkb) { return kW4SuUs * nkb + 1.f; }   // ... for a super-tile that it has alone
 
 // One token tile (T <= kW4DecodeT): how many super-units per CTA.  Candidates are the balanced stream-K cut (every SM the same
 // number of units, but most CTAs then straddle two super-tiles: two fix-ups at the tail) and the aligned cuts nkb / d
@@ -713,8 +717,9 @@ static W4Plan plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool defer = fal
   // deferred reduction (the consumer kernel sums the partials): no in-kernel fix-up, a CTA that straddles two super-tiles only
   // pays a mid-loop accumulator drain (~1 us)
   auto cost = [&](int su, bool aligned, int d) {
-    const float fix = defer ? (aligned ? 0.f : 1.0f) : (aligned ? (d == 1 ? 1.0f : 4.5f + 0.2f * d) : 10.0f);
-    return 0.35f * kW4R * su + fix;
+    if (!defer && aligned && d == 1) return w4_whole_us(su);
+    const float fix = defer ? (aligned ? 0.f : 1.0f) : (aligned ? 4.5f + 0.2f * d : 10.0f);
+    return kW4SuUs * su + fix;
   };
   float best_cost = cost(best, pl.nkb % best == 0, pl.nkb / best);
   for (int d = 1; d <= 8; d *= 2) {
@@ -730,7 +735,8 @@ static W4Plan plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool defer = fal
     const char* e = getenv("B200_W4_SU");
     env_su = e ? atoi(e) : 0;
   }
-  if (env_su > 0 && (total + env_su - 1) / env_su <= sms) pl.su_per_cta = env_su;
+  pl.forced = env_su > 0 && (total + env_su - 1) / env_su <= sms;
+  if (pl.forced) pl.su_per_cta = env_su;
   pl.n_ctas = (total + pl.su_per_cta - 1) / pl.su_per_cta;
   pl.max_contrib = (pl.nkb + pl.su_per_cta - 1) / pl.su_per_cta + 1;
   if (pl.su_per_cta % pl.nkb == 0) pl.max_contrib = 1;
@@ -813,7 +819,7 @@ extern "C" int b200_gptq_pack(const void* qweight, const void* qzeros, const voi
 
 // bytes of split-K partials the int4 GEMM may write for this shape (the tile counters sit in the first 64 KiB)
 // The plan a launch uses: the stream-K cut needs the workspace (partials + one counter pair per super-tile) and every CTA
-// resident at once (the fix-up spins on its peers); otherwise each CTA takes whole super-tiles.
+// resident at once (the fix-up spins on its peers); otherwise each CTA takes whole super-tiles.  Clusters are compared with whichever of the two would run.
 // clusters[d]: clusters of d CTAs that the chip holds (NULL: none).  The largest cluster whose super-tiles all fit in one wave, where it costs less: adding up
 // through shared memory takes 2.5 us and 0.8 for each CTA whose sums are read (64 tokens: 64 KB of them).  That is less than a cut that straddles
 // super-tiles, more so the more contributors one has, and about as much as an aligned cut's, which has 8 contributors where the chip holds 15 clusters of
@@ -823,23 +829,22 @@ extern "C" int b200_gptq_pack(const void* qweight, const void* qzeros, const voi
 static W4Plan launch_plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool has_workspace, bool defer = false, const int* clusters = nullptr) {
   float cost;
   W4Plan pl = plan_w4(T, N, K, sms, defer, &cost);
-  if (!defer && clusters) {
-    int d = kW4MostCluster;
-    while (d > 1 && (d > pl.nkb || clusters[d] < pl.n_super)) --d;
-    const int su = (pl.nkb + d - 1) / d;
-    if (pl.nkb % pl.su_per_cta != 0) cost += 0.2f * pl.max_contrib;
-    if (d > 1 && 0.35f * kW4R * su + 2.5f + 0.8f * d < cost) {
-      pl.cluster = d;
-      pl.su_per_cta = su;
-      pl.n_ctas = pl.n_super * d;
-      pl.max_contrib = 1;
-      return pl;
-    }
-  }
   if (defer) return pl;  // the caller checked: one token tile, workspace present; no counters, no co-residency requirement
   if (pl.max_contrib > 1 && (!has_workspace || (int64_t)pl.n_super * 8 > kW4CounterBytes || pl.n_ctas > sms)) {
     pl.su_per_cta = pl.nkb;
     pl.n_ctas = pl.n_super;
+    pl.max_contrib = 1;
+    cost = w4_whole_us(pl.nkb);
+  }
+  if (!clusters || pl.forced) return pl;
+  int d = kW4MostCluster;
+  while (d > 1 && (d > pl.nkb || clusters[d] < pl.n_super)) --d;
+  const int su = (pl.nkb + d - 1) / d;
+  if (pl.su_per_cta < pl.nkb && pl.nkb % pl.su_per_cta != 0) cost += 0.2f * pl.max_contrib;
+  if (d > 1 && kW4SuUs * su + 2.5f + 0.8f * d < cost) {
+    pl.cluster = d;
+    pl.su_per_cta = su;
+    pl.n_ctas = pl.n_super * d;
     pl.max_contrib = 1;
   }
   return pl;
