@@ -139,6 +139,12 @@ def test_int4_clusters_beside_what_else_can_run(lib):
         assert r.stdout.strip() == want, r.stdout + r.stderr
 
 
+def test_int4_counters_fit(lib):
+    """a counter of four bytes for each super-tile that CTAs share, in the workspace's first 64 KB; where they don't fit nothing is shared"""
+    fit, above = _plan(lib, 1, 64, 256 * 16384, 512), _plan(lib, 1, 64, 256 * 16385, 512)
+    assert fit["contrib"] > 1 and fit["units_per_cta"] % fit["nkb"] != 0 and above["contrib"] == 1 and above["ctas"] == 16385
+
+
 def test_bad_arguments(lib):
     out = (ctypes.c_int32 * 8)()
     assert lib.b200_debug_gemm_plan(2, 1, 128, 128, SMS, out) != 0

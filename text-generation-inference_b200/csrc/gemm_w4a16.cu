@@ -818,7 +818,7 @@ extern "C" int b200_gptq_pack(const void* qweight, const void* qzeros, const voi
 }
 
 // bytes of split-K partials the int4 GEMM may write for this shape (the tile counters sit in the first 64 KiB)
-// The plan a launch uses: the stream-K cut needs the workspace (partials + one counter pair per super-tile) and every CTA
+// The plan a launch uses: the stream-K cut needs the workspace (partials + one counter per super-tile) and every CTA
 // resident at once (the fix-up spins on its peers); otherwise each CTA takes whole super-tiles.  Clusters are compared with whichever of the two would run.
 // clusters[d]: clusters of d CTAs that the chip holds (NULL: none).  The largest cluster whose super-tiles all fit in one wave, where it costs less: adding up
 // through shared memory takes 2.5 us and 0.8 for each CTA whose sums are read (64 tokens: 64 KB of them).  That is less than a cut that straddles
@@ -830,7 +830,7 @@ static W4Plan launch_plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool has_
   float cost;
   W4Plan pl = plan_w4(T, N, K, sms, defer, &cost);
   if (defer) return pl;  // the caller checked: one token tile, workspace present; no counters, no co-residency requirement
-  if (pl.max_contrib > 1 && (!has_workspace || (int64_t)pl.n_super * 8 > kW4CounterBytes || pl.n_ctas > sms)) {
+  if (pl.max_contrib > 1 && (!has_workspace || (int64_t)pl.n_super * (int64_t)sizeof(unsigned) > kW4CounterBytes || pl.n_ctas > sms)) {
     pl.su_per_cta = pl.nkb;
     pl.n_ctas = pl.n_super;
     pl.max_contrib = 1;
