@@ -127,6 +127,15 @@ def test_int4_clusters(lib, N, K, cluster, T):
     assert none["cluster"] == 0 and [none[k] for k in ("units_per_cta", "ctas", "contrib")] == [_plan(lib, 1, T, N, K)[k] for k in ("units_per_cta", "ctas", "contrib")]
 
 
+@pytest.mark.parametrize("K,N,T,clusters", [(28672, 8192, 9, 0), (28672, 8192, 32, 0), (14336, 10240, 32, 0), (14336, 10240, 128, 1), (11008, 10240, 9, 0), (11008, 10240, 128, 1),
+                                            (8192, 10240, 16, 0), (8192, 12288, 9, 0), (11008, 1024, 32, 1), (5632, 2048, 9, 1), (5632, 2048, 128, 1)])
+def test_int4_clusters_by_tokens(lib, K, N, T, clusters):
+    """on the side that took less on B200, where the other cut straddles super-tiles"""
+    none = _plan(lib, 1, T, N, K)
+    assert none["nkb"] % none["units_per_cta"] != 0
+    assert (_w4_plan(lib, T, N, K)["cluster"] > 0) == clusters
+
+
 def test_int4_clusters_beside_what_else_can_run(lib):
     """without a workspace the other cut is whole super-tiles, whatever a cut through a workspace would take; a cut that is forced stays"""
     assert _w4_plan(lib, 64, 4096, 4096)["cluster"] == 0 and _w4_plan(lib, 64, 4096, 4096, workspace=0)["cluster"] == 6

@@ -820,12 +820,21 @@ extern "C" int b200_gptq_pack(const void* qweight, const void* qzeros, const voi
 // bytes of split-K partials the int4 GEMM may write for this shape (the tile counters sit in the first 64 KiB)
 // The plan a launch uses: the stream-K cut needs the workspace (partials + one counter per super-tile) and every CTA
 // resident at once (the fix-up spins on its peers); otherwise each CTA takes whole super-tiles.  Clusters are compared with whichever of the two would run.
-// clusters[d]: clusters of d CTAs that the chip holds (NULL: none).  The largest cluster whose super-tiles all fit in one wave, where it costs less: adding up
-// through shared memory takes 2.5 us and 0.8 for each CTA whose sums are read (64 tokens: 64 KB of them).  That is less than a cut that straddles
-// super-tiles, more so the more contributors one has, and about as much as an aligned cut's, which has 8 contributors where the chip holds 15 clusters of
-// 8 or fewer of more CTAs.  us, through global memory / clusters, at 9, 64 and 128 tokens: 5632 -> 2048 (clusters of 8) 9.9 / 7.3, 13.2 / 10.2, 17.8 / 15.5; 4096 ->
-// 12288 (of 2) 12.8 / 12.2, 16.2 / 15.4, 23.0 / 22.1; the other side of the line: 4096 -> 4096 (of 6) 7.4 / 8.1, 9.3 / 11.4, 12.7 / 15.8; 14336 -> 4096 12.6 / 14.3,
-// 14.5 / 17.9, 20.1 / 25.0; 4096 -> 6144 (of 5) 8.7 / 9.4, 11.3 / 12.9, 15.4 / 17.2.
+// clusters[d]: clusters of d CTAs that the chip holds (NULL: none).  The largest cluster whose super-tiles all fit in one wave, where it takes less.  Against whole super-tiles
+// and aligned cuts, in the units of plan_w4: adding up through shared memory takes 2.5 us and 0.8 for each CTA whose sums are read, about as much as an aligned cut's
+// fix-up, which has 8 contributors where the chip holds 15 clusters of 8 or fewer of more CTAs.  Us, through global memory / clusters, at 9, 64 and 128 tokens: 4096 ->
+// 12288 (of 2) 12.2 / 12.1, 15.9 / 15.2, 23.0 / 21.6; 5120 -> 5120 (of 7) 8.9 / 8.6, 11.5 / 11.6, 16.2 / 16.3; the other side: 4096 -> 4096 (of 6) 6.9 / 7.2, 9.1 / 10.4,
+// 12.5 / 14.7; 4096 -> 6144 (of 5) 8.3 / 8.6, 11.0 / 11.7, 15.1 / 15.9.
+// Against cuts that straddle super-tiles (w4_clusters_less): few tokens, whose fix-up is short, against the SMs that clusters leave idle.
+// 5632 -> 2048 (of 8) 8.3 / 6.7, 11.3 / 9.9, 15.8 / 14.7; 28672 -> 8192 (of 4) 29.4 / 31.9, 38.0 / 37.7, 56.5 / 54.7; 14336 -> 10240 (of 3) 21.8 / 23.4, 27.2 / 26.5, 39.4 / 37.2.
+// In 1133 measured calls with clusters to choose, what is taken is 0.5 % slower on average than the better of the two; 26 take 1 to 6 % more than
+// without clusters, one 22 % (12544 -> 11392 at 32 tokens, 22.7 / 27.8: 45 clusters, as many as the chip holds, whose time varies from call to call).
+// us by which clusters of d CTAs, su super-units each, differ from a cut that straddles super-tiles, below 0; fitted to 570 calls of 9 to 128 tokens on B200: a super-unit's
+// time at the token tile, a share of the memory for each CTA, the end of a super-tile
+static bool w4_clusters_less(int64_t T, const W4Plan& cut, int d, int su) {
+  const float unit = cut.TN <= 32 ? 0.44f : cut.TN <= 64 ? 0.48f : 0.71f;
+  return unit * (su - cut.su_per_cta) + 0.049f * (cut.n_super * d - cut.n_ctas) + 0.4f + (0.0067f * d - 0.06f) * T < 0.f;
+}
 static W4Plan launch_plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool has_workspace, bool defer = false, const int* clusters = nullptr) {
   float cost;
   W4Plan pl = plan_w4(T, N, K, sms, defer, &cost);
@@ -840,8 +849,8 @@ static W4Plan launch_plan_w4(int64_t T, int64_t N, int64_t K, int sms, bool has_
   int d = kW4MostCluster;
   while (d > 1 && (d > pl.nkb || clusters[d] < pl.n_super)) --d;
   const int su = (pl.nkb + d - 1) / d;
-  if (pl.su_per_cta < pl.nkb && pl.nkb % pl.su_per_cta != 0) cost += 0.2f * pl.max_contrib;
-  if (d > 1 && kW4SuUs * su + 2.5f + 0.8f * d < cost) {
+  const bool straddles = pl.su_per_cta < pl.nkb && pl.nkb % pl.su_per_cta != 0;
+  if (d > 1 && (straddles ? w4_clusters_less(T, pl, d, su) : kW4SuUs * su + 2.5f + 0.8f * d < cost)) {
     pl.cluster = d;
     pl.su_per_cta = su;
     pl.n_ctas = pl.n_super * d;
