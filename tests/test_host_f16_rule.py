@@ -17,12 +17,14 @@ def on_pairs():
 
 @pytest.mark.parametrize("T,K,N", [(65, 4096, 4096), (65, 5632, 2048), (65, 11008, 4096), (65, 16384, 2048), (65, 28672, 2048), (65, 20480, 5120), (128, 4096, 4096),
                                    (128, 5632, 2048), (128, 11008, 4096), (128, 16384, 2048), (128, 28672, 2048), (128, 20480, 5120), (256, 11008, 4096),
-                                   (256, 16384, 2048), (256, 28672, 2048), (256, 20480, 5120)])
+                                   (256, 16384, 2048), (256, 28672, 2048), (256, 20480, 5120), (65, 28672, 8192), (128, 28672, 8192), (256, 28672, 8192), (65, 5632, 9216),
+                                   (128, 8192, 9216)])
 def test_streamed(on_pairs, T, K, N):
     assert on_pairs(T, K, N) == 0
 
 
-@pytest.mark.parametrize("T,K,N", [(128, 2048, 2560), (256, 2048, 2560), (256, 4096, 4096), (128, 4096, 22016), (256, 4096, 22016), (257, 11008, 4096), (200, 2048, 2048)])
+@pytest.mark.parametrize("T,K,N", [(128, 2048, 2560), (256, 2048, 2560), (256, 4096, 4096), (128, 4096, 22016), (256, 4096, 22016), (257, 11008, 4096), (200, 2048, 2048), (224, 24576, 6144), (192, 16384, 8192),
+                                   (224, 8192, 8192)])
 def test_on_pairs(on_pairs, T, K, N):
     assert on_pairs(T, K, N) == 1
 

@@ -42,9 +42,9 @@ constexpr int kTileM = 128;  // features per tile
 constexpr int kTileK = 64;   // fp16 elements per k-block = one 128-byte swizzle row
 // Calls of more than kF16DecodeT tokens may go to the SM pairs (gemm_pair.cuh), calls of more than kF16MostT all do; between the two f16_cluster_us, or
 // f16_stream_us where no cluster shares a tile, says which kernel takes less.  Measured on B200 in replayed graphs (us, this kernel / pairs) at 65 tokens: 4096 ->
-// 4096 11.1 / 12.7, 4096 -> 22016 38.8 / 38.8, 5632 -> 2048 11.0 / 16.1, 11008 -> 4096 19.4 / 27.9, 16384 -> 2048 17.6 / 37.2, 28672 -> 2048 25.9 / 62.5, 28672 ->
-// 8192 78 / 94, 20480 -> 5120 42 / 59, 2048 -> 2560 8.1 / 7.7; at 128: 12.3 / 12.9, 45.0 / 41.3, 12.4 / 15.7, 20.5 / 28.1, 19.0 / 37.5, 27.3 / 62.8, 93 / 111, 40 /
-// 62, 9.3 / 8.1; at 256: 16.0 / 15.1, 74 / 51, 15.8 / 15.8, 26.6 / 34.2, 25.6 / 37.6, 37.0 / 62.9, 143 / 129, 54 / 66, 12.8 / 9.2.
+// 4096 11.7 / 13.2, 4096 -> 22016 38.8 / 38.8, 5632 -> 2048 10.7 / 15.4, 11008 -> 4096 20.3 / 28.4, 16384 -> 2048 18.6 / 38.0, 28672 -> 2048 27.1 / 63.2, 28672 ->
+// 8192 79 / 93, 20480 -> 5120 38 / 52, 2048 -> 2560 8.2 / 7.8; at 128: 13.0 / 13.6, 45.0 / 41.3, 12.0 / 15.6, 21.3 / 28.7, 20.0 / 38.0, 28.6 / 63.5, 84 / 97, 40 /
+// 61, 9.5 / 8.2; at 256: 16.8 / 15.8, 74 / 51, 16.2 / 16.2, 26.9 / 34.9, 26.6 / 38.5, 37.8 / 63.5, 114 / 117 (129 / 142 under the power cap), 54 / 66, 12.9 / 9.3.
 // Up to 64 tokens the pairs take wide outputs only (feature tiles that no wave of clusters holds), from kF16PairT tokens on; us, this kernel / pairs, at 16
 // and 64 tokens: 2048 -> 11264 10.9 / 10.6 and 13.0 / 11.7, 2048 -> 32000 24.1 / 22.8 and 29.0 / 24.3, 4096 -> 12288 18.9 / 18.9 and 21.1 / 20.4, 5120 ->
 // 15360 25.8 / 26.6 and 28.4 / 28.4, 4096 -> 22016 (a wave and a sixth) 31.4 / 34.7 and 37.0 / 38.5.
@@ -434,13 +434,16 @@ static float f16_stream_us(const F16Plan& pl, int64_t T) {
   return unit * pl.units_per_cta + straddle * (4.f + (float)T * (0.0125f * contrib + 0.035f));
 }
 
-// The same where clusters of d CTAs share a tile: its own k-blocks, at the rate of a CTA or of the memory, and the end of a tile, which grows with the tokens whose sums go
-// through shared memory.  Fitted to the times at kF16DecodeT: within 9 % of all of them.  (By the model of the fix-up through global memory too many went to the pairs; us, so /
-// now: 5632 -> 2048 at 65 and 200 tokens 15.5 / 10.7, 16.1 / 15.2; 11008 -> 4096 at 200 35.0 / 26.8; 8192 -> 4096 at 128 23.2 / 18.3; 20480 -> 5120 at 65 53.8 / 40.7.)
+// The same where clusters of d CTAs share a tile: its own k-blocks, at the rate of a CTA or, above 128 tokens, of the memory, and the end of a tile, which grows with the
+// tokens whose sums go through shared memory.  The line to pair_plan's time is what is fitted, not the time itself (that is off by more than 10 % at 200 of 790 shapes, by 40 % at
+// the widest): of 792 calls of 1024 .. 28672 -> 512 .. 9216 at 65 to 256 tokens what is taken is 0.1 % slower on average than the better of the two kernels, of the 360 larger ones
+// under the power cap 0.5 %; 7 are 1 to 4 % slower than by the model without clusters.  (By that model, too many went to the pairs; us, so / now: 5632 -> 2048 at 65
+// and 200 tokens 15.5 / 10.7, 16.1 / 15.2; 11008 -> 4096 at 200 35.0 / 26.8; 8192 -> 4096 at 128 22.7 / 17.7; 20480 -> 5120 at 65 51.7 / 38.1.  With up to 0.0025 us for each
+// CTA below 129 tokens still too many, 5632 -> 9216 at 65 24.1 / 22.0; with 0.0031 above too few, 24576 -> 6144 at 224 87.6 / 83.4, under the power cap 16384 -> 9216 at 256 95.4 / 88.7.)
 static float f16_cluster_us(int64_t T, int64_t N, int64_t K, int d) {
   const int64_t nkb = (K + kTileK - 1) / kTileK, ctas = (N + kTileM - 1) / kTileM * d;
-  const float unit = T <= 128 ? fmaxf(0.26f, 0.0025f * ctas) : fmaxf(0.355f, 0.0031f * ctas);
-  return unit * ((nkb + d - 1) / d) + 4.8f + 0.0212f * T;
+  const float unit = T <= 128 ? 0.25f : fmaxf(0.385f, 0.0033f * ctas);
+  return unit * ((nkb + d - 1) / d) + 5.1f + 0.0212f * T;
 }
 
 }  // namespace b200
