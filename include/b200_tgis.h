@@ -37,7 +37,7 @@ void b200_debug_w4_flags(int flags); /* debug timing experiments (results invali
 void b200_debug_w4_trace(void* device_buffer); /* debug: [n_ctas][64] u64 phase timestamps of int4 GEMM launches; NULL = off */
 /* tests, host only: 1 if an fp16 call with a workspace takes the SM pairs where the chip holds clusters[d] clusters of d = 2 .. 8 CTAs, 0 if not */
 int b200_debug_f16_on_pairs(int64_t T, int64_t N, int64_t K, int sms, const int32_t* clusters9);
-int b200_debug_pair_plan(int kind, int64_t T, int64_t N, int64_t K, int sms, int32_t* out8); /* tests, host only: whether a launch takes the SM pairs (of 65 to 256 tokens: where no cluster shares a tile), and how; kind 0 fp16, 1 int4, 2 bfloat16 with fp32 results; out = {taken, token tile, token tiles, feature tiles, pairs, k-blocks per stage, pieces of k, stages of a piece} */
+int b200_debug_pair_plan(int kind, int64_t T, int64_t N, int64_t K, int sms, int32_t* out8); /* tests, host only: whether a launch takes the SM pairs (of up to 64 tokens: with the clusters that the present device holds, or those of a B200 without one; of 65 to 256: where no cluster shares a tile), and how; kind 0 fp16, 1 int4, 2 bfloat16 with fp32 results; out = {taken, token tile, token tiles, feature tiles, pairs, k-blocks per stage, pieces of k, stages of a piece} */
 int b200_debug_gemm_plan(int kind, int64_t T, int64_t N, int64_t K, int sms, int32_t* out8); /* tests, host only: stream-K plan of a launch of up to 256 (int4: 128) tokens that no cluster shares tiles of; kind 0 fp16, 1 int4; out = {token tile, k-blocks, feature (super-)tiles, 1, units per CTA, CTAs, contributor slots, tiles per unit} */
 /* tests: how an int4 launch of up to 128 tokens is cut where the chip holds clusters[d] clusters of d = 2 .. 8 CTAs (NULL: as many as the present device does, otherwise host
  * only); out = {token tile, k-blocks, super-tiles, CTAs of a cluster that shares a super-tile or 0, super-units per CTA, CTAs, contributor slots, 2} */

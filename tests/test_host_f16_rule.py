@@ -37,3 +37,10 @@ def test_without_clusters(on_pairs):
             assert _lib.load().b200_debug_pair_plan(0, T, N, K, 148, out) == 0
             if T > 64:
                 assert on_pairs(T, K, N, (0,) * 9) == out[0], (T, K, N)
+
+
+@pytest.mark.parametrize("T", [17, 64])
+def test_up_to_64_tokens_by_the_table_given(on_pairs, T):
+    """wide outputs go to the pairs unless clusters hold their feature tiles, whatever device there is"""
+    assert on_pairs(T, 2048, 11264) == 1 and on_pairs(T, 2048, 11264, (0, 0, 88) + (0,) * 6) == 0 and on_pairs(T, 2048, 11264, (0,) * 9) == 1
+    assert on_pairs(16, 2048, 11264) == 0

@@ -485,7 +485,7 @@ extern "C" int b200_debug_pair_plan(int kind, int64_t T, int64_t N, int64_t K, i
   }
   const int64_t n_kb = kind == 1 ? 2 * ((K + 127) / 128) : (K + kPairK - 1) / kPairK;
   const PairPlan pl = pair_plan(T, N, n_kb, kind == 1, sms, kind == 1 ? 1 : f16_pieces(T, N, K, sms));
-  const int taken = kind == 1 ? T > kW4DecodeT : f16_takes_pairs(kind == 2 ? 2 : 0, T, N, K, true, sms, nullptr);
+  const int taken = kind == 1 ? T > kW4DecodeT : f16_takes_pairs(kind == 2 ? 2 : 0, T, N, K, true, sms, T <= kF16DecodeT ? f16_clusters() : nullptr);
   const int32_t v[8] = {taken, pl.tn, pl.n_tt, pl.n_m, pl.n_pairs, pl.per_stage, pl.pieces, pl.piece_stages};
   for (int i = 0; i < 8; ++i) out[i] = v[i];
   return B200_OK;
@@ -522,7 +522,7 @@ extern "C" int64_t b200_gemm_workspace_bytes_max(int64_t N, int64_t K) {
   return best;
 }
 
-// whether a call's kernel is that of gemm_pair.cuh; clusters: as f16_cluster, for calls of more than kF16DecodeT tokens (NULL: none)
+// whether a call's kernel is that of gemm_pair.cuh; clusters: as f16_cluster (NULL: none)
 static bool f16_takes_pairs(int fmt, int64_t T, int64_t N, int64_t K, bool workspace, int sms, const int* clusters) {
   if (T <= kF16PairT || (fmt == 2 && T <= kF16MostT)) return false;
   if (T > kF16MostT || (!workspace && T > kF16DecodeT)) return true;
@@ -531,7 +531,7 @@ static bool f16_takes_pairs(int fmt, int64_t T, int64_t N, int64_t K, bool works
     // Wide outputs: both stream the weights at the memory's rate, the pairs without fix-ups; but the pairs' last wave has to be a full one, and over
     // three waves and more the fix-ups no longer show (4096 -> 128256 at 64 tokens 168 us, 96 % of the memory's rate).
     const int64_t n_m = (N + kPairM - 1) / kPairM, pairs = sms / 2, waves = (n_m + pairs - 1) / pairs;
-    return f16_cluster(N, K, f16_clusters()) == 0 && workspace && waves <= 2 && (waves == 1 || n_m * 5 >= waves * pairs * 4);
+    return (!clusters || f16_cluster(N, K, clusters) == 0) && workspace && waves <= 2 && (waves == 1 || n_m * 5 >= waves * pairs * 4);
   }
   if ((int64_t)pl.n_tiles_n * 4 > kCounterBytes) return true;
   const int d = clusters ? f16_cluster(N, K, clusters) : 0;
