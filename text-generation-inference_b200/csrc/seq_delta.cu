@@ -140,10 +140,12 @@ __global__ void __launch_bounds__(kPrepThreads, TAPS <= 4 ? 4 : 2) delta_prepare
 // 32 heads: 3600 tokens 246 / 108, 400 31.4 / 19.9.
 constexpr int kRunTok = 16, kRunMinTokens = 384;
 
-// kPerSm: blocks of an SM that registers are left for.  Three (80 registers, a few spilled) from kRunBlocksMany blocks on, where they save a round of blocks; two
-// (116, none spilled) below.  us of a call with the memory's part, two / three: 16 heads 4 x 256 - 768 tokens (854 blocks) 210.8 / 206.4, 16 x 250 353 / 344, 32 heads 6 x
-// 400 - 800 659 / 641; 16 heads 4 x 200 - 250 (420) 110.6 / 112.3, 6 x 96 - 120 (322) 77.1 / 80.8.
-constexpr int kRunBlocksMany = 3 * 148;
+// kPerSm: blocks of an SM that registers are left for: two (116, none spilled) or three (80, a few spilled).  With few blocks the spills show, with many the third block
+// hides more of the memory's latency.  Us, two / three, in a replayed graph, 16 heads in 4 sequences: 273 blocks 14.0 / 16.5, 420 16.7 / 16.8, 462 18.8 / 16.6, 903 34.5 / 29.4, 1862 72 / 59.  The
+// line lies where calls with the memory's part behind them change sides (176 calls, 16 and 32 heads, 1, 4 and 16 sequences of 400 to 4200 tokens in all): up to 441 blocks three take up to 9 %
+// longer (4 x 125 tokens 68.0 / 71.9; 32 heads from 338 blocks on 2 to 3 % less), 448 to 504 from 2.4 % longer (16 x 50 tokens) to 4.7 % less (32 heads, 4 x 125),
+// above up to 5 % less (4 x 500 210.9 / 205.7, 4 x 1050 412 / 401).
+constexpr int kRunBlocksMany = 3;   // blocks for each SM above which three are
 template <typename TP, int kPerSm>
 __global__ void __launch_bounds__(256, kPerSm) delta_prepare_run_kernel(
     const float* __restrict__ u, int64_t ld, int col0, int taps, const TP* __restrict__ w, float* conv_state,
@@ -726,7 +728,7 @@ extern "C" int b200_seq_delta_prepare(const float* u, int64_t ld, int col0, int 
 #define DPRUN(N)                                                                                                                                                  \
   B200_SEQ_DISPATCH(dt, E, B200_LAUNCH((delta_prepare_run_kernel<E, N>), grid, dim3(256), 0, st, u, ld, col0, taps, (const E*)w, conv_state, state_slots, cu_q, B, \
                                        position_ids, raw, ldr, col_b, dec, ldd, col_a, channels, (const E*)A_log, (const E*)dt_bias, q_scale, out, H, kv_heads, dk, dv))
-    if ((int64_t)grid.x * grid.y > kRunBlocksMany) DPRUN(3);
+    if ((int64_t)grid.x * grid.y > (int64_t)kRunBlocksMany * b200_num_sms()) DPRUN(3);
     else DPRUN(2);
 #undef DPRUN
     b200_count_launches(1);
