@@ -757,20 +757,20 @@ extern "C" int b200_seq_talk_attn_splits(int dt, int64_t T, int B, int H, int G,
 }
 
 // Prompts without a mix take the tcgen05 kernel: tiles of 128 (token, head) rows, so it wants steps of enough tokens per sequence to fill them.
-// Measured on B200 (us, the m16n8k16 kernel / this one; 16 / 4 heads, d = 128): 1618 + 2000 tokens in chunks of 2048 343 / 101, 1000 108 / 39, 16 x 24 after
-// 4000 cached 134 / 90, 2 x 40 after 100 32 / 25, 24 after 500 38 / 32; with one bfloat16 value per weight 4 x 16 after 1900 55 / 53, 4 x 8 48 / 50.
+// Measured on B200 (us, the m16n8k16 kernel in up to 32 runs of keys / this one, in replayed graphs; 16 / 4 heads, d = 128): one prompt of 1000 tokens 99 / 29, of 2000 256 / 53, of 4000
+// 715 / 93, 2 x 500 behind 1000 keys 134 / 39, 8 x 500 behind 8000 2312 / 365, 24 tokens behind none 19 / 11.
 // What it needs beside that: heads of 64 or 128 columns, whole 128-row tiles (128 % (heads / kv_heads) == 0), pages of 16 tokens, and 16-byte pieces; and a
 // shape that talk_mma_plan accepts: those rounded queries and weights to bfloat16 before, the others (at d = 128: 16 / 16, 32 / 32, 32 / 16, 64 / 16 ... heads,
 // and everything under B200_SEQ_ATTN_MMA=0) are computed in fp32 and stay so.
 constexpr int kTalkPromptTokens = 24;  // average tokens per sequence from which on
 
 // Few items over many keys are a matter of latency: the m16n8k16 kernel cuts the keys into runs then, this one does not.  `keys`: a bound of
-// the keys that a query sees, as far as the host knows it (the block table's width, a chunk, a window).  Models of both, from 80 steps measured on
-// B200.  Us, m16n8k16 / this one, no chunk, no window: 16 / 4 heads of 128, 24 tokens behind 2000 keys 56 / 51, behind 30 000 454 / 475, 200 behind 8000 181 /
-// 145; 8 / 2 heads of 64, 24 behind 500 36 / 27, 64 behind 8000 77 / 141, 500 behind 8000 103 / 150; 16 / 8 heads of 64, 24 x 16 sequences behind 4000 108 / 127, a
-// prompt of 4000 beside 100 single tokens behind 1500 527 / 248.
-// (The first of each pair was measured in at most kTalkModelRuns runs of keys, with queries ahead of the first keys.  In up to 32 runs that kernel takes less - 32 tokens
-// behind 1000 keys, 16 / 4 heads of 128, 30.4 where this one is taken and takes 33.1 - so the line lies on this one's side.)
+// the keys that a query sees, as far as the host knows it (the block table's width, a chunk, a window).  Models of both, of that kernel in at most
+// kTalkModelRuns runs.  In the up to 32 runs that it takes now, and since this one lost the divisions and the late items of its tiles, the line lies on this one's side: of 790 calls
+// (16 / 4 and 32 / 8 heads of 128, 8 / 2 of 64, 24 to 4000 tokens in 1 to 101 sequences behind up to 30 000 keys) none that goes to the other kernel would take less here, and
+// 78 that are taken here would take less there (us, that / this: 24 tokens behind 1000 keys, 8 / 2 heads of 64, 16.5 / 20.9; 16 / 4 heads of 128, 24 behind 4000 40 / 80, 100 behind
+// 8000 78 / 152).  They stay: that kernel has one bfloat16 value for each weight where this one has two halves, and is 20 to 30 % further from float64 (24 tokens behind
+// 2000 keys 2.05e-3 / 1.69e-3, 2 x 64 behind 4000 2.19e-3 / 1.69e-3).
 constexpr int kTalkModelRuns = 8;
 static bool talk_prompt_pays(int64_t T, int B, int H, int G, int d, int dv, int64_t keys, int QT, int nsplit) {
   const int tokens = 128 / (H / G), sms = b200_num_sms();
