@@ -378,7 +378,7 @@ typedef struct {
   int64_t* next_ids; /* optional [rows] greedy ids (sharded head: needs p2p_argmax) */
   const int64_t* banned_ids; /* optional [rows], see b200_argmax */
   /* decode-sized steps (T <= 128): */
-  int32_t defer_splitk; /* 1: linears leave split-K partials to their consumer kernels (B200SplitK) */
+  int32_t defer_splitk; /* 1: linears leave split-K partials to their consumer kernels (B200SplitK), but for int4 ones of more than eight tokens on a single rank */
   int32_t _pad2;
   void* p2p_norm;   /* tensor parallel: b200_p2p_create window for b200_p2p_allreduce_rmsnorm (the layer boundary runs inside the
                        step, no host-side collective), or NULL: the caller all-reduces `hidden` between the block calls */

@@ -28,8 +28,8 @@
 //                 4 HADD2 (exact q - zero), 4 HMUL2 (x scale: bit-identical to the formula of record) -> tcgen05.st into a
 //                 ring of A-operand tiles in TMEM (64 columns each), an arrival at the super-unit's barrier.  Teams run on their own clocks.
 //   warps 20, 21  MMA issue, alternate super-units: wait for the super-unit's barrier (its activation tile and the 8 team-warp
-//                 quarters of its two A tiles), then for the turn, 16 x tcgen05.mma.kind::f16 (A from TMEM, B from shared memory), ONE tcgen05.commit that
-//                 frees the activation stage and both A stages
+//                 quarters of its two A tiles), then for the turn, 16 x tcgen05.mma.kind::f16 (A from TMEM, B from shared memory), a tcgen05.commit that frees both
+//                 A stages (su_done) and one that frees the activation stage (x_empty)
 //   warps 0..3    epilogue: tcgen05.ld of a finished super-tile, then fp16 store / fused SiLU(gate) * up store / fp32
 //                 partial store when the super-tile is shared with other CTAs; they sleep while they wait
 // Decode (T <= 128) is weight-streaming / HBM-bound: the (super-tile, k-block) space is cut into contiguous ranges, one
@@ -37,8 +37,8 @@
 // Super-tiles shared by several CTAs are finished after the main loop by ALL their contributors: each sums one slice over
 // the contributors' fp32 partials in contributor order (deterministic, unlike the reference kernel's fp16 atomicAdd across
 // K slices; a reduce-scatter, so the tail costs one partial's worth of L2 reads per CTA however many CTAs share it).
-// The contributors wait for one another: all CTAs of the grid are co-resident (grid <= #SMs, one CTA per SM).  Where that cut would have many contributors
-// or few SMs, the CTAs of a cluster share a super-tile instead and add their parts through shared memory (launch_plan_w4).
+// The contributors wait for one another: all CTAs of the grid are co-resident (grid <= #SMs, one CTA per SM).  Where that takes less,
+// the CTAs of a cluster share a super-tile instead and add their parts through shared memory (launch_plan_w4).
 //
 // mbarrier rule used throughout: a thread that waits on a barrier observes every phase of it in order, or an earlier
 // observation implies the skipped phase completed (see the ring-depth static_asserts).  Polls whose result is wanted
@@ -195,7 +195,7 @@ gemm_w4a16_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Params p) 
   uint64_t* empty_w = full_w + C::kWStages;
   uint64_t* su_full = empty_w + C::kWStages;    // [kXStages] super-unit j's inputs are there, its activation tile and the 8 team-warp quarters of its two A tiles
   uint64_t* x_empty = su_full + C::kXStages;    // [kXStages] the MMAs that read the stage's activation tile have completed
-  uint64_t* su_done = x_empty + C::kXStages;    // [kSuRing] MMA commit of super-unit j -> barrier j % kSuRing: its x stage and its A stages are free
+  uint64_t* su_done = x_empty + C::kXStages;    // [kSuRing] MMA commit of super-unit j -> barrier j % kSuRing: its A stages are free
   uint64_t* tmem_full = su_done + C::kSuRing;   // [2]
   uint64_t* tmem_empty = tmem_full + 2;         // [2]
   uint64_t* turn = tmem_empty + 2;              // [2] hand-over between the two MMA warps

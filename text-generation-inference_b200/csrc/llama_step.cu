@@ -8,7 +8,8 @@
 // Two things move between kernels at decode sizes (T <= 128), without changing a result by more than the order of fp32 sums:
 //   * deferred split-K (s->defer_splitk): a linear leaves its K-slices' fp32 partials in the workspace and the kernel that
 //     consumes its output anyway (residual + RMSNorm, RoPE + KV write, SiLU * up) sums them while it reads - the GEMM no longer
-//     waits for its slowest CTA and re-reads the partials itself (include/b200_tgis.h "B200SplitK");
+//     waits for its slowest CTA and re-reads the partials itself (include/b200_tgis.h "B200SplitK").  Not so int4 linears of more
+//     than eight tokens on a single rank, which finish in their own kernel (finishes());
 //   * the tensor-parallel layer boundary (s->p2p_norm): all-reduce over NVLink peer memory + residual + RMSNorm in one
 //     kernel (b200_p2p_allreduce_rmsnorm), fed directly by the row-parallel linear's partials.  The whole sharded step is then
 //     one C call like the single-rank one; without a window the caller all-reduces `hidden` (NCCL) between the block calls.
