@@ -95,3 +95,23 @@ def test_a_result_off_any_eight_bytes(T):
         got.append(room[off:off + T * N].clone())
         assert all(float(v) == 7.0 for v in torch.cat([room[:off], room[off + T * N:]]))
     assert torch.equal(*got)
+
+
+# 32 feature tiles of four CTAs each, 172 that 148 CTAs straddle; clusters of four
+@pytest.mark.parametrize("T,N,K", [(4, 4096, 4096), (16, 22016, 1024), (16, 4096, 4096)])
+def test_results_off_any_eight_bytes(T, N, K):
+    """with a workspace, so that CTAs share feature tiles through it or in clusters: the bits of a y on eight bytes"""
+    import ctypes
+    import tgis_b200  # noqa: F401
+    from tgis_b200 import _lib
+    lib, (x, w, bias) = _lib.load(), _data(T, N, K, torch.float16)
+    ws = torch.zeros(lib.b200_gemm_workspace_bytes(T, N, K), dtype=torch.uint8, device=DEV)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+
+    def call(y):
+        assert lib.b200_gemm_f16(p(x), p(w), p(bias), p(y), T, N, K, p(ws), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        return y
+    room = torch.full((T * N + 2,), 7.0, dtype=torch.float16, device=DEV)
+    want = call(torch.empty(T, N, dtype=torch.float16, device=DEV))
+    _near(want, x, w, bias, 2 ** -11)
+    assert torch.equal(call(room[1:-1].view(T, N)), want) and float(room[0]) == 7.0 == float(room[-1])

@@ -306,7 +306,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
         if (s_is_last) {
           const float* base = p.partial + (size_t)tile * p.max_contrib * (TN * kTileM);
           const int n_vec = min(p.T, TN) * (kTileM / 4);
-          const bool vec_ok = (p.N & 3) == 0;
+          const bool vec_ok = (p.N & 3) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
           for (int idx0 = etid; idx0 < n_vec; idx0 += 256) {
             float4 acc[2];
             float4 ld[2][4];
