@@ -138,13 +138,18 @@ struct W4Params {
   unsigned long long* trace;  // debug: per-CTA phase timestamps (globaltimer ns), NULL in production
 };
 
-// four features of a token at y; p.y may start off any four halves (rows are a multiple of 32 long, so the first address says it for all)
+// four features of a token at y; p.y may start off any four halves (rows are a multiple of 32 long, so the first address says it for all).  Single stores in a loop:
+// unrolled in all three endings they lengthened the kernel for everybody (4096 -> 28672 with the SiLU at 64 tokens, replayed graph, 21.25 us, so 21.14)
 __device__ __forceinline__ void w4_store(const W4Params& p, __half* y, uint2 o) {
   if ((reinterpret_cast<uintptr_t>(p.y) & 7) == 0) {
     *reinterpret_cast<uint2*>(y) = o;
   } else {
-    const __half* h = reinterpret_cast<const __half*>(&o);
-    for (int j = 0; j < 4; ++j) y[j] = h[j];
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) {
+      reinterpret_cast<unsigned short*>(y)[j] = (unsigned short)o.x;
+      o.x = __funnelshift_r(o.x, o.y, 16);
+      o.y >>= 16;
+    }
   }
 }
 
